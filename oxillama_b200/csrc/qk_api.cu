@@ -195,6 +195,11 @@ static int upload_impl(qk_ctx *c, int type, const uint8_t *w, size_t n_cols, siz
     delete h;
     return QK_CUDA_ERROR;
   }
+  if (qk_gemm_tc_supported(h->L, 1) && (e = qk_gemm_tc_map(h->L, h->dev, h->tmap)) != cudaSuccess) {
+    c->err = std::string("weights upload: tensor map: ") + cudaGetErrorString(e);
+    free_weights(h);
+    return QK_CUDA_ERROR;
+  }
   uint8_t *raw = nullptr;
   int st = QK_OK;
   do {
@@ -324,6 +329,23 @@ extern "C" int qk_weights_cache_evict(qk_ctx *c, const uint8_t *w) {
 }
 
 // ------------------------------------------------------------ device entry points
+static int ensure_scratch(qk_ctx *c, size_t need) {
+  if (need <= c->scratch_cap) return QK_OK;
+  CK(c, cudaDeviceSynchronize());
+  cudaFree(c->scratch);
+  c->scratch = nullptr, c->scratch_cap = 0;
+  CK(c, cudaMalloc(&c->scratch, need + need / 4));
+  c->scratch_cap = need + need / 4;
+  return QK_OK;
+}
+
+static int tc_call(qk_ctx *c, const QkTcCall &call, cudaStream_t s) {
+  int st = ensure_scratch(c, qk_gemm_tc_scratch_bytes(call, c->sm_count));
+  if (st) return st;
+  CK(c, qk_launch_gemm_tc(call, c->status_dev, c->scratch, c->sm_count, s));
+  return QK_OK;
+}
+
 static int gemm_dispatch(qk_ctx *c, const qk_weights *h, const float *x, float *y, size_t m,
                          size_t ldy, cudaStream_t s) {
   if (h->L.rows == 0 || m == 0) return QK_OK;
@@ -331,28 +353,11 @@ static int gemm_dispatch(qk_ctx *c, const qk_weights *h, const float *x, float *
     CK(c, cudaMemset2DAsync(y, ldy * sizeof(float), 0, h->L.rows * sizeof(float), m, s));
     return QK_OK;
   }
-  auto ensure_scratch = [&](size_t need) -> int {
-    if (need <= c->scratch_cap) return QK_OK;
-    CK(c, cudaDeviceSynchronize());
-    cudaFree(c->scratch);
-    c->scratch = nullptr, c->scratch_cap = 0;
-    CK(c, cudaMalloc(&c->scratch, need * 2));
-    c->scratch_cap = need * 2;
-    return QK_OK;
-  };
   if (!c->force_simple && m <= QK_GEMV_MAX_M && qk_gemv_fast_supported(h->L, (uint32_t)m)) {
-    int st = ensure_scratch(qk_gemv_fast_scratch_bytes(h->L, (uint32_t)m));
+    int st = ensure_scratch(c, qk_gemv_fast_scratch_bytes(h->L, (uint32_t)m));
     if (st) return st;
     CK(c, qk_launch_gemv_fast(h->L, h->dev, x, y, (uint32_t)m, ldy, c->status_dev, c->scratch,
                               c->sm_count, s));
-    return QK_OK;
-  }
-  // 5 .. 16 rows of a tall Q4_K matrix: the streaming fp16-MMA kernel (measured faster than
-  // the tcgen05 kernel from eight 8-row chunks per SM up; below that it is not)
-  if (!c->force_simple && !qk_knob("QK_NO_SB") && qk_gemm_sb_preferred(h->L, (uint32_t)m, c->sm_count)) {
-    int st = ensure_scratch(qk_gemm_sb_scratch_bytes(h->L, (uint32_t)m));
-    if (st) return st;
-    CK(c, qk_launch_gemm_sb(h->L, h->dev, x, y, (uint32_t)m, ldy, c->status_dev, c->scratch, c->sm_count, s));
     return QK_OK;
   }
   // The tensor-core path rounds its operands to fp16; batches the decode kernels take keep
@@ -363,11 +368,10 @@ static int gemm_dispatch(qk_ctx *c, const qk_weights *h, const float *x, float *
   const bool tc_small = m <= QK_GEMV_MAX_M && m > 1 && qk_gemv_fast_supported(h->L, 1);
   if (!c->force_simple && (m > QK_GEMV_MAX_M || tc_small) && m < (1u << 30) &&
       qk_gemm_tc_supported(h->L, (uint32_t)m)) {
-    int st = ensure_scratch(qk_gemm_tc_scratch_bytes(h->L, (uint32_t)m));
-    if (st) return st;
-    CK(c, qk_launch_gemm_tc(h->L, h->dev, x, y, (uint32_t)m, ldy, c->status_dev, c->scratch,
-                            c->sm_count, s));
-    return QK_OK;
+    QkTcCall call = {};
+    call.L = &h->L, call.maps[0] = h->tmap, call.n = call.n_act = 1;
+    call.x = x, call.m = (uint32_t)m, call.y = y, call.ldy = ldy;
+    return tc_call(c, call, s);
   }
   CK(c, qk_launch_gemm_simple(h->L, h->dev, x, y, (uint32_t)m, ldy, s));
   return QK_OK;
@@ -463,7 +467,7 @@ extern "C" int qk_moe_ffn_dev(qk_ctx *c, const qk_weights *const *gate, const qk
               down[e]->L.type == down[0]->L.type && qk_gemm_tc_supported(gate[e]->L, 1) &&
               qk_gemm_tc_supported(down[e]->L, 1);
   if (grouped) {
-    const size_t cap = qk_gemm_tc_group_cap((uint32_t)tokens), rows = n_local * cap;
+    const size_t cap = tokens, rows = n_local * cap;
     const size_t o_ids = 0, o_wts = o_ids + al(slots * 4), o_cnt = o_wts + al(slots * 4);
     const size_t o_lists = o_cnt + al(n_local * 4), o_pos = o_lists + al(n_local * slots * 4);
     const size_t o_g = o_pos + al(slots * 4), o_u = o_g + rows * inter * 4;  // u directly behind g
@@ -475,43 +479,32 @@ extern "C" int qk_moe_ffn_dev(qk_ctx *c, const qk_weights *const *gate, const qk
     int *pos = (int *)(base + o_pos);
     float *wts = (float *)(base + o_wts), *g = (float *)(base + o_g), *u = (float *)(base + o_u);
     float *o = (float *)(base + o_o);
-    size_t sneed = qk_gemm_tc_grouped_scratch_bytes(gate[0]->L, (uint32_t)n_local, (uint32_t)tokens);
-    const size_t sdown = qk_gemm_tc_grouped_scratch_bytes(down[0]->L, (uint32_t)n_local, (uint32_t)tokens);
-    if (sdown > sneed) sneed = sdown;
-    if (sneed > c->scratch_cap) {
-      CK(c, cudaDeviceSynchronize());
-      cudaFree(c->scratch);
-      c->scratch = nullptr, c->scratch_cap = 0;
-      CK(c, cudaMalloc(&c->scratch, sneed));
-      c->scratch_cap = sneed;
-    }
-    const uint8_t *wgu[QK_MAX_GROUPS], *wd[QK_MAX_GROUPS];
-    const bool one_launch = 2 * n_local <= QK_MAX_GROUPS;  // gate and up as 2 n groups over n activation groups
-    for (size_t e = 0; e < n_local; e++) wd[e] = down[e]->dev;
     CK(c, qk_launch_moe_route(logits_dev, (uint32_t)tokens, (uint32_t)n_exp, (uint32_t)top_k, ids, wts, s));
     CK(c, qk_launch_moe_lists(ids, (uint32_t)tokens, (uint32_t)top_k, (uint32_t)expert_begin, (uint32_t)n_local,
                               cnt, lists, pos, s));
-    if (one_launch) {
-      // u directly behind g: groups 0 .. n - 1 write g, groups n .. 2 n - 1 write u
-      u = g + rows * inter;
-      for (size_t e = 0; e < n_local; e++) wgu[e] = gate[e]->dev, wgu[n_local + e] = up[e]->dev;
-      CK(c, qk_launch_gemm_tc_grouped(gate[0]->L, wgu, (uint32_t)(2 * n_local), (uint32_t)n_local, cnt,
-                                      (uint32_t)tokens, x_dev, lists, (uint32_t)slots, (uint32_t)top_k, g, inter,
-                                      c->status_dev, c->scratch, c->sm_count, s));
-    } else {
-      for (size_t e = 0; e < n_local; e++) wgu[e] = gate[e]->dev;
-      CK(c, qk_launch_gemm_tc_grouped(gate[0]->L, wgu, (uint32_t)n_local, (uint32_t)n_local, cnt, (uint32_t)tokens,
-                                      x_dev, lists, (uint32_t)slots, (uint32_t)top_k, g, inter, c->status_dev,
-                                      c->scratch, c->sm_count, s));
-      for (size_t e = 0; e < n_local; e++) wgu[e] = up[e]->dev;
-      CK(c, qk_launch_gemm_tc_grouped(up[0]->L, wgu, (uint32_t)n_local, (uint32_t)n_local, cnt, (uint32_t)tokens,
-                                      x_dev, lists, (uint32_t)slots, (uint32_t)top_k, u, inter, c->status_dev,
-                                      c->scratch, c->sm_count, s));
+    QkTcCall gu = {};
+    gu.L = &gate[0]->L, gu.n_act = (uint32_t)n_local, gu.counts = cnt, gu.m = (uint32_t)tokens;
+    gu.expect = (uint32_t)((slots + n_exp - 1) / n_exp), gu.xcap = gu.ycap = (uint32_t)cap;
+    gu.x = x_dev, gu.lists = lists, gu.list_stride = (uint32_t)slots, gu.list_div = (uint32_t)top_k;
+    gu.y = g, gu.ldy = inter;
+    // gate and up as 2 n groups over n activation groups (groups n .. 2 n - 1 write u, behind g)
+    const bool one_launch = 2 * n_local <= QK_MAX_GROUPS;
+    for (size_t e = 0; e < n_local; e++) gu.maps[e] = gate[e]->tmap;
+    if (one_launch)
+      for (size_t e = 0; e < n_local; e++) gu.maps[n_local + e] = up[e]->tmap;
+    gu.n = (uint32_t)(one_launch ? 2 * n_local : n_local);
+    if ((st = tc_call(c, gu, s))) return st;
+    if (!one_launch) {
+      for (size_t e = 0; e < n_local; e++) gu.maps[e] = up[e]->tmap;
+      gu.y = u;
+      if ((st = tc_call(c, gu, s))) return st;
     }
-    CK(c, qk_launch_moe_silu_mul_grouped(g, u, cnt, (uint32_t)n_local, (uint32_t)tokens, (uint32_t)cap,
-                                         (uint32_t)inter, s));
-    CK(c, qk_launch_gemm_tc_grouped(down[0]->L, wd, (uint32_t)n_local, (uint32_t)n_local, cnt, (uint32_t)tokens, u, nullptr, 0, 1, o,
-                                    hidden, c->status_dev, c->scratch, c->sm_count, s));
+    // silu(g) * u is formed where the down projection's activations are converted
+    QkTcCall dn = {};
+    dn.L = &down[0]->L, dn.n = dn.n_act = (uint32_t)n_local, dn.counts = cnt, dn.m = (uint32_t)tokens, dn.expect = gu.expect;
+    dn.xcap = dn.ycap = (uint32_t)cap, dn.x = g, dn.x2 = u, dn.y = o, dn.ldy = hidden;
+    for (size_t e = 0; e < n_local; e++) dn.maps[e] = down[e]->tmap;
+    if ((st = tc_call(c, dn, s))) return st;
     CK(c, qk_launch_moe_combine(o, ids, pos, wts, (uint32_t)tokens, (uint32_t)top_k, (uint32_t)expert_begin,
                                 (uint32_t)n_local, (uint32_t)cap, (uint32_t)hidden, y_dev, s));
     return QK_OK;
@@ -583,16 +576,23 @@ extern "C" int qk_ffn_dev(qk_ctx *c, const qk_weights *gate, const qk_weights *u
                      inter > 0 && m <= QK_GEMV_MAX_M && qk_gemv_dual_supported(gate->L, (uint32_t)m);
   if (fused) {
     // gate and up in one launch (they share the split activations), silu(g) * u in its reducer
-    const size_t sneed = qk_gemv_mma_scratch_bytes(gate->L, (uint32_t)m);
-    if (sneed > c->scratch_cap) {
-      CK(c, cudaDeviceSynchronize());
-      cudaFree(c->scratch);
-      c->scratch = nullptr, c->scratch_cap = 0;
-      CK(c, cudaMalloc(&c->scratch, sneed * 2));
-      c->scratch_cap = sneed * 2;
-    }
+    int st = ensure_scratch(c, qk_gemv_mma_scratch_bytes(gate->L, (uint32_t)m));
+    if (st) return st;
     CK(c, qk_launch_gemv_dual(gate->L, gate->dev, up->dev, x_dev, h, (uint32_t)m, inter, c->status_dev, c->scratch,
                               c->sm_count, s));
+  } else if (!c->force_simple && m > QK_GEMV_MAX_M && m < (1u << 30) && hidden > 0 && inter > 0 && gate->L.type == up->L.type &&
+             qk_gemm_tc_supported(gate->L, (uint32_t)m) && qk_gemm_tc_supported(down->L, (uint32_t)m)) {
+    // Batches: gate and up as one tensor-core launch over the activations converted once, and
+    // silu(g) * u formed where the down projection's activations are converted.
+    QkTcCall gu = {};
+    gu.L = &gate->L, gu.maps[0] = gate->tmap, gu.maps[1] = up->tmap, gu.n = 2, gu.n_act = 1;
+    gu.x = x_dev, gu.m = (uint32_t)m, gu.xcap = gu.ycap = (uint32_t)m, gu.y = h, gu.ldy = inter;
+    int st = tc_call(c, gu, s);
+    if (st) return st;
+    QkTcCall dn = {};
+    dn.L = &down->L, dn.maps[0] = down->tmap, dn.n = dn.n_act = 1;
+    dn.x = h, dn.x2 = u, dn.m = (uint32_t)m, dn.y = y_dev, dn.ldy = down->L.rows;
+    return tc_call(c, dn, s);
   } else {
     int st = gemm_dispatch(c, gate, x_dev, h, m, inter, s);
     if (st) return st;

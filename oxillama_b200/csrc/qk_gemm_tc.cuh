@@ -1,0 +1,1120 @@
+// Batched dequant-matmul (more than four activation rows) on the 5th-generation tensor cores.
+//
+//   y[t][n] = sum_k  w(n, k) * x[t][k]          w as the format's dequant_block gives it, rounded to fp16
+//
+// A real dense contraction, so it goes to tcgen05.mma: 128 weight rows are the MMA's M, up to
+// 256 activation rows (tokens) its N, fp16 operands, f32 accumulation in tensor memory.
+//
+// Both the accumulator and the expanded weights live in tensor memory: a thread that owns a
+// weight row expands its columns in registers and stores them with tcgen05.st straight into the
+// lane and columns from which the MMA reads its A operand.  Nothing of the weights passes through
+// shared memory a second time: no proxy fence, no swizzled stores, and the MMA reads only the
+// activations from there.  (Measured: with A in tensor memory an MMA takes max(12, N / 2) cycles,
+// with A in shared memory 47 at least; issued by a warp that walks the loop together, the MMA
+// predicated on one lane -- a lone thread behind lane == 0 needs 98 cycles per MMA.)
+//
+// Two forms of the kernel.  CG = 1: one CTA works on 128 rows, for tiles of up to 64 tokens, where
+// the expansion is the bound and the hand-overs inside one SM are the shortest.  CG = 2: a pair of
+// CTAs (the two SMs of a TPC) works on 256 rows with cta_group::2, each loading half of the tokens:
+// at 256 tokens one SM alone would have to load 64 bytes a cycle of activations, which L2 does not
+// deliver to all SMs (measured: 53 at 2700 cycles per 256 columns instead of 2048).
+//
+// Persistent; the work of a CTA (pair) is a list of segments (output tile, run of 256-column
+// super-blocks):
+//   warp 0      MMA issuer (of both CTAs, in the first of a pair)
+//   warp 1      activation producer: TMA tiles (128-byte swizzle) of the fp16 activations
+//   warp 2      weight producer: one TMA box per super-block brings the packed bytes of 128 rows
+//               (16 chunks x 8 rows) into a ring; it starts before the previous kernel has ended
+//   warp 3      allocates and frees the tensor memory
+//   warps 4-19  two sets of eight warps that take the super-blocks in turn, one thread per row and
+//               128 columns
+//   warps 20-23 epilogue: accumulator -> y (or the workspace of a split tile)
+// Tensor memory: two accumulator halves of up to 128 tokens in columns 0-255 and the expanded
+// weights of two super-blocks behind them; up to 64 tokens, halves of 64 in columns 0-127 and three
+// super-blocks.  A tile of up to 128 tokens uses one half, the halves alternating from tile to tile;
+// a wider tile uses both.  An SM stores 32 bytes a cycle, so writing out a half takes the time of
+// about 32 of its MMAs: at the ends of a wide tile the two super-blocks there are issued first half
+// by first half, then second half by second half, so that one half is written out under the MMAs of
+// the other and the tensor pipe does not wait.
+//
+// Tiles are dealt out in whole waves; the remainder that would leave SMs idle is cut along K into
+// equal runs of super-blocks over all CTAs (pairs).  A tile cut this way has several contributors: each
+// leaves its f32 partial in a workspace and counts itself in, and whoever comes last adds the
+// partials in a fixed order (so the result does not depend on who that is: the same bits on every
+// run) and writes y.  Nobody waits for another CTA.
+//
+// The activations are converted to fp16 once per call by qk_x16_kernel, the columns of every
+// 64-group in the order in which the packed words yield their weights (both operands use the same
+// order, so the sum is unchanged).  fp16 operands put the result at ~5e-4 of the output's
+// inf-norm against the f32 reference (its stated tolerance is 1e-3).
+//
+// Every mbarrier wait is time-bounded; a wait that runs out raises QK_DEV_TIMEOUT and the CTA
+// falls through to the common exit, which lets the copies in flight land and frees its tensor
+// memory.
+#pragma once
+#include <cuda.h>
+
+#include <cfloat>
+#include <cmath>
+#include <cstdlib>
+#include <cstring>
+
+#include "qk_kernels.h"
+#include "qk_pipe.cuh"
+
+namespace qktc {
+
+using namespace qkpipe;
+
+constexpr uint32_t BM = 128;       // weight rows per CTA
+constexpr int NDW = 16;            // expanding warps: two sets of eight
+constexpr int FIRST_DW = 4, FIRST_EW = FIRST_DW + NDW;
+constexpr int NTHREADS = (FIRST_EW + 4) * 32;
+constexpr uint32_t MAX_BN = 256;   // most tokens per tile: two accumulator halves of 128
+constexpr int MAX_WST = 12, MAX_BST = 6;
+
+struct TcSmem {
+  uint32_t w_full, w_empty, b_full, b_empty, a_full, a_empty, d_full, d_empty, drain, tmem_slot, pre, scales, lut;
+  uint32_t w, b;                   // ring bases
+  uint32_t w_stage, b_stage;       // bytes per stage
+  uint32_t w_stages, b_stages;
+};
+
+// One call, as every role of the kernel sees it.
+struct TcArgs {
+  QkLayout L;
+  TcSmem S;
+  const float *xscale;
+  float *y;
+  float *part;                     // partial tiles: two slots per CTA, [bn][128] f32 each
+  unsigned *cnt;                   // arrivals per (split tile, half, CTA of the pair); zeroed by the conversion kernel
+  unsigned *status;
+  uint64_t ldy;
+  uint32_t m;                      // activation rows (of every group, unless counted on the device)
+  uint32_t bn, hn;                 // token rows per tile and of its first accumulator half (bn, if that is 128 at most); multiples of 16
+  uint32_t tok_blocks;             // token blocks per group (upper bound where the counts are on the device)
+  uint32_t row_blocks;             // 128- or 256-row blocks per matrix
+  uint32_t min_run;                // fewest super-blocks worth a CTA in the split part
+  uint32_t n, n_act;               // weight matrices; distinct activation groups (group e reads e % n_act)
+  uint32_t xcap, ycap;             // rows reserved per group in the activation and output arrays
+  uint32_t once;                   // weights are read once: evict-first in L2
+  const int *counts;               // device: live rows per activation group, or null (m rows each)
+};
+// Tensor maps: the matrices, and the fp16 activations as boxes of 64 columns x h tokens x the steps of
+// a stage: h = hn, or one of the quarters of it where the live tokens of a group are known on the
+// device only.
+template <int NG>
+struct TcMaps {
+  CUtensorMap x[NG > 1 ? 4 : 1];
+  CUtensorMap w[NG];
+};
+
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+// The whole warp waits: one poll where the phase is already over, else the bounded loop.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity));
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// Issued by the lane that has `lead` set; the whole warp walks the producing loops, so that what the
+// compiler knows to be uniform stays in uniform registers (a lone thread needs 500 cycles per copy).
+__device__ __forceinline__ void expect_tx(uint32_t bar, uint32_t bytes, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
+      "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes), "r"(lead)
+      : "memory");
+}
+// `bar`: a barrier of this CTA or, with CG = 2, of either CTA of the pair (cluster address).
+template <int CG>
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar, uint32_t lead) {
+#define QK_TMA(GROUP)                                                                                                     \
+  asm volatile(                                                                                                           \
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %6, 0;\n\t"                                                                   \
+      "@q cp.async.bulk.tensor.3d" GROUP ".shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n\t}" ::"r"(dst), \
+      "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar), "r"(lead)                                                               \
+      : "memory")
+  if (CG == 1) QK_TMA("");
+  else QK_TMA(".cta_group::2");
+#undef QK_TMA
+}
+__device__ __forceinline__ void tma_load_3d_hint(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar,
+                                                 uint64_t policy, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %7, 0;\n\t"
+      "@q cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4}], "
+      "[%5], %6;\n\t}" ::"r"(dst),
+      "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar), "l"(policy), "r"(lead)
+      : "memory");
+}
+// Shared-memory descriptor of a K-major operand tile, 128-byte swizzle, rows 128 bytes apart, 8-row
+// groups 1024 bytes apart: the low word holds the address / 16, the rest is constant.
+constexpr uint32_t UMMA_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t umma_desc_lo(uint32_t smem_addr) { return ((smem_addr >> 4) & 0x3FFFu) | (1u << 16); }
+// D[128 CG x N] (+)= A[128 CG x 16] B[N x 16]^T with A in tensor memory, issued by the lane that has
+// `lead` set.  The whole warp walks the issuing loop: in code that the compiler knows to be uniform
+// the operands stay in uniform registers.
+template <int CG>
+__device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint32_t bdesc_lo, uint32_t idesc,
+                                            uint32_t accumulate, uint32_t lead) {
+#define QK_UMMA(GROUP)                                                              \
+  asm volatile(                                                                     \
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 d;\n\t"                                   \
+      "mov.b64 d, {%2, %6};\n\t"                                                    \
+      "setp.ne.b32 p, %4, 0;\n\t"                                                   \
+      "setp.ne.b32 q, %5, 0;\n\t"                                                   \
+      "@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], [%1], d, %3, p;\n\t}"    \
+      :                                                                             \
+      : "r"(tmem_d), "r"(tmem_a), "r"(bdesc_lo), "r"(idesc), "r"(accumulate), "r"(lead), "n"(UMMA_DESC_HI) \
+      : "memory")
+  if (CG == 1) QK_UMMA("1");
+  else QK_UMMA("2");
+#undef QK_UMMA
+}
+// Arrives on the barrier (of both CTAs of a pair) once the MMAs issued so far have retired.
+template <int CG>
+__device__ __forceinline__ void umma_commit(uint32_t bar, uint32_t lead) {
+  if (CG == 1)
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(lead)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t.reg .b16 m;\n\tmov.b16 m, 3;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n\t}" ::"r"(bar), "r"(lead)
+        : "memory");
+}
+// The same shared-memory address in the first CTA of a pair.
+template <int CG>
+__device__ __forceinline__ uint32_t in_first(uint32_t addr) {
+  if (CG == 1) return addr;
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(0));
+  return r;
+}
+// Arrives on a barrier of either CTA.  What it orders is tensor-memory work, which the tcgen05 fences
+// around it order; a release at cluster scope would also wait for every store to global memory that
+// this thread still has in flight (measured: 1000 cycles per arrival).
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(addr),
+      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+      "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(addr));
+}
+
+// Barrier of the four epilogue warps that also tells whether any thread came with `v` set.
+__device__ __forceinline__ bool any_of_128(bool v) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.or.pred p, 1, 128, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(r)
+      : "r"((uint32_t)v)
+      : "memory");
+  return r != 0;
+}
+__device__ __forceinline__ float4 ldcg4(const float *p) { return __ldcg(reinterpret_cast<const float4 *>(p)); }
+
+// ---------------------------------------------------------------- weight formats
+// What differs between the formats is how a thread fetches the packed bytes of half a super-block
+// (one weight row x 128 columns: half hh) from the staged super-block and expands them, 32 columns
+// at a time.  Each format expands in the order its packed words yield values; src(p) names the
+// column (inside the super-block) that lands at position p, and the activations are laid out in the
+// same order, so the contraction is unchanged.
+//
+//   BB, BPS   bytes of a block of one row; blocks per super-block.  A staged super-block is
+//             [16 chunks][BPS blocks][8 rows x BB bytes], block-major as in HBM
+//   Pk        the packed bytes of half a super-block; load() fetches them (p: the row's chunk)
+//   expand    32 columns (quarter q = 0 .. 3 of the half) -> sixteen half2
+template <int T>
+struct WFmt;
+
+__device__ __forceinline__ uint32_t h2_bits(__half2 v) { return *reinterpret_cast<uint32_t *>(&v); }
+__device__ __forceinline__ __half2 bits_h2(uint32_t v) { return *reinterpret_cast<__half2 *>(&v); }
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t d;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+  return d;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t addr) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ uint32_t lds16(uint32_t addr) {
+  uint32_t v;
+  asm volatile("{\n\t.reg .u16 t;\n\tld.shared.u16 t, [%1];\n\tcvt.u32.u16 %0, t;\n\t}" : "=r"(v) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ uint32_t word(const uint4 &v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+// Four nibble pairs of one packed word -> 8 halves: low nibbles q become 1024 + q
+// (0x6400 | q), high nibbles 64 + q (0x5400 | q << 4, no shift needed); values come out
+// as pairs (byte 0, byte 2), (byte 1, byte 3) of the low nibbles, then of the high ones.
+__device__ __forceinline__ void nibbles_to_magic(uint32_t w, uint32_t e[4]) {
+  const uint32_t wj = w >> 8;
+  e[0] = (w & 0x000F000Fu) | 0x64006400u, e[1] = (wj & 0x000F000Fu) | 0x64006400u;
+  e[2] = (w & 0x00F000F0u) | 0x54005400u, e[3] = (wj & 0x00F000F0u) | 0x54005400u;
+}
+// Four unsigned bytes -> halves 1024 + b, in byte order.
+__device__ __forceinline__ void bytes_to_magic(uint32_t w, uint32_t &lo, uint32_t &hi) {
+  lo = prmt(w, 0x64646464u, 0x4140), hi = prmt(w, 0x64646464u, 0x4342);
+}
+
+template <>
+struct WFmt<QK_T_Q4_K> {  // d, dmin, 12 bytes of 6-bit scales / mins, 128 bytes of nibbles (reference/q4_k.rs:27-102)
+  static constexpr uint32_t BB = 144, BPS = 1, LUT = 0;
+  __device__ static void fill_lut(unsigned char *, uint32_t, uint32_t) {}
+  struct Pk { uint4 h, q[4]; };
+  // position 8 i + j of a 64-group <- column 4 i + {0,2,1,3}[j & 3] + 32 (j >> 2): byte 4 i + b of
+  // the group's 32 holds column 4 i + b (low nibble) and 32 + 4 i + b (high nibble)
+  __host__ __device__ static uint32_t src(uint32_t p) {
+    const uint32_t g = p >> 6, i = (p >> 3) & 7u, j = p & 7u, jj = j & 3u;
+    return 64 * g + 4 * i + (jj == 1 ? 2 : jj == 2 ? 1 : jj) + 32 * (j >> 2);
+  }
+  // [8 rows x 16 header | 4 groups x 8 rows x 32 nibble bytes]
+  __device__ static void load(Pk &k, uint32_t p, uint32_t rr, uint32_t hh) {
+    const uint32_t n = p + 128 + hh * 512 + rr * 32;
+    k.h = lds128(p + rr * 16), k.q[0] = lds128(n), k.q[1] = lds128(n + 16), k.q[2] = lds128(n + 256), k.q[3] = lds128(n + 272);
+  }
+  struct Sc { __half2 s[2], m[2]; };  // per 64-group: (low nibbles, high nibbles) of scale and of -min
+  __device__ static void scales(const Pk &k, uint32_t hh, Sc &c) {
+    // Sub-blocks 4 hh .. 4 hh + 3.  d * sc and dmin * mn have 17 bits at most, so the fp16 products
+    // are the f32 ones rounded once.
+    const uint32_t scw = hh ? ((k.h.w & 0x0F0F0F0Fu) | ((k.h.y >> 2) & 0x30303030u)) : (k.h.y & 0x3F3F3F3Fu);
+    const uint32_t mnw = hh ? (((k.h.w >> 4) & 0x0F0F0F0Fu) | ((k.h.z >> 2) & 0x30303030u)) : (k.h.z & 0x3F3F3F3Fu);
+    const __half2 k1024 = __float2half2_rn(1024.f), d = __low2half2(bits_h2(k.h.x)), m = __hneg2(__high2half2(bits_h2(k.h.x)));
+#pragma unroll
+    for (int g = 0; g < 2; g++) {
+      c.s[g] = __hmul2(__hsub2(bits_h2(prmt(scw, 0x64646464u, g ? 0x4342u : 0x4140u)), k1024), d);
+      c.m[g] = __hmul2(__hsub2(bits_h2(prmt(mnw, 0x64646464u, g ? 0x4342u : 0x4140u)), k1024), m);
+    }
+  }
+  // q exact after the subtraction, then one fused q * scale - min
+  __device__ static void expand(const Pk &k, const Sc &c, uint32_t, int q, uint32_t (&o)[16], uint32_t) {
+    const __half2 k_lo = __float2half2_rn(1024.f), k_hi = __float2half2_rn(64.f);
+    const __half2 s_lo = __low2half2(c.s[q >> 1]), s_hi = __high2half2(c.s[q >> 1]);
+    const __half2 m_lo = __low2half2(c.m[q >> 1]), m_hi = __high2half2(c.m[q >> 1]);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      uint32_t e[4];
+      nibbles_to_magic(word(k.q[q], i), e);
+      o[4 * i + 0] = h2_bits(__hfma2(__hsub2(bits_h2(e[0]), k_lo), s_lo, m_lo));
+      o[4 * i + 1] = h2_bits(__hfma2(__hsub2(bits_h2(e[1]), k_lo), s_lo, m_lo));
+      o[4 * i + 2] = h2_bits(__hfma2(__hsub2(bits_h2(e[2]), k_hi), s_hi, m_hi));
+      o[4 * i + 3] = h2_bits(__hfma2(__hsub2(bits_h2(e[3]), k_hi), s_hi, m_hi));
+    }
+  }
+};
+
+template <>
+struct WFmt<QK_T_Q8_0> {  // block of 32: f16 d, 32 int8 (reference/q8_0.rs)
+  static constexpr uint32_t BB = 34, BPS = 8, LUT = 0;
+  __device__ static void fill_lut(unsigned char *, uint32_t, uint32_t) {}
+  struct Pk { uint4 q[8]; uint32_t d[4]; };
+  __host__ __device__ static uint32_t src(uint32_t p) { return p; }
+  // A block's 8 rows: [2 granules x 8 rows x 16 int8][8 x d].  Blocks past the end of the row
+  // are zero-filled by the copy: d = 0.
+  __device__ static void load(Pk &k, uint32_t p, uint32_t rr, uint32_t hh) {
+    p += hh * 4 * 272;
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+      k.q[2 * b] = lds128(p + b * 272 + rr * 16), k.q[2 * b + 1] = lds128(p + b * 272 + 128 + rr * 16);
+      k.d[b] = lds16(p + b * 272 + 256 + 2 * rr);
+    }
+  }
+  struct Sc {};
+  __device__ static void scales(const Pk &, uint32_t, Sc &) {}
+  __device__ static void expand(const Pk &k, const Sc &, uint32_t, int q, uint32_t (&o)[16], uint32_t) {
+    const __half2 off = __float2half2_rn(1152.f);  // 1024 + 128: (1024 + (q ^ 0x80)) - 1152 = q, exact; q * d rounded once
+    const __half2 d = __low2half2(bits_h2(k.d[q]));
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      uint32_t a, b2;
+      bytes_to_magic(word(k.q[2 * q + (i >> 2)], i & 3) ^ 0x80808080u, a, b2);
+      o[2 * i] = h2_bits(__hmul2(__hsub2(bits_h2(a), off), d));
+      o[2 * i + 1] = h2_bits(__hmul2(__hsub2(bits_h2(b2), off), d));
+    }
+  }
+};
+
+template <>
+struct WFmt<QK_T_Q4_0> {  // block of 32: f16 d, 16 bytes; byte j = elements 2 j (low nibble) and 2 j + 1 (high) (reference/q4_0.rs:36-46)
+  static constexpr uint32_t BB = 18, BPS = 8, LUT = 0;
+  __device__ static void fill_lut(unsigned char *, uint32_t, uint32_t) {}
+  struct Pk { uint4 q[4]; uint32_t d[4]; };
+  // a word yields its eight elements as (byte 0, byte 2), (byte 1, byte 3) low nibbles, then the
+  // same of the high nibbles
+  __host__ __device__ static uint32_t src(uint32_t p) {
+    const uint32_t order = 0x73516240u;  // positions 0..7 <- elements 0, 4, 2, 6, 1, 5, 3, 7 of the word
+    return (p & ~7u) + ((order >> (4 * (p & 7u))) & 7u);
+  }
+  // A block's 8 rows: [8 rows x 16 nibble bytes][8 x d].
+  __device__ static void load(Pk &k, uint32_t p, uint32_t rr, uint32_t hh) {
+    p += hh * 4 * 144;
+#pragma unroll
+    for (int b = 0; b < 4; b++) k.q[b] = lds128(p + b * 144 + rr * 16), k.d[b] = lds16(p + b * 144 + 128 + 2 * rr);
+  }
+  struct Sc {};
+  __device__ static void scales(const Pk &, uint32_t, Sc &) {}
+  __device__ static void expand(const Pk &k, const Sc &, uint32_t, int q, uint32_t (&o)[16], uint32_t) {
+    const __half2 off_lo = __float2half2_rn(1032.f), off_hi = __float2half2_rn(72.f);  // (K + q) - (K + 8) = q - 8, exact
+    const __half2 d = __low2half2(bits_h2(k.d[q]));
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      uint32_t e[4];
+      nibbles_to_magic(word(k.q[q], i), e);
+      o[4 * i + 0] = h2_bits(__hmul2(__hsub2(bits_h2(e[0]), off_lo), d));
+      o[4 * i + 1] = h2_bits(__hmul2(__hsub2(bits_h2(e[1]), off_lo), d));
+      o[4 * i + 2] = h2_bits(__hmul2(__hsub2(bits_h2(e[2]), off_hi), d));
+      o[4 * i + 3] = h2_bits(__hmul2(__hsub2(bits_h2(e[3]), off_hi), d));
+    }
+  }
+};
+
+template <>
+struct WFmt<QK_T_Q6_K> {  // super-block of 256: ql 128, qh 64, 16 int8 scales, f16 d (reference/q6_k.rs)
+  static constexpr uint32_t BB = 210, BPS = 1, LUT = 0;
+  __device__ static void fill_lut(unsigned char *, uint32_t, uint32_t) {}
+  // half hh = ql[64 hh ..], qh[32 hh ..]; its quarter q (columns 32 q ..) = nibble q >> 1 of ql bytes
+  // 32 (q & 1) + l and bit pair 2 q of qh byte l
+  struct Pk { uint4 ql[4], qh[2]; uint2 sc; uint32_t d; };
+  __host__ __device__ static uint32_t src(uint32_t p) { return p; }
+  // A block's 8 rows: [12 granules x 8 rows x 16 bytes of ql+qh][8 rows x 16 scales][8 x d].
+  __device__ static void load(Pk &k, uint32_t p, uint32_t rr, uint32_t hh) {
+    const uint32_t q = p + rr * 16;
+#pragma unroll
+    for (int i = 0; i < 4; i++) k.ql[i] = lds128(q + (4 * hh + i) * 128);
+    k.qh[0] = lds128(q + (8 + 2 * hh) * 128), k.qh[1] = lds128(q + (9 + 2 * hh) * 128);
+    k.sc = lds64(q + 1536 + 8 * hh);
+    k.d = lds16(p + 1664 + 2 * rr);
+  }
+  struct Sc { float d; };
+  __device__ static void scales(const Pk &k, uint32_t, Sc &c) { c.d = h2f_bits(k.d); }
+  __device__ static void expand(const Pk &k, const Sc &c, uint32_t, int q, uint32_t (&o)[16], uint32_t) {
+    const __half2 off = __float2half2_rn(1056.f);  // (1024 + q) - 1056 = q - 32, exact; then one rounding in the product
+    const uint32_t scw = (q >> 1) ? k.sc.y : k.sc.x;
+    __half2 s[2];  // 16 columns per scale
+#pragma unroll
+    for (int i = 0; i < 2; i++) s[i] = __float2half2_rn(c.d * (float)(int)(signed char)((scw >> (16 * (q & 1) + 8 * i)) & 0xFF));
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const uint32_t lw = word(k.ql[2 * (q & 1) + (i >> 2)], i & 3), hw = word(k.qh[i >> 2], i & 3);
+      const uint32_t hi = q == 0 ? hw << 4 : q == 1 ? hw << 2 : q == 2 ? hw : hw >> 2;
+      const uint32_t q6 = (((q >> 1) ? lw >> 4 : lw) & 0x0F0F0F0Fu) | (hi & 0x30303030u);
+      uint32_t a, b2;
+      bytes_to_magic(q6, a, b2);
+      o[2 * i] = h2_bits(__hmul2(__hsub2(bits_h2(a), off), s[i >> 2]));
+      o[2 * i + 1] = h2_bits(__hmul2(__hsub2(bits_h2(b2), off), s[i >> 2]));
+    }
+  }
+};
+
+template <>
+struct WFmt<QK_T_IQ4_XS> {  // super-block of 256: f16 d, scales_h, scales_l[4], 128 nibble bytes (reference/iq4_xs.rs:47-97)
+  // sub-block s = nibble bytes 16 s ..; byte j holds elements 2 j (low) and 2 j + 1 (high); value =
+  // d (ls - 32) K[nibble] with the non-linear table K (iq_shared.rs:16-18).  A table in shared memory
+  // maps a byte straight to the half2 (K[low], K[high]) of its two adjacent elements; every lane has
+  // a copy of its own in its own bank (32 KB), so the look-ups of a warp never conflict.
+  static constexpr uint32_t BB = 136, BPS = 1, LUT = 32768;
+  struct Pk { uint4 q[4]; uint2 h; };
+  __host__ __device__ static uint32_t src(uint32_t p) { return p; }
+  __device__ static void fill_lut(unsigned char *lut, uint32_t tid, uint32_t nthreads) {
+    constexpr uint32_t K0 = 0xBFAD9881u, K1 = 0xF6EADDCFu, K2 = 0x26190D01u, K3 = 0x71594535u;  // K[0..15] as bytes
+    auto val = [&](uint32_t i) {
+      const uint32_t w = i < 8 ? (i < 4 ? K0 : K1) : (i < 12 ? K2 : K3);
+      return (float)(int)(signed char)((w >> (8 * (i & 3u))) & 0xFFu);
+    };
+    for (uint32_t i = tid; i < 256 * 32; i += nthreads)
+      reinterpret_cast<uint32_t *>(lut)[i] = h2_bits(__floats2half2_rn(val((i >> 5) & 15u), val(i >> 9)));
+  }
+  // A block's 8 rows: [8 granules x 8 rows x 16 nibble bytes][8 rows x 8 header bytes].
+  __device__ static void load(Pk &k, uint32_t p, uint32_t rr, uint32_t hh) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) k.q[i] = lds128(p + (4 * hh + i) * 128 + rr * 16);
+    k.h = lds64(p + 1024 + rr * 8);
+  }
+  struct Sc { float d; uint32_t ls; };  // ls: the half's four 6-bit scales, one per byte
+  __device__ static void scales(const Pk &k, uint32_t hh, Sc &c) {
+    c.d = h2f_bits(k.h.x);
+    const uint32_t sl = hh ? k.h.y >> 16 : k.h.y, sh = k.h.x >> (16 + 8 * hh);
+    c.ls = (sl & 0x0Fu) | ((sl & 0xF0u) << 4) | ((sl & 0xF00u) << 8) | ((sl & 0xF000u) << 12);
+    c.ls |= ((sh & 3u) << 4) | ((sh & 0xCu) << 10) | ((sh & 0x30u) << 16) | ((sh & 0xC0u) << 22);
+  }
+  // lut: this lane's copy (byte b at lut + 128 b)
+  __device__ static void expand(const Pk &k, const Sc &c, uint32_t, int q, uint32_t (&o)[16], uint32_t lut) {
+    const __half2 dl = __float2half2_rn(c.d * (float)((int)((c.ls >> (8 * q)) & 0x3Fu) - 32));
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const uint32_t w = word(k.q[q], i);
+      o[4 * i + 0] = h2_bits(__hmul2(bits_h2(lds32(lut + ((w << 7) & 0x7F80u))), dl));
+      o[4 * i + 1] = h2_bits(__hmul2(bits_h2(lds32(lut + ((w >> 1) & 0x7F80u))), dl));
+      o[4 * i + 2] = h2_bits(__hmul2(bits_h2(lds32(lut + ((w >> 9) & 0x7F80u))), dl));
+      o[4 * i + 3] = h2_bits(__hmul2(bits_h2(lds32(lut + ((w >> 17) & 0x7F80u))), dl));
+    }
+  }
+};
+
+// ---------------------------------------------------------------- activations -> fp16
+// X16[t][256 s + p] = x[t][256 s + src(p)] / scale[t] in fp16, where scale[t] is the power
+// of two that puts the row's largest magnitude in [512, 1024): the division is exact, no
+// activation overflows or falls into fp16's subnormals, and the epilogue multiplies the
+// row of results by scale[t] again (also exact).  Columns >= cols are zero.  One CTA per token
+// row; a row of up to 16384 columns is read once and stays in registers between the maximum and
+// the conversion (a thread's eight positions come from two float4s whatever the format's order).
+// GLU: the row is silu(x) * x2, formed here (crates/oxillama-arch/src/common/swiglu.rs:15-21, each
+// step rounded), so the hidden activations of a feed-forward block are never written out in f32.
+constexpr int CT = 512, CCH = 4;  // threads; chunks of eight positions a thread keeps
+struct ConvArgs {
+  const float *x, *x2;
+  __half *out;
+  float *scales;
+  unsigned *zero;                 // arrival counters of the matmul that follows, cleared here
+  const int *counts, *lists;      // grouped: live rows per group; rows to gather (row t of group e = x[lists[e][t] / list_div])
+  uint32_t m, cols, Kp, n_zero, cap, list_stride, list_div;
+};
+
+__device__ __forceinline__ float silu_mul(float g, float u) {
+  const float sg = __fdiv_rn(1.f, __fadd_rn(1.f, expf(-g)));
+  return __fmul_rn(__fmul_rn(g, sg), u);
+}
+// The eight activations of positions 8 c .. 8 c + 7.
+template <int T, bool GLU>
+__device__ __forceinline__ void conv_load(const float *__restrict__ x, const float *__restrict__ x2, uint32_t c,
+                                          uint32_t cols, bool vec, float (&v)[8]) {
+  const uint32_t ka = T == QK_T_Q4_K ? (c >> 3) * 64 + (c & 7u) * 4 : c * 8, kb = T == QK_T_Q4_K ? ka + 32 : ka + 4;
+  float a[4], b[4];
+  auto quad = [&](uint32_t k, float (&q)[4]) {
+    if (vec && k + 4 <= cols) {
+      const float4 f = __ldg(reinterpret_cast<const float4 *>(x + k));
+      q[0] = f.x, q[1] = f.y, q[2] = f.z, q[3] = f.w;
+      if (GLU) {
+        const float4 u = __ldg(reinterpret_cast<const float4 *>(x2 + k));
+        q[0] = silu_mul(q[0], u.x), q[1] = silu_mul(q[1], u.y), q[2] = silu_mul(q[2], u.z), q[3] = silu_mul(q[3], u.w);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        q[i] = k + i < cols ? __ldg(x + k + i) : 0.f;
+        if (GLU && k + i < cols) q[i] = silu_mul(q[i], __ldg(x2 + k + i));
+      }
+    }
+  };
+  quad(ka, a), quad(kb, b);
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    uint32_t e;  // which of the eight loaded values lands at position j
+    if (T == QK_T_Q4_K) e = (j & 4) + ((j & 3) == 1 ? 2 : (j & 3) == 2 ? 1 : (j & 3));
+    else e = WFmt<T>::src((uint32_t)j);
+    v[j] = e < 4 ? a[e & 3] : b[e & 3];
+  }
+}
+
+template <int T, bool GLU>
+__global__ void __launch_bounds__(CT) qk_x16_kernel(const ConvArgs A) {
+  __shared__ float red[CT / 32];
+  pdl_launch_dependents();
+  pdl_wait();
+  if (blockIdx.x == 0)
+    for (uint32_t i = threadIdx.x; i < A.n_zero; i += CT) A.zero[i] = 0u;
+  const uint32_t t = blockIdx.x;
+  const float *xr = A.x + (uint64_t)t * A.cols, *ur = A.x2 + (uint64_t)t * A.cols;
+  if (A.counts) {
+    const uint32_t e = t / A.cap, tl = t % A.cap;
+    if (tl >= (uint32_t)A.counts[e]) return;  // rows past the live ones: never stored, their values do not matter
+    if (A.lists) xr = A.x + (uint64_t)(A.lists[(uint64_t)e * A.list_stride + tl] / (int)A.list_div) * A.cols;
+  }
+  const bool vec = (A.cols & 3u) == 0 && (((uintptr_t)xr | (GLU ? (uintptr_t)ur : 0u)) & 15u) == 0;
+  const uint32_t nch = A.Kp / 8;
+  float v[CCH][8];
+  float amax = 0.f;
+#pragma unroll
+  for (int i = 0; i < CCH; i++) {
+    const uint32_t c = threadIdx.x + i * CT;
+    if (c < nch) {
+      conv_load<T, GLU>(xr, ur, c, A.cols, vec, v[i]);
+#pragma unroll
+      for (int j = 0; j < 8; j++) amax = fmaxf(amax, fabsf(v[i][j]));
+    }
+  }
+  for (uint32_t c = threadIdx.x + CCH * CT; c < nch; c += CT) {  // wider rows: read again below
+    float w[8];
+    conv_load<T, GLU>(xr, ur, c, A.cols, vec, w);
+#pragma unroll
+    for (int j = 0; j < 8; j++) amax = fmaxf(amax, fabsf(w[j]));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
+  __syncthreads();
+  amax = red[0];
+#pragma unroll
+  for (int w = 1; w < CT / 32; w++) amax = fmaxf(amax, red[w]);
+  float scale = 1.f;
+  if (amax > 0.f && amax <= FLT_MAX) {  // finite and non-zero (a NaN row keeps scale 1 and stays NaN)
+    int e;
+    frexpf(amax, &e);  // amax = f * 2^e, f in [0.5, 1)
+    scale = ldexpf(1.f, e - 10);
+  }
+  const float inv = 1.f / scale;  // a power of two: exact
+  if (threadIdx.x == 0) A.scales[t] = scale;
+  __half *orow = A.out + (uint64_t)t * A.Kp;
+  auto put = [&](uint32_t c, const float (&w)[8]) {
+    uint32_t h[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) h[j] = h2_bits(__floats2half2_rn(w[2 * j] * inv, w[2 * j + 1] * inv));
+    *reinterpret_cast<uint4 *>(orow + 8ull * c) = make_uint4(h[0], h[1], h[2], h[3]);
+  };
+#pragma unroll
+  for (int i = 0; i < CCH; i++) {
+    const uint32_t c = threadIdx.x + i * CT;
+    if (c < nch) put(c, v[i]);
+  }
+  for (uint32_t c = threadIdx.x + CCH * CT; c < nch; c += CT) {
+    float w[8];
+    conv_load<T, GLU>(xr, ur, c, A.cols, vec, w);
+    put(c, w);
+  }
+}
+
+// ---------------------------------------------------------------- schedule
+// The segments of one CTA (pair), the same list for every role: first its run of the split tiles
+// (tiles 0 .. R - 1, R = the remainder of the tile count over the pairs, their R * nsb super-blocks cut
+// into equal runs), then whole tiles R + pair, + pairs, ..
+struct Sched {
+  uint32_t nsb, R, base, rem, b, e, first_tile, n_split, n_seg, me, pairs;
+  template <int CG>
+  __device__ __forceinline__ void init(uint32_t tiles, uint32_t nsb_, uint32_t min_run) {
+    nsb = nsb_, me = blockIdx.x / CG, pairs = gridDim.x / CG;
+    const uint32_t whole = tiles / pairs;
+    R = tiles - whole * pairs;
+    const uint32_t total = R * nsb, runs = total / min_run;
+    const uint32_t n = runs < pairs ? (runs ? runs : 1u) : pairs;  // pairs that share the split part
+    base = total / n, rem = total - base * n;                             // the first `rem` runs are one longer
+    b = e = first_tile = n_split = 0;
+    if (R && me < n) {
+      b = start_of(me), e = start_of(me + 1);
+      first_tile = b / nsb;
+      n_split = (e - 1) / nsb - first_tile + 1;
+    }
+    n_seg = n_split + whole;
+  }
+  __device__ __forceinline__ uint32_t start_of(uint32_t pair) const { return pair * base + (pair < rem ? pair : rem); }
+  __device__ __forceinline__ uint32_t owner_of(uint32_t sb) const {  // pair whose run holds super-block sb of the split part
+    const uint32_t longer = rem * (base + 1);
+    return sb < longer ? sb / (base + 1) : rem + (sb - longer) / base;
+  }
+  __device__ __forceinline__ void get(uint32_t i, uint32_t &tile, uint32_t &s0, uint32_t &s1) const {
+    if (i < n_split) {
+      tile = first_tile + i;
+      s0 = i == 0 ? b - tile * nsb : 0u;
+      s1 = i + 1 == n_split ? e - tile * nsb : nsb;
+    } else {
+      tile = R + me + (i - n_split) * pairs, s0 = 0, s1 = nsb;
+    }
+  }
+};
+// Where a tile lies: its matrix, row block, first token inside the group and live tokens of that group.
+struct TileAt {
+  uint32_t g, rb, t0, live, n;  // n: tokens the MMA covers, a multiple of 16
+};
+
+// The super-blocks of a segment in the order the MMAs take them: one at a time (`half` 0, then 1),
+// but at either end of a wide tile two at a time (both under half 0, then both under half 1).
+// Calls step(sb, half, which of the two, last use of the super-block's weights, end of the segment) -> false to stop.
+template <class Step>
+__device__ __forceinline__ bool walk_segment(uint32_t s0, uint32_t s1, bool wide, Step &&step) {
+  for (uint32_t sb = s0; sb < s1;) {
+    const uint32_t two = wide && s1 - sb >= 2 && (sb == s0 || s1 - sb == 2) ? 2u : 1u;
+    for (uint32_t h = 0; h < (wide ? 2u : 1u); h++)
+      for (uint32_t k = 0; k < two; k++)
+        if (!step(sb + k, h, k, h == (wide ? 1u : 0u), sb + k + 1 == s1)) return false;
+    sb += two;
+  }
+  return true;
+}
+
+// ---------------------------------------------------------------- main kernel
+// T: weight format.  CG: CTAs per tile (see the top).  NG: 1 = one matrix; otherwise up to NG matrices
+// of one shape and format (the projections of a feed-forward block, the experts of a mixture), each
+// multiplying its own group of activation rows.
+template <int T, int CG, int NG>
+__global__ void __launch_bounds__(NTHREADS, 1)
+    qk_gemm_tc_kernel(const __grid_constant__ TcArgs A, const __grid_constant__ TcMaps<NG> M) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  using F = WFmt<T>;
+  const TcSmem &S = A.S;
+  const uint32_t sbase = smem_u32(smem);
+  const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const uint32_t rank = CG == 1 ? 0u : blockIdx.x & 1u;  // in the pair; rank 0 issues the MMAs of both
+  // Tensor memory: two accumulator halves, then na buffers of 128 columns for the expanded weights.
+  const bool narrow = A.hn <= 64;
+  const uint32_t na = narrow ? 3u : 2u, d_step = narrow ? 64u : 128u, a_col = 2 * d_step;
+
+  pdl_launch_dependents();
+  if (threadIdx.x == 0) {
+    for (uint32_t s = 0; s < S.w_stages; s++) mbar_init(sbase + S.w_full + s * 8, 1), mbar_init(sbase + S.w_empty + s * 8, NDW / 2);
+    for (uint32_t s = 0; s < S.b_stages; s++) mbar_init(sbase + S.b_full + s * 8, 1), mbar_init(sbase + S.b_empty + s * 8, 1);
+    for (uint32_t s = 0; s < 3; s++) mbar_init(sbase + S.a_full + s * 8, CG * NDW / 2), mbar_init(sbase + S.a_empty + s * 8, 1);
+    for (uint32_t s = 0; s < 2; s++) mbar_init(sbase + S.d_full + s * 8, 1), mbar_init(sbase + S.d_empty + s * 8, CG * 4);
+    mbar_init(sbase + S.drain, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (threadIdx.x == 32) asm volatile("prefetch.tensormap [%0];" ::"l"(&M.x[0]) : "memory");
+  if (threadIdx.x == 64 && NG == 1) asm volatile("prefetch.tensormap [%0];" ::"l"(&M.w[0]) : "memory");
+  if (F::LUT) F::fill_lut(smem + S.lut, threadIdx.x, NTHREADS);
+  if (warp == 3) {
+    if (CG == 1) {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + S.tmem_slot), "r"(512u) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + S.tmem_slot), "r"(512u) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+  }
+  uint32_t *pre = reinterpret_cast<uint32_t *>(smem + S.pre);  // tiles before group g (device-counted groups)
+  const bool counted = NG > 1 && A.counts;
+  if (counted) {
+    pdl_wait();  // the counts are the work of an earlier kernel
+    if (threadIdx.x == 0) {
+      uint32_t s = 0;
+      for (uint32_t g = 0; g < A.n; g++) {
+        pre[g] = s;
+        s += A.row_blocks * (((uint32_t)A.counts[g % A.n_act] + A.bn - 1) / A.bn);
+      }
+      pre[A.n] = s;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (CG == 2) cluster_sync();  // the other CTA's barriers are initialised, its tensor memory is there
+  tc_fence_after();
+  const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(smem + S.tmem_slot);
+
+  Sched sc{};
+  sc.template init<CG>(counted ? pre[A.n] : A.n * A.row_blocks * A.tok_blocks, (A.L.cols + 255u) / 256u, A.min_run);
+  auto at = [&](uint32_t tile) {
+    TileAt q;
+    uint32_t tb;
+    if (counted) {
+      uint32_t g = 0;
+      while (tile >= pre[g + 1]) g++;
+      q.g = g, q.live = (uint32_t)__ldg(A.counts + g % A.n_act);
+      const uint32_t r = tile - pre[g], nt = (q.live + A.bn - 1) / A.bn;
+      q.rb = r / nt, tb = r % nt;
+    } else {  // a row block's token blocks are neighbours: its weights are read by CTAs that run at the same time
+      tb = tile % A.tok_blocks;
+      const uint32_t r = tile / A.tok_blocks;
+      q.g = NG > 1 ? r / A.row_blocks : 0u, q.rb = NG > 1 ? r % A.row_blocks : r, q.live = A.m;
+    }
+    q.t0 = tb * A.bn;
+    const uint32_t left = q.live - q.t0;
+    q.n = left >= A.bn ? A.bn : ((left + 15u) & ~15u);
+    return q;
+  };
+  const bool both = A.bn > 128;  // a tile owns both accumulator halves
+  // Token rows that an activation box brings: each CTA of a pair loads half of the n tokens.
+  const uint32_t hq = A.hn / (4 * CG);
+  auto box_rows = [&](uint32_t n) { return NG > 1 ? (n / CG + hq - 1) / hq * hq : A.hn / CG; };
+
+  bool dead = false;
+  if (warp == 0 && rank == 0) {
+    // ======================= MMA issuer =======================
+    const uint32_t lead = elect_one() ? 1u : 0u;
+    uint32_t bs = 0, bph = 0, ab = 0, aph = 0, dph = 0;  // dph bit h: parity of the next wait for half h; bit 2 + h: it was used before
+    for (uint32_t i = 0; i < sc.n_seg && !dead; i++) {
+      uint32_t tile, s0, s1;
+      sc.get(i, tile, s0, s1);
+      const TileAt q = at(tile);
+      const bool wide = q.n > A.hn;
+      uint32_t begun = 0;      // halves whose accumulator this segment has taken over
+      uint32_t ab1 = 0;        // (two super-blocks at a time) buffers are walked again under the second half
+      const bool ok = walk_segment(s0, s1, wide, [&](uint32_t, uint32_t h, uint32_t k, bool last, bool end) {
+        const uint32_t n = h ? q.n - A.hn : wide ? A.hn : q.n, dh = both ? h : i & 1u;
+        const uint32_t step16 = box_rows(n) * 8u;  // a step of the activation stage, in units of 16 bytes
+        const uint32_t idesc = (1u << 4) | ((n >> 3) << 17) | ((CG * BM >> 4) << 24), d = tmem + dh * d_step;
+        uint32_t acc = 1u;
+        if (!(begun & (1u << h))) {
+          begun |= 1u << h, acc = 0u;
+          if ((dph >> (2 + dh)) & 1u) {
+            if (!warp_wait(sbase + S.d_empty + dh * 8, (dph >> dh) & 1u)) return false;
+            dph ^= 1u << dh;
+          }
+          dph |= 4u << dh;
+        }
+        if (h == 0) {
+          if (k == 0) ab1 = ab;
+          if (!warp_wait(sbase + S.a_full + ab * 8, aph)) return false;
+          tc_fence_after();
+        } else if (k == 0) {
+          ab = ab1;
+        }
+        const uint32_t a = tmem + a_col + ab * 128u;
+        if (!warp_wait(sbase + S.b_full + bs * 8, bph)) return false;
+        const uint32_t bd = umma_desc_lo(sbase + S.b + bs * S.b_stage);
+#pragma unroll
+        for (uint32_t g = 0; g < 4; g++)
+#pragma unroll
+          for (uint32_t j = 0; j < 4; j++) umma_f16_ta<CG>(d, a + g * 32 + j * 8, bd + g * step16 + j * 2, idesc, g || j ? 1u : acc, lead);
+        umma_commit<CG>(sbase + S.b_empty + bs * 8, lead);
+        if (++bs == S.b_stages) bs = 0, bph ^= 1u;
+        if (last) umma_commit<CG>(sbase + S.a_empty + ab * 8, lead);
+        if (end) umma_commit<CG>(sbase + S.d_full + dh * 8, lead);
+        if (++ab == na) {
+          ab = 0;
+          if (h == 0) aph ^= 1u;
+        }
+        return true;
+      });
+      if (!ok) dead = true;
+    }
+    if (dead) {  // let what was issued retire before the CTA gives its memory back
+      if (lead) atomicOr(A.status, QK_DEV_TIMEOUT);
+      umma_commit<CG>(sbase + S.drain, lead);
+      (void)mbar_wait_bounded(sbase + S.drain, 0);
+    }
+  } else if (warp == 1) {
+    // ======================= activation producer =======================
+    const uint32_t lead = elect_one() ? 1u : 0u;
+    pdl_wait();  // X16 belongs to the previous kernel until it has finished
+    const uint32_t full0 = in_first<CG>(sbase + S.b_full);
+    uint32_t bs = 0, bph = 0, rounds = 0, bar = sbase + S.b_full, dst = sbase + S.b, full = full0;
+    const uint32_t to_empty = S.b_empty - S.b_full, nst = S.b_stages, stage = S.b_stage;
+    for (uint32_t i = 0; i < sc.n_seg && !dead; i++) {
+      uint32_t tile, s0, s1;
+      sc.get(i, tile, s0, s1);
+      const TileAt q = at(tile);
+      const bool wide = q.n > A.hn;
+      const uint32_t row0 = (NG > 1 ? (q.g % A.n_act) * A.xcap : 0u) + q.t0;
+      const bool ok = walk_segment(s0, s1, wide, [&](uint32_t sb, uint32_t h, uint32_t, bool, bool) {
+        const uint32_t n = h ? q.n - A.hn : wide ? A.hn : q.n, rows = box_rows(n);
+        const uint32_t r0 = row0 + (h ? A.hn : 0u) + (rank ? n / 2 : 0u);
+        const CUtensorMap *map = &M.x[NG > 1 ? rows / hq - 1 : 0];
+        if (rounds && !warp_wait(bar + to_empty, bph ^ 1u)) return false;
+        // the halves of both CTAs land on the barrier of rank 0, which alone announces them
+        if (rank == 0) expect_tx(bar, rows * 512u * CG, lead);
+        tma_load_3d<CG>(dst, map, 0, (int)r0, (int)(sb * 4), full, lead);
+        bs++, bar += 8, full += 8, dst += stage;
+        if (bs == nst) bs = 0, bph ^= 1u, rounds = 1, bar = sbase + S.b_full, full = full0, dst = sbase + S.b;
+        return true;
+      });
+      if (!ok) dead = true;
+    }
+    if (dead) {
+      if (lead) atomicOr(A.status, QK_DEV_TIMEOUT);
+      if (rank == 0)  // copies in flight land before the CTAs end
+        for (uint32_t k = 0; k < nst; k++)
+          if (rounds || k < bs) (void)mbar_wait_bounded(sbase + S.b_full + k * 8, k < bs ? bph : bph ^ 1u);
+    }
+  } else if (warp == 2) {
+    // ======================= weight producer =======================
+    // The weights are immutable: their stream starts before the previous kernel has ended.
+    const uint32_t lead = elect_one() ? 1u : 0u;
+    uint64_t policy;
+    if (A.once) policy = stream_policy();
+    else asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(policy));
+    uint32_t ws = 0, wph = 0, rounds = 0, bar = sbase + S.w_full, dst = sbase + S.w;
+    const uint32_t to_empty = S.w_empty - S.w_full, nst = S.w_stages, stage = S.w_stage;
+    for (uint32_t i = 0; i < sc.n_seg && !dead; i++) {
+      uint32_t tile, s0, s1;
+      sc.get(i, tile, s0, s1);
+      const TileAt q = at(tile);
+      const CUtensorMap *map = &M.w[NG > 1 ? q.g : 0];
+      for (uint32_t sb = s0; sb < s1; sb++) {
+        if (rounds && !warp_wait(bar + to_empty, wph ^ 1u)) {
+          dead = true;
+          break;
+        }
+        expect_tx(bar, stage, lead);
+        tma_load_3d_hint(dst, map, 0, (int)(sb * F::BPS), (int)(q.rb * (16 * CG) + rank * 16), bar, policy, lead);
+        ws++, bar += 8, dst += stage;
+        if (ws == nst) ws = 0, wph ^= 1u, rounds = 1, bar = sbase + S.w_full, dst = sbase + S.w;
+      }
+    }
+    if (dead) {
+      if (lead) atomicOr(A.status, QK_DEV_TIMEOUT);
+      for (uint32_t k = 0; k < nst; k++)
+        if (rounds || k < ws) (void)mbar_wait_bounded(sbase + S.w_full + k * 8, k < ws ? wph : wph ^ 1u);
+    }
+  } else if (warp >= FIRST_EW) {
+    // ======================= epilogue warps =======================
+    // Warp `quarter` owns accumulator lanes (weight rows) 32 quarter .. + 32 of every half.
+    const uint32_t quarter = warp & 3u, r = 32 * quarter + lane;
+    const uint32_t tlane = tmem + ((32 * quarter) << 16);
+    const uint32_t d_empty = in_first<CG>(sbase + S.d_empty);
+    float *scales = reinterpret_cast<float *>(smem + S.scales) + quarter * 128;  // this warp's copy of a half's token scales
+    volatile uint32_t *told = reinterpret_cast<volatile uint32_t *>(smem + S.scales + 2048);
+    uint32_t dph = 0;
+    pdl_wait();  // y, the scales and the workspace belong to the previous kernel until it has finished
+    const uint64_t ldy = A.ldy;
+    for (uint32_t i = 0; i < sc.n_seg && !dead; i++) {
+      uint32_t tile, s0, s1;
+      sc.get(i, tile, s0, s1);
+      const TileAt q = at(tile);
+      const bool wide = q.n > A.hn;
+      const bool split = i < sc.n_split && (s0 != 0 || s1 != sc.nsb);
+      const uint32_t row0 = (q.rb * CG + rank) * BM, row = row0 + r;
+      const float *sp = A.xscale + (NG > 1 ? (q.g % A.n_act) * A.xcap : 0u) + q.t0;
+      float *yt = A.y + (uint64_t)((NG > 1 ? q.g * A.ycap : 0u) + q.t0) * ldy;  // the tile's first token
+      // partial tiles: [slot][token][128 rows]
+      const uint32_t slot = A.bn * BM;
+      float *mine = A.part + (blockIdx.x * 2 + (i == 0 ? 0u : 1u)) * slot + r;
+      for (uint32_t h = 0; h < (wide ? 2u : 1u); h++) {
+        const uint32_t dh = both ? h : i & 1u, hoff = h * A.hn;  // first token of the half inside the tile
+        const uint32_t n = h ? q.n - A.hn : wide ? A.hn : q.n;
+        const uint32_t live = min(q.live - q.t0 - hoff, n);      // tokens to write
+        if (!split) {
+          __syncwarp();
+#pragma unroll
+          for (uint32_t k = 0; k < 4; k++) scales[k * 32 + lane] = k * 32 + lane < live ? __ldg(sp + hoff + k * 32 + lane) : 0.f;
+          __syncwarp();
+        }
+        if (!warp_wait(sbase + S.d_full + dh * 8, (dph >> dh) & 1u)) {
+          dead = true;
+          break;
+        }
+        dph ^= 1u << dh;
+        tc_fence_after();
+        float *yp = yt + (uint64_t)hoff * ldy + row, *pp = mine + hoff * BM;
+        for (uint32_t c = 0; c < n; c += 16, pp += 16 * BM) {
+          uint32_t v[16];
+          tmem_ld16(tlane + dh * d_step + c, v);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (c + 16 == n) {  // read to the end: the half is free for its next tile
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(d_empty + dh * 8);
+          }
+          if (split) {
+#pragma unroll
+            for (uint32_t j = 0; j < 16; j++) __stcg(pp + j * BM, __uint_as_float(v[j]));
+          } else {
+            const float4 *f4 = reinterpret_cast<const float4 *>(scales + c);
+            if (row0 + 32 * quarter + 32 <= A.L.rows && c + 16 <= live) {  // warp-uniform: all of it is wanted
+#pragma unroll
+              for (uint32_t j4 = 0; j4 < 4; j4++) {
+                const float4 f = f4[j4];
+                *yp = __uint_as_float(v[4 * j4]) * f.x, yp += ldy;
+                *yp = __uint_as_float(v[4 * j4 + 1]) * f.y, yp += ldy;
+                *yp = __uint_as_float(v[4 * j4 + 2]) * f.z, yp += ldy;
+                *yp = __uint_as_float(v[4 * j4 + 3]) * f.w, yp += ldy;
+              }
+            } else {
+#pragma unroll
+              for (uint32_t j = 0; j < 16; j++, yp += ldy)
+                if (row < A.L.rows && c + j < live) *yp = __uint_as_float(v[j]) * scales[c + j];
+            }
+          }
+        }
+      }
+      if (!split) continue;
+      // Count in, once both halves are in the workspace (the accumulators are free by now); the last
+      // contributor adds the partials up, in the order of their K runs.
+      const uint32_t i0 = sc.owner_of(tile * sc.nsb), i1 = sc.owner_of((tile + 1) * sc.nsb - 1);
+      __threadfence();
+      if (any_of_128(dead)) {
+        dead = true;
+        continue;
+      }
+      if (warp == FIRST_EW && lane == 0) *told = atomicAdd(A.cnt + tile * 2 + rank, 1u);
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      if (*told != i1 - i0) continue;
+      __threadfence();
+      // lane: rows 4 lane .. + 3; the four warps share the tokens, four at a time
+      const uint32_t live = min(q.live - q.t0, q.n), rw = row0 + 4 * lane;
+      const bool vec = row0 + BM <= A.L.rows && (ldy & 3u) == 0 && ((uintptr_t)A.y & 15u) == 0;
+      for (uint32_t c = 4 * quarter; c < live; c += 16) {
+        float4 s[4];
+#pragma unroll
+        for (uint32_t j = 0; j < 4; j++) s[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+        for (uint32_t p = i0; p <= i1; p++) {
+          const float *src = A.part + ((p * CG + rank) * 2 + (sc.start_of(p) / sc.nsb == tile ? 0u : 1u)) * slot + c * BM + 4 * lane;
+          float4 o[4];
+#pragma unroll
+          for (uint32_t j = 0; j < 4; j++) o[j] = ldcg4(src + j * BM);  // (token rows past the live ones exist: n is a multiple of 16)
+#pragma unroll
+          for (uint32_t j = 0; j < 4; j++) s[j].x += o[j].x, s[j].y += o[j].y, s[j].z += o[j].z, s[j].w += o[j].w;
+        }
+        float *yp = yt + (uint64_t)c * ldy + rw;
+#pragma unroll
+        for (uint32_t j = 0; j < 4; j++, yp += ldy) {
+          if (c + j >= live) break;
+          const float f = __ldg(sp + c + j);
+          const float4 v = make_float4(s[j].x * f, s[j].y * f, s[j].z * f, s[j].w * f);
+          if (vec) {
+            *reinterpret_cast<float4 *>(yp) = v;
+          } else {
+            if (rw < A.L.rows) yp[0] = v.x;
+            if (rw + 1 < A.L.rows) yp[1] = v.y;
+            if (rw + 2 < A.L.rows) yp[2] = v.z;
+            if (rw + 3 < A.L.rows) yp[3] = v.w;
+          }
+        }
+      }
+    }
+    if (dead && lane == 0) atomicOr(A.status, QK_DEV_TIMEOUT);
+  } else if (warp >= FIRST_DW) {
+    // ======================= expanding warps =======================
+    // Set `set` takes every second super-block; in it, warp (hh, quarter) the columns [128 hh, + 128)
+    // and the tensor-memory lanes 32 quarter .. + 32.
+    const uint32_t set = (warp - FIRST_DW) >> 3, hh = ((warp - FIRST_DW) >> 2) & 1u, quarter = warp & 3u;
+    const uint32_t r = 32 * quarter + lane, rr = r & 7u;               // weight row inside the tile, inside its chunk
+    constexpr uint32_t CHB = 8 * F::BB * F::BPS;                       // a chunk's bytes of one super-block
+    const uint32_t lut = sbase + S.lut + lane * 4;
+    uint32_t n_sb = 0;
+    for (uint32_t i = 0; i < sc.n_seg; i++) {
+      uint32_t tile, s0, s1;
+      sc.get(i, tile, s0, s1);
+      n_sb += s1 - s0;
+    }
+    const uint32_t w_bytes = S.w_stage, nst = S.w_stages, w0 = sbase + S.w + (r >> 3) * CHB;
+    const uint32_t ta0 = tmem + ((32 * quarter) << 16) + a_col + hh * 64u, a_full0 = in_first<CG>(sbase + S.a_full);
+    uint32_t ws = set % nst, wph = set / nst & 1u;      // ring stage and parity of this set's next super-block
+    uint32_t ab = set, auses = 0;                       // its buffer, and how often that has been used (set < na)
+    for (uint32_t j = set; j < n_sb; j += 2) {
+      if (!warp_wait(sbase + S.w_full + ws * 8, wph)) {
+        dead = true;  // warp-uniform: these warps execute .aligned tcgen05 instructions
+        break;
+      }
+      typename F::Pk pk;
+      F::load(pk, w0 + ws * w_bytes, rr, hh);
+      typename F::Sc c;
+      F::scales(pk, hh, c);
+      uint32_t o[16];
+      F::expand(pk, c, hh, 0, o, lut);
+      // the MMAs that read this buffer's previous contents must have retired
+      if (auses && !warp_wait(sbase + S.a_empty + ab * 8, (auses - 1) & 1u)) {
+        dead = true;
+        break;
+      }
+      tc_fence_after();
+      const uint32_t ta = ta0 + ab * 128u;
+      tmem_st16(ta, o);
+#pragma unroll
+      for (int k = 1; k < 4; k++) {
+        F::expand(pk, c, hh, k, o, lut);
+        if (k == 3) {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(sbase + S.w_empty + ws * 8);  // every lane holds its packed bytes
+        }
+        tmem_st16(ta + 16 * k, o);
+      }
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(a_full0 + ab * 8);
+      ws += 2;
+      if (ws >= nst) ws -= nst, wph ^= 1u;
+      ab += 2;
+      if (ab >= na) ab -= na, auses++;
+    }
+    if (dead && lane == 0) atomicOr(A.status, QK_DEV_TIMEOUT);
+  }
+
+  // common exit: the tensor memory is always returned
+  tc_fence_before();
+  __syncthreads();
+  if (CG == 2) cluster_sync();  // neither CTA leaves while the other may still arrive on its barriers or read its operands
+  tc_fence_after();
+  if (warp == 3) {
+    if (CG == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+  }
+}
+
+// ---------------------------------------------------------------- host side
+constexpr uint32_t SMEM_BUDGET = 226u * 1024u;
+
+struct TcPlan {
+  TcSmem S;
+  uint32_t cg, smem, bn, hn, tok_blocks, row_blocks, nsb, min_run, grid, xrows;
+  size_t o_scale, o_cnt, o_part, bytes;
+};
+// qk_gemm_tc.cu
+bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P);
+bool x_map(CUtensorMap *m, __half *x16, uint32_t xrows, uint32_t Kp, uint32_t rows);
+
+inline cudaLaunchAttribute pdl_attr() {
+  cudaLaunchAttribute a = {};
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  return a;
+}
+
+template <int T, int CG, int NG>
+cudaError_t launch_main(const TcPlan &P, const TcArgs &A, __half *x16, const QkTcCall &c, cudaStream_t s) {
+  auto kern = qk_gemm_tc_kernel<T, CG, NG>;
+  static QkPerDevice attr_set;
+  if (attr_set.first()) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BUDGET);
+    if (e != cudaSuccess) return attr_set.reset(), e;
+  }
+  TcMaps<NG> M;
+  for (uint32_t k = 0; k < (NG > 1 ? 4u : 1u); k++)
+    if (!x_map(&M.x[k], x16, P.xrows, P.nsb * 256u, NG > 1 ? P.hn / (4 * CG) * (k + 1) : P.hn / CG)) return cudaErrorInvalidValue;
+  for (uint32_t g = 0; g < (NG == 1 ? 1u : c.n); g++) memcpy(&M.w[g], c.maps[g], sizeof(CUtensorMap));
+  cudaLaunchAttribute at[2] = {pdl_attr(), {}};
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = 2, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(P.grid), cfg.blockDim = dim3(NTHREADS), cfg.dynamicSmemBytes = P.smem, cfg.stream = s;
+  cfg.attrs = at, cfg.numAttrs = CG == 2 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kern, A, M);
+}
+
+template <int T>
+cudaError_t launch_fmt(const QkTcCall &c, unsigned *status, unsigned char *scratch, int sm_count, cudaStream_t s) {
+  const QkLayout &L = *c.L;
+  TcPlan P;
+  if (!make_plan(c, sm_count, &P)) return cudaErrorInvalidConfiguration;
+  const uint32_t Kp = P.nsb * 256u;
+  __half *x16 = reinterpret_cast<__half *>(scratch);
+  float *scales = reinterpret_cast<float *>(scratch + P.o_scale);
+  unsigned *cnt = reinterpret_cast<unsigned *>(scratch + P.o_cnt);
+  ConvArgs C = {};
+  C.x = c.x, C.x2 = c.x2, C.out = x16, C.scales = scales, C.zero = cnt, C.n_zero = (uint32_t)sm_count * 2;
+  C.counts = c.counts, C.lists = c.lists, C.m = c.m, C.cols = L.cols, C.Kp = Kp, C.cap = c.xcap;
+  C.list_stride = c.list_stride, C.list_div = c.list_div ? c.list_div : 1u;
+  cudaLaunchAttribute at = pdl_attr();
+  cudaLaunchConfig_t c0 = {};
+  c0.gridDim = dim3(c.counts || c.n_act > 1 ? c.n_act * c.xcap : c.m), c0.blockDim = dim3(CT), c0.stream = s, c0.attrs = &at, c0.numAttrs = 1;
+  cudaError_t e = c.x2 ? cudaLaunchKernelEx(&c0, qk_x16_kernel<T, true>, C) : cudaLaunchKernelEx(&c0, qk_x16_kernel<T, false>, C);
+  if (e != cudaSuccess) return e;
+
+  TcArgs A;
+  A.L = L, A.S = P.S, A.xscale = scales, A.y = c.y, A.part = reinterpret_cast<float *>(scratch + P.o_part), A.cnt = cnt;
+  A.status = status, A.ldy = c.ldy, A.m = c.m, A.bn = P.bn, A.hn = P.hn, A.tok_blocks = P.tok_blocks, A.row_blocks = P.row_blocks;
+  A.min_run = P.min_run, A.n = c.n, A.n_act = c.n_act, A.xcap = c.xcap, A.ycap = c.ycap, A.once = P.tok_blocks == 1, A.counts = c.counts;
+  if (c.n == 1 && !c.counts) return P.cg == 1 ? launch_main<T, 1, 1>(P, A, x16, c, s) : launch_main<T, 2, 1>(P, A, x16, c, s);
+  return P.cg == 1 ? launch_main<T, 1, QK_MAX_GROUPS>(P, A, x16, c, s) : launch_main<T, 2, QK_MAX_GROUPS>(P, A, x16, c, s);
+}
+
+}  // namespace qktc
+
+// One translation unit per format.
+#define QK_TC_DEFINE(NAME, T)                                                                                          \
+  cudaError_t qk_tc_##NAME##_launch(const QkTcCall &c, unsigned *status, unsigned char *scratch, int sm_count, cudaStream_t s) { \
+    return qktc::launch_fmt<T>(c, status, scratch, sm_count, s);                                                      \
+  }

@@ -293,6 +293,7 @@ extern "C" int qk_weights_upload_gguf(qk_ctx *c, const qk_gguf *g, const char *n
     if (e != cudaSuccess) break;
     if ((e = cudaMemsetAsync(h->dev, 0, tiled, c->stream)) != cudaSuccess) break;
     if (nbytes == 0) break;
+    if (qk_gemm_tc_supported(h->L, 1) && (e = qk_gemm_tc_map(h->L, h->dev, h->tmap)) != cudaSuccess) break;
     if ((e = cudaMalloc(&raw, nbytes)) != cudaSuccess) break;
     for (int i = 0; i < 2 && e == cudaSuccess; i++) {
       e = cudaHostAlloc((void **)&stage[i], piece < nbytes ? piece : nbytes, cudaHostAllocDefault);

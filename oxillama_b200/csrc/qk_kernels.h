@@ -112,54 +112,37 @@ cudaError_t qk_launch_gemv_fast(const QkLayout &L, const uint8_t *tiled, const f
                                 uint32_t m, uint64_t ldy, unsigned *status, unsigned char *scratch,
                                 int sm_count, cudaStream_t s);
 
-// Small batches (1 .. 16 rows) of Q4_K on the fp16 mma.sync with the decode path's streaming
-// structure.  `scratch`: qk_gemm_sb_scratch_bytes(L, m) bytes.  _preferred: the shapes where
-// it was measured faster than the tcgen05 kernel (5 .. 16 rows, at least eight chunks per SM).
-bool qk_gemm_sb_supported(const QkLayout &L, uint32_t m);
-bool qk_gemm_sb_preferred(const QkLayout &L, uint32_t m, int sm_count);
-size_t qk_gemm_sb_scratch_bytes(const QkLayout &L, uint32_t m);
-cudaError_t qk_launch_gemm_sb(const QkLayout &L, const uint8_t *tiled, const float *x, float *y, uint32_t m,
-                              uint64_t ldy, unsigned *status, unsigned char *scratch, int sm_count, cudaStream_t s);
-
-// Q4_K batched matmul on tcgen05 / TMEM (any m; used for m > QK_GEMV_MAX_M).  `scratch`
-// holds the fp16 copy of the activations: qk_gemm_tc_scratch_bytes(L, m) bytes.
-bool qk_gemm_tc_supported(const QkLayout &L, uint32_t m);
-
-// Grouped form (mixture-of-experts projections): `n` weight matrices of one shape and format,
-// group e multiplying its own activation rows [e * cap, e * cap + counts[e]) (counts on the
-// device: no host round trip sizes the launch) into output rows of the same numbers.
-// Optionally the activation rows are gathered on the fly: row (e, i) = x[lists[e * list_stride
-// + i] / list_div].  One conversion launch and one matmul launch for all groups.
+// Batched matmul on tcgen05 / TMEM (used for m > QK_GEMV_MAX_M).  One call multiplies `n` weight
+// matrices of one shape and format, each by its own group of activation rows: n = 1 is the ordinary
+// matmul; the projections of a feed-forward block or the experts of a mixture go together.
 #define QK_MAX_GROUPS 16
-struct QkGroups {
-  uint32_t n;                        // 0: one matrix (the ordinary call)
-  uint32_t n_act;                    // groups e and e + n_act read the same activation rows (gate and up of an expert)
-  uint32_t rbpg, tbpg;               // 128-row blocks and token blocks per group
-  const int *counts;                 // device: valid activation rows per group
-  const uint8_t *w[QK_MAX_GROUPS];   // each group's tiled weights
+struct QkTcCall {
+  const QkLayout *L;                 // of every matrix
+  const void *maps[QK_MAX_GROUPS];   // their tensor maps (qk_gemm_tc_map, 128 bytes each)
+  uint32_t n, n_act;                 // matrices; activation groups: matrix e multiplies group e % n_act
+  // Activation row i of group e is x row e * xcap + i; with `lists` (device) it is x row
+  // lists[e * list_stride + i] / list_div.  x2 != null: the row is silu(x) * x2 instead.
+  const float *x, *x2;
+  const int *lists;
+  uint32_t list_stride, list_div;
+  // m rows per group, or (counts != null, on the device) counts[e] of at most m; `expect`: the rows of an average group
+  const int *counts;
+  uint32_t m, expect, xcap, ycap;
+  float *y;                          // output row i of matrix e: y + (e * ycap + i) * ldy
+  uint64_t ldy;
 };
-uint32_t qk_gemm_tc_group_cap(uint32_t max_rows_per_group);  // activation rows reserved per group
-size_t qk_gemm_tc_grouped_scratch_bytes(const QkLayout &L, uint32_t n_groups, uint32_t max_rows_per_group);
-// n_act: number of distinct activation groups (n_groups a multiple of it; counts_dev, x and the
-// lists describe n_act groups, y holds n_groups * cap rows: group e + k n_act multiplies the
-// activations of group e).
-cudaError_t qk_launch_gemm_tc_grouped(const QkLayout &L, const uint8_t *const *tiled, uint32_t n_groups, uint32_t n_act,
-                                      const int *counts_dev, uint32_t max_rows_per_group, const float *x,
-                                      const int *lists, uint32_t list_stride, uint32_t list_div, float *y,
-                                      uint64_t ldy, unsigned *status, unsigned char *scratch, int sm_count,
-                                      cudaStream_t s);
-size_t qk_gemm_tc_scratch_bytes(const QkLayout &L, uint32_t m);
-cudaError_t qk_launch_gemm_tc(const QkLayout &L, const uint8_t *tiled, const float *x, float *y,
-                              uint32_t m, uint64_t ldy, unsigned *status, unsigned char *scratch,
-                              int sm_count, cudaStream_t s);
+bool qk_gemm_tc_supported(const QkLayout &L, uint32_t m);
+// The tensor map (128 bytes, 64-byte aligned) through which the kernel fetches a matrix.
+cudaError_t qk_gemm_tc_map(const QkLayout &L, uint8_t *tiled, void *map);
+// Scratch of a call: the fp16 activations, their scales and the partial tiles of a K split.
+size_t qk_gemm_tc_scratch_bytes(const QkTcCall &c, int sm_count);
+cudaError_t qk_launch_gemm_tc(const QkTcCall &c, unsigned *status, unsigned char *scratch, int sm_count, cudaStream_t s);
 
 // Mixture-of-experts glue (routing, token lists, gather, silu * up, weighted scatter-add).
 cudaError_t qk_launch_moe_route(const float *logits, uint32_t tokens, uint32_t n_exp, uint32_t top_k,
                                 int *ids, float *wts, cudaStream_t s);
 cudaError_t qk_launch_moe_lists(const int *ids, uint32_t tokens, uint32_t top_k, uint32_t expert_begin,
                                 uint32_t n_local, int *counts, int *lists, int *pos, cudaStream_t s);
-cudaError_t qk_launch_moe_silu_mul_grouped(const float *g, float *u, const int *counts, uint32_t n_local,
-                                           uint32_t max_rows, uint32_t cap, uint32_t inter, cudaStream_t s);
 cudaError_t qk_launch_moe_combine(const float *o, const int *ids, const int *pos, const float *wts, uint32_t tokens,
                                   uint32_t top_k, uint32_t expert_begin, uint32_t n_local, uint32_t cap,
                                   uint32_t hidden, float *y, cudaStream_t s);

@@ -115,22 +115,6 @@ __global__ void __launch_bounds__(256)
     dst[c] = __fadd_rn(dst[c], __fmul_rn(w, o[(uint64_t)i * hidden + c]));
 }
 
-
-// Grouped form of the element-wise step: u[(e, i)] <- silu(g[(e, i)]) * u[(e, i)] for the live rows
-// i < counts[e] of every local expert; rows are `cap` apart per expert (moe.rs:96-112).
-__global__ void __launch_bounds__(256)
-    qk_moe_silu_mul_grouped_kernel(const float *__restrict__ g, float *__restrict__ u, const int *__restrict__ counts,
-                                   uint32_t cap, uint32_t inter) {
-  const uint32_t e = blockIdx.y, i = blockIdx.x;
-  if ((int)i >= counts[e]) return;
-  const uint64_t base = ((uint64_t)e * cap + i) * inter;
-  for (uint32_t c = threadIdx.x; c < inter; c += 256) {
-    const float v = g[base + c];
-    const float sig = __fdiv_rn(1.f, __fadd_rn(1.f, expf(-v)));
-    u[base + c] = __fmul_rn(u[base + c], __fmul_rn(v, sig));
-  }
-}
-
 // y[token] = sum over the token's slots, in slot order, of w[slot] * o[(expert, position)] for
 // the slots whose expert is local (moe.rs:232-255 accumulates in that order); a token none of
 // whose experts is local gets zeros.
@@ -187,12 +171,6 @@ cudaError_t qk_launch_moe_lists(const int *ids, uint32_t tokens, uint32_t top_k,
                                 uint32_t n_local, int *counts, int *lists, int *pos, cudaStream_t s) {
   if (n_local == 0) return cudaSuccess;
   qk_moe_lists_kernel<<<n_local, 32, 0, s>>>(ids, tokens, top_k, expert_begin, counts, lists, pos);
-  return cudaGetLastError();
-}
-cudaError_t qk_launch_moe_silu_mul_grouped(const float *g, float *u, const int *counts, uint32_t n_local,
-                                           uint32_t max_rows, uint32_t cap, uint32_t inter, cudaStream_t s) {
-  if (n_local == 0 || max_rows == 0 || inter == 0) return cudaSuccess;
-  qk_moe_silu_mul_grouped_kernel<<<dim3(max_rows, n_local), 256, 0, s>>>(g, u, counts, cap, inter);
   return cudaGetLastError();
 }
 cudaError_t qk_launch_moe_combine(const float *o, const int *ids, const int *pos, const float *wts, uint32_t tokens,

@@ -142,6 +142,7 @@ extern "C" int qk_shutdown(qk_ctx *c) {
   if (c->sa) cudaFree(c->sa);
   if (c->sb) cudaFree(c->sb);
   cudaFreeHost((void *)c->status_host);
+  if (c->hx) cudaFreeHost(c->hx);
   if (c->scratch) cudaFree(c->scratch);
   if (c->moe) cudaFree(c->moe);
   if (c->ffn) cudaFree(c->ffn);
@@ -353,12 +354,21 @@ static int gemm_dispatch(qk_ctx *c, const qk_weights *h, const float *x, float *
     CK(c, cudaMemset2DAsync(y, ldy * sizeof(float), 0, h->L.rows * sizeof(float), m, s));
     return QK_OK;
   }
-  if (!c->force_simple && m <= QK_GEMV_MAX_M && qk_gemv_fast_supported(h->L, (uint32_t)m)) {
-    int st = ensure_scratch(c, qk_gemv_fast_scratch_bytes(h->L, (uint32_t)m));
-    if (st) return st;
-    CK(c, qk_launch_gemv_fast(h->L, h->dev, x, y, (uint32_t)m, ldy, c->status_dev, c->scratch,
-                              c->sm_count, s));
-    return QK_OK;
+  // Formats without a tensor-core matmul (Q5_K, Q3_K, Q2_K) take a batch of any size on the decode
+  // kernels, as many rows at a time as these take: the weights are streamed once per four rows, where
+  // the generic kernel decodes them byte by byte once per eight.
+  if (!c->force_simple && qk_gemv_fast_supported(h->L, 1) && (m <= QK_GEMV_MAX_M || !qk_gemm_tc_supported(h->L, 1))) {
+    size_t step = m < QK_GEMV_MAX_M ? m : QK_GEMV_MAX_M;
+    while (step > 1 && !qk_gemv_fast_supported(h->L, (uint32_t)step)) step--;
+    if (step == m || !qk_gemm_tc_supported(h->L, 1)) {
+      int st = ensure_scratch(c, qk_gemv_fast_scratch_bytes(h->L, (uint32_t)step));
+      if (st) return st;
+      for (size_t i = 0; i < m; i += step) {
+        const uint32_t k = (uint32_t)(m - i < step ? m - i : step);
+        CK(c, qk_launch_gemv_fast(h->L, h->dev, x + i * h->L.cols, y + i * ldy, k, ldy, c->status_dev, c->scratch, c->sm_count, s));
+      }
+      return QK_OK;
+    }
   }
   // The tensor-core path rounds its operands to fp16; batches the decode kernels take keep
   // f32-grade activations.  Decode-sized calls the decode kernels cannot take (K not a
@@ -572,11 +582,10 @@ extern "C" int qk_ffn_dev(qk_ctx *c, const qk_weights *gate, const qk_weights *u
     c->ffn_cap = need;
   }
   float *h = (float *)c->ffn, *u = h + m * inter;
-  const bool fused = !c->force_simple && gate->L.type == QK_T_Q4_K && up->L.type == QK_T_Q4_K && hidden > 0 &&
-                     inter > 0 && m <= QK_GEMV_MAX_M && qk_gemv_dual_supported(gate->L, (uint32_t)m);
+  const bool fused = !c->force_simple && gate->L.type == up->L.type && hidden > 0 && inter > 0 && m <= QK_GEMV_MAX_M && qk_gemv_dual_supported(gate->L, (uint32_t)m);
   if (fused) {
     // gate and up in one launch (they share the split activations), silu(g) * u in its reducer
-    int st = ensure_scratch(c, qk_gemv_mma_scratch_bytes(gate->L, (uint32_t)m));
+    int st = ensure_scratch(c, qk_gemv_fast_scratch_bytes(gate->L, (uint32_t)m));
     if (st) return st;
     CK(c, qk_launch_gemv_dual(gate->L, gate->dev, up->dev, x_dev, h, (uint32_t)m, inter, c->status_dev, c->scratch,
                               c->sm_count, s));
@@ -678,6 +687,19 @@ extern "C" int qk_dequant_matrix(qk_ctx *c, int type, const uint8_t *w, size_t w
   return st;
 }
 
+static int host_stage(qk_ctx *c) {
+  if (c->hx) return QK_OK;
+  unsigned char *p = nullptr, *d = nullptr;
+  CK(c, cudaHostAlloc((void **)&p, 2 * QK_HOST_STAGE, cudaHostAllocMapped | cudaHostAllocPortable));
+  cudaError_t e = cudaHostGetDevicePointer((void **)&d, p, 0);
+  if (e != cudaSuccess) {
+    cudaFreeHost(p);
+    CK(c, e);
+  }
+  c->hx = p, c->hx_dev = d, c->hy = p + QK_HOST_STAGE, c->hy_dev = d + QK_HOST_STAGE;
+  return QK_OK;
+}
+
 static int host_gemm(qk_ctx *c, int type, const uint8_t *w, size_t w_len, size_t n, size_t k,
                      const float *x, float *y, size_t m) {
   std::lock_guard<std::mutex> g(c->mu);
@@ -685,26 +707,42 @@ static int host_gemm(qk_ctx *c, int type, const uint8_t *w, size_t w_len, size_t
   qk_weights *h = nullptr;
   int st = cached(c, type, w, w_len, n, k, &h);
   if (st) return st;
-  size_t xb = m * k * sizeof(float), yb = m * n * sizeof(float);
-  if ((st = grow(c, &c->sa, &c->sa_cap, xb ? xb : 4))) return st;
-  if ((st = grow(c, &c->sb, &c->sb_cap, yb ? yb : 4))) return st;
-  if (xb) CK(c, cudaMemcpyAsync(c->sa, x, xb, cudaMemcpyHostToDevice, c->stream));
-  // Decode-sized calls into pinned host memory: the kernels that serve M <= 4 only store y
-  // (a few KB, 32 contiguous bytes per 8-row chunk), so they write it straight through the
-  // mapping and the device-to-host copy with its launch drops out.
-  float *ydev = (float *)c->sb;
-  bool mapped = false;
-  if (yb && m <= QK_GEMV_MAX_M && !c->force_simple && qk_gemv_fast_supported(h->L, (uint32_t)m)) {
+  const size_t xb = m * k * sizeof(float), yb = m * n * sizeof(float);
+  const bool stage_x = xb <= QK_HOST_STAGE, stage_y = yb <= QK_HOST_STAGE;
+  if ((stage_x || stage_y) && (st = host_stage(c))) return st;
+  // Decode-sized calls: the kernels that serve M <= 4 split the activations once, before the matvec,
+  // straight out of the mapped staging (a copy and its hand-over to the kernel drop out), and store y
+  // (a few KB, 32 contiguous bytes per 8-row chunk) straight through the mapping, into the caller's
+  // buffer if that is pinned, else into the staging.
+  const bool decode = m <= QK_GEMV_MAX_M && k > 0 && !c->force_simple && qk_gemv_fast_supported(h->L, (uint32_t)m);
+  float *ydev = nullptr;
+  bool direct = false;
+  if (decode) {
     cudaPointerAttributes pa;
-    if (cudaPointerGetAttributes(&pa, y) == cudaSuccess && pa.type == cudaMemoryTypeHost &&
-        pa.devicePointer)
-      ydev = (float *)pa.devicePointer, mapped = true;
+    if (cudaPointerGetAttributes(&pa, y) == cudaSuccess && pa.type == cudaMemoryTypeHost && pa.devicePointer)
+      ydev = (float *)pa.devicePointer, direct = true;
     else
       (void)cudaGetLastError();
+    if (!direct && stage_y) ydev = (float *)c->hy_dev;
   }
-  if ((st = gemm_dispatch(c, h, (const float *)c->sa, ydev, m, n, c->stream))) return st;
-  if (yb && !mapped) CK(c, cudaMemcpyAsync(y, c->sb, yb, cudaMemcpyDeviceToHost, c->stream));
+  if (!ydev) {
+    if ((st = grow(c, &c->sb, &c->sb_cap, yb ? yb : 4))) return st;
+    ydev = (float *)c->sb;
+  }
+  if (stage_x) memcpy(c->hx, x, xb);
+  if (decode && stage_x) {
+    if ((st = ensure_scratch(c, qk_gemv_fast_scratch_bytes(h->L, (uint32_t)m)))) return st;
+    CK(c, qk_launch_gemv_fast(h->L, h->dev, (const float *)c->hx_dev, ydev, (uint32_t)m, n, c->status_dev, c->scratch,
+                              c->sm_count, c->stream, true));
+  } else {
+    if ((st = grow(c, &c->sa, &c->sa_cap, xb ? xb : 4))) return st;
+    if (xb) CK(c, cudaMemcpyAsync(c->sa, stage_x ? (const void *)c->hx : x, xb, cudaMemcpyHostToDevice, c->stream));
+    if ((st = gemm_dispatch(c, h, (const float *)c->sa, ydev, m, n, c->stream))) return st;
+  }
+  const bool from_dev = ydev == (float *)c->sb;
+  if (from_dev) CK(c, cudaMemcpyAsync(stage_y ? (void *)c->hy : y, c->sb, yb, cudaMemcpyDeviceToHost, c->stream));
   CK(c, cudaStreamSynchronize(c->stream));
+  if (!direct && stage_y) memcpy(y, c->hy, yb);
   return take_device_status(c);  // a bounded wait that ran out leaves y invalid: say so
 }
 

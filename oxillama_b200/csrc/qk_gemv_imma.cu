@@ -1,5 +1,5 @@
-// Decode matvec (1..4 activation rows) for Q8_0, Q4_0, IQ4_XS and Q6_K: the instantiations
-// of the integer-MMA decode kernel (qk_gemv_skel.cuh) with the policies of qk_dec_fmts.cuh
+// Decode matvec (1..4 activation rows): the instantiations
+// of the integer-MMA decode kernel (qk_gemv_skel.cuh) with the policies of qk_dec_fmts.cuh and qk_dec_kq.cuh
 // live in qk_dec_<format>.cu; this is the per-type dispatch of the decode path.
 #include "qk_kernels.h"
 
@@ -9,11 +9,14 @@
   size_t qk_dec_##NAME##_scratch(const QkLayout &L, uint32_t m);                                                \
   cudaError_t qk_dec_##NAME##_launch(const QkLayout &L, const uint8_t *tiled, const float *x, float *y,         \
                                      uint32_t m, uint64_t ldy, unsigned *status, unsigned char *scratch,        \
-                                     int sm_count, cudaStream_t s, const QkPeers *peers);
+                                     int sm_count, cudaStream_t s, const QkPeers *peers, const uint8_t *tiled2, bool host_x);
 QK_DEC_DECLARE(q80)
 QK_DEC_DECLARE(q40)
 QK_DEC_DECLARE(iq4xs)
 QK_DEC_DECLARE(q6k)
+QK_DEC_DECLARE(q5k)
+QK_DEC_DECLARE(q3k)
+QK_DEC_DECLARE(q2k)
 
 #define QK_BY_TYPE(L, call_q4k, call)            \
   switch ((L).type) {                            \
@@ -27,6 +30,12 @@ QK_DEC_DECLARE(q6k)
       return call(iq4xs);                        \
     case QK_T_Q6_K:                              \
       return call(q6k);                          \
+    case QK_T_Q5_K:                              \
+      return call(q5k);                          \
+    case QK_T_Q3_K:                              \
+      return call(q3k);                          \
+    case QK_T_Q2_K:                              \
+      return call(q2k);                          \
     default:                                     \
       break;                                     \
   }
@@ -48,23 +57,38 @@ size_t qk_gemv_fast_scratch_bytes(const QkLayout &L, uint32_t m) {
 
 cudaError_t qk_launch_gemv_fast(const QkLayout &L, const uint8_t *tiled, const float *x, float *y,
                                 uint32_t m, uint64_t ldy, unsigned *status, unsigned char *scratch,
-                                int sm_count, cudaStream_t s) {
-#define CALL(F) qk_dec_##F##_launch(L, tiled, x, y, m, ldy, status, scratch, sm_count, s, nullptr)
-  QK_BY_TYPE(L, qk_launch_gemv_mma(L, tiled, x, y, m, ldy, status, scratch, sm_count, s), CALL)
+                                int sm_count, cudaStream_t s, bool host_x) {
+#define CALL(F) qk_dec_##F##_launch(L, tiled, x, y, m, ldy, status, scratch, sm_count, s, nullptr, nullptr, host_x)
+  QK_BY_TYPE(L, qk_launch_gemv_mma(L, tiled, x, y, m, ldy, status, scratch, sm_count, s, nullptr, nullptr, host_x), CALL)
 #undef CALL
   return cudaErrorNotSupported;
 }
 
 // ---- the same kernels with the output fan-out of a row-sharded layer built in
-bool qk_gemv_peer_supported(const QkLayout &L, uint32_t m) { return qk_gemv_fast_supported(L, m); }
+bool qk_gemv_peer_supported(const QkLayout &L, uint32_t m) {
+  return L.type != QK_T_Q5_K && L.type != QK_T_Q3_K && L.type != QK_T_Q2_K && qk_gemv_fast_supported(L, m);
+}
 
 size_t qk_gemv_peer_scratch_bytes(const QkLayout &L, uint32_t m) { return qk_gemv_fast_scratch_bytes(L, m); }
 
 cudaError_t qk_launch_gemv_peer(const QkLayout &L, const uint8_t *tiled, const float *x, uint32_t m,
                                 uint64_t ldy, unsigned *status, unsigned char *scratch, int sm_count,
                                 cudaStream_t s, const QkPeers *peers) {
-#define CALL(F) qk_dec_##F##_launch(L, tiled, x, nullptr, m, ldy, status, scratch, sm_count, s, peers)
+#define CALL(F) qk_dec_##F##_launch(L, tiled, x, nullptr, m, ldy, status, scratch, sm_count, s, peers, nullptr, false)
   QK_BY_TYPE(L, qk_launch_gemv_mma(L, tiled, x, nullptr, m, ldy, status, scratch, sm_count, s, peers), CALL)
+#undef CALL
+  return cudaErrorNotSupported;
+}
+
+// ---- gate and up projection of a feed-forward block in one launch:
+// h[i][j] = silu(gate_j . x_i) * (up_j . x_i)
+bool qk_gemv_dual_supported(const QkLayout &L, uint32_t m) { return L.type != QK_T_Q6_K && qk_gemv_fast_supported(L, m); }
+
+cudaError_t qk_launch_gemv_dual(const QkLayout &L, const uint8_t *gate_tiled, const uint8_t *up_tiled, const float *x,
+                                float *h, uint32_t m, uint64_t ldh, unsigned *status, unsigned char *scratch,
+                                int sm_count, cudaStream_t s) {
+#define CALL(F) qk_dec_##F##_launch(L, gate_tiled, x, h, m, ldh, status, scratch, sm_count, s, nullptr, up_tiled, false)
+  QK_BY_TYPE(L, qk_launch_gemv_mma(L, gate_tiled, x, h, m, ldh, status, scratch, sm_count, s, nullptr, up_tiled), CALL)
 #undef CALL
   return cudaErrorNotSupported;
 }

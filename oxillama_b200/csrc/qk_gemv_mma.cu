@@ -20,17 +20,8 @@ size_t qk_gemv_mma_scratch_bytes(const QkLayout &L, uint32_t m) { return scratch
 
 cudaError_t qk_launch_gemv_mma(const QkLayout &L, const uint8_t *tiled, const float *x, float *y,
                                uint32_t m, uint64_t ldy, unsigned *status, unsigned char *scratch,
-                               int sm_count, cudaStream_t s, const QkPeers *peers) {
-  return launch<DecQ4K>(L, tiled, x, y, m, ldy, status, scratch, sm_count, s, peers);
-}
-
-// Gate and up projection of a feed-forward block in one launch: h[i][j] = silu(gate_j . x_i) * (up_j . x_i).
-bool qk_gemv_dual_supported(const QkLayout &L, uint32_t m) { return qk_gemv_mma_supported(L, m); }
-
-cudaError_t qk_launch_gemv_dual(const QkLayout &L, const uint8_t *gate_tiled, const uint8_t *up_tiled, const float *x,
-                                float *h, uint32_t m, uint64_t ldh, unsigned *status, unsigned char *scratch,
-                                int sm_count, cudaStream_t s) {
-  return launch<DecQ4K>(L, gate_tiled, x, h, m, ldh, status, scratch, sm_count, s, nullptr, up_tiled);
+                               int sm_count, cudaStream_t s, const QkPeers *peers, const uint8_t *tiled2, bool host_x) {
+  return launch<DecQ4K>(L, tiled, x, y, m, ldy, status, scratch, sm_count, s, peers, tiled2, host_x);
 }
 
 // Same matvec, always through qk_xsplit_kernel + the x image in `scratch` (never the

@@ -178,8 +178,14 @@ __global__ void __launch_bounds__(256)
   if (wait_slots) {  // x is gathered from other GPUs: read it from the tagged slots as it arrives
     if (!load_quad_slots(wait_slots + (uint64_t)m * wait_ld, *wait_epoch, e0, cols, v)) atomicOr(status, QK_DEV_TIMEOUT);
   } else {
+    const float *xr = x + (uint64_t)m * cols + e0;
+    if ((cols & 3u) == 0 && ((uintptr_t)x & 15u) == 0 && e0 + 4 <= cols) {
+      const float4 q = __ldg(reinterpret_cast<const float4 *>(xr));
+      v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+    } else {
 #pragma unroll
-    for (int i = 0; i < 4; i++) v[i] = (e0 + i < cols) ? __ldg(x + (uint64_t)m * cols + e0 + i) : 0.f;
+      for (int i = 0; i < 4; i++) v[i] = (e0 + i < cols) ? __ldg(xr + i) : 0.f;
+    }
   }
   float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
   float s4 = (v[0] + v[1]) + (v[2] + v[3]);
@@ -806,14 +812,14 @@ inline bool split_in_cta(const PlanMma &P, uint32_t m) {
 template <class F, int M>
 cudaError_t launch_mma_m(const QkLayout &L, const uint8_t *W, const float *x, float *y,
                          uint64_t ldy, unsigned *status, unsigned char *ximg, int sm_count,
-                         const PlanMma &P, cudaStream_t s, const QkPeers *peers, const uint8_t *W2 = nullptr) {
+                         const PlanMma &P, cudaStream_t s, const QkPeers *peers, const uint8_t *W2, bool host_x) {
   // Warp groups: a group owns every G-th chunk.  A stage must always be consumed by
   // the same group (a waiter on an mbarrier may be at most one phase ahead of it),
   // so the ring depth is a multiple of G * ktiles; P.groups was chosen to allow that.
   const int cw = P.cw;
   const bool peer = peers != nullptr;
 #define QK_LAUNCH1(CWV, GV, PV)                                                                               \
-  return split_in_cta(P, M)                                                                                   \
+  return !host_x && split_in_cta(P, M)                                                                                   \
              ? launch_mma<F, M, true, CWV, GV, PV>(L, W, x, y, ldy, status, ximg, sm_count, P, s, peers, W2)  \
              : launch_mma<F, M, false, CWV, GV, PV>(L, W, x, y, ldy, status, ximg, sm_count, P, s, peers, W2)
 #define QK_LAUNCH(CWV, GV)                \
@@ -823,11 +829,12 @@ cudaError_t launch_mma_m(const QkLayout &L, const uint8_t *W, const float *x, fl
         QK_LAUNCH1(CWV, GV, 2);           \
       }                                   \
     }                                     \
-    if (peer) {                           \
-      QK_LAUNCH1(CWV, GV, 1);             \
-    } else {                              \
-      QK_LAUNCH1(CWV, GV, 0);             \
+    if constexpr (F::HAS_PEER) {          \
+      if (peer) {                         \
+        QK_LAUNCH1(CWV, GV, 1);           \
+      }                                   \
     }                                     \
+    QK_LAUNCH1(CWV, GV, 0);               \
   } while (0)
   if constexpr (M == 1)
     if (cw == 12) QK_LAUNCH(12, 3);
@@ -874,18 +881,18 @@ size_t scratch_bytes(const QkLayout &L, uint32_t m) {
 template <class F>
 cudaError_t launch(const QkLayout &L, const uint8_t *tiled, const float *x, float *y, uint32_t m, uint64_t ldy,
                    unsigned *status, unsigned char *scratch, int sm_count, cudaStream_t s, const QkPeers *peers,
-                   const uint8_t *tiled2 = nullptr) {
+                   const uint8_t *tiled2 = nullptr, bool host_x = false) {
   PlanMma P;
   if (!make_plan_mma(L, m, &P, F::XSB)) return cudaErrorInvalidConfiguration;
   if (m < 1 || m > (uint32_t)F::MAX_M) return cudaErrorInvalidConfiguration;
-  if (tiled2 && (!F::HAS_DUAL || peers)) return cudaErrorInvalidConfiguration;
-  if (m == 1) return launch_mma_m<F, 1>(L, tiled, x, y, ldy, status, scratch, sm_count, P, s, peers, tiled2);
+  if ((tiled2 && (!F::HAS_DUAL || peers)) || (peers && !F::HAS_PEER)) return cudaErrorInvalidConfiguration;
+  if (m == 1) return launch_mma_m<F, 1>(L, tiled, x, y, ldy, status, scratch, sm_count, P, s, peers, tiled2, host_x);
   if constexpr (F::MAX_M >= 2)
-    if (m == 2) return launch_mma_m<F, 2>(L, tiled, x, y, ldy, status, scratch, sm_count, P, s, peers, tiled2);
+    if (m == 2) return launch_mma_m<F, 2>(L, tiled, x, y, ldy, status, scratch, sm_count, P, s, peers, tiled2, host_x);
   if constexpr (F::MAX_M >= 3)
-    if (m == 3) return launch_mma_m<F, 3>(L, tiled, x, y, ldy, status, scratch, sm_count, P, s, peers, tiled2);
+    if (m == 3) return launch_mma_m<F, 3>(L, tiled, x, y, ldy, status, scratch, sm_count, P, s, peers, tiled2, host_x);
   if constexpr (F::MAX_M >= 4)
-    if (m == 4) return launch_mma_m<F, 4>(L, tiled, x, y, ldy, status, scratch, sm_count, P, s, peers, tiled2);
+    if (m == 4) return launch_mma_m<F, 4>(L, tiled, x, y, ldy, status, scratch, sm_count, P, s, peers, tiled2, host_x);
   return cudaErrorInvalidConfiguration;
 }
 
@@ -897,12 +904,12 @@ cudaError_t launch(const QkLayout &L, const uint8_t *tiled, const float *x, floa
   size_t qk_dec_##NAME##_scratch(const QkLayout &L, uint32_t m) { return qkdec::scratch_bytes<F>(L, m); }       \
   cudaError_t qk_dec_##NAME##_launch(const QkLayout &L, const uint8_t *tiled, const float *x, float *y,         \
                                      uint32_t m, uint64_t ldy, unsigned *status, unsigned char *scratch,        \
-                                     int sm_count, cudaStream_t s, const QkPeers *peers) {                      \
-    return qkdec::launch<F>(L, tiled, x, y, m, ldy, status, scratch, sm_count, s, peers);                       \
+                                     int sm_count, cudaStream_t s, const QkPeers *peers, const uint8_t *tiled2, bool host_x) { \
+    return qkdec::launch<F>(L, tiled, x, y, m, ldy, status, scratch, sm_count, s, peers, tiled2, host_x);       \
   }
 #define QK_DEC_DECLARE(NAME)                                                                                    \
   bool qk_dec_##NAME##_supported(const QkLayout &L, uint32_t m);                                                \
   size_t qk_dec_##NAME##_scratch(const QkLayout &L, uint32_t m);                                                \
   cudaError_t qk_dec_##NAME##_launch(const QkLayout &L, const uint8_t *tiled, const float *x, float *y,         \
                                      uint32_t m, uint64_t ldy, unsigned *status, unsigned char *scratch,        \
-                                     int sm_count, cudaStream_t s, const QkPeers *peers);
+                                     int sm_count, cudaStream_t s, const QkPeers *peers, const uint8_t *tiled2, bool host_x);

@@ -17,6 +17,10 @@ struct qk_weights {
   uint64_t fp = 0;  // content fingerprint of the host buffer it was uploaded from (host-pointer cache only)
 };
 
+// Host calls of up to this many bytes go through the context's own pinned staging: a driver copy from
+// or to pageable memory costs more than the memcpy (larger ones are left to the driver, which overlaps).
+#define QK_HOST_STAGE ((size_t)256 << 10)
+
 struct qk_ctx {
   int device;
   int sm_count;
@@ -35,6 +39,9 @@ struct qk_ctx {
   // scratch for the host-pointer entry points
   void *sa = nullptr, *sb = nullptr;
   size_t sa_cap = 0, sb_cap = 0;
+  // pinned, device-mapped staging of those calls' activations and results (QK_HOST_STAGE bytes each,
+  // made by the first such call)
+  unsigned char *hx = nullptr, *hx_dev = nullptr, *hy = nullptr, *hy_dev = nullptr;
   // weight cache for the host-pointer entry points
   typedef std::tuple<const void *, size_t, int, size_t, size_t, uint64_t> Key;
   std::map<Key, qk_weights *> cache;

@@ -89,7 +89,8 @@ bool qk_gemv_mma_supported(const QkLayout &L, uint32_t m);
 size_t qk_gemv_mma_scratch_bytes(const QkLayout &L, uint32_t m);
 cudaError_t qk_launch_gemv_mma(const QkLayout &L, const uint8_t *tiled, const float *x, float *y,
                                uint32_t m, uint64_t ldy, unsigned *status, unsigned char *scratch,
-                               int sm_count, cudaStream_t s, const QkPeers *peers = nullptr);
+                               int sm_count, cudaStream_t s, const QkPeers *peers = nullptr,
+                               const uint8_t *tiled2 = nullptr, bool host_x = false);
 cudaError_t qk_launch_gemv_mma_split(const QkLayout &L, const uint8_t *tiled, const float *x,
                                      float *y, uint32_t m, uint64_t ldy, unsigned *status,
                                      unsigned char *scratch, int sm_count, cudaStream_t s);
@@ -101,16 +102,17 @@ cudaError_t qk_launch_gemv_peer(const QkLayout &L, const uint8_t *tiled, const f
                                 uint64_t ldy, unsigned *status, unsigned char *scratch, int sm_count,
                                 cudaStream_t s, const QkPeers *peers);
 // Gate and up projection of a feed-forward block in one launch (two matrices of the same
-// shape and format, Q4_K): h[i * ldh + j] = silu(gate_j . x_i) * (up_j . x_i).  Scratch as
-// qk_gemv_mma_scratch_bytes.
+// shape and format): h[i * ldh + j] = silu(gate_j . x_i) * (up_j . x_i).  Scratch as
+// qk_gemv_fast_scratch_bytes.
 bool qk_gemv_dual_supported(const QkLayout &L, uint32_t m);
 cudaError_t qk_launch_gemv_dual(const QkLayout &L, const uint8_t *gate_tiled, const uint8_t *up_tiled, const float *x,
                                 float *h, uint32_t m, uint64_t ldh, unsigned *status, unsigned char *scratch,
                                 int sm_count, cudaStream_t s);
 size_t qk_gemv_fast_scratch_bytes(const QkLayout &L, uint32_t m);
+// host_x: x is mapped host memory; it is read once (split by a kernel of its own), not by every CTA.
 cudaError_t qk_launch_gemv_fast(const QkLayout &L, const uint8_t *tiled, const float *x, float *y,
                                 uint32_t m, uint64_t ldy, unsigned *status, unsigned char *scratch,
-                                int sm_count, cudaStream_t s);
+                                int sm_count, cudaStream_t s, bool host_x = false);
 
 // Batched matmul on tcgen05 / TMEM (used for m > QK_GEMV_MAX_M).  One call multiplies `n` weight
 // matrices of one shape and format, each by its own group of activation rows: n = 1 is the ordinary

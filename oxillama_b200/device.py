@@ -13,9 +13,20 @@ import torch
 from .kernels import Context, QuantError, default_context
 
 
-def _stream_ptr(stream=None) -> C.c_void_p:
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return C.c_void_p(s.cuda_stream)
+_F32 = torch.float32
+# A decode step is hundreds of calls of a few microseconds, so what a call costs in Python counts:
+# the raw handle of the current stream without building a Stream object, plain integers where the
+# typed entry points take pointers, one expression for the checks of the ordinary case.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
+
+
+def _stream_ptr(stream=None) -> int:
+    if stream is not None:
+        return stream.cuda_stream
+    if _raw_stream is not None:
+        return _raw_stream(_device())
+    return torch.cuda.current_stream().cuda_stream
 
 
 class DeviceWeights:
@@ -76,20 +87,26 @@ class DeviceWeights:
 
     def gemv(self, x: torch.Tensor, y: torch.Tensor, stream=None) -> None:
         """y[0:rows] = W x (overwrites)."""
-        self._chk(x, torch.float32, self.cols, "input")
-        self._chk(y, torch.float32, self.rows, "output")
-        self.ctx.check(self.ctx.lib.qk_gemv_dev(self.ctx.handle, self.handle, C.c_void_p(x.data_ptr()),
-                                                C.c_void_p(y.data_ptr()), _stream_ptr(stream)))
+        if not (x.is_cuda and x.dtype is _F32 and x.is_contiguous() and x.numel() >= self.cols
+                and y.is_cuda and y.dtype is _F32 and y.is_contiguous() and y.numel() >= self.rows):
+            self._chk(x, _F32, self.cols, "input")
+            self._chk(y, _F32, self.rows, "output")
+        ctx = self.ctx
+        st = ctx.lib.qk_gemv_dev(ctx.handle, self.handle, x.data_ptr(), y.data_ptr(), _stream_ptr(stream))
+        if st:
+            ctx.check(st)
 
     def gemm(self, x: torch.Tensor, y: torch.Tensor, m: int, ldy: int | None = None,
              col_offset: int = 0, stream=None) -> None:
         """y[i, col_offset + j] = dot(W row j, x row i); y has row pitch ldy (default rows)."""
         ldy = self.rows if ldy is None else ldy
-        self._chk(x, torch.float32, m * self.cols, "input")
-        self._chk(y, torch.float32, (m - 1) * ldy + col_offset + self.rows if m else 0, "output")
-        self.ctx.check(self.ctx.lib.qk_gemm_dev(
-            self.ctx.handle, self.handle, C.c_void_p(x.data_ptr()),
-            C.c_void_p(y.data_ptr() + 4 * col_offset), m, ldy, _stream_ptr(stream)))
+        self._chk(x, _F32, m * self.cols, "input")
+        self._chk(y, _F32, (m - 1) * ldy + col_offset + self.rows if m else 0, "output")
+        ctx = self.ctx
+        st = ctx.lib.qk_gemm_dev(ctx.handle, self.handle, x.data_ptr(), y.data_ptr() + 4 * col_offset, m, ldy,
+                                 _stream_ptr(stream))
+        if st:
+            ctx.check(st)
 
     def dequant(self, out: torch.Tensor, stream=None) -> None:
         self._chk(out, torch.float32, self.rows * self.cols, "output")
@@ -120,8 +137,10 @@ def ffn(gate: DeviceWeights, up: DeviceWeights, down: DeviceWeights, x: torch.Te
         stream=None) -> None:
     """y[m x down.rows] = down(silu(gate x) * up x): the dense branch of the reference's
     `feed_forward` (crates/oxillama-arch/src/llama/model.rs:281-310) as one call (`qk_ffn_dev`)."""
-    DeviceWeights._chk(x, torch.float32, m * gate.cols, "input")
-    DeviceWeights._chk(y, torch.float32, m * down.rows, "output")
+    DeviceWeights._chk(x, _F32, m * gate.cols, "input")
+    DeviceWeights._chk(y, _F32, m * down.rows, "output")
     ctx = gate.ctx
-    ctx.check(ctx.lib.qk_ffn_dev(ctx.handle, gate.handle, up.handle, down.handle, C.c_void_p(x.data_ptr()),
-                                 C.c_void_p(y.data_ptr()), m, _stream_ptr(stream)))
+    st = ctx.lib.qk_ffn_dev(ctx.handle, gate.handle, up.handle, down.handle, x.data_ptr(), y.data_ptr(), m,
+                            _stream_ptr(stream))
+    if st:
+        ctx.check(st)

@@ -463,35 +463,19 @@ extern "C" int qk_moe_ffn_dev(qk_ctx *c, const qk_weights *const *gate, const qk
     return QK_OK;
   };
 
-  // Grouped route: batches of more than a handful of tokens, experts of one format the
-  // tensor-core kernel takes.  Every projection is one conversion launch (which also gathers
-  // the routed rows) and one matmul launch over all local experts; the per-expert token
-  // counts stay on the device and nothing is read back, so the whole call is a fixed
-  // sequence of launches with no host synchronisation.  An expert may receive every token:
-  // the activation arrays reserve `cap` rows per expert, of which only the live ones are
-  // touched.
-  bool grouped = !c->force_simple && !qk_knob("QK_NO_MOE_GROUPED") && tokens > 16 && n_local <= QK_MAX_GROUPS &&
-                 hidden > 0 && inter > 0;
+  // Experts of one format (per projection) that the tensor-core kernel takes go together, every
+  // projection in one launch over all local experts; the token counts stay on the device and nothing is
+  // read back, so the whole call is a fixed sequence of launches with no host synchronisation.
+  bool grouped = !c->force_simple && n_local <= QK_MAX_GROUPS && n_local <= QK_MOE_MAX && hidden > 0 && inter > 0;
   for (size_t e = 0; e < n_local && grouped; e++)
     grouped = gate[e]->L.type == gate[0]->L.type && up[e]->L.type == gate[0]->L.type &&
               down[e]->L.type == down[0]->L.type && qk_gemm_tc_supported(gate[e]->L, 1) &&
               qk_gemm_tc_supported(down[e]->L, 1);
-  if (grouped) {
-    const size_t cap = tokens, rows = n_local * cap;
-    const size_t o_ids = 0, o_wts = o_ids + al(slots * 4), o_cnt = o_wts + al(slots * 4);
-    const size_t o_lists = o_cnt + al(n_local * 4), o_pos = o_lists + al(n_local * slots * 4);
-    const size_t o_g = o_pos + al(slots * 4), o_u = o_g + rows * inter * 4;  // u directly behind g
-    const size_t o_o = al(o_u + rows * inter * 4), need = o_o + al(rows * hidden * 4);
-    int st = grow_moe(need);
-    if (st) return st;
-    unsigned char *base = (unsigned char *)c->moe;
-    int *ids = (int *)(base + o_ids), *cnt = (int *)(base + o_cnt), *lists = (int *)(base + o_lists);
-    int *pos = (int *)(base + o_pos);
-    float *wts = (float *)(base + o_wts), *g = (float *)(base + o_g), *u = (float *)(base + o_u);
-    float *o = (float *)(base + o_o);
-    CK(c, qk_launch_moe_route(logits_dev, (uint32_t)tokens, (uint32_t)n_exp, (uint32_t)top_k, ids, wts, s));
-    CK(c, qk_launch_moe_lists(ids, (uint32_t)tokens, (uint32_t)top_k, (uint32_t)expert_begin, (uint32_t)n_local,
-                              cnt, lists, pos, s));
+  // gate / up / down of the experts' rows in `lists` (counts in cnt) on the tensor cores: outputs at o,
+  // `cap` rows apart per expert (an expert may receive every token; only the live rows are touched)
+  const size_t cap = tokens, rows = n_local * cap;
+  auto on_tensor_cores = [&](const int *cnt, const int *lists, float *g, float *o) -> int {
+    float *u = g + rows * inter;
     QkTcCall gu = {};
     gu.L = &gate[0]->L, gu.n_act = (uint32_t)n_local, gu.counts = cnt, gu.m = (uint32_t)tokens;
     gu.expect = (uint32_t)((slots + n_exp - 1) / n_exp), gu.xcap = gu.ycap = (uint32_t)cap;
@@ -503,7 +487,8 @@ extern "C" int qk_moe_ffn_dev(qk_ctx *c, const qk_weights *const *gate, const qk
     if (one_launch)
       for (size_t e = 0; e < n_local; e++) gu.maps[n_local + e] = up[e]->tmap;
     gu.n = (uint32_t)(one_launch ? 2 * n_local : n_local);
-    if ((st = tc_call(c, gu, s))) return st;
+    int st = tc_call(c, gu, s);
+    if (st) return st;
     if (!one_launch) {
       for (size_t e = 0; e < n_local; e++) gu.maps[e] = up[e]->tmap;
       gu.y = u;
@@ -514,13 +499,62 @@ extern "C" int qk_moe_ffn_dev(qk_ctx *c, const qk_weights *const *gate, const qk
     dn.L = &down[0]->L, dn.n = dn.n_act = (uint32_t)n_local, dn.counts = cnt, dn.m = (uint32_t)tokens, dn.expect = gu.expect;
     dn.xcap = dn.ycap = (uint32_t)cap, dn.x = g, dn.x2 = u, dn.y = o, dn.ldy = hidden;
     for (size_t e = 0; e < n_local; e++) dn.maps[e] = down[e]->tmap;
-    if ((st = tc_call(c, dn, s))) return st;
-    CK(c, qk_launch_moe_combine(o, ids, pos, wts, (uint32_t)tokens, (uint32_t)top_k, (uint32_t)expert_begin,
+    return tc_call(c, dn, s);
+  };
+
+  if (grouped && tokens > QK_MOE_DEC_TOKENS) {
+    const size_t o_ids = 0, o_wts = o_ids + al(slots * 4), o_cnt = o_wts + al(slots * 4);
+    const size_t o_lists = o_cnt + al(n_local * 4), o_pos = o_lists + al(n_local * slots * 4);
+    const size_t o_g = o_pos + al(slots * 4), o_o = o_g + al(2 * rows * inter * 4), need = o_o + al(rows * hidden * 4);
+    int st = grow_moe(need);
+    if (st) return st;
+    unsigned char *base = (unsigned char *)c->moe;
+    int *ids = (int *)(base + o_ids), *cnt = (int *)(base + o_cnt), *lists = (int *)(base + o_lists);
+    int *pos = (int *)(base + o_pos);
+    float *wts = (float *)(base + o_wts), *g = (float *)(base + o_g), *o = (float *)(base + o_o);
+    CK(c, qk_launch_moe_route(logits_dev, (uint32_t)tokens, (uint32_t)n_exp, (uint32_t)top_k, ids, wts, s));
+    CK(c, qk_launch_moe_lists(ids, (uint32_t)tokens, (uint32_t)top_k, (uint32_t)expert_begin, (uint32_t)n_local,
+                              cnt, lists, pos, s));
+    if ((st = on_tensor_cores(cnt, lists, g, o))) return st;
+    CK(c, qk_launch_moe_combine(o, nullptr, nullptr, ids, pos, wts, (uint32_t)tokens, (uint32_t)top_k, (uint32_t)expert_begin,
                                 (uint32_t)n_local, (uint32_t)cap, (uint32_t)hidden, y_dev, s));
     return QK_OK;
   }
 
-  // Few tokens (decode): per expert, on the decode kernels, sized by the token counts read back.
+  // A handful of tokens: the experts with up to QK_MOE_DEC_ROWS rows on the decode kernels (f32-grade
+  // sums, as a plain matmul of that many rows), any others on the tensor cores beside them.
+  const uint32_t rg = grouped ? qk_moe_dec_rows(gate[0]->L) : 0, rd = grouped ? qk_moe_dec_rows(down[0]->L) : 0;
+  const uint32_t per_job = rg < rd ? rg : rd;
+  if (grouped && per_job) {
+    const bool big_too = tokens > QK_MOE_DEC_ROWS;
+    const size_t ig = qk_moe_dec_image_bytes(gate[0]->L), id = qk_moe_dec_image_bytes(down[0]->L);
+    const size_t o_jobs = 0, o_ids = al(sizeof(QkMoeJobs)), o_wts = o_ids + al(slots * 4), o_big = o_wts + al(slots * 4);
+    const size_t o_lists = o_big + al(n_local * 4), o_pos = o_lists + al(n_local * slots * 4), o_ig = o_pos + al(slots * 4);
+    const size_t o_h = o_ig + al(tokens * ig), o_id = o_h + al(slots * inter * 4), o_o = o_id + al(slots * id);
+    const size_t o_g = o_o + al(slots * hidden * 4), o_ob = o_g + (big_too ? al(2 * rows * inter * 4) : 0);
+    int st = grow_moe(o_ob + (big_too ? al(rows * hidden * 4) : 0));
+    if (st) return st;
+    unsigned char *base = (unsigned char *)c->moe;
+    QkMoeJobs *jobs = (QkMoeJobs *)(base + o_jobs);
+    int *ids = (int *)(base + o_ids), *big = (int *)(base + o_big), *lists = (int *)(base + o_lists), *pos = (int *)(base + o_pos);
+    float *wts = (float *)(base + o_wts), *h = (float *)(base + o_h), *o = (float *)(base + o_o), *ob = (float *)(base + o_ob);
+    const uint8_t *wg[QK_MOE_MAX], *wu[QK_MOE_MAX], *wd[QK_MOE_MAX];
+    for (size_t e = 0; e < n_local; e++) wg[e] = gate[e]->dev, wu[e] = up[e]->dev, wd[e] = down[e]->dev;
+    CK(c, qk_launch_moe_plan(logits_dev, (uint32_t)tokens, (uint32_t)n_exp, (uint32_t)top_k, (uint32_t)expert_begin,
+                             (uint32_t)n_local, per_job, ids, wts, big, lists, pos, jobs, s));
+    CK(c, qk_launch_moe_dec_split(gate[0]->L, x_dev, (uint32_t)tokens, base + o_ig, s));
+    CK(c, qk_launch_moe_dec(gate[0]->L, wg, wu, (uint32_t)n_local, per_job, jobs, base + o_ig, (uint32_t)top_k, h, inter,
+                            c->status_dev, c->sm_count, s));
+    CK(c, qk_launch_moe_dec_split(down[0]->L, h, (uint32_t)slots, base + o_id, s));
+    CK(c, qk_launch_moe_dec(down[0]->L, wd, nullptr, (uint32_t)n_local, per_job, jobs, base + o_id, 1, o, hidden, c->status_dev,
+                            c->sm_count, s));
+    if (big_too && (st = on_tensor_cores(big, lists, (float *)(base + o_g), ob))) return st;
+    CK(c, qk_launch_moe_combine(ob, o, big, ids, pos, wts, (uint32_t)tokens, (uint32_t)top_k, (uint32_t)expert_begin,
+                                (uint32_t)n_local, (uint32_t)cap, (uint32_t)hidden, y_dev, s));
+    return QK_OK;
+  }
+
+  // Other formats, mixed formats, more experts: one after the other, sized by the token counts read back.
   // scratch: ids, wts, counts, lists, then the per-expert activations (sized for every token)
   const size_t o_ids = 0, o_wts = o_ids + al(slots * 4), o_cnt = o_wts + al(slots * 4);
   const size_t o_lists = o_cnt + al(n_local * 4), o_xe = o_lists + al(n_local * slots * 4);

@@ -92,3 +92,54 @@ cudaError_t qk_launch_gemv_dual(const QkLayout &L, const uint8_t *gate_tiled, co
 #undef CALL
   return cudaErrorNotSupported;
 }
+
+// ---- mixture-of-experts projections of a handful of tokens (qk_gemv_moe.cuh)
+#define QK_MOE_DEC_DECLARE(NAME)                                                                                         \
+  uint32_t qk_moe_dec_##NAME##_rows(const QkLayout &L);                                                                  \
+  size_t qk_moe_dec_##NAME##_image(const QkLayout &L);                                                                   \
+  cudaError_t qk_moe_dec_##NAME##_split(const QkLayout &L, const float *x, uint32_t rows, unsigned char *img, cudaStream_t s); \
+  cudaError_t qk_moe_dec_##NAME##_launch(const QkLayout &L, const uint8_t *const *w, const uint8_t *const *w2, uint32_t n, \
+                                         uint32_t rows_per_job, const QkMoeJobs *jobs, const unsigned char *img,         \
+                                         uint32_t div, float *y, uint64_t ldy, unsigned *status, int sm_count, cudaStream_t s);
+QK_MOE_DEC_DECLARE(q4k)
+QK_MOE_DEC_DECLARE(q80)
+QK_MOE_DEC_DECLARE(q40)
+QK_MOE_DEC_DECLARE(iq4xs)
+QK_MOE_DEC_DECLARE(q6k)
+#define QK_MOE_BY_TYPE(L, SUFFIX, ARGS)              \
+  switch ((L).type) {                                \
+    case QK_T_Q4_K:                                  \
+      return qk_moe_dec_q4k_##SUFFIX ARGS;           \
+    case QK_T_Q8_0:                                  \
+      return qk_moe_dec_q80_##SUFFIX ARGS;           \
+    case QK_T_Q4_0:                                  \
+      return qk_moe_dec_q40_##SUFFIX ARGS;           \
+    case QK_T_IQ4_XS:                                \
+      return qk_moe_dec_iq4xs_##SUFFIX ARGS;         \
+    case QK_T_Q6_K:                                  \
+      return qk_moe_dec_q6k_##SUFFIX ARGS;           \
+    default:                                         \
+      break;                                         \
+  }
+
+uint32_t qk_moe_dec_rows(const QkLayout &L) {
+  QK_MOE_BY_TYPE(L, rows, (L))
+  return 0;
+}
+
+size_t qk_moe_dec_image_bytes(const QkLayout &L) {
+  QK_MOE_BY_TYPE(L, image, (L))
+  return 0;
+}
+
+cudaError_t qk_launch_moe_dec_split(const QkLayout &L, const float *x, uint32_t rows, unsigned char *img, cudaStream_t s) {
+  QK_MOE_BY_TYPE(L, split, (L, x, rows, img, s))
+  return cudaErrorNotSupported;
+}
+
+cudaError_t qk_launch_moe_dec(const QkLayout &L, const uint8_t *const *w, const uint8_t *const *w2, uint32_t n,
+                              uint32_t rows_per_job, const QkMoeJobs *jobs, const unsigned char *img, uint32_t div, float *y,
+                              uint64_t ldy, unsigned *status, int sm_count, cudaStream_t s) {
+  QK_MOE_BY_TYPE(L, launch, (L, w, w2, n, rows_per_job, jobs, img, div, y, ldy, status, sm_count, s))
+  return cudaErrorNotSupported;
+}

@@ -114,6 +114,30 @@ cudaError_t qk_launch_gemv_fast(const QkLayout &L, const uint8_t *tiled, const f
                                 uint32_t m, uint64_t ldy, unsigned *status, unsigned char *scratch,
                                 int sm_count, cudaStream_t s, bool host_x = false);
 
+// Mixture-of-experts projections of a handful of tokens on the decode kernels, all experts hit in one
+// launch (qk_gemv_moe.cuh).  The job list is made on the device: one expert and one or two rows each.
+#define QK_MOE_MAX 16       // most local experts
+#define QK_MOE_DEC_TOKENS 16  // most tokens of such a call
+#define QK_MOE_DEC_ROWS 4   // experts with more rows than this go to the tensor cores
+struct QkMoeJobs {
+  uint32_t n, pad[3];
+  struct {
+    uint32_t expert, rows, slot[2];  // slots = token * top_k + k
+  } job[2 * QK_MOE_MAX];
+};
+// Routing, token lists and job list in one kernel: ids / wts as qk_launch_moe_route; big[e] = rows of
+// expert e where these exceed QK_MOE_DEC_ROWS, else 0; lists / pos as qk_launch_moe_lists.
+cudaError_t qk_launch_moe_plan(const float *logits, uint32_t tokens, uint32_t n_exp, uint32_t top_k, uint32_t expert_begin,
+                               uint32_t n_local, uint32_t rows_per_job, int *ids, float *wts, int *big, int *lists, int *pos,
+                               QkMoeJobs *jobs, cudaStream_t s);
+uint32_t qk_moe_dec_rows(const QkLayout &L);  // rows a job may have: 2, 1, or 0 where the format or shape is not served
+size_t qk_moe_dec_image_bytes(const QkLayout &L);  // scratch per split activation row
+cudaError_t qk_launch_moe_dec_split(const QkLayout &L, const float *x, uint32_t rows, unsigned char *img, cudaStream_t s);
+// y[slot][row] = w[expert] row . image(slot / div), or with w2 the silu(gate) * up of both.
+cudaError_t qk_launch_moe_dec(const QkLayout &L, const uint8_t *const *w, const uint8_t *const *w2, uint32_t n,
+                              uint32_t rows_per_job, const QkMoeJobs *jobs, const unsigned char *img, uint32_t div, float *y,
+                              uint64_t ldy, unsigned *status, int sm_count, cudaStream_t s);
+
 // Batched matmul on tcgen05 / TMEM (used for m > QK_GEMV_MAX_M).  One call multiplies `n` weight
 // matrices of one shape and format, each by its own group of activation rows: n = 1 is the ordinary
 // matmul; the projections of a feed-forward block or the experts of a mixture go together.
@@ -145,9 +169,11 @@ cudaError_t qk_launch_moe_route(const float *logits, uint32_t tokens, uint32_t n
                                 int *ids, float *wts, cudaStream_t s);
 cudaError_t qk_launch_moe_lists(const int *ids, uint32_t tokens, uint32_t top_k, uint32_t expert_begin,
                                 uint32_t n_local, int *counts, int *lists, int *pos, cudaStream_t s);
-cudaError_t qk_launch_moe_combine(const float *o, const int *ids, const int *pos, const float *wts, uint32_t tokens,
-                                  uint32_t top_k, uint32_t expert_begin, uint32_t n_local, uint32_t cap,
-                                  uint32_t hidden, float *y, cudaStream_t s);
+// y[token] = sum in slot order of wts * output row; the rows of expert e lie at o + e * cap (position
+// pos inside), or, where `by_slot` is given and big[e] == 0, at by_slot + slot.
+cudaError_t qk_launch_moe_combine(const float *o, const float *by_slot, const int *big, const int *ids, const int *pos,
+                                  const float *wts, uint32_t tokens, uint32_t top_k, uint32_t expert_begin,
+                                  uint32_t n_local, uint32_t cap, uint32_t hidden, float *y, cudaStream_t s);
 cudaError_t qk_launch_moe_gather(const float *x, const int *list, uint32_t n, uint32_t top_k,
                                  uint32_t hidden, float *xe, cudaStream_t s);
 cudaError_t qk_launch_moe_silu_mul(const float *g, float *u, uint64_t n, cudaStream_t s);

@@ -1,23 +1,29 @@
 // Mixture-of-experts FFN around the quantized matmuls (crates/oxillama-arch/src/common/moe.rs:184-258):
 // routing, the per-expert token lists, and the element-wise steps between the three
-// matmuls of an expert (moe.rs:75-126).  The matmuls themselves are the ordinary
-// dequant-matmul kernels: for decode-sized calls run once per expert on the tokens routed to
-// it, for batches as one grouped launch per projection over all local experts (the _grouped
-// kernels below work on arrays that reserve `cap` rows per expert, live below counts[e]).
+// matmuls of an expert (moe.rs:75-126).  The matmuls themselves are the ordinary dequant-matmul
+// kernels: one grouped launch per projection over all local experts, on the decode kernels
+// (qk_gemv_moe.cuh) for a handful of tokens, else on the tensor cores.
 #include <cfloat>
 
 #include "qk_kernels.h"
+#include "qk_pipe.cuh"
+
+using namespace qkpipe;
 
 namespace {
+
+cudaLaunchAttribute pdl_attr() {
+  cudaLaunchAttribute a = {};
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  return a;
+}
 
 // One thread per token: softmax over all experts, the top_k largest in descending order
 // (equal values keep ascending expert order, as a stable sort would), weights
 // renormalised by the selected sum (moe.rs:200-248).
-__global__ void __launch_bounds__(128)
-    qk_moe_route_kernel(const float *__restrict__ logits, uint32_t tokens, uint32_t n_exp,
-                        uint32_t top_k, int *__restrict__ ids, float *__restrict__ wts) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= tokens) return;
+__device__ __forceinline__ void route_token(const float *__restrict__ logits, uint32_t t, uint32_t n_exp, uint32_t top_k,
+                                            int *ids, float *wts) {
   const float *l = logits + (uint64_t)t * n_exp;
   const uint32_t ek = top_k < n_exp ? top_k : n_exp;
   float mx = -INFINITY;
@@ -47,6 +53,54 @@ __global__ void __launch_bounds__(128)
     w = ssum > 1e-9f ? __fdiv_rn(w, ssum) : __fdiv_rn(1.f, (float)ek);
   }
   for (uint32_t k = ek; k < top_k; k++) ids[(uint64_t)t * top_k + k] = -1, wts[(uint64_t)t * top_k + k] = 0.f;
+}
+
+__global__ void __launch_bounds__(128)
+    qk_moe_route_kernel(const float *__restrict__ logits, uint32_t tokens, uint32_t n_exp,
+                        uint32_t top_k, int *__restrict__ ids, float *__restrict__ wts) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < tokens) route_token(logits, t, n_exp, top_k, ids, wts);
+}
+
+// A handful of tokens: the whole plan of a call in one block.
+__global__ void __launch_bounds__(32)
+    qk_moe_plan_kernel(const float *__restrict__ logits, uint32_t tokens, uint32_t n_exp, uint32_t top_k, uint32_t expert_begin,
+                       uint32_t n_local, uint32_t rows_per_job, int *ids, float *wts, int *big, int *lists, int *pos,
+                       QkMoeJobs *jobs) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const uint32_t lane = threadIdx.x;
+  if (lane < tokens) route_token(logits, lane, n_exp, top_k, ids, wts);
+  __syncwarp();
+  const uint32_t n = tokens * top_k;
+  uint32_t count = 0, first[QK_MOE_DEC_ROWS] = {};
+  if (lane < n_local) {
+    const int want = (int)(expert_begin + lane);
+    for (uint32_t i = 0; i < n; i++) {
+      if (ids[i] != want) continue;
+#pragma unroll
+      for (uint32_t k = 0; k < QK_MOE_DEC_ROWS; k++)
+        if (k == count) first[k] = i;
+      lists[lane * n + count] = (int)i;
+      pos[i] = (int)count++;
+    }
+    big[lane] = count > QK_MOE_DEC_ROWS ? (int)count : 0;
+  }
+  const uint32_t mine = count > QK_MOE_DEC_ROWS ? 0u : (count + rows_per_job - 1) / rows_per_job;
+  uint32_t end = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t v = __shfl_up_sync(0xffffffffu, end, o);
+    if (lane >= (uint32_t)o) end += v;
+  }
+  if (lane == 31) jobs->n = end;
+#pragma unroll
+  for (uint32_t k = 0; k < QK_MOE_DEC_ROWS; k++) {
+    if (k % rows_per_job || k >= count || !mine) continue;
+    const bool two = rows_per_job == 2 && k + 1 < count;
+    auto &j = jobs->job[end - mine + k / rows_per_job];
+    j.expert = lane, j.rows = two ? 2u : 1u, j.slot[0] = first[k], j.slot[1] = two ? first[k + 1 < QK_MOE_DEC_ROWS ? k + 1 : k] : 0u;
+  }
 }
 
 // One warp per local expert: the (token, slot) pairs routed to it, in token order.
@@ -115,24 +169,29 @@ __global__ void __launch_bounds__(256)
     dst[c] = __fadd_rn(dst[c], __fmul_rn(w, o[(uint64_t)i * hidden + c]));
 }
 
-// y[token] = sum over the token's slots, in slot order, of w[slot] * o[(expert, position)] for
-// the slots whose expert is local (moe.rs:232-255 accumulates in that order); a token none of
-// whose experts is local gets zeros.
+// y[token] = sum over the token's slots, in slot order, of w[slot] * its expert's output row, for the
+// slots whose expert is local (moe.rs:232-255 accumulates in that order); a token none of whose experts
+// is local gets zeros.
 __global__ void __launch_bounds__(256)
-    qk_moe_combine_kernel(const float *__restrict__ o, const int *__restrict__ ids, const int *__restrict__ pos,
-                          const float *__restrict__ wts, uint32_t top_k, uint32_t expert_begin, uint32_t n_local,
-                          uint32_t cap, uint32_t hidden, float *__restrict__ y) {
-  const uint32_t t = blockIdx.x;
-  for (uint32_t c = threadIdx.x; c < hidden; c += 256) {
-    float acc = 0.f;
-    for (uint32_t k = 0; k < top_k; k++) {
-      const int id = ids[(uint64_t)t * top_k + k];
-      if (id < (int)expert_begin || id >= (int)(expert_begin + n_local)) continue;
-      const uint64_t row = (uint64_t)(id - (int)expert_begin) * cap + (uint32_t)pos[(uint64_t)t * top_k + k];
-      acc = __fadd_rn(acc, __fmul_rn(wts[(uint64_t)t * top_k + k], o[row * hidden + c]));
-    }
-    y[(uint64_t)t * hidden + c] = acc;
+    qk_moe_combine_kernel(const float *__restrict__ o, const float *__restrict__ by_slot, const int *__restrict__ big,
+                          const int *__restrict__ ids, const int *__restrict__ pos, const float *__restrict__ wts,
+                          uint32_t top_k, uint32_t expert_begin, uint32_t n_local, uint32_t cap, uint32_t hidden,
+                          float *__restrict__ y) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const uint32_t t = blockIdx.x, c = blockIdx.y * 256 + threadIdx.x;
+  if (c >= hidden) return;
+  float acc = 0.f;
+  for (uint32_t k = 0; k < top_k; k++) {
+    const uint32_t slot = t * top_k + k;
+    const int id = ids[slot];
+    if (id < (int)expert_begin || id >= (int)(expert_begin + n_local)) continue;
+    const uint32_t e = (uint32_t)(id - (int)expert_begin);
+    const float *row = by_slot && !big[e] ? by_slot + (uint64_t)slot * hidden
+                                          : o + ((uint64_t)e * cap + (uint32_t)pos[slot]) * hidden;
+    acc = __fadd_rn(acc, __fmul_rn(wts[slot], row[c]));
   }
+  y[(uint64_t)t * hidden + c] = acc;
 }
 
 // out[i][:] = x[idx[i]][:]: the rows a rank sends to another rank, in send order.
@@ -173,12 +232,24 @@ cudaError_t qk_launch_moe_lists(const int *ids, uint32_t tokens, uint32_t top_k,
   qk_moe_lists_kernel<<<n_local, 32, 0, s>>>(ids, tokens, top_k, expert_begin, counts, lists, pos);
   return cudaGetLastError();
 }
-cudaError_t qk_launch_moe_combine(const float *o, const int *ids, const int *pos, const float *wts, uint32_t tokens,
-                                  uint32_t top_k, uint32_t expert_begin, uint32_t n_local, uint32_t cap,
-                                  uint32_t hidden, float *y, cudaStream_t s) {
+cudaError_t qk_launch_moe_plan(const float *logits, uint32_t tokens, uint32_t n_exp, uint32_t top_k, uint32_t expert_begin,
+                               uint32_t n_local, uint32_t rows_per_job, int *ids, float *wts, int *big, int *lists, int *pos,
+                               QkMoeJobs *jobs, cudaStream_t s) {
+  if (tokens == 0 || tokens > QK_MOE_DEC_TOKENS || n_local > QK_MOE_MAX || rows_per_job < 1 || rows_per_job > 2) return cudaErrorInvalidValue;
+  cudaLaunchAttribute at = pdl_attr();
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(1), c.blockDim = dim3(32), c.stream = s, c.attrs = &at, c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, qk_moe_plan_kernel, logits, tokens, n_exp, top_k, expert_begin, n_local, rows_per_job, ids, wts, big,
+                            lists, pos, jobs);
+}
+cudaError_t qk_launch_moe_combine(const float *o, const float *by_slot, const int *big, const int *ids, const int *pos,
+                                  const float *wts, uint32_t tokens, uint32_t top_k, uint32_t expert_begin,
+                                  uint32_t n_local, uint32_t cap, uint32_t hidden, float *y, cudaStream_t s) {
   if (tokens == 0 || hidden == 0) return cudaSuccess;
-  qk_moe_combine_kernel<<<tokens, 256, 0, s>>>(o, ids, pos, wts, top_k, expert_begin, n_local, cap, hidden, y);
-  return cudaGetLastError();
+  cudaLaunchAttribute at = pdl_attr();
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(tokens, (hidden + 255) / 256), c.blockDim = dim3(256), c.stream = s, c.attrs = &at, c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, qk_moe_combine_kernel, o, by_slot, big, ids, pos, wts, top_k, expert_begin, n_local, cap, hidden, y);
 }
 cudaError_t qk_launch_moe_gather(const float *x, const int *list, uint32_t n, uint32_t top_k,
                                  uint32_t hidden, float *xe, cudaStream_t s) {

@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "qk_internal.h"
+#include "qk_moe_plan.cuh"
 
 #define CK(ctx, call)                                                                     \
   do {                                                                                    \
@@ -540,12 +541,12 @@ extern "C" int qk_moe_ffn_dev(qk_ctx *c, const qk_weights *const *gate, const qk
     float *wts = (float *)(base + o_wts), *h = (float *)(base + o_h), *o = (float *)(base + o_o), *ob = (float *)(base + o_ob);
     const uint8_t *wg[QK_MOE_MAX], *wu[QK_MOE_MAX], *wd[QK_MOE_MAX];
     for (size_t e = 0; e < n_local; e++) wg[e] = gate[e]->dev, wu[e] = up[e]->dev, wd[e] = down[e]->dev;
-    CK(c, qk_launch_moe_plan(logits_dev, (uint32_t)tokens, (uint32_t)n_exp, (uint32_t)top_k, (uint32_t)expert_begin,
-                             (uint32_t)n_local, per_job, ids, wts, big, lists, pos, jobs, s));
-    CK(c, qk_launch_moe_dec_split(gate[0]->L, x_dev, (uint32_t)tokens, base + o_ig, s));
+    const qkmoe::PlanArgs plan = {logits_dev, (uint32_t)tokens, (uint32_t)n_exp, (uint32_t)top_k, (uint32_t)expert_begin,
+                                  (uint32_t)n_local, per_job, ids, wts, big, lists, pos, jobs};
+    CK(c, qk_launch_moe_dec_split(gate[0]->L, x_dev, (uint32_t)tokens, base + o_ig, &plan, s));
     CK(c, qk_launch_moe_dec(gate[0]->L, wg, wu, (uint32_t)n_local, per_job, jobs, base + o_ig, (uint32_t)top_k, h, inter,
                             c->status_dev, c->sm_count, s));
-    CK(c, qk_launch_moe_dec_split(down[0]->L, h, (uint32_t)slots, base + o_id, s));
+    CK(c, qk_launch_moe_dec_split(down[0]->L, h, (uint32_t)slots, base + o_id, nullptr, s));
     CK(c, qk_launch_moe_dec(down[0]->L, wd, nullptr, (uint32_t)n_local, per_job, jobs, base + o_id, 1, o, hidden, c->status_dev,
                             c->sm_count, s));
     if (big_too && (st = on_tensor_cores(big, lists, (float *)(base + o_g), ob))) return st;

@@ -43,12 +43,15 @@ __device__ __forceinline__ uint32_t lds16o(uint32_t addr) {
   asm volatile("{\n\t.reg .u16 t;\n\tld.shared.u16 t, [%1+%2];\n\tcvt.u32.u16 %0, t;\n\t}" : "=r"(v) : "r"(addr), "n"(OFF));
   return v;
 }
-__device__ __forceinline__ void mma_s8s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+__device__ __forceinline__ void mma_s8s8(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                          uint32_t b0, uint32_t b1) {
+  int r[4];
   asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%10,%11,%12,%13};"
-      : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0), "r"(0), "r"(0), "r"(0));
+      "{%10,%10,%10,%10};"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0x4B400000));
+#pragma unroll
+  for (int i = 0; i < 4; i++) c[i] = __int_as_float(r[i]);
 }
 __device__ __forceinline__ float digit_weight(uint32_t tig) {
   return tig == 0 ? 1.f : tig == 1 ? 1.f / 254.f : tig == 2 ? 1.f / (254.f * 254.f) : 0.f;
@@ -93,7 +96,7 @@ struct DecQ80 {
   static constexpr uint32_t COLB = 8 * 272, XSB = 8;
   static constexpr int MAX_M = 4;
   static constexpr bool HAS_DUAL = true, HAS_PEER = true;
-  static constexpr bool SPLIT_PRODUCER = false;  // the tile producer as a warp of its own (measured per format)
+  static constexpr bool SPLIT_PRODUCER = true;  // the tile producer as a warp of its own (measured per format)
   // digit order inside a 32-column block: the lane's 8 bytes are columns 4 tig .. + 3 and
   // 16 + 4 tig .. + 3, the two 4-byte pieces of its A fragment (bytes 4 tig of both 16-byte granules)
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
@@ -143,14 +146,14 @@ struct DecQ80 {
 #pragma unroll
     for (int m = 0; m < M; m++) {
       const float tx = d0 * D.xs[m].x, ty = d1 * D.xs[m].z;
-      int c[4][4];
+      float c[4][4];
 #pragma unroll
       for (int gq = 0; gq < 4; gq++)
         mma_s8s8(c[gq], D.a[gq][0], D.a[gq][1], D.a[gq][2], D.a[gq][3], D.b[m][gq].x, D.b[m][gq].y);
 #pragma unroll
       for (int gq = 0; gq < 4; gq++) {
-        acc[m][0] = fmaf(__shfl_sync(0xffffffffu, tx, gq, 4), __int2float_rn(c[gq][0]), acc[m][0]);
-        acc[m][1] = fmaf(__shfl_sync(0xffffffffu, ty, gq, 4), __int2float_rn(c[gq][3]), acc[m][1]);
+        acc[m][0] = fmaf(__shfl_sync(0xffffffffu, tx, gq, 4), c[gq][0] - MMA_BIAS, acc[m][0]);
+        acc[m][1] = fmaf(__shfl_sync(0xffffffffu, ty, gq, 4), c[gq][3] - MMA_BIAS, acc[m][1]);
       }
     }
   }
@@ -164,7 +167,7 @@ struct DecQ40 {
   static constexpr uint32_t COLB = 8 * 144, XSB = 8;
   static constexpr int MAX_M = 4;
   static constexpr bool HAS_DUAL = true, HAS_PEER = true;
-  static constexpr bool SPLIT_PRODUCER = false;  // the tile producer as a warp of its own (measured per format)
+  static constexpr bool SPLIT_PRODUCER = true;  // the tile producer as a warp of its own (measured per format)
   // The lane's word (bytes 4 tig .. + 3 of the block) holds elements 8 tig .. + 7: low
   // nibbles the even ones, high nibbles the odd ones.  Digits go evens first, then odds,
   // inside every group of 8 columns.
@@ -222,14 +225,14 @@ struct DecQ40 {
       const float tx = d0 * D.xs[m].x, ty = d1 * D.xs[m].z;
       acc[m][2] = fmaf(8.f * d0, D.xs[m].y, acc[m][2]);  // the zero point: 8 d Sx
       acc[m][2] = fmaf(8.f * d1, D.xs[m].w, acc[m][2]);
-      int c[4][4];
+      float c[4][4];
 #pragma unroll
       for (int gq = 0; gq < 4; gq++)
         mma_u8s8(c[gq], a[gq][0], a[gq][1], a[gq][2], a[gq][3], D.b[m][gq].x, D.b[m][gq].y);
 #pragma unroll
       for (int gq = 0; gq < 4; gq++) {
-        acc[m][0] = fmaf(__shfl_sync(0xffffffffu, tx, gq, 4), __int2float_rn(c[gq][0]), acc[m][0]);
-        acc[m][1] = fmaf(__shfl_sync(0xffffffffu, ty, gq, 4), __int2float_rn(c[gq][3]), acc[m][1]);
+        acc[m][0] = fmaf(__shfl_sync(0xffffffffu, tx, gq, 4), c[gq][0] - MMA_BIAS, acc[m][0]);
+        acc[m][1] = fmaf(__shfl_sync(0xffffffffu, ty, gq, 4), c[gq][3] - MMA_BIAS, acc[m][1]);
       }
     }
   }
@@ -245,7 +248,7 @@ struct DecIQ4XS {
   static constexpr uint32_t COLB = 1088, XSB = 8;
   static constexpr int MAX_M = 4;
   static constexpr bool HAS_DUAL = true, HAS_PEER = true;
-  static constexpr bool SPLIT_PRODUCER = false;  // the tile producer as a warp of its own (measured per format)
+  static constexpr bool SPLIT_PRODUCER = true;  // the tile producer as a warp of its own (measured per format)
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
                                                       uint32_t w1, uint32_t w2) {
     store_digits_natural(row_img, PS, e0, w0, w1, w2);
@@ -319,14 +322,14 @@ struct DecIQ4XS {
 #pragma unroll
     for (int m = 0; m < M; m++) {
       const float tx = sc0 * D.xs[m].x, ty = sc1 * D.xs[m].z;
-      int c[4][4];
+      float c[4][4];
 #pragma unroll
       for (int gq = 0; gq < 4; gq++)
         mma_s8s8(c[gq], a[gq][0], a[gq][1], a[gq][2], a[gq][3], D.b[m][gq].x, D.b[m][gq].y);
 #pragma unroll
       for (int gq = 0; gq < 4; gq++) {
-        acc[m][0] = fmaf(__shfl_sync(0xffffffffu, tx, gq, 4), __int2float_rn(c[gq][0]), acc[m][0]);
-        acc[m][1] = fmaf(__shfl_sync(0xffffffffu, ty, gq, 4), __int2float_rn(c[gq][3]), acc[m][1]);
+        acc[m][0] = fmaf(__shfl_sync(0xffffffffu, tx, gq, 4), c[gq][0] - MMA_BIAS, acc[m][0]);
+        acc[m][1] = fmaf(__shfl_sync(0xffffffffu, ty, gq, 4), c[gq][3] - MMA_BIAS, acc[m][1]);
       }
     }
   }
@@ -435,7 +438,7 @@ struct DecQ6K {
       float z = ds[0] * x0.z;
       z = fmaf(ds[1], x0.w, z), z = fmaf(ds[2], x1.z, z), z = fmaf(ds[3], x1.w, z);
       acc[m][2] = fmaf(32.f, z, acc[m][2]);
-      int c[8][4];
+      float c[8][4];
 #pragma unroll
       for (int i = 0; i < 8; i++)
         mma_u8s8(c[i], a[i][0], 0u, a[i][1], 0u, D.b[m][i] & LN.m0, D.b[m][i] & LN.m1);
@@ -447,8 +450,8 @@ struct DecQ6K {
           const int src = 2 * G + (k >> 1);
           const float ta = __shfl_sync(0xffffffffu, t[2 * (k & 1)], src, 4);
           const float tb = __shfl_sync(0xffffffffu, t[2 * (k & 1) + 1], src, 4);
-          acc[m][0] = fmaf(ta, __int2float_rn(c[G * 4 + k][0]), acc[m][0]);
-          acc[m][1] = fmaf(tb, __int2float_rn(c[G * 4 + k][1]), acc[m][1]);
+          acc[m][0] = fmaf(ta, c[G * 4 + k][0] - MMA_BIAS, acc[m][0]);
+          acc[m][1] = fmaf(tb, c[G * 4 + k][1] - MMA_BIAS, acc[m][1]);
         }
     }
   }

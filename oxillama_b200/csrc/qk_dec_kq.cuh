@@ -92,14 +92,14 @@ struct DecQ5K {
       const float tx = ds0 * D.xs[m].x, ty = ds1 * D.xs[m].z;
       acc[m][2] = fmaf(dm0, D.xs[m].y, acc[m][2]);
       acc[m][2] = fmaf(dm1, D.xs[m].w, acc[m][2]);
-      int c[4][4];
+      float c[4][4];
 #pragma unroll
       for (int gq = 0; gq < 4; gq++)
         mma_u8s8(c[gq], a[gq][0], a[gq][1], a[gq][2], a[gq][3], D.b[m][gq].x, D.b[m][gq].y);
 #pragma unroll
       for (int gq = 0; gq < 4; gq++) {
-        acc[m][0] = fmaf(__shfl_sync(0xffffffffu, tx, gq, 4), __int2float_rn(c[gq][0]), acc[m][0]);
-        acc[m][1] = fmaf(__shfl_sync(0xffffffffu, ty, gq, 4), __int2float_rn(c[gq][3]), acc[m][1]);
+        acc[m][0] = fmaf(__shfl_sync(0xffffffffu, tx, gq, 4), c[gq][0] - MMA_BIAS, acc[m][0]);
+        acc[m][1] = fmaf(__shfl_sync(0xffffffffu, ty, gq, 4), c[gq][3] - MMA_BIAS, acc[m][1]);
       }
     }
   }
@@ -146,13 +146,13 @@ __device__ __forceinline__ void mma_strips(const D &d, const LN &ln, const uint3
     float z = off[0] * x0.z;
     z = fmaf(off[1], x0.w, z), z = fmaf(off[2], x1.z, z), z = fmaf(off[3], x1.w, z);
     acc[m][2] += z;
-    int c[8][4];
+    float c[8][4];
 #pragma unroll
     for (int i = 0; i < 8; i++) mma_u8s8(c[i], a[i][0], 0u, a[i][1], 0u, d.b[m][i] & ln.m0, d.b[m][i] & ln.m1);
 #pragma unroll
     for (int i = 0; i < 8; i++) {  // block i = 4 G + k: its scales live in lane 2 G + k / 2 of the quad, entries 2 (k & 1), + 1
-      acc[m][0] = fmaf(__shfl_sync(0xffffffffu, t[2 * (i & 1)], i >> 1, 4), __int2float_rn(c[i][0]), acc[m][0]);
-      acc[m][1] = fmaf(__shfl_sync(0xffffffffu, t[2 * (i & 1) + 1], i >> 1, 4), __int2float_rn(c[i][1]), acc[m][1]);
+      acc[m][0] = fmaf(__shfl_sync(0xffffffffu, t[2 * (i & 1)], i >> 1, 4), c[i][0] - MMA_BIAS, acc[m][0]);
+      acc[m][1] = fmaf(__shfl_sync(0xffffffffu, t[2 * (i & 1) + 1], i >> 1, 4), c[i][1] - MMA_BIAS, acc[m][1]);
     }
   }
 }

@@ -125,7 +125,7 @@ struct DecQ4K {
       acc[m][2] = fmaf(dm0, D.xs[m].y, acc[m][2]);
       acc[m][2] = fmaf(dm1, D.xs[m].w, acc[m][2]);
       // four MMAs back to back (one per 32-byte group), then their scaling
-      int c[4][4];
+      float c[4][4];
 #pragma unroll
       for (int gq = 0; gq < 4; gq++)
         mma_u8s8(c[gq], D.w[gq].x & 0x0F0F0F0Fu, D.w[gq].x, D.w[gq].y & 0x0F0F0F0Fu, D.w[gq].y,
@@ -135,8 +135,8 @@ struct DecQ4K {
         // lane gq of this lane's group of four (width 4: the source lane is an immediate)
         const float sx = __shfl_sync(0xffffffffu, tx, gq, 4);
         const float sy = __shfl_sync(0xffffffffu, ty, gq, 4);
-        acc[m][0] = fmaf(sx, __int2float_rn(c[gq][0]), acc[m][0]);
-        acc[m][1] = fmaf(sy, __int2float_rn(c[gq][3] - c[gq][1]), acc[m][1]);
+        acc[m][0] = fmaf(sx, c[gq][0] - MMA_BIAS, acc[m][0]);
+        acc[m][1] = fmaf(sy, c[gq][3] - c[gq][1], acc[m][1]);
       }
     }
   }

@@ -97,7 +97,8 @@ cudaError_t qk_launch_gemv_dual(const QkLayout &L, const uint8_t *gate_tiled, co
 #define QK_MOE_DEC_DECLARE(NAME)                                                                                         \
   uint32_t qk_moe_dec_##NAME##_rows(const QkLayout &L);                                                                  \
   size_t qk_moe_dec_##NAME##_image(const QkLayout &L);                                                                   \
-  cudaError_t qk_moe_dec_##NAME##_split(const QkLayout &L, const float *x, uint32_t rows, unsigned char *img, cudaStream_t s); \
+  cudaError_t qk_moe_dec_##NAME##_split(const QkLayout &L, const float *x, uint32_t rows, unsigned char *img, \
+                                        const qkmoe::PlanArgs *plan, cudaStream_t s); \
   cudaError_t qk_moe_dec_##NAME##_launch(const QkLayout &L, const uint8_t *const *w, const uint8_t *const *w2, uint32_t n, \
                                          uint32_t rows_per_job, const QkMoeJobs *jobs, const unsigned char *img,         \
                                          uint32_t div, float *y, uint64_t ldy, unsigned *status, int sm_count, cudaStream_t s);
@@ -132,8 +133,9 @@ size_t qk_moe_dec_image_bytes(const QkLayout &L) {
   return 0;
 }
 
-cudaError_t qk_launch_moe_dec_split(const QkLayout &L, const float *x, uint32_t rows, unsigned char *img, cudaStream_t s) {
-  QK_MOE_BY_TYPE(L, split, (L, x, rows, img, s))
+cudaError_t qk_launch_moe_dec_split(const QkLayout &L, const float *x, uint32_t rows, unsigned char *img,
+                                    const qkmoe::PlanArgs *plan, cudaStream_t s) {
+  QK_MOE_BY_TYPE(L, split, (L, x, rows, img, plan, s))
   return cudaErrorNotSupported;
 }
 

@@ -30,15 +30,15 @@ cudaError_t qk_launch_gemv_mma_split(const QkLayout &L, const uint8_t *tiled, co
                                      float *y, uint32_t m, uint64_t ldy, unsigned *status,
                                      unsigned char *scratch, int sm_count, cudaStream_t s) {
   PlanMma P;
-  if (!make_plan_mma(L, m, &P, DecQ4K::XSB, true)) return cudaErrorInvalidConfiguration;
+  if (!make_plan_mma(L, m, &P, DecQ4K::XSB)) return cudaErrorInvalidConfiguration;
 #define QK_SPLIT(MV)                                                                                       \
   switch (P.groups) {                                                                                      \
     case 4:                                                                                                \
-      return launch_mma<DecQ4K, MV, false, 8, 4>(L, tiled, x, y, ldy, status, scratch, sm_count, P, s);   \
+      return launch_mma<DecQ4K, MV, false, MAX_CW, 4>(L, tiled, x, y, ldy, status, scratch, sm_count, P, s);   \
     case 2:                                                                                                \
-      return launch_mma<DecQ4K, MV, false, 8, 2>(L, tiled, x, y, ldy, status, scratch, sm_count, P, s);   \
+      return launch_mma<DecQ4K, MV, false, MAX_CW, 2>(L, tiled, x, y, ldy, status, scratch, sm_count, P, s);   \
     default:                                                                                               \
-      return launch_mma<DecQ4K, MV, false, 8, 1>(L, tiled, x, y, ldy, status, scratch, sm_count, P, s);   \
+      return launch_mma<DecQ4K, MV, false, MAX_CW, 1>(L, tiled, x, y, ldy, status, scratch, sm_count, P, s);   \
   }
   switch (m) {
     case 1:

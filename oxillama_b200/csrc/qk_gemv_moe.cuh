@@ -17,6 +17,7 @@
 // three tokens, 250 us against 71 us of weight stream.
 #pragma once
 #include "qk_gemv_skel.cuh"
+#include "qk_moe_plan.cuh"
 
 namespace qkdec {
 
@@ -26,7 +27,7 @@ struct MoeArgs {
   const QkMoeJobs *jobs;
   const unsigned char *img;          // split rows; row = slot / div
   uint64_t img_stride;
-  uint32_t div;
+  uint32_t div, rows;               // rows: most rows of a job
   uint32_t early;                    // the job list is older than the previous kernel: weights may be fetched before it ends
   float *y;                          // y[slot][row]
   uint64_t ldy;
@@ -40,13 +41,18 @@ struct MoeSeg {
   uint32_t e, rows, slot0, slot1, chunk, n, ord, pad;  // first chunk, chunks, ordinal of the first (in chunks of either matrix)
 };
 
-template <class F>
+// Rows of activations -> split images.  With PLAN the first block makes the call's plan meanwhile.
+template <class F, bool PLAN>
 __global__ void __launch_bounds__(256)
     qk_moe_split_kernel(const float *__restrict__ x, uint32_t rows, uint32_t cols, uint32_t Kp, uint32_t PS,
-                        unsigned char *__restrict__ img, uint64_t stride) {
+                        unsigned char *__restrict__ img, uint64_t stride, const qkmoe::PlanArgs P) {
   pdl_launch_dependents();
   pdl_wait();
-  const uint32_t quads = Kp / 4, it = blockIdx.x * 256 + threadIdx.x;
+  if (PLAN && blockIdx.x == 0) {
+    qkmoe::plan_block(P);
+    return;
+  }
+  const uint32_t quads = Kp / 4, it = (blockIdx.x - (PLAN ? 1u : 0u)) * 256 + threadIdx.x;
   if (it >= rows * quads) return;  // warp-uniform: quads is a multiple of 64
   const uint32_t r = it / quads, e0 = (it % quads) * 4;
   float v[4];
@@ -69,8 +75,8 @@ __global__ void __launch_bounds__(256)
 }
 
 template <class F, bool DUAL, int G>
-__global__ void __launch_bounds__(320, 1) qk_gemv_moe_kernel(const __grid_constant__ MoeArgs A) {
-  constexpr int CW = 8, WG = CW / G;
+__global__ void __launch_bounds__((MAX_CW + 2) * 32, 1) qk_gemv_moe_kernel(const __grid_constant__ MoeArgs A) {
+  constexpr int CW = MAX_CW, WG = CW / G;
   constexpr uint32_t ND = DUAL ? 2 : 1;
   extern __shared__ __align__(128) unsigned char smem[];
   const QkLayout &L = A.L;
@@ -192,11 +198,11 @@ __global__ void __launch_bounds__(320, 1) qk_gemv_moe_kernel(const __grid_consta
           dead = true;
           break;
         }
-        const float *red = reinterpret_cast<const float *>(smem + S.red) + slot * (WG * 2 * 8);
+        const float *red = reinterpret_cast<const float *>(smem + S.red) + slot * (WG * A.rows * 8);
         if (lane < 8 * q.rows) {
           float v = 0.f;
 #pragma unroll
-          for (int wv = 0; wv < WG; wv++) v += red[(wv * 2 + m) * 8 + r];
+          for (int wv = 0; wv < WG; wv++) v += red[(wv * A.rows + m) * 8 + r];
           const uint32_t row = (q.chunk + i / ND) * 8 + r;
           if (DUAL && (i & 1u) == 0) {
             gate_v = v;
@@ -262,18 +268,13 @@ __global__ void __launch_bounds__(320, 1) qk_gemv_moe_kernel(const __grid_consta
           auto tile_body = [&](auto full_tag) {
             constexpr bool FULL = decltype(full_tag)::value;
             constexpr int NSB = NBT / WG;
-            Data d0, d1;
-            if (FULL || wl < nbt) F::template load<M, 0, WG>(d0, B, LN);
-            static_for<0, (NSB + 1) / 2>([&](auto pt) {
-              constexpr int J = 2 * decltype(pt)::value;
-              const uint32_t sb0 = wl + J * WG, sb1 = sb0 + WG, sb2 = sb1 + WG;
-              if constexpr (J + 1 < NSB)
-                if (FULL || sb1 < nbt) F::template load<M, J + 1, WG>(d1, B, LN);
-              if (FULL || sb0 < nbt) F::template compute<M>(d0, LN, acc);
-              if constexpr (J + 2 < NSB)
-                if (FULL || sb2 < nbt) F::template load<M, J + 2, WG>(d0, B, LN);
-              if constexpr (J + 1 < NSB)
-                if (FULL || sb1 < nbt) F::template compute<M>(d1, LN, acc);
+            static_for<0, NSB>([&](auto jt) {
+              constexpr int J = decltype(jt)::value;
+              if (FULL || wl + J * WG < nbt) {
+                Data D;
+                F::template load<M, J, WG>(D, B, LN);
+                F::template compute<M>(D, LN, acc);
+              }
             });
           };
           if (nbt == NBT) tile_body(std::true_type{});
@@ -281,13 +282,13 @@ __global__ void __launch_bounds__(320, 1) qk_gemv_moe_kernel(const __grid_consta
           if (++st == (uint32_t)nstage) st = 0, fph ^= 1;
         }
         if (dead) break;
-        float *red = reinterpret_cast<float *>(smem + S.red) + slot * (WG * 2 * 8);
+        float *red = reinterpret_cast<float *>(smem + S.red) + slot * (WG * A.rows * 8);
 #pragma unroll
         for (int m = 0; m < M; m++) {
           float v = F::finish(acc[m], LN);
           v += __shfl_xor_sync(0xffffffffu, v, 1);
           v += __shfl_xor_sync(0xffffffffu, v, 2);
-          if (tig == 0) red[(wl * 2 + m) * 8 + g] = v;
+          if (tig == 0) red[(wl * A.rows + m) * 8 + g] = v;
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(sbase + S.redfull + slot * 8);
@@ -308,9 +309,9 @@ struct PlanMoe {
   PlanMma P;
   uint32_t seg, total;
 };
-// The decode kernel's plan (8 warps) for two activation rows; the run table goes behind the ring.
+// The decode kernel's plan for `rows` activation rows; the run table goes behind the ring.
 inline bool make_plan_moe(const QkLayout &L, uint32_t rows, uint32_t xsb, PlanMoe *p) {
-  if (!make_plan_mma(L, rows, &p->P, xsb, true)) return false;
+  if (!make_plan_mma(L, rows, &p->P, xsb)) return false;
   const uint32_t table = 2 * QK_MOE_MAX * sizeof(MoeSeg) + 16;
   // (the plan leaves 1 KB of the budget unused; the table takes a stage's place where it does not fit)
   while (p->P.total + table > 227u * 1024u) {
@@ -336,14 +337,15 @@ uint32_t moe_rows(const QkLayout &L) {  // activation rows a job may have: 2, 1 
 }
 
 template <class F>
-cudaError_t moe_split(const QkLayout &L, const float *x, uint32_t rows, unsigned char *img, cudaStream_t s) {
+cudaError_t moe_split(const QkLayout &L, const float *x, uint32_t rows, unsigned char *img, const qkmoe::PlanArgs *plan, cudaStream_t s) {
   const uint32_t Kp = L.nb * L.bs;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t c = {};
-  c.gridDim = dim3((rows * (Kp / 4) + 255) / 256), c.blockDim = dim3(256), c.stream = s, c.attrs = at, c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, qk_moe_split_kernel<F>, x, rows, L.cols, Kp, Kp + 64, img, (uint64_t)moe_image_stride<F>(L));
+  c.gridDim = dim3((rows * (Kp / 4) + 255) / 256 + (plan ? 1 : 0)), c.blockDim = dim3(256), c.stream = s, c.attrs = at, c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, plan ? qk_moe_split_kernel<F, true> : qk_moe_split_kernel<F, false>, x, rows, L.cols, Kp, Kp + 64, img,
+                            (uint64_t)moe_image_stride<F>(L), plan ? *plan : qkmoe::PlanArgs{});
 }
 
 template <class F, bool DUAL, int G>
@@ -358,7 +360,7 @@ cudaError_t moe_launch_g(const MoeArgs &A, uint32_t smem, int sm_count, cudaStre
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t c = {};
-  c.gridDim = dim3((unsigned)sm_count), c.blockDim = dim3(320), c.dynamicSmemBytes = smem, c.stream = s, c.attrs = at, c.numAttrs = 1;
+  c.gridDim = dim3((unsigned)sm_count), c.blockDim = dim3((MAX_CW + 2) * 32), c.dynamicSmemBytes = smem, c.stream = s, c.attrs = at, c.numAttrs = 1;
   return cudaLaunchKernelEx(&c, kern, A);
 }
 
@@ -370,7 +372,7 @@ cudaError_t moe_launch(const QkLayout &L, const uint8_t *const *w, const uint8_t
   PlanMoe p;
   if (n > QK_MOE_MAX || !make_plan_moe(L, rows_per_job, F::XSB, &p)) return cudaErrorInvalidConfiguration;
   MoeArgs A = {};
-  A.L = L, A.jobs = jobs, A.img = img, A.img_stride = moe_image_stride<F>(L), A.div = div, A.early = w2 == nullptr;
+  A.L = L, A.jobs = jobs, A.img = img, A.img_stride = moe_image_stride<F>(L), A.div = div, A.rows = rows_per_job, A.early = w2 == nullptr;
   for (uint32_t e = 0; e < n; e++) A.w[e] = w[e], A.w[QK_MOE_MAX + e] = w2 ? w2[e] : nullptr;
   A.y = y, A.ldy = ldy, A.status = status, A.S = p.P.S, A.Kp = p.P.Kp, A.stage_bytes = p.P.stage_bytes, A.seg = p.seg;
   A.nstage = p.P.nstage, A.nslot = p.P.nslot;
@@ -389,8 +391,9 @@ cudaError_t moe_launch(const QkLayout &L, const uint8_t *const *w, const uint8_t
 #define QK_MOE_DEC_DEFINE(NAME, F)                                                                                       \
   uint32_t qk_moe_dec_##NAME##_rows(const QkLayout &L) { return qkdec::moe_rows<F>(L); }                                 \
   size_t qk_moe_dec_##NAME##_image(const QkLayout &L) { return qkdec::moe_image_stride<F>(L); }                          \
-  cudaError_t qk_moe_dec_##NAME##_split(const QkLayout &L, const float *x, uint32_t rows, unsigned char *img, cudaStream_t s) { \
-    return qkdec::moe_split<F>(L, x, rows, img, s);                                                                      \
+  cudaError_t qk_moe_dec_##NAME##_split(const QkLayout &L, const float *x, uint32_t rows, unsigned char *img, \
+                                        const qkmoe::PlanArgs *plan, cudaStream_t s) {                                   \
+    return qkdec::moe_split<F>(L, x, rows, img, plan, s);                                                                      \
   }                                                                                                                      \
   cudaError_t qk_moe_dec_##NAME##_launch(const QkLayout &L, const uint8_t *const *w, const uint8_t *const *w2, uint32_t n, \
                                          uint32_t rows_per_job, const QkMoeJobs *jobs, const unsigned char *img,         \

@@ -18,7 +18,7 @@
 //
 // qk_gemv_imma_kernel, persistent, one CTA per SM: a producer warp streams 8-row
 // tiles into a ring of shared-memory stages with cp.async.bulk (mbarrier completion);
-// the compute warps (8 in four groups; 12 in three for short matrices) first split x
+// the compute warps (16, in four groups or fewer) first split x
 // into the digit planes and scale table in shared memory, then a group takes every
 // G-th chunk, each warp its share of the tile's 256-column spans, and leaves its row
 // partials in a small ring; the producer warp sums a chunk's partials, writes the outputs
@@ -61,7 +61,7 @@ namespace qkdec {
 
 using namespace qkpipe;
 
-constexpr int MAX_CW = 16;                      // compute warps: 8 or 16 (+ one producer warp)
+constexpr int MAX_CW = 16;                      // compute warps (+ one or two producer / reducer warps)
 constexpr uint32_t NBT = QK_TILE_ELEMS / 256;   // super-blocks per full k-tile (16)
 constexpr int MAX_STAGE = 12;
 constexpr int MAX_SLOT = MAX_STAGE + 1;
@@ -109,17 +109,20 @@ __device__ __forceinline__ void static_for(Fn &&f) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void mma_u8s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
+// The accumulators start at the bit pattern of 1.5 * 2^23, so the integer sums (|v| < 2^22: at most 32 x
+// 255 x 127) come out as the floats 12582912 + v: one subtraction, or the difference of two of them,
+// gives the exact sum on a full-rate pipe where an int-to-float conversion runs at half rate.
+constexpr float MMA_BIAS = 12582912.f;
+__device__ __forceinline__ void mma_u8s8(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
                                          uint32_t a3, uint32_t b0, uint32_t b1) {
+  int r[4];
   asm(  // a pure function of its operands: left free for the scheduler to interleave
       "mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%10,%11,%12,%13};"
-      : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0), "r"(0), "r"(0), "r"(0));
-}
-// Exact int -> float for |v| < 2^22 on the full-rate pipes (no I2F).
-__device__ __forceinline__ float small_int_to_float(int v) {
-  return __int_as_float(0x4B400000 + v) - 12582912.0f;
+      "{%10,%10,%10,%10};"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0x4B400000));
+#pragma unroll
+  for (int i = 0; i < 4; i++) c[i] = __int_as_float(r[i]);
 }
 
 // Four activations of one 32-column block -> their three balanced base-254 digits, one
@@ -327,8 +330,8 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
                            uint32_t stage_bytes, SmemMma S, uint32_t Kp, QkPeers peers, int npre) {
   constexpr int WG = CW / G;  // warps per group; a group owns every G-th chunk
   // The tile producer as a warp of its own (F::SPLIT_PRODUCER) or as a second job of the reducer
-  // warp: measured per format (Q4_K 14336 x 4096: 8.2 -> 7.8 us with its own warp; Q6_K
-  // 128256 x 4096: 85 -> 90 us).
+  // warp: measured per format (IQ4_XS 14336 x 4096: 11.3 -> 10.95 us with its own warp; Q6_K
+  // 128256 x 4096: 79.2 -> 79.9 us).
   constexpr bool SPLIT = F::SPLIT_PRODUCER;
   constexpr int XW = CW + 1 + (SPLIT ? 1 : 0);  // first warp behind the compute, reducer and producer warps
   constexpr bool PEER = MODE == 1, DUAL = MODE == 2;
@@ -595,10 +598,11 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
         break;
       }
       QK_STAMP(warp == 0 && tstamp < 30, 2 + 2 * tstamp);
-      // software pipeline over this warp's columns (fully unrolled, two register
-      // buffers): the next column's loads are in flight while the current one is
-      // decoded, multiplied and scaled.  A full tile (all but the last k-tile of a K that
-      // is not a multiple of the tile width) runs without the per-column bound checks.
+      // One column at a time (fully unrolled): four warps per scheduler hide the latencies.  (Eight warps
+      // with the next column's loads in a second register buffer left a scheduler two warps to choose
+      // from: 14336 x 4096, 8.0 us at one row, 12.7 at two, 23.5 at four, against 7.9, 11.5, 17.7.)  A full
+      // tile (all but the last k-tile of a K that is not a multiple of the tile width) runs without the
+      // per-column bound checks.
       // every shared-memory load of a column is a compile-time offset from these per-tile bases
       const typename F::Base B = F::base(LN, tile, kt);
       auto load_sb = [&](Data &D, auto jt) { F::template load<M, decltype(jt)::value, WG>(D, B, LN); };
@@ -606,18 +610,12 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
       auto tile_body = [&](auto full_tag) {
         constexpr bool FULL = decltype(full_tag)::value;
         constexpr int NSB = NBT / WG;  // columns of a full tile per warp
-        Data d0, d1;
-        if (FULL || wl < nbt) load_sb(d0, std::integral_constant<int, 0>{});
-        static_for<0, (NSB + 1) / 2>([&](auto pt) {
-          constexpr int J = 2 * decltype(pt)::value;
-          const uint32_t sb0 = wl + J * WG, sb1 = sb0 + WG, sb2 = sb1 + WG;
-          if constexpr (J + 1 < NSB)
-            if (FULL || sb1 < nbt) load_sb(d1, std::integral_constant<int, J + 1>{});
-          if (FULL || sb0 < nbt) compute_sb(d0);
-          if constexpr (J + 2 < NSB)
-            if (FULL || sb2 < nbt) load_sb(d0, std::integral_constant<int, J + 2>{});
-          if constexpr (J + 1 < NSB)
-            if (FULL || sb1 < nbt) compute_sb(d1);
+        static_for<0, NSB>([&](auto jt) {
+          if (FULL || wl + decltype(jt)::value * WG < nbt) {
+            Data D;
+            load_sb(D, jt);
+            compute_sb(D);
+          }
         });
       };
       if (nbt == NBT)
@@ -652,34 +650,11 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
 struct PlanMma {
   SmemMma S;
   uint32_t Kp, stage_bytes, total;
-  int nstage, nslot, groups, cw;
+  int nstage, nslot, groups;
 };
 
-// Compute warps per CTA (+ one producer / reducer warp).  With 16 the register budget is 96
-// per thread and the column pipeline spills; 8 warps (up to 255 registers) stream as fast or
-// faster at every M (14336 x 4096, M = 1: 8.2 us against 8.8 us).  12 warps in three groups
-// (128 registers) start and finish sooner when a CTA has few chunks: 3.3 against 3.8 us at
-// 1024 rows, 4.6 against 4.7 us at 4096, level from 14336 rows on.  Q6_K, whose fragment
-// assembly costs the most arithmetic per byte, is bound by its compute warps with 8 of them:
-// 12 take the 128256 x 4096 matvec from 86.4 to 74.1 us (0.76 -> 0.89 of the copy bandwidth),
-// so it takes 12 at every row count (IQ4_XS gains 1 %, Q4_K loses 2 % at 14336 rows and both
-// keep 8).  QK_CW overrides (developer knob: 8, 12 or 16).
-inline int compute_warps(const QkLayout &L, uint32_t m) {
-  static int cw_env = -1;
-  if (cw_env < 0) {
-    const char *e = qk_knob("QK_CW");
-    const int v = e ? atoi(e) : 0;
-    cw_env = (v == 8 || v == 12 || v == 16) ? v : 0;
-  }
-  if (m >= 2) return cw_env == 16 ? 16 : 8;  // the 12-warp kernel is built for M = 1 only
-  if (cw_env) return cw_env;
-  return (L.ktiles == 1 && (L.chunks <= 1024 || L.type == QK_T_Q6_K)) ? 12 : 8;
-}
-
-// force_cw8: always the 8-warp kernel (the route that takes its split activations from a
-// caller-provided image is built for 8 warps only).
 // xsb: bytes per 32-column block in the activation scale table (F::XSB).
-inline bool make_plan_mma(const QkLayout &L, uint32_t m, PlanMma *P, uint32_t xsb, bool force_cw8 = false) {
+inline bool make_plan_mma(const QkLayout &L, uint32_t m, PlanMma *P, uint32_t xsb) {
   if (L.nb == 0 || L.chunks == 0) return false;  // nothing to stream: the callers handle empty shapes
   uint32_t Kp = L.nb * L.bs;
   if (Kp % 256u) return false;  // the kernels walk K in spans of 256 columns
@@ -716,15 +691,7 @@ inline bool make_plan_mma(const QkLayout &L, uint32_t m, PlanMma *P, uint32_t xs
   int groups = 1;
   const char *ge = qk_knob("QK_GROUPS");
   const int gmax = ge ? atoi(ge) : 4;
-  int cw = force_cw8 ? 8 : compute_warps(L, m);
-  if (cw == 12) {  // three groups of four warps, if the ring can hold three chunks
-    const int unit = 3 * (int)L.ktiles;
-    if (nstage / unit >= 1 && (nstage / unit) * unit >= (int)L.ktiles + 1)
-      groups = 3, nstage = (nstage / unit) * unit;
-    else
-      cw = 8;
-  }
-  for (int gtry = 4; gtry >= 2 && cw != 12; gtry >>= 1) {
+  for (int gtry = 4; gtry >= 2; gtry >>= 1) {
     const int unit = gtry * (int)L.ktiles;
     if (gtry <= gmax && nstage / unit >= 1 && (nstage / unit) * unit >= (int)L.ktiles + 1) {
       groups = gtry;
@@ -732,7 +699,7 @@ inline bool make_plan_mma(const QkLayout &L, uint32_t m, PlanMma *P, uint32_t xs
       break;
     }
   }
-  P->S = S, P->Kp = Kp, P->stage_bytes = stage_bytes, P->nstage = nstage, P->nslot = nstage + 1, P->groups = groups, P->cw = cw;
+  P->S = S, P->Kp = Kp, P->stage_bytes = stage_bytes, P->nstage = nstage, P->nslot = nstage + 1, P->groups = groups;
   P->total = off + nstage * stage_bytes;
   return true;
 }
@@ -781,17 +748,16 @@ cudaError_t launch_mma(const QkLayout &L, const uint8_t *W, const float *x, floa
   QkPeers pv = {};
   if (peers) pv = *peers;
   // Weight tiles issued before the wait on the previous kernel; the rest of the ring follows
-  // the activation loads.  Measured at 14336 x 4096, M = 1, 8 warps: with the producer a warp
-  // of its own 1 tile 8.04 us, 2 7.81, 3 7.97; with the reducer issuing 1 tile 8.2 us, 2 8.3,
-  // 3 8.6; M = 2: 2 tiles 13.1 us, 3 12.9, 4 12.7.  The 12-warp plans with one tile instead of
-  // two: within 1 % over the layer's shapes (Q4_0 4096^2 4.7 -> 4.5 us, Q8_0 4096^2 5.2 -> 5.3).
+  // the activation loads.  Measured at Q4_K 14336 x 4096: M = 1 1 tile 8.09 us, 2 7.88, 3 8.12; M = 2
+  // 1 tile 11.2 us, 3 11.5, 4 11.7 (Q8_0 4096^2: 6.4, 7.0, 7.3): the more activations there are to
+  // bring in, the more a tile ahead of them costs.
   // QK_PRE overrides (developer knob).
   static int npre_env = -1;
   if (npre_env < 0) {
     const char *e = qk_knob("QK_PRE");
     npre_env = e ? atoi(e) : 0;
   }
-  int npre = npre_env > 0 ? npre_env : (M == 1 ? ((F::SPLIT_PRODUCER || CW == 12) ? 2 : 1) : (M == 2 ? 4 : 3));
+  int npre = npre_env > 0 ? npre_env : (M == 1 ? 2 : 1);
   if (npre > P.nstage) npre = P.nstage;
   return cudaLaunchKernelEx(&cfg, kern, L, W, W2, x, (const unsigned char *)ximg, y, ldy, status,
                             P.nstage, P.nslot, P.stage_bytes, P.S, P.Kp, pv, npre);
@@ -816,7 +782,6 @@ cudaError_t launch_mma_m(const QkLayout &L, const uint8_t *W, const float *x, fl
   // Warp groups: a group owns every G-th chunk.  A stage must always be consumed by
   // the same group (a waiter on an mbarrier may be at most one phase ahead of it),
   // so the ring depth is a multiple of G * ktiles; P.groups was chosen to allow that.
-  const int cw = P.cw;
   const bool peer = peers != nullptr;
 #define QK_LAUNCH1(CWV, GV, PV)                                                                               \
   return !host_x && split_in_cta(P, M)                                                                                   \
@@ -836,27 +801,13 @@ cudaError_t launch_mma_m(const QkLayout &L, const uint8_t *W, const float *x, fl
     }                                     \
     QK_LAUNCH1(CWV, GV, 0);               \
   } while (0)
-  if constexpr (M == 1)
-    if (cw == 12) QK_LAUNCH(12, 3);
-#ifdef QK_DEV_KNOBS  // the 16-warp variants exist for experiments only (QK_CW=16)
-  if (cw == 16) {
-    switch (P.groups) {
-      case 4:
-        QK_LAUNCH(16, 4);
-      case 2:
-        QK_LAUNCH(16, 2);
-      default:
-        QK_LAUNCH(16, 1);
-    }
-  }
-#endif
   switch (P.groups) {
     case 4:
-      QK_LAUNCH(8, 4);
+      QK_LAUNCH(MAX_CW, 4);
     case 2:
-      QK_LAUNCH(8, 2);
+      QK_LAUNCH(MAX_CW, 2);
     default:
-      QK_LAUNCH(8, 1);
+      QK_LAUNCH(MAX_CW, 1);
   }
 #undef QK_LAUNCH1
 #undef QK_LAUNCH

@@ -125,14 +125,13 @@ struct QkMoeJobs {
     uint32_t expert, rows, slot[2];  // slots = token * top_k + k
   } job[2 * QK_MOE_MAX];
 };
-// Routing, token lists and job list in one kernel: ids / wts as qk_launch_moe_route; big[e] = rows of
-// expert e where these exceed QK_MOE_DEC_ROWS, else 0; lists / pos as qk_launch_moe_lists.
-cudaError_t qk_launch_moe_plan(const float *logits, uint32_t tokens, uint32_t n_exp, uint32_t top_k, uint32_t expert_begin,
-                               uint32_t n_local, uint32_t rows_per_job, int *ids, float *wts, int *big, int *lists, int *pos,
-                               QkMoeJobs *jobs, cudaStream_t s);
 uint32_t qk_moe_dec_rows(const QkLayout &L);  // rows a job may have: 2, 1, or 0 where the format or shape is not served
 size_t qk_moe_dec_image_bytes(const QkLayout &L);  // scratch per split activation row
-cudaError_t qk_launch_moe_dec_split(const QkLayout &L, const float *x, uint32_t rows, unsigned char *img, cudaStream_t s);
+// plan != null: the same launch also makes the plan (qk_moe_plan.cuh): ids / wts as qk_launch_moe_route,
+// big[e] = rows of expert e where these exceed QK_MOE_DEC_ROWS, else 0, lists / pos as qk_launch_moe_lists.
+namespace qkmoe { struct PlanArgs; }
+cudaError_t qk_launch_moe_dec_split(const QkLayout &L, const float *x, uint32_t rows, unsigned char *img,
+                                    const qkmoe::PlanArgs *plan, cudaStream_t s);
 // y[slot][row] = w[expert] row . image(slot / div), or with w2 the silu(gate) * up of both.
 cudaError_t qk_launch_moe_dec(const QkLayout &L, const uint8_t *const *w, const uint8_t *const *w2, uint32_t n,
                               uint32_t rows_per_job, const QkMoeJobs *jobs, const unsigned char *img, uint32_t div, float *y,

@@ -6,6 +6,7 @@
 #include <cfloat>
 
 #include "qk_kernels.h"
+#include "qk_moe_plan.cuh"
 #include "qk_pipe.cuh"
 
 using namespace qkpipe;
@@ -19,88 +20,11 @@ cudaLaunchAttribute pdl_attr() {
   return a;
 }
 
-// One thread per token: softmax over all experts, the top_k largest in descending order
-// (equal values keep ascending expert order, as a stable sort would), weights
-// renormalised by the selected sum (moe.rs:200-248).
-__device__ __forceinline__ void route_token(const float *__restrict__ logits, uint32_t t, uint32_t n_exp, uint32_t top_k,
-                                            int *ids, float *wts) {
-  const float *l = logits + (uint64_t)t * n_exp;
-  const uint32_t ek = top_k < n_exp ? top_k : n_exp;
-  float mx = -INFINITY;
-  for (uint32_t i = 0; i < n_exp; i++) mx = fmaxf(mx, l[i]);
-  float es = 0.f;
-  for (uint32_t i = 0; i < n_exp; i++) es = __fadd_rn(es, expf(__fsub_rn(l[i], mx)));
-  auto prob = [&](uint32_t i) {
-    const float e = expf(__fsub_rn(l[i], mx));
-    return es > 0.f ? __fdiv_rn(e, es) : __fdiv_rn(1.f, (float)n_exp);
-  };
-  float ssum = 0.f;
-  for (uint32_t k = 0; k < ek; k++) {  // k-th largest not yet taken; ties to the lower index
-    float best = -1.f;
-    uint32_t bi = 0;
-    for (uint32_t i = 0; i < n_exp; i++) {
-      bool taken = false;
-      for (uint32_t j = 0; j < k; j++) taken |= ids[(uint64_t)t * top_k + j] == (int)i;
-      const float p = prob(i);
-      if (!taken && p > best) best = p, bi = i;
-    }
-    ids[(uint64_t)t * top_k + k] = (int)bi;
-    wts[(uint64_t)t * top_k + k] = best;
-    ssum = __fadd_rn(ssum, best);
-  }
-  for (uint32_t k = 0; k < ek; k++) {
-    float &w = wts[(uint64_t)t * top_k + k];
-    w = ssum > 1e-9f ? __fdiv_rn(w, ssum) : __fdiv_rn(1.f, (float)ek);
-  }
-  for (uint32_t k = ek; k < top_k; k++) ids[(uint64_t)t * top_k + k] = -1, wts[(uint64_t)t * top_k + k] = 0.f;
-}
-
 __global__ void __launch_bounds__(128)
     qk_moe_route_kernel(const float *__restrict__ logits, uint32_t tokens, uint32_t n_exp,
                         uint32_t top_k, int *__restrict__ ids, float *__restrict__ wts) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < tokens) route_token(logits, t, n_exp, top_k, ids, wts);
-}
-
-// A handful of tokens: the whole plan of a call in one block.
-__global__ void __launch_bounds__(32)
-    qk_moe_plan_kernel(const float *__restrict__ logits, uint32_t tokens, uint32_t n_exp, uint32_t top_k, uint32_t expert_begin,
-                       uint32_t n_local, uint32_t rows_per_job, int *ids, float *wts, int *big, int *lists, int *pos,
-                       QkMoeJobs *jobs) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const uint32_t lane = threadIdx.x;
-  if (lane < tokens) route_token(logits, lane, n_exp, top_k, ids, wts);
-  __syncwarp();
-  const uint32_t n = tokens * top_k;
-  uint32_t count = 0, first[QK_MOE_DEC_ROWS] = {};
-  if (lane < n_local) {
-    const int want = (int)(expert_begin + lane);
-    for (uint32_t i = 0; i < n; i++) {
-      if (ids[i] != want) continue;
-#pragma unroll
-      for (uint32_t k = 0; k < QK_MOE_DEC_ROWS; k++)
-        if (k == count) first[k] = i;
-      lists[lane * n + count] = (int)i;
-      pos[i] = (int)count++;
-    }
-    big[lane] = count > QK_MOE_DEC_ROWS ? (int)count : 0;
-  }
-  const uint32_t mine = count > QK_MOE_DEC_ROWS ? 0u : (count + rows_per_job - 1) / rows_per_job;
-  uint32_t end = mine;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t v = __shfl_up_sync(0xffffffffu, end, o);
-    if (lane >= (uint32_t)o) end += v;
-  }
-  if (lane == 31) jobs->n = end;
-#pragma unroll
-  for (uint32_t k = 0; k < QK_MOE_DEC_ROWS; k++) {
-    if (k % rows_per_job || k >= count || !mine) continue;
-    const bool two = rows_per_job == 2 && k + 1 < count;
-    auto &j = jobs->job[end - mine + k / rows_per_job];
-    j.expert = lane, j.rows = two ? 2u : 1u, j.slot[0] = first[k], j.slot[1] = two ? first[k + 1 < QK_MOE_DEC_ROWS ? k + 1 : k] : 0u;
-  }
+  if (t < tokens) qkmoe::route_token(logits, t, n_exp, top_k, ids, wts);
 }
 
 // One warp per local expert: the (token, slot) pairs routed to it, in token order.
@@ -231,16 +155,6 @@ cudaError_t qk_launch_moe_lists(const int *ids, uint32_t tokens, uint32_t top_k,
   if (n_local == 0) return cudaSuccess;
   qk_moe_lists_kernel<<<n_local, 32, 0, s>>>(ids, tokens, top_k, expert_begin, counts, lists, pos);
   return cudaGetLastError();
-}
-cudaError_t qk_launch_moe_plan(const float *logits, uint32_t tokens, uint32_t n_exp, uint32_t top_k, uint32_t expert_begin,
-                               uint32_t n_local, uint32_t rows_per_job, int *ids, float *wts, int *big, int *lists, int *pos,
-                               QkMoeJobs *jobs, cudaStream_t s) {
-  if (tokens == 0 || tokens > QK_MOE_DEC_TOKENS || n_local > QK_MOE_MAX || rows_per_job < 1 || rows_per_job > 2) return cudaErrorInvalidValue;
-  cudaLaunchAttribute at = pdl_attr();
-  cudaLaunchConfig_t c = {};
-  c.gridDim = dim3(1), c.blockDim = dim3(32), c.stream = s, c.attrs = &at, c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, qk_moe_plan_kernel, logits, tokens, n_exp, top_k, expert_begin, n_local, rows_per_job, ids, wts, big,
-                            lists, pos, jobs);
 }
 cudaError_t qk_launch_moe_combine(const float *o, const float *by_slot, const int *big, const int *ids, const int *pos,
                                   const float *wts, uint32_t tokens, uint32_t top_k, uint32_t expert_begin,

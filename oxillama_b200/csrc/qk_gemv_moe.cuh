@@ -82,7 +82,7 @@ __global__ void __launch_bounds__((MAX_CW + 2) * 32, 1) qk_gemv_moe_kernel(const
   const QkLayout &L = A.L;
   const SmemMma &S = A.S;
   const uint32_t sbase = smem_u32(smem);
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int nstage = A.nstage, nslot = A.nslot;
   MoeSeg *segs = reinterpret_cast<MoeSeg *>(smem + A.seg);
   volatile uint32_t *meta = reinterpret_cast<volatile uint32_t *>(smem + A.seg + 2 * QK_MOE_MAX * sizeof(MoeSeg));  // segments, chunks
@@ -133,29 +133,30 @@ __global__ void __launch_bounds__((MAX_CW + 2) * 32, 1) qk_gemv_moe_kernel(const
 
   if (warp == CW + 1) {
     // ================= producer warp =================
-    uint32_t sg = 0, k = 0, which = 0, pkt = 0, pst = 0, item = 0;
-    const uint32_t my_items = n_chunks * L.ktiles;
+    const uint32_t lead = elect_lead();
+    const uint32_t my_items = __shfl_sync(0xffffffffu, n_chunks, 0) * L.ktiles;
+    uint32_t sg = 0, left = 0, which = 0, pkt = 0, pst = 0, item = 0;
+    const uint8_t *W0 = nullptr, *W1 = nullptr;  // the next chunk in the gate (or only) and the up matrix
     const uint64_t policy = stream_policy();
-    auto issue = [&]() {  // lane 0 only
-      const MoeSeg &q = segs[sg];
-      const uint8_t *W = A.w[q.e + (which ? QK_MOE_MAX : 0)];
-      const uint32_t bytes = QK_TILE_ROWS * qk_tile_nb(L, pkt) * L.bb, bar = sbase + S.full + pst * 8;
-      mbar_expect_tx(bar, bytes);
-      bulk_g2s_stream(sbase + S.stage + pst * A.stage_bytes, W + qk_tile_offset(L, q.chunk + k, pkt), bytes, bar, policy);
+    auto issue = [&]() {  // the whole warp
+      if (left == 0) {
+        const MoeSeg &q = segs[sg++];
+        const uint32_t e = __shfl_sync(0xffffffffu, q.e, 0), c0 = __shfl_sync(0xffffffffu, q.chunk, 0);
+        left = __shfl_sync(0xffffffffu, q.n, 0);
+        W0 = A.w[e] + (uint64_t)c0 * L.chunk_bytes;
+        if (DUAL) W1 = A.w[e + QK_MOE_MAX] + (uint64_t)c0 * L.chunk_bytes;
+      }
+      const uint32_t bytes = QK_TILE_ROWS * qk_tile_nb(L, pkt) * L.bb;
+      stream_tile(sbase + S.stage + pst * A.stage_bytes, (which ? W1 : W0) + pkt * L.tile_bytes, bytes, sbase + S.full + pst * 8, policy, lead);
       if (++pkt == L.ktiles) {
         pkt = 0;
-        if (++which == ND) {
-          which = 0;
-          if (++k == q.n) k = 0, sg++;
-        }
+        if (++which == ND) which = 0, left--, W0 += L.chunk_bytes, W1 += L.chunk_bytes;
       }
       if (++pst == (uint32_t)nstage) pst = 0;
     };
     auto issue_upto = [&](uint32_t limit) {
       const uint32_t end = limit < my_items ? limit : my_items;
-      if (lane == 0)
-        for (uint32_t i = item; i < end; i++) issue();
-      if (end > item) item = end;
+      for (; item < end; item++) issue();
     };
     issue_upto((uint32_t)nstage);
     uint32_t slot = 0, sph = 0;

@@ -337,7 +337,7 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
   constexpr bool PEER = MODE == 1, DUAL = MODE == 2;
   extern __shared__ __align__(128) unsigned char smem[];
   const uint32_t sbase = smem_u32(smem);
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
   // chunks of this CTA, in the order it takes them; with two matrices every 8-row group counts twice
   const uint32_t my_chunks =
@@ -359,26 +359,25 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
   // tile issue state and helpers of whichever warp streams the tiles
   uint32_t pc = 0, pkt = 0, pst = 0;  // chunk ordinal, k-tile and stage of the next item
   const uint64_t policy = stream_policy();
-  auto issue = [&]() {                // lane 0 only
+  uint32_t lead = 0;                  // the lane that issues, in the warp that does
+  auto issue = [&]() {                // the whole warp
     const uint32_t chunk = blockIdx.x + (DUAL ? pc >> 1 : pc) * gridDim.x;
     const uint8_t *Wc = (DUAL && (pc & 1u)) ? W2 : W;
     const uint32_t bytes = QK_TILE_ROWS * qk_tile_nb(L, pkt) * L.bb;
     const uint32_t bar = sbase + S.full + pst * 8;
-    mbar_expect_tx(bar, bytes);
-    bulk_g2s_stream(sbase + S.stage + pst * stage_bytes, Wc + qk_tile_offset(L, chunk, pkt), bytes, bar, policy);
+    stream_tile(sbase + S.stage + pst * stage_bytes, Wc + qk_tile_offset(L, chunk, pkt), bytes, bar, policy, lead);
     if (++pkt == L.ktiles) pkt = 0, pc++;
     if (++pst == (uint32_t)nstage) pst = 0;
   };
   uint32_t item = 0;  // items issued so far; kept in step by every lane
   auto issue_upto = [&](uint32_t limit) {
     const uint32_t end = limit < my_items ? limit : my_items;
-    if (lane == 0)
-      for (uint32_t i = item; i < end; i++) issue();
-    if (end > item) item = end;
+    for (; item < end; item++) issue();
   };
   if (SPLIT && warp == CW + 1) {
+    lead = elect_lead();
     // ================= producer warp =================
-    // Lane 0 streams the tiles: the first ring fill, then the k-tiles of chunk c + (ring depth)
+    // It streams the tiles: the first ring fill, then the k-tiles of chunk c + (ring depth)
     // as soon as the compute warps have handed chunk c over (they are done with its stages
     // then).  A warp of its own, because a copy instruction does not return until the copy
     // unit has room for it -- a third of a microsecond and more under a saturated stream --
@@ -438,6 +437,7 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
     // the tiles (!SPLIT) it refills the chunk's stages first: gating the refills on the
     // reduction bounds how far the compute warps can run ahead, which is what makes the ring
     // of `nslot` partial buffers safe without a second handshake.
+    if (!SPLIT) lead = elect_lead();
     if (!SPLIT) issue_upto((uint32_t)npre);  // weights are immutable: their prefetch need not wait for the previous kernel
     pdl_wait();  // the x image and y belong to the previous kernel until it has finished
     QK_STAMP(true, 120);

@@ -47,6 +47,25 @@ __device__ __forceinline__ void bulk_g2s_stream(uint32_t dst, const void *src, u
       "l"(src), "r"(bytes), "r"(bar), "l"(policy)
       : "memory");
 }
+// One lane of a converged warp.
+__device__ __forceinline__ uint32_t elect_lead() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p;
+}
+// expect_tx and the streaming copy by the lane with `lead` set, the whole warp walking the issuing loop:
+// what the compiler knows to be uniform then stays in uniform registers, where the copy instruction
+// wants its operands.  (A lone thread behind lane == 0 took 600 ns per copy in the mixture-of-experts
+// decode kernel and was its bottleneck.)
+__device__ __forceinline__ void stream_tile(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar, uint64_t policy,
+                                            uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%3], %2;\n\t"
+      "@q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;\n\t}" ::"r"(dst),
+      "l"(src), "r"(bytes), "r"(bar), "l"(policy), "r"(lead)
+      : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(

@@ -35,7 +35,7 @@ namespace qktc {
 // has not been given yet, two phases back, and take that for its own).  Narrow tiles are bound by the
 // weight stream and give it what they can; wide ones need four activation stages first (a stage is
 // refilled only after the MMAs that read it have retired).
-static bool plan_smem(uint32_t hn, uint32_t cg, uint32_t w_stage, uint32_t lut, TcSmem *S, uint32_t *total) {
+static bool plan_smem(uint32_t hn, uint32_t cg, uint32_t cs, uint32_t w_stage, uint32_t lut, TcSmem *S, uint32_t *total) {
   TcSmem s;
   uint32_t off = 0;
   s.w_full = off, off += MAX_WST * 8;
@@ -53,6 +53,7 @@ static bool plan_smem(uint32_t hn, uint32_t cg, uint32_t w_stage, uint32_t lut, 
   s.scales = off, off += 4 * 512 + 16;  // a copy of a half's token scales per epilogue warp, and one word
   off = (off + 127u) & ~127u;
   s.lut = off, off += lut;
+  s.red = off, off += cs > 1 ? cs * ((hn + cs - 1) / cs) * BM * 4 : 0;  // the cluster's partial sums of this CTA's tokens
   off = (off + 1023u) & ~1023u;
   s.w_stage = w_stage, s.b_stage = (hn / cg) * 512u;  // this CTA's tokens, a super-block's four steps
   const uint32_t room = SMEM_BUDGET - off;
@@ -72,16 +73,19 @@ static bool plan_smem(uint32_t hn, uint32_t cg, uint32_t w_stage, uint32_t lut, 
 
 static uint32_t round_up(uint32_t v, uint32_t to) { return (v + to - 1) / to * to; }
 
-// Form of the kernel, token-tile width and K split by predicted time (cycles of the slowest CTA):
-// whole waves of tiles, then the split remainder with its partials.  A super-block costs, whichever
-// is longest, its 16 MMAs of N / 2 cycles, its expansion, or a round of hand-overs (expanding warps
-// -> issuer -> tensor pipe -> back) over the buffers in flight.
+// Form of the kernel, token-tile width and K split by predicted time: cycles of the slowest CTA.  The
+// constants are a fit to 46 shapes (300 x 8192 .. 14336 x 4096, 8 .. 2048 tokens, Q4_K, Q6_K, Q8_0, Q4_0), each
+// timed with every tile width and split: the prediction is 10 % off (rms), the form it picks 0.8 % slower than
+// the fastest (mean).  A super-block takes as long as its expansion, which loads of wider activations slow down,
+// or in a pair the round of hand-overs (expanding warps -> issuer -> tensor pipe -> back).  A tile whose
+// partials go through the workspace costs some 8000 cycles and 58 per token (writing them out, the fence, the
+// counter, reading them back); through the cluster 5300, whatever its width.
 bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
   const QkLayout &L = *c.L;
   const uint32_t w_stage = 16u * 8u * L.bb * (256u / L.bs), lut = L.type == QK_T_IQ4_XS ? WFmt<QK_T_IQ4_XS>::LUT : 0u;
   const bool many = c.n > 1 || c.counts;
   TcPlan p;
-  p.nsb = (L.cols + 255u) / 256u;
+  p.nsb = (L.cols + 255u) / 256u, p.cs = 1;
   auto half_of = [&](uint32_t bn, uint32_t cg) {
     const uint32_t h = bn <= 128 ? bn : round_up((bn + 1) / 2, 16);
     return many ? round_up(h, 32 * cg) : h;  // groups: boxes come in quarters of whole 8-row swizzle atoms per CTA
@@ -99,8 +103,11 @@ bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
     p.row_blocks = (L.rows + p.cg * BM - 1) / (p.cg * BM);
     p.grid = (uint32_t)sm_count / p.cg;
   } else {
-    const float expand = L.type == QK_T_Q6_K ? 850.f : 700.f;
+    const float expand = L.type == QK_T_Q6_K ? 1440.f : 1110.f;
     float best = FLT_MAX;
+    auto take = [&](float t, uint32_t cg, uint32_t cs, uint32_t bn, uint32_t tbr, uint32_t rbs, uint32_t run, uint32_t grid) {
+      if (t < best) best = t, p.cg = cg, p.cs = cs, p.bn = bn, p.tok_blocks = tbr, p.row_blocks = rbs, p.min_run = run, p.grid = grid;
+    };
     const uint32_t tb0 = (c.m + MAX_BN - 1) / MAX_BN;
     for (uint32_t cg = 1; cg <= 2; cg++) {
       const uint32_t units = (uint32_t)sm_count / cg, rbs = (L.rows + cg * BM - 1) / (cg * BM);
@@ -109,13 +116,12 @@ bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
         const uint32_t bn = round_up((c.m + tbk - 1) / tbk, 16);
         if (k && bn < 32) break;
         if (cg == 1 && bn > 64) continue;
-        const uint32_t tbr = (c.m + bn - 1) / bn;
-        const float mma = 8.f * bn, chain = (cg == 1 ? 1900.f : 2300.f) / (bn <= 64 ? 3.f : 2.f);
-        const float sb = fmaxf(fmaxf(mma, expand), chain);
+        const uint32_t tbr = (c.m + bn - 1) / bn, own = bn / cg;
+        const float sb = fmaxf(expand + (own > 16 ? 5.f * (own - 16) : 0.f), cg == 2 ? 1060.f + 6.1f * bn : 0.f), out = bn * 19.f;
         const uint64_t tiles = (uint64_t)c.n * rbs * tbr;
         for (uint32_t run = 1; run <= 16; run <<= 1) {
           const uint32_t R = (uint32_t)(tiles % units), total = R * p.nsb;
-          float t = (float)(tiles / units) * (p.nsb * sb + (bn > 128 ? 2000.f : 300.f));
+          float t = (float)(tiles / units) * (p.nsb * sb + (bn > 128 ? 7000.f : 100.f)) + out;
           uint32_t grid = units;
           if (R) {
             uint32_t sk = total / run;
@@ -126,16 +132,21 @@ bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
             }
             const float len = (float)((total + sk - 1) / sk), contrib = (float)sk / R;
             t += len * sb;
-            if (contrib > 1.01f) t += 4000.f + contrib * bn * 8.f;
+            if (contrib > 1.01f) t += 7800.f + bn * (58.f + 5.f * contrib);
           }
-          t += bn * 16.f;  // writing out the last tile
-          if (t < best * 0.995f) best = t, p.cg = cg, p.bn = bn, p.tok_blocks = tbr, p.row_blocks = rbs, p.min_run = run, p.grid = grid;
+          take(t, cg, 1, bn, tbr, rbs, run, grid);
         }
+        // One tile per cluster of cs CTAs.  At most as many as fit at a time: 32 clusters of four, 14 of eight on
+        // 148 SMs (1024 x 4096 by 37: 8.5 us as 8 clusters of eight, 12.8 as 16).  Clusters of two are never the fastest.
+        if (cg == 1 && c.n == 1)
+          for (uint32_t cs = 4; cs <= 8 && cs <= p.nsb; cs <<= 1)
+            if (tiles * cs <= (uint32_t)sm_count * (cs == 4 ? 14u : 12u) / 16u)
+              take((float)((p.nsb + cs - 1) / cs) * sb + 5300.f + out, 1, cs, bn, tbr, rbs, 1, (uint32_t)tiles * cs);
       }
     }
   }
   p.hn = half_of(p.bn, p.cg);
-  if (!plan_smem(p.hn, p.cg, w_stage, lut, &p.S, &p.smem)) return false;
+  if (!plan_smem(p.hn, p.cg, p.cs, w_stage, lut, &p.S, &p.smem)) return false;
   p.xrows = c.counts || c.n_act > 1 ? c.n_act * c.xcap : p.tok_blocks * p.bn;
   const size_t Kp = (size_t)p.nsb * 256u;
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };

@@ -67,14 +67,14 @@ namespace qktc {
 using namespace qkpipe;
 
 constexpr uint32_t BM = 128;       // weight rows per CTA
-constexpr int NDW = 16;            // expanding warps: two sets of eight
-constexpr int FIRST_DW = 4, FIRST_EW = FIRST_DW + NDW;
-constexpr int NTHREADS = (FIRST_EW + 4) * 32;
+constexpr int FIRST_DW = 4;        // first expanding warp
+constexpr int NDW = 16;            // expanding warps: two sets of eight (three sets of 64 registers a thread: 3 to 10 % slower)
+constexpr int FIRST_EW = FIRST_DW + NDW, NTHREADS = (FIRST_EW + 4) * 32;
 constexpr uint32_t MAX_BN = 256;   // most tokens per tile: two accumulator halves of 128
 constexpr int MAX_WST = 12, MAX_BST = 6;
 
 struct TcSmem {
-  uint32_t w_full, w_empty, b_full, b_empty, a_full, a_empty, d_full, d_empty, drain, tmem_slot, pre, scales, lut;
+  uint32_t w_full, w_empty, b_full, b_empty, a_full, a_empty, d_full, d_empty, drain, tmem_slot, pre, scales, lut, red;
   uint32_t w, b;                   // ring bases
   uint32_t w_stage, b_stage;       // bytes per stage
   uint32_t w_stages, b_stages;
@@ -97,6 +97,7 @@ struct TcArgs {
   uint32_t min_run;                // fewest super-blocks worth a CTA in the split part
   uint32_t n, n_act;               // weight matrices; distinct activation groups (group e reads e % n_act)
   uint32_t xcap, ycap;             // rows reserved per group in the activation and output arrays
+  uint32_t cs;                     // CTAs of a cluster that share a tile along K (CG = 1, one segment each); 1 = see Sched
   uint32_t once;                   // weights are read once: evict-first in L2
   const int *counts;               // device: live rows per activation group, or null (m rows each)
 };
@@ -204,6 +205,10 @@ __device__ __forceinline__ uint32_t in_first(uint32_t addr) {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+// Stores at the same shared-memory address of CTA `rank` of the cluster.
+__device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t rank, float v) {
+  asm volatile("{\n\t.reg .u32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.shared::cluster.f32 [a], %2;\n\t}" ::"r"(addr), "r"(rank), "f"(v) : "memory");
+}
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -245,8 +250,11 @@ __device__ __forceinline__ float4 ldcg4(const float *p) { return __ldcg(reinterp
 //
 //   BB, BPS   bytes of a block of one row; blocks per super-block.  A staged super-block is
 //             [16 chunks][BPS blocks][8 rows x BB bytes], block-major as in HBM
-//   Pk        the packed bytes of half a super-block; load() fetches them (p: the row's chunk)
-//   expand    32 columns (quarter q = 0 .. 3 of the half) -> sixteen half2
+//   Hd        what the four quarters share (scales), head() fetches it (p: the row's chunk)
+//   Qt        the packed bytes of quarter k (32 columns); quarter() fetches them
+//   expand    quarter k -> sixteen half2
+// (The four quarters are unrolled; as a rolled loop of a quarter of the code they take the same time,
+// Q4_K 14336 x 4096 by 64 tokens 18.1 against 18.6 us.)
 template <int T>
 struct WFmt;
 
@@ -285,42 +293,40 @@ template <>
 struct WFmt<QK_T_Q4_K> {  // d, dmin, 12 bytes of 6-bit scales / mins, 128 bytes of nibbles (reference/q4_k.rs:27-102)
   static constexpr uint32_t BB = 144, BPS = 1, LUT = 0;
   __device__ static void fill_lut(unsigned char *, uint32_t, uint32_t) {}
-  struct Pk { uint4 h, q[4]; };
   // position 8 i + j of a 64-group <- column 4 i + {0,2,1,3}[j & 3] + 32 (j >> 2): byte 4 i + b of
   // the group's 32 holds column 4 i + b (low nibble) and 32 + 4 i + b (high nibble)
   __host__ __device__ static uint32_t src(uint32_t p) {
     const uint32_t g = p >> 6, i = (p >> 3) & 7u, j = p & 7u, jj = j & 3u;
     return 64 * g + 4 * i + (jj == 1 ? 2 : jj == 2 ? 1 : jj) + 32 * (j >> 2);
   }
+  struct Hd { uint32_t scw, mnw, d; };  // the half's four 6-bit scales and minima, one per byte; d and dmin
+  struct Qt { uint4 q; };
   // [8 rows x 16 header | 4 groups x 8 rows x 32 nibble bytes]
-  __device__ static void load(Pk &k, uint32_t p, uint32_t rr, uint32_t hh) {
-    const uint32_t n = p + 128 + hh * 512 + rr * 32;
-    k.h = lds128(p + rr * 16), k.q[0] = lds128(n), k.q[1] = lds128(n + 16), k.q[2] = lds128(n + 256), k.q[3] = lds128(n + 272);
+  __device__ static void head(Hd &c, uint32_t p, uint32_t rr, uint32_t hh) {
+    const uint4 h = lds128(p + rr * 16);
+    c.scw = hh ? ((h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u)) : (h.y & 0x3F3F3F3Fu);
+    c.mnw = hh ? (((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u)) : (h.z & 0x3F3F3F3Fu);
+    c.d = h.x;
   }
-  struct Sc { __half2 s[2], m[2]; };  // per 64-group: (low nibbles, high nibbles) of scale and of -min
-  __device__ static void scales(const Pk &k, uint32_t hh, Sc &c) {
-    // Sub-blocks 4 hh .. 4 hh + 3.  d * sc and dmin * mn have 17 bits at most, so the fp16 products
-    // are the f32 ones rounded once.
-    const uint32_t scw = hh ? ((k.h.w & 0x0F0F0F0Fu) | ((k.h.y >> 2) & 0x30303030u)) : (k.h.y & 0x3F3F3F3Fu);
-    const uint32_t mnw = hh ? (((k.h.w >> 4) & 0x0F0F0F0Fu) | ((k.h.z >> 2) & 0x30303030u)) : (k.h.z & 0x3F3F3F3Fu);
-    const __half2 k1024 = __float2half2_rn(1024.f), d = __low2half2(bits_h2(k.h.x)), m = __hneg2(__high2half2(bits_h2(k.h.x)));
-#pragma unroll
-    for (int g = 0; g < 2; g++) {
-      c.s[g] = __hmul2(__hsub2(bits_h2(prmt(scw, 0x64646464u, g ? 0x4342u : 0x4140u)), k1024), d);
-      c.m[g] = __hmul2(__hsub2(bits_h2(prmt(mnw, 0x64646464u, g ? 0x4342u : 0x4140u)), k1024), m);
-    }
+  __device__ static void quarter(Qt &t, uint32_t p, uint32_t rr, uint32_t hh, uint32_t k) {
+    t.q = lds128(p + 128 + hh * 512 + rr * 32 + (k >> 1) * 256 + (k & 1u) * 16);
   }
-  // q exact after the subtraction, then one fused q * scale - min
-  __device__ static void expand(const Pk &k, const Sc &c, uint32_t, int q, uint32_t (&o)[16], uint32_t) {
-    const __half2 k_lo = __float2half2_rn(1024.f), k_hi = __float2half2_rn(64.f);
-    const __half2 s_lo = __low2half2(c.s[q >> 1]), s_hi = __high2half2(c.s[q >> 1]);
-    const __half2 m_lo = __low2half2(c.m[q >> 1]), m_hi = __high2half2(c.m[q >> 1]);
+  // d * sc and dmin * mn have 17 bits at most, so the fp16 products are the f32 ones rounded once.
+  // q is exact after the subtraction, then one fused q * scale - min.
+  __device__ static void expand(const Qt &t, const Hd &c, uint32_t k, uint32_t (&o)[16], uint32_t) {
+    const __half2 k1024 = __float2half2_rn(1024.f), k_hi = __float2half2_rn(64.f);
+    const __half2 d = __low2half2(bits_h2(c.d)), m = __hneg2(__high2half2(bits_h2(c.d)));
+    const uint32_t lo = 0x4040u + (k >> 1) * 0x0202u, hi = lo + 0x0101u;  // the 64-group's two sub-blocks
+    const __half2 s_lo = __hmul2(__hsub2(bits_h2(prmt(c.scw, 0x64646464u, lo)), k1024), d);
+    const __half2 s_hi = __hmul2(__hsub2(bits_h2(prmt(c.scw, 0x64646464u, hi)), k1024), d);
+    const __half2 m_lo = __hmul2(__hsub2(bits_h2(prmt(c.mnw, 0x64646464u, lo)), k1024), m);
+    const __half2 m_hi = __hmul2(__hsub2(bits_h2(prmt(c.mnw, 0x64646464u, hi)), k1024), m);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
       uint32_t e[4];
-      nibbles_to_magic(word(k.q[q], i), e);
-      o[4 * i + 0] = h2_bits(__hfma2(__hsub2(bits_h2(e[0]), k_lo), s_lo, m_lo));
-      o[4 * i + 1] = h2_bits(__hfma2(__hsub2(bits_h2(e[1]), k_lo), s_lo, m_lo));
+      nibbles_to_magic(word(t.q, i), e);
+      o[4 * i + 0] = h2_bits(__hfma2(__hsub2(bits_h2(e[0]), k1024), s_lo, m_lo));
+      o[4 * i + 1] = h2_bits(__hfma2(__hsub2(bits_h2(e[1]), k1024), s_lo, m_lo));
       o[4 * i + 2] = h2_bits(__hfma2(__hsub2(bits_h2(e[2]), k_hi), s_hi, m_hi));
       o[4 * i + 3] = h2_bits(__hfma2(__hsub2(bits_h2(e[3]), k_hi), s_hi, m_hi));
     }
@@ -331,27 +337,23 @@ template <>
 struct WFmt<QK_T_Q8_0> {  // block of 32: f16 d, 32 int8 (reference/q8_0.rs)
   static constexpr uint32_t BB = 34, BPS = 8, LUT = 0;
   __device__ static void fill_lut(unsigned char *, uint32_t, uint32_t) {}
-  struct Pk { uint4 q[8]; uint32_t d[4]; };
   __host__ __device__ static uint32_t src(uint32_t p) { return p; }
+  struct Hd {};
+  struct Qt { uint4 q[2]; uint32_t d; };
+  __device__ static void head(Hd &, uint32_t, uint32_t, uint32_t) {}
   // A block's 8 rows: [2 granules x 8 rows x 16 int8][8 x d].  Blocks past the end of the row
   // are zero-filled by the copy: d = 0.
-  __device__ static void load(Pk &k, uint32_t p, uint32_t rr, uint32_t hh) {
-    p += hh * 4 * 272;
-#pragma unroll
-    for (int b = 0; b < 4; b++) {
-      k.q[2 * b] = lds128(p + b * 272 + rr * 16), k.q[2 * b + 1] = lds128(p + b * 272 + 128 + rr * 16);
-      k.d[b] = lds16(p + b * 272 + 256 + 2 * rr);
-    }
+  __device__ static void quarter(Qt &t, uint32_t p, uint32_t rr, uint32_t hh, uint32_t k) {
+    p += (hh * 4 + k) * 272;
+    t.q[0] = lds128(p + rr * 16), t.q[1] = lds128(p + 128 + rr * 16), t.d = lds16(p + 256 + 2 * rr);
   }
-  struct Sc {};
-  __device__ static void scales(const Pk &, uint32_t, Sc &) {}
-  __device__ static void expand(const Pk &k, const Sc &, uint32_t, int q, uint32_t (&o)[16], uint32_t) {
+  __device__ static void expand(const Qt &t, const Hd &, uint32_t, uint32_t (&o)[16], uint32_t) {
     const __half2 off = __float2half2_rn(1152.f);  // 1024 + 128: (1024 + (q ^ 0x80)) - 1152 = q, exact; q * d rounded once
-    const __half2 d = __low2half2(bits_h2(k.d[q]));
+    const __half2 d = __low2half2(bits_h2(t.d));
 #pragma unroll
     for (int i = 0; i < 8; i++) {
       uint32_t a, b2;
-      bytes_to_magic(word(k.q[2 * q + (i >> 2)], i & 3) ^ 0x80808080u, a, b2);
+      bytes_to_magic(word(t.q[i >> 2], i & 3) ^ 0x80808080u, a, b2);
       o[2 * i] = h2_bits(__hmul2(__hsub2(bits_h2(a), off), d));
       o[2 * i + 1] = h2_bits(__hmul2(__hsub2(bits_h2(b2), off), d));
     }
@@ -362,28 +364,27 @@ template <>
 struct WFmt<QK_T_Q4_0> {  // block of 32: f16 d, 16 bytes; byte j = elements 2 j (low nibble) and 2 j + 1 (high) (reference/q4_0.rs:36-46)
   static constexpr uint32_t BB = 18, BPS = 8, LUT = 0;
   __device__ static void fill_lut(unsigned char *, uint32_t, uint32_t) {}
-  struct Pk { uint4 q[4]; uint32_t d[4]; };
   // a word yields its eight elements as (byte 0, byte 2), (byte 1, byte 3) low nibbles, then the
   // same of the high nibbles
   __host__ __device__ static uint32_t src(uint32_t p) {
     const uint32_t order = 0x73516240u;  // positions 0..7 <- elements 0, 4, 2, 6, 1, 5, 3, 7 of the word
     return (p & ~7u) + ((order >> (4 * (p & 7u))) & 7u);
   }
+  struct Hd {};
+  struct Qt { uint4 q; uint32_t d; };
+  __device__ static void head(Hd &, uint32_t, uint32_t, uint32_t) {}
   // A block's 8 rows: [8 rows x 16 nibble bytes][8 x d].
-  __device__ static void load(Pk &k, uint32_t p, uint32_t rr, uint32_t hh) {
-    p += hh * 4 * 144;
-#pragma unroll
-    for (int b = 0; b < 4; b++) k.q[b] = lds128(p + b * 144 + rr * 16), k.d[b] = lds16(p + b * 144 + 128 + 2 * rr);
+  __device__ static void quarter(Qt &t, uint32_t p, uint32_t rr, uint32_t hh, uint32_t k) {
+    p += (hh * 4 + k) * 144;
+    t.q = lds128(p + rr * 16), t.d = lds16(p + 128 + 2 * rr);
   }
-  struct Sc {};
-  __device__ static void scales(const Pk &, uint32_t, Sc &) {}
-  __device__ static void expand(const Pk &k, const Sc &, uint32_t, int q, uint32_t (&o)[16], uint32_t) {
+  __device__ static void expand(const Qt &t, const Hd &, uint32_t, uint32_t (&o)[16], uint32_t) {
     const __half2 off_lo = __float2half2_rn(1032.f), off_hi = __float2half2_rn(72.f);  // (K + q) - (K + 8) = q - 8, exact
-    const __half2 d = __low2half2(bits_h2(k.d[q]));
+    const __half2 d = __low2half2(bits_h2(t.d));
 #pragma unroll
     for (int i = 0; i < 4; i++) {
       uint32_t e[4];
-      nibbles_to_magic(word(k.q[q], i), e);
+      nibbles_to_magic(word(t.q, i), e);
       o[4 * i + 0] = h2_bits(__hmul2(__hsub2(bits_h2(e[0]), off_lo), d));
       o[4 * i + 1] = h2_bits(__hmul2(__hsub2(bits_h2(e[1]), off_lo), d));
       o[4 * i + 2] = h2_bits(__hmul2(__hsub2(bits_h2(e[2]), off_hi), d));
@@ -396,32 +397,32 @@ template <>
 struct WFmt<QK_T_Q6_K> {  // super-block of 256: ql 128, qh 64, 16 int8 scales, f16 d (reference/q6_k.rs)
   static constexpr uint32_t BB = 210, BPS = 1, LUT = 0;
   __device__ static void fill_lut(unsigned char *, uint32_t, uint32_t) {}
-  // half hh = ql[64 hh ..], qh[32 hh ..]; its quarter q (columns 32 q ..) = nibble q >> 1 of ql bytes
-  // 32 (q & 1) + l and bit pair 2 q of qh byte l
-  struct Pk { uint4 ql[4], qh[2]; uint2 sc; uint32_t d; };
+  // half hh = ql[64 hh ..], qh[32 hh ..]; its quarter k (columns 32 k ..) = nibble k >> 1 of ql bytes
+  // 32 (k & 1) + l and bit pair 2 k of qh byte l
   __host__ __device__ static uint32_t src(uint32_t p) { return p; }
+  struct Hd { uint4 qh[2]; uint2 sc; float d; };
+  struct Qt { uint4 ql[2]; };
   // A block's 8 rows: [12 granules x 8 rows x 16 bytes of ql+qh][8 rows x 16 scales][8 x d].
-  __device__ static void load(Pk &k, uint32_t p, uint32_t rr, uint32_t hh) {
+  __device__ static void head(Hd &c, uint32_t p, uint32_t rr, uint32_t hh) {
     const uint32_t q = p + rr * 16;
-#pragma unroll
-    for (int i = 0; i < 4; i++) k.ql[i] = lds128(q + (4 * hh + i) * 128);
-    k.qh[0] = lds128(q + (8 + 2 * hh) * 128), k.qh[1] = lds128(q + (9 + 2 * hh) * 128);
-    k.sc = lds64(q + 1536 + 8 * hh);
-    k.d = lds16(p + 1664 + 2 * rr);
+    c.qh[0] = lds128(q + (8 + 2 * hh) * 128), c.qh[1] = lds128(q + (9 + 2 * hh) * 128);
+    c.sc = lds64(q + 1536 + 8 * hh);
+    c.d = h2f_bits(lds16(p + 1664 + 2 * rr));
   }
-  struct Sc { float d; };
-  __device__ static void scales(const Pk &k, uint32_t, Sc &c) { c.d = h2f_bits(k.d); }
-  __device__ static void expand(const Pk &k, const Sc &c, uint32_t, int q, uint32_t (&o)[16], uint32_t) {
+  __device__ static void quarter(Qt &t, uint32_t p, uint32_t rr, uint32_t hh, uint32_t k) {
+    const uint32_t q = p + rr * 16 + (4 * hh + 2 * (k & 1u)) * 128;
+    t.ql[0] = lds128(q), t.ql[1] = lds128(q + 128);
+  }
+  __device__ static void expand(const Qt &t, const Hd &c, uint32_t k, uint32_t (&o)[16], uint32_t) {
     const __half2 off = __float2half2_rn(1056.f);  // (1024 + q) - 1056 = q - 32, exact; then one rounding in the product
-    const uint32_t scw = (q >> 1) ? k.sc.y : k.sc.x;
+    const uint32_t scw = ((k >> 1) ? c.sc.y : c.sc.x) >> (16 * (k & 1u)), nib = 4 * (k >> 1), rot = (4 - 2 * k) & 31u;
     __half2 s[2];  // 16 columns per scale
 #pragma unroll
-    for (int i = 0; i < 2; i++) s[i] = __float2half2_rn(c.d * (float)(int)(signed char)((scw >> (16 * (q & 1) + 8 * i)) & 0xFF));
+    for (int i = 0; i < 2; i++) s[i] = __float2half2_rn(c.d * (float)(int)(signed char)((scw >> (8 * i)) & 0xFF));
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-      const uint32_t lw = word(k.ql[2 * (q & 1) + (i >> 2)], i & 3), hw = word(k.qh[i >> 2], i & 3);
-      const uint32_t hi = q == 0 ? hw << 4 : q == 1 ? hw << 2 : q == 2 ? hw : hw >> 2;
-      const uint32_t q6 = (((q >> 1) ? lw >> 4 : lw) & 0x0F0F0F0Fu) | (hi & 0x30303030u);
+      const uint32_t lw = word(t.ql[i >> 2], i & 3) >> nib, hw = word(c.qh[i >> 2], i & 3);
+      const uint32_t q6 = (lw & 0x0F0F0F0Fu) | (__funnelshift_l(hw, hw, rot) & 0x30303030u);
       uint32_t a, b2;
       bytes_to_magic(q6, a, b2);
       o[2 * i] = h2_bits(__hmul2(__hsub2(bits_h2(a), off), s[i >> 2]));
@@ -437,7 +438,6 @@ struct WFmt<QK_T_IQ4_XS> {  // super-block of 256: f16 d, scales_h, scales_l[4],
   // maps a byte straight to the half2 (K[low], K[high]) of its two adjacent elements; every lane has
   // a copy of its own in its own bank (32 KB), so the look-ups of a warp never conflict.
   static constexpr uint32_t BB = 136, BPS = 1, LUT = 32768;
-  struct Pk { uint4 q[4]; uint2 h; };
   __host__ __device__ static uint32_t src(uint32_t p) { return p; }
   __device__ static void fill_lut(unsigned char *lut, uint32_t tid, uint32_t nthreads) {
     constexpr uint32_t K0 = 0xBFAD9881u, K1 = 0xF6EADDCFu, K2 = 0x26190D01u, K3 = 0x71594535u;  // K[0..15] as bytes
@@ -448,25 +448,23 @@ struct WFmt<QK_T_IQ4_XS> {  // super-block of 256: f16 d, scales_h, scales_l[4],
     for (uint32_t i = tid; i < 256 * 32; i += nthreads)
       reinterpret_cast<uint32_t *>(lut)[i] = h2_bits(__floats2half2_rn(val((i >> 5) & 15u), val(i >> 9)));
   }
+  struct Hd { float d; uint32_t ls; };  // ls: the half's four 6-bit scales, one per byte
+  struct Qt { uint4 q; };
   // A block's 8 rows: [8 granules x 8 rows x 16 nibble bytes][8 rows x 8 header bytes].
-  __device__ static void load(Pk &k, uint32_t p, uint32_t rr, uint32_t hh) {
-#pragma unroll
-    for (int i = 0; i < 4; i++) k.q[i] = lds128(p + (4 * hh + i) * 128 + rr * 16);
-    k.h = lds64(p + 1024 + rr * 8);
-  }
-  struct Sc { float d; uint32_t ls; };  // ls: the half's four 6-bit scales, one per byte
-  __device__ static void scales(const Pk &k, uint32_t hh, Sc &c) {
-    c.d = h2f_bits(k.h.x);
-    const uint32_t sl = hh ? k.h.y >> 16 : k.h.y, sh = k.h.x >> (16 + 8 * hh);
+  __device__ static void head(Hd &c, uint32_t p, uint32_t rr, uint32_t hh) {
+    const uint2 h = lds64(p + 1024 + rr * 8);
+    c.d = h2f_bits(h.x);
+    const uint32_t sl = hh ? h.y >> 16 : h.y, sh = h.x >> (16 + 8 * hh);
     c.ls = (sl & 0x0Fu) | ((sl & 0xF0u) << 4) | ((sl & 0xF00u) << 8) | ((sl & 0xF000u) << 12);
     c.ls |= ((sh & 3u) << 4) | ((sh & 0xCu) << 10) | ((sh & 0x30u) << 16) | ((sh & 0xC0u) << 22);
   }
+  __device__ static void quarter(Qt &t, uint32_t p, uint32_t rr, uint32_t hh, uint32_t k) { t.q = lds128(p + (4 * hh + k) * 128 + rr * 16); }
   // lut: this lane's copy (byte b at lut + 128 b)
-  __device__ static void expand(const Pk &k, const Sc &c, uint32_t, int q, uint32_t (&o)[16], uint32_t lut) {
-    const __half2 dl = __float2half2_rn(c.d * (float)((int)((c.ls >> (8 * q)) & 0x3Fu) - 32));
+  __device__ static void expand(const Qt &t, const Hd &c, uint32_t k, uint32_t (&o)[16], uint32_t lut) {
+    const __half2 dl = __float2half2_rn(c.d * (float)((int)((c.ls >> (8 * k)) & 0x3Fu) - 32));
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-      const uint32_t w = word(k.q[q], i);
+      const uint32_t w = word(t.q, i);
       o[4 * i + 0] = h2_bits(__hmul2(bits_h2(lds32(lut + ((w << 7) & 0x7F80u))), dl));
       o[4 * i + 1] = h2_bits(__hmul2(bits_h2(lds32(lut + ((w >> 1) & 0x7F80u))), dl));
       o[4 * i + 2] = h2_bits(__hmul2(bits_h2(lds32(lut + ((w >> 9) & 0x7F80u))), dl));
@@ -484,7 +482,13 @@ struct WFmt<QK_T_IQ4_XS> {  // super-block of 256: f16 d, scales_h, scales_l[4],
 // the conversion (a thread's eight positions come from two float4s whatever the format's order).
 // GLU: the row is silu(x) * x2, formed here (crates/oxillama-arch/src/common/swiglu.rs:15-21, each
 // step rounded), so the hidden activations of a feed-forward block are never written out in f32.
-constexpr int CT = 512, CCH = 4;  // threads; chunks of eight positions a thread keeps
+//
+// CT threads keep CCH chunks of eight positions each.  512 threads are the faster conversion, but their
+// CTAs and those of the matmul (24 warps of 80 registers) do not fit on an SM together: the matmul's CTA
+// there starts, sets itself up and fetches its first weights only when the conversion is over.  From 64 rows
+// of up to 4096 columns (so many CTAs that few SMs are without one) 256 threads of 40 registers run beside
+// a matmul of 72 registers.  Q4_K 4096 x 4096: 37 rows 11.1 (apart) against 11.5 us (beside), 64 rows 13.8
+// against 12.6, 128 rows 19.7 against 18.3.
 struct ConvArgs {
   const float *x, *x2;
   __half *out;
@@ -530,8 +534,21 @@ __device__ __forceinline__ void conv_load(const float *__restrict__ x, const flo
   }
 }
 
-template <int T, bool GLU>
-__global__ void __launch_bounds__(CT) qk_x16_kernel(const ConvArgs A) {
+__device__ __forceinline__ float conv_scale(float amax) {
+  if (!(amax > 0.f && amax <= FLT_MAX)) return 1.f;  // zero, or not finite (a NaN row stays NaN)
+  int e;
+  frexpf(amax, &e);  // amax = f * 2^e, f in [0.5, 1)
+  return ldexpf(1.f, e - 10);
+}
+__device__ __forceinline__ void conv_store(__half *orow, uint32_t c, const float (&w)[8], float inv) {
+  uint32_t h[4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) h[j] = h2_bits(__floats2half2_rn(w[2 * j] * inv, w[2 * j + 1] * inv));
+  *reinterpret_cast<uint4 *>(orow + 8ull * c) = make_uint4(h[0], h[1], h[2], h[3]);
+}
+
+template <int T, bool GLU, int CT, int CCH>
+__global__ void __launch_bounds__(CT, CT == 256 ? 6 : 1) qk_x16_kernel(const ConvArgs A) {
   __shared__ float red[CT / 32];
   pdl_launch_dependents();
   pdl_wait();
@@ -570,43 +587,40 @@ __global__ void __launch_bounds__(CT) qk_x16_kernel(const ConvArgs A) {
   amax = red[0];
 #pragma unroll
   for (int w = 1; w < CT / 32; w++) amax = fmaxf(amax, red[w]);
-  float scale = 1.f;
-  if (amax > 0.f && amax <= FLT_MAX) {  // finite and non-zero (a NaN row keeps scale 1 and stays NaN)
-    int e;
-    frexpf(amax, &e);  // amax = f * 2^e, f in [0.5, 1)
-    scale = ldexpf(1.f, e - 10);
-  }
+  const float scale = conv_scale(amax);
   const float inv = 1.f / scale;  // a power of two: exact
   if (threadIdx.x == 0) A.scales[t] = scale;
   __half *orow = A.out + (uint64_t)t * A.Kp;
-  auto put = [&](uint32_t c, const float (&w)[8]) {
-    uint32_t h[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) h[j] = h2_bits(__floats2half2_rn(w[2 * j] * inv, w[2 * j + 1] * inv));
-    *reinterpret_cast<uint4 *>(orow + 8ull * c) = make_uint4(h[0], h[1], h[2], h[3]);
-  };
 #pragma unroll
   for (int i = 0; i < CCH; i++) {
     const uint32_t c = threadIdx.x + i * CT;
-    if (c < nch) put(c, v[i]);
+    if (c < nch) conv_store(orow, c, v[i], inv);
   }
   for (uint32_t c = threadIdx.x + CCH * CT; c < nch; c += CT) {
     float w[8];
     conv_load<T, GLU>(xr, ur, c, A.cols, vec, w);
-    put(c, w);
+    conv_store(orow, c, w, inv);
   }
 }
 
 // ---------------------------------------------------------------- schedule
-// The segments of one CTA (pair), the same list for every role: first its run of the split tiles
-// (tiles 0 .. R - 1, R = the remainder of the tile count over the pairs, their R * nsb super-blocks cut
-// into equal runs), then whole tiles R + pair, + pairs, ..
+// The segments of one CTA (pair), the same list for every role: first whole tiles R + pair, + pairs, ..
+// (R = the remainder of the tile count over the pairs), then its run of the split tiles 0 .. R - 1, whose
+// R * nsb super-blocks are cut into equal runs.  (The split part last, so that all warps of the CTA can add
+// the partials up: four warps alone have 16 KB of loads in flight, 25 us for a tile of 256 x 256 from two
+// runs, and a whole tile's main loop behind it does not hide that.)
 struct Sched {
-  uint32_t nsb, R, base, rem, b, e, first_tile, n_split, n_seg, me, pairs;
+  uint32_t nsb, R, base, rem, b, e, first_tile, n_split, whole, n_seg, me, pairs;
+  // One tile per cluster of cs CTAs, K cut into cs runs.
+  __device__ __forceinline__ void init_cluster(uint32_t nsb_, uint32_t cs) {
+    const uint32_t k = blockIdx.x % cs;
+    nsb = nsb_, first_tile = blockIdx.x / cs, n_split = n_seg = 1, whole = 0, R = pairs = gridDim.x / cs;
+    b = first_tile * nsb + k * nsb / cs, e = first_tile * nsb + (k + 1) * nsb / cs;
+  }
   template <int CG>
   __device__ __forceinline__ void init(uint32_t tiles, uint32_t nsb_, uint32_t min_run) {
     nsb = nsb_, me = blockIdx.x / CG, pairs = gridDim.x / CG;
-    const uint32_t whole = tiles / pairs;
+    whole = tiles / pairs;
     R = tiles - whole * pairs;
     const uint32_t total = R * nsb, runs = total / min_run;
     const uint32_t n = runs < pairs ? (runs ? runs : 1u) : pairs;  // pairs that share the split part
@@ -625,12 +639,12 @@ struct Sched {
     return sb < longer ? sb / (base + 1) : rem + (sb - longer) / base;
   }
   __device__ __forceinline__ void get(uint32_t i, uint32_t &tile, uint32_t &s0, uint32_t &s1) const {
-    if (i < n_split) {
-      tile = first_tile + i;
-      s0 = i == 0 ? b - tile * nsb : 0u;
-      s1 = i + 1 == n_split ? e - tile * nsb : nsb;
+    if (i >= whole) {
+      tile = first_tile + i - whole;
+      s0 = i == whole ? b - tile * nsb : 0u;
+      s1 = i + 1 == n_seg ? e - tile * nsb : nsb;
     } else {
-      tile = R + me + (i - n_split) * pairs, s0 = 0, s1 = nsb;
+      tile = R + me + i * pairs, s0 = 0, s1 = nsb;
     }
   }
 };
@@ -658,8 +672,9 @@ __device__ __forceinline__ bool walk_segment(uint32_t s0, uint32_t s1, bool wide
 // T: weight format.  CG: CTAs per tile (see the top).  NG: 1 = one matrix; otherwise up to NG matrices
 // of one shape and format (the projections of a feed-forward block, the experts of a mixture), each
 // multiplying its own group of activation rows.
-template <int T, int CG, int NG>
-__global__ void __launch_bounds__(NTHREADS, 1)
+// REGS: registers per thread: 80, or 72 to leave room for CTAs of the conversion beside it.
+template <int T, int CG, int NG, int REGS>
+__global__ void __maxnreg__(REGS)
     qk_gemm_tc_kernel(const __grid_constant__ TcArgs A, const __grid_constant__ TcMaps<NG> M) {
   extern __shared__ __align__(1024) unsigned char smem[];
   using F = WFmt<T>;
@@ -673,11 +688,12 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 
   pdl_launch_dependents();
   if (threadIdx.x == 0) {
-    for (uint32_t s = 0; s < S.w_stages; s++) mbar_init(sbase + S.w_full + s * 8, 1), mbar_init(sbase + S.w_empty + s * 8, NDW / 2);
+    for (uint32_t s = 0; s < S.w_stages; s++) mbar_init(sbase + S.w_full + s * 8, 1), mbar_init(sbase + S.w_empty + s * 8, 8);
     for (uint32_t s = 0; s < S.b_stages; s++) mbar_init(sbase + S.b_full + s * 8, 1), mbar_init(sbase + S.b_empty + s * 8, 1);
-    for (uint32_t s = 0; s < 3; s++) mbar_init(sbase + S.a_full + s * 8, CG * NDW / 2), mbar_init(sbase + S.a_empty + s * 8, 1);
+    for (uint32_t s = 0; s < 3; s++) mbar_init(sbase + S.a_full + s * 8, CG * 8), mbar_init(sbase + S.a_empty + s * 8, 1);
     for (uint32_t s = 0; s < 2; s++) mbar_init(sbase + S.d_full + s * 8, 1), mbar_init(sbase + S.d_empty + s * 8, CG * 4);
     mbar_init(sbase + S.drain, 1);
+    *reinterpret_cast<volatile uint32_t *>(smem + S.scales + 2052) = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -708,12 +724,14 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   }
   tc_fence_before();
   __syncthreads();
-  if (CG == 2) cluster_sync();  // the other CTA's barriers are initialised, its tensor memory is there
+  const bool clustered = CG == 2 || (NG == 1 && A.cs > 1);
+  if (clustered) cluster_sync();  // the other CTAs run, their barriers are initialised, their tensor memory is there
   tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(smem + S.tmem_slot);
 
   Sched sc{};
-  sc.template init<CG>(counted ? pre[A.n] : A.n * A.row_blocks * A.tok_blocks, (A.L.cols + 255u) / 256u, A.min_run);
+  if (CG == 1 && NG == 1 && A.cs > 1) sc.init_cluster((A.L.cols + 255u) / 256u, A.cs);
+  else sc.template init<CG>(counted ? pre[A.n] : A.n * A.row_blocks * A.tok_blocks, (A.L.cols + 255u) / 256u, A.min_run);
   auto at = [&](uint32_t tile) {
     TileAt q;
     uint32_t tb;
@@ -737,6 +755,48 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   // Token rows that an activation box brings: each CTA of a pair loads half of the n tokens.
   const uint32_t hq = A.hn / (4 * CG);
   auto box_rows = [&](uint32_t n) { return NG > 1 ? (n / CG + hq - 1) / hq * hq : A.hn / CG; };
+
+  // The last contributor of a split tile adds the partials up, in the order of their K runs: a warp four
+  // tokens at a time, a lane four rows.
+  auto add_up = [&](uint32_t tile) {
+    __threadfence();
+    const TileAt q = at(tile);
+    const uint32_t i0 = sc.owner_of(tile * sc.nsb), i1 = sc.owner_of((tile + 1) * sc.nsb - 1), slot = A.bn * BM;
+    const uint32_t live = min(q.live - q.t0, q.n), row0 = (q.rb * CG + rank) * BM, rw = row0 + 4 * lane;
+    const float *sp = A.xscale + (NG > 1 ? (q.g % A.n_act) * A.xcap : 0u) + q.t0;
+    float *yt = A.y + (uint64_t)((NG > 1 ? q.g * A.ycap : 0u) + q.t0) * A.ldy;
+    const bool vec = row0 + BM <= A.L.rows && (A.ldy & 3u) == 0 && ((uintptr_t)A.y & 15u) == 0;
+    for (uint32_t c = 4 * warp; c < live; c += NTHREADS / 8) {
+      float4 s[4];
+#pragma unroll
+      for (uint32_t j = 0; j < 4; j++) s[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+      for (uint32_t p = i0; p <= i1; p++) {
+        const float *src = A.part + ((p * CG + rank) * 2 + (sc.start_of(p) / sc.nsb == tile ? 0u : 1u)) * slot + c * BM + 4 * lane;
+        float4 o[4];
+#pragma unroll
+        for (uint32_t j = 0; j < 4; j++) o[j] = ldcg4(src + j * BM);  // (token rows past the live ones exist: n is a multiple of 16)
+#pragma unroll
+        for (uint32_t j = 0; j < 4; j++) s[j].x += o[j].x, s[j].y += o[j].y, s[j].z += o[j].z, s[j].w += o[j].w;
+      }
+      float *yp = yt + (uint64_t)c * A.ldy + rw;
+#pragma unroll
+      for (uint32_t j = 0; j < 4; j++, yp += A.ldy) {
+        if (c + j >= live) break;
+        const float f = __ldg(sp + c + j);
+        const float4 v = make_float4(s[j].x * f, s[j].y * f, s[j].z * f, s[j].w * f);
+        if (vec) {
+          *reinterpret_cast<float4 *>(yp) = v;
+        } else {
+          if (rw < A.L.rows) yp[0] = v.x;
+          if (rw + 1 < A.L.rows) yp[1] = v.y;
+          if (rw + 2 < A.L.rows) yp[2] = v.z;
+          if (rw + 3 < A.L.rows) yp[3] = v.w;
+        }
+      }
+    }
+  };
+  volatile uint32_t *last = reinterpret_cast<volatile uint32_t *>(smem + S.scales + 2052);  // split segments that this CTA adds up at its end
 
   bool dead = false;
   if (warp == 0 && rank == 0) {
@@ -873,13 +933,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       sc.get(i, tile, s0, s1);
       const TileAt q = at(tile);
       const bool wide = q.n > A.hn;
-      const bool split = i < sc.n_split && (s0 != 0 || s1 != sc.nsb);
+      const bool split = s0 != 0 || s1 != sc.nsb;
       const uint32_t row0 = (q.rb * CG + rank) * BM, row = row0 + r;
       const float *sp = A.xscale + (NG > 1 ? (q.g % A.n_act) * A.xcap : 0u) + q.t0;
       float *yt = A.y + (uint64_t)((NG > 1 ? q.g * A.ycap : 0u) + q.t0) * ldy;  // the tile's first token
       // partial tiles: [slot][token][128 rows]
       const uint32_t slot = A.bn * BM;
-      float *mine = A.part + (blockIdx.x * 2 + (i == 0 ? 0u : 1u)) * slot + r;
+      float *mine = A.part + (blockIdx.x * 2 + (i == sc.whole ? 0u : 1u)) * slot + r;
       for (uint32_t h = 0; h < (wide ? 2u : 1u); h++) {
         const uint32_t dh = both ? h : i & 1u, hoff = h * A.hn;  // first token of the half inside the tile
         const uint32_t n = h ? q.n - A.hn : wide ? A.hn : q.n;
@@ -906,7 +966,16 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(d_empty + dh * 8);
           }
-          if (split) {
+          if (CG == 1 && NG == 1 && A.cs > 1) {
+            // to the CTA of the cluster that adds up the token
+            const uint32_t own = (q.n + A.cs - 1) / A.cs, at = sbase + S.red + (blockIdx.x % A.cs * own * BM + r) * 4;
+            uint32_t to = c / own, t = c % own;
+#pragma unroll
+            for (uint32_t j = 0; j < 16; j++) {
+              st_cluster(at + t * (BM * 4), to, __uint_as_float(v[j]));
+              if (++t == own) t = 0, to++;
+            }
+          } else if (split) {
 #pragma unroll
             for (uint32_t j = 0; j < 16; j++) __stcg(pp + j * BM, __uint_as_float(v[j]));
           } else {
@@ -929,6 +998,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         }
       }
       if (!split) continue;
+      if (CG == 1 && NG == 1 && A.cs > 1) break;  // see below
       // Count in, once both halves are in the workspace (the accumulators are free by now); the last
       // contributor adds the partials up, in the order of their K runs.
       const uint32_t i0 = sc.owner_of(tile * sc.nsb), i1 = sc.owner_of((tile + 1) * sc.nsb - 1);
@@ -940,39 +1010,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       if (warp == FIRST_EW && lane == 0) *told = atomicAdd(A.cnt + tile * 2 + rank, 1u);
       asm volatile("bar.sync 1, 128;" ::: "memory");
       if (*told != i1 - i0) continue;
-      __threadfence();
-      // lane: rows 4 lane .. + 3; the four warps share the tokens, four at a time
-      const uint32_t live = min(q.live - q.t0, q.n), rw = row0 + 4 * lane;
-      const bool vec = row0 + BM <= A.L.rows && (ldy & 3u) == 0 && ((uintptr_t)A.y & 15u) == 0;
-      for (uint32_t c = 4 * quarter; c < live; c += 16) {
-        float4 s[4];
-#pragma unroll
-        for (uint32_t j = 0; j < 4; j++) s[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 2
-        for (uint32_t p = i0; p <= i1; p++) {
-          const float *src = A.part + ((p * CG + rank) * 2 + (sc.start_of(p) / sc.nsb == tile ? 0u : 1u)) * slot + c * BM + 4 * lane;
-          float4 o[4];
-#pragma unroll
-          for (uint32_t j = 0; j < 4; j++) o[j] = ldcg4(src + j * BM);  // (token rows past the live ones exist: n is a multiple of 16)
-#pragma unroll
-          for (uint32_t j = 0; j < 4; j++) s[j].x += o[j].x, s[j].y += o[j].y, s[j].z += o[j].z, s[j].w += o[j].w;
-        }
-        float *yp = yt + (uint64_t)c * ldy + rw;
-#pragma unroll
-        for (uint32_t j = 0; j < 4; j++, yp += ldy) {
-          if (c + j >= live) break;
-          const float f = __ldg(sp + c + j);
-          const float4 v = make_float4(s[j].x * f, s[j].y * f, s[j].z * f, s[j].w * f);
-          if (vec) {
-            *reinterpret_cast<float4 *>(yp) = v;
-          } else {
-            if (rw < A.L.rows) yp[0] = v.x;
-            if (rw + 1 < A.L.rows) yp[1] = v.y;
-            if (rw + 2 < A.L.rows) yp[2] = v.z;
-            if (rw + 3 < A.L.rows) yp[3] = v.w;
-          }
-        }
-      }
+      if (warp == FIRST_EW && lane == 0) *last |= 1u << (i - sc.whole);  // all warps add them up, below
     }
     if (dead && lane == 0) atomicOr(A.status, QK_DEV_TIMEOUT);
   } else if (warp >= FIRST_DW) {
@@ -991,19 +1029,18 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     }
     const uint32_t w_bytes = S.w_stage, nst = S.w_stages, w0 = sbase + S.w + (r >> 3) * CHB;
     const uint32_t ta0 = tmem + ((32 * quarter) << 16) + a_col + hh * 64u, a_full0 = in_first<CG>(sbase + S.a_full);
-    uint32_t ws = set % nst, wph = set / nst & 1u;      // ring stage and parity of this set's next super-block
+    uint32_t ws = set, wph = 0;      // ring stage and parity of this set's next super-block
     uint32_t ab = set, auses = 0;                       // its buffer, and how often that has been used (set < na)
     for (uint32_t j = set; j < n_sb; j += 2) {
       if (!warp_wait(sbase + S.w_full + ws * 8, wph)) {
         dead = true;  // warp-uniform: these warps execute .aligned tcgen05 instructions
         break;
       }
-      typename F::Pk pk;
-      F::load(pk, w0 + ws * w_bytes, rr, hh);
-      typename F::Sc c;
-      F::scales(pk, hh, c);
-      uint32_t o[16];
-      F::expand(pk, c, hh, 0, o, lut);
+      const uint32_t p = w0 + ws * w_bytes;
+      typename F::Hd hd;
+      typename F::Qt qt;
+      F::quarter(qt, p, rr, hh, 0);
+      F::head(hd, p, rr, hh);
       // the MMAs that read this buffer's previous contents must have retired
       if (auses && !warp_wait(sbase + S.a_empty + ab * 8, (auses - 1) & 1u)) {
         dead = true;
@@ -1011,16 +1048,17 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
       tc_fence_after();
       const uint32_t ta = ta0 + ab * 128u;
-      tmem_st16(ta, o);
 #pragma unroll
-      for (int k = 1; k < 4; k++) {
-        F::expand(pk, c, hh, k, o, lut);
-        if (k == 3) {
-          __syncwarp();
-          if (lane == 0) mbar_arrive(sbase + S.w_empty + ws * 8);  // every lane holds its packed bytes
-        }
+      for (uint32_t k = 0; k < 4; k++) {
+        typename F::Qt next;
+        F::quarter(next, p, rr, hh, k < 3 ? k + 1 : 3);
+        uint32_t o[16];
+        F::expand(qt, hd, k, o, lut);
         tmem_st16(ta + 16 * k, o);
+        qt = next;
       }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(sbase + S.w_empty + ws * 8);  // every lane holds its packed bytes
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
       __syncwarp();
@@ -1036,20 +1074,36 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   // common exit: the tensor memory is always returned
   tc_fence_before();
   __syncthreads();
-  if (CG == 2) cluster_sync();  // neither CTA leaves while the other may still arrive on its barriers or read its operands
+  if (clustered) cluster_sync();  // neither CTA leaves while the other may still arrive on its barriers or read its operands
   tc_fence_after();
+  if (CG == 1 && NG == 1 && A.cs > 1 && warp >= FIRST_EW) {
+    // The partial sums of this CTA's tokens have arrived: add them up in the order of their K runs.
+    const TileAt q = at(sc.first_tile);
+    const uint32_t own = (q.n + A.cs - 1) / A.cs, k = blockIdx.x % A.cs, r = 32 * (warp & 3u) + lane, row = q.rb * BM + r;
+    const float *red = reinterpret_cast<const float *>(smem + S.red) + r;
+    const uint32_t left = q.live - q.t0, t1 = min((k + 1) * own, min(left, q.n));
+    if (row < A.L.rows)
+      for (uint32_t t = k * own; t < t1; t++) {
+        float v = 0.f;
+        for (uint32_t p = 0; p < A.cs; p++) v += red[(p * own + t - k * own) * BM];
+        A.y[(uint64_t)(q.t0 + t) * A.ldy + row] = v * __ldg(A.xscale + q.t0 + t);
+      }
+  }
   if (warp == 3) {
     if (CG == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
     else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
   }
+  if (*last)
+    for (uint32_t i = 0; i < sc.n_split; i++)
+      if (*last >> i & 1u) add_up(sc.first_tile + i);
 }
 
 // ---------------------------------------------------------------- host side
-constexpr uint32_t SMEM_BUDGET = 226u * 1024u;
+constexpr uint32_t SMEM_BUDGET = 225u * 1024u;  // leaves room for a CTA of the conversion
 
 struct TcPlan {
   TcSmem S;
-  uint32_t cg, smem, bn, hn, tok_blocks, row_blocks, nsb, min_run, grid, xrows;
+  uint32_t cg, cs, smem, bn, hn, tok_blocks, row_blocks, nsb, min_run, grid, xrows;
   size_t o_scale, o_cnt, o_part, bytes;
 };
 // qk_gemm_tc.cu
@@ -1063,9 +1117,9 @@ inline cudaLaunchAttribute pdl_attr() {
   return a;
 }
 
-template <int T, int CG, int NG>
+template <int T, int CG, int NG, int REGS = 80>
 cudaError_t launch_main(const TcPlan &P, const TcArgs &A, __half *x16, const QkTcCall &c, cudaStream_t s) {
-  auto kern = qk_gemm_tc_kernel<T, CG, NG>;
+  auto kern = qk_gemm_tc_kernel<T, CG, NG, REGS>;
   static QkPerDevice attr_set;
   if (attr_set.first()) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BUDGET);
@@ -1077,12 +1131,15 @@ cudaError_t launch_main(const TcPlan &P, const TcArgs &A, __half *x16, const QkT
   for (uint32_t g = 0; g < (NG == 1 ? 1u : c.n); g++) memcpy(&M.w[g], c.maps[g], sizeof(CUtensorMap));
   cudaLaunchAttribute at[2] = {pdl_attr(), {}};
   at[1].id = cudaLaunchAttributeClusterDimension;
-  at[1].val.clusterDim.x = 2, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
+  at[1].val.clusterDim.x = CG == 2 ? 2 : P.cs, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(P.grid), cfg.blockDim = dim3(NTHREADS), cfg.dynamicSmemBytes = P.smem, cfg.stream = s;
-  cfg.attrs = at, cfg.numAttrs = CG == 2 ? 2 : 1;
+  cfg.attrs = at, cfg.numAttrs = CG == 2 || P.cs > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, A, M);
 }
+
+// Formats whose expansion runs as fast on 72 registers (Q6_K does not: 4096 x 14336 by 512 66.0 against 63.0 us).
+constexpr bool beside_of(int t) { return t != QK_T_Q6_K; }
 
 template <int T>
 cudaError_t launch_fmt(const QkTcCall &c, unsigned *status, unsigned char *scratch, int sm_count, cudaStream_t s) {
@@ -1097,17 +1154,24 @@ cudaError_t launch_fmt(const QkTcCall &c, unsigned *status, unsigned char *scrat
   C.x = c.x, C.x2 = c.x2, C.out = x16, C.scales = scales, C.zero = cnt, C.n_zero = (uint32_t)sm_count * 2;
   C.counts = c.counts, C.lists = c.lists, C.m = c.m, C.cols = L.cols, C.Kp = Kp, C.cap = c.xcap;
   C.list_stride = c.list_stride, C.list_div = c.list_div ? c.list_div : 1u;
+  const bool beside = beside_of(T) && c.n == 1 && !c.counts && c.m >= 64 && Kp <= 4096;
   cudaLaunchAttribute at = pdl_attr();
   cudaLaunchConfig_t c0 = {};
-  c0.gridDim = dim3(c.counts || c.n_act > 1 ? c.n_act * c.xcap : c.m), c0.blockDim = dim3(CT), c0.stream = s, c0.attrs = &at, c0.numAttrs = 1;
-  cudaError_t e = c.x2 ? cudaLaunchKernelEx(&c0, qk_x16_kernel<T, true>, C) : cudaLaunchKernelEx(&c0, qk_x16_kernel<T, false>, C);
+  c0.gridDim = dim3(c.counts || c.n_act > 1 ? c.n_act * c.xcap : c.m), c0.blockDim = dim3(beside ? 256 : 512), c0.stream = s, c0.attrs = &at, c0.numAttrs = 1;
+  cudaError_t e;
+  if (beside) e = c.x2 ? cudaLaunchKernelEx(&c0, qk_x16_kernel<T, true, 256, 2>, C) : cudaLaunchKernelEx(&c0, qk_x16_kernel<T, false, 256, 2>, C);
+  else e = c.x2 ? cudaLaunchKernelEx(&c0, qk_x16_kernel<T, true, 512, 4>, C) : cudaLaunchKernelEx(&c0, qk_x16_kernel<T, false, 512, 4>, C);
   if (e != cudaSuccess) return e;
 
   TcArgs A;
   A.L = L, A.S = P.S, A.xscale = scales, A.y = c.y, A.part = reinterpret_cast<float *>(scratch + P.o_part), A.cnt = cnt;
   A.status = status, A.ldy = c.ldy, A.m = c.m, A.bn = P.bn, A.hn = P.hn, A.tok_blocks = P.tok_blocks, A.row_blocks = P.row_blocks;
-  A.min_run = P.min_run, A.n = c.n, A.n_act = c.n_act, A.xcap = c.xcap, A.ycap = c.ycap, A.once = P.tok_blocks == 1, A.counts = c.counts;
-  if (c.n == 1 && !c.counts) return P.cg == 1 ? launch_main<T, 1, 1>(P, A, x16, c, s) : launch_main<T, 2, 1>(P, A, x16, c, s);
+  A.cs = P.cs, A.min_run = P.min_run, A.n = c.n, A.n_act = c.n_act, A.xcap = c.xcap, A.ycap = c.ycap, A.once = P.tok_blocks == 1, A.counts = c.counts;
+  if (c.n == 1 && !c.counts) {
+    if constexpr (beside_of(T))
+      if (beside) return P.cg == 1 ? launch_main<T, 1, 1, 72>(P, A, x16, c, s) : launch_main<T, 2, 1, 72>(P, A, x16, c, s);
+    return P.cg == 1 ? launch_main<T, 1, 1>(P, A, x16, c, s) : launch_main<T, 2, 1>(P, A, x16, c, s);
+  }
   return P.cg == 1 ? launch_main<T, 1, QK_MAX_GROUPS>(P, A, x16, c, s) : launch_main<T, 2, QK_MAX_GROUPS>(P, A, x16, c, s);
 }
 

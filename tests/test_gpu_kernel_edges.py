@@ -1,0 +1,148 @@
+"""GPU kernels at the sizes where their tiling can go wrong: remainders of every tile, the smallest
+call, both sides of each dispatch rule.  The reference is the f64 product of the oracle's dequantised
+weights.
+
+Bounds, per output (a: largest |w| of the 32-column block, x: the activation, sums over a row):
+  * fp16 operands: a term carries at most four independent roundings to 11 bits (the scale, the
+    minimum, the weight, the activation), each uniform within 2^-11 of its value, so the error of a sum
+    has sigma <= 2^-11 sqrt(4 / 3) sqrt(sum a^2 x^2); 7 sigma.
+  * f32-grade sums: block sums are exact, the activation lies on a 254^3 grid of its block's largest
+    value, and the f32 additions over two terms per block each round within 2^-24:
+    sigma <= 2^-23 (1 + sqrt(2 K / 32)) sqrt(sum a^2 xmax^2); 7 sigma.
+"""
+import numpy as np
+import pytest
+
+import oracle_lib as O
+from oxillama_b200 import synth as S
+
+pytestmark = pytest.mark.gpu
+
+TC_TYPES = [S.Q4_K, S.Q8_0, S.Q4_0, S.Q6_K, S.IQ4_XS]
+
+
+def block_max(a):
+    """|a| replaced by the largest of its 32-column block."""
+    pad = -a.shape[1] % 32
+    b = np.pad(np.abs(a), ((0, 0), (0, pad))).reshape(a.shape[0], -1, 32).max(axis=2)
+    return np.repeat(b, 32, axis=1)[:, : a.shape[1]].astype(np.float64)
+
+
+def assert_product(y, x, wd, half):
+    import torch
+    xd, w = torch.from_numpy(x).cuda().double(), torch.from_numpy(wd).cuda().double()
+    ref = (xd @ w.T).cpu().numpy()
+    a = torch.from_numpy(block_max(wd) ** 2).cuda()
+    xx = x.astype(np.float64) if half else block_max(x)
+    s = np.sqrt((torch.from_numpy(xx ** 2).cuda() @ a.T).cpu().numpy())
+    sigma = 2.0 ** -11 * np.sqrt(4 / 3) if half else 2.0 ** -23 * (1 + np.sqrt(2 * x.shape[1] / 32))
+    assert np.all(np.isfinite(y))
+    assert np.all(np.abs(y - ref) <= 7 * sigma * s + 1e-30), float((np.abs(y - ref) / (sigma * s + 1e-30)).max())
+
+
+def device_product(t, w, x, rows, cols, m):
+    import torch
+    from oxillama_b200.device import DeviceWeights, check_device_status
+    dw = DeviceWeights(t, w, rows, cols)
+    y = torch.full((m, rows), float("nan"), device="cuda")
+    xd = torch.from_numpy(x).cuda()
+    if m == 1:
+        dw.gemv(xd, y)
+    else:
+        dw.gemm(xd, y, m)
+    check_device_status()
+    dw.free()
+    return y.cpu().numpy()
+
+
+# Rows around the 128- and 256-row tiles, columns around super-blocks, tokens around the tile widths
+# (16 .. 64 in one CTA, up to 256 in a pair, several token blocks); K split over many CTAs (128 x 8192),
+# over few (2048 rows), a tile with both accumulator halves of unequal width (129, 300 tokens).
+@pytest.mark.parametrize("rows,cols,m", [(1, 256, 5), (127, 512, 16), (129, 768, 17), (257, 2048, 64), (128, 8192, 65), (300, 1280, 128),
+                                         (2048, 1024, 129), (513, 2304, 257), (640, 512, 300), (384, 256, 700)])
+@pytest.mark.parametrize("t", TC_TYPES)
+def test_tensor_core_matmul_edges(t, rows, cols, m):
+    if t in (S.Q8_0, S.Q4_0):
+        cols += 32 * (m % 7)  # a last super-block that is not whole
+    w, x = S.gen_weight(t, rows, cols, seed=m), S.gen_acts(m, cols, seed=m)
+    assert_product(device_product(t, w, x, rows, cols, m), x, O.dequant_matrix(t, w, rows, cols), True)
+
+
+# One to five rows (five: the tensor cores, or chunks of rows for the formats without them); fewer rows
+# than a chunk, a ragged last chunk, several 2048-column tiles with a short last one, fewer chunks than SMs and more.
+@pytest.mark.parametrize("rows,cols", [(1, 256), (9, 2048), (1190, 2304), (37, 14336), (5003, 512)])
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("t", TC_TYPES + [S.Q5_K, S.Q3_K, S.Q2_K])
+def test_decode_kernel_edges(t, m, rows, cols):
+    w, x = S.gen_weight(t, rows, cols, seed=rows + m), S.gen_acts(m, cols, seed=rows + m)
+    # (more than one row of 14336 columns may not fit the shared memory beside the tiles: tensor cores)
+    half = t in TC_TYPES and (m > (2 if t == S.Q6_K else 4) or (m > 1 and cols > 8192))
+    assert_product(device_product(t, w, x, rows, cols, m), x, O.dequant_matrix(t, w, rows, cols), half)
+
+
+# Gate and up in one launch (up to four rows), as two groups of one matmul with silu(g) * u in the
+# conversion (more), and one after the other (different formats).
+@pytest.mark.parametrize("tgu,td,hidden,inter", [(S.Q4_0, S.Q8_0, 544, 1056), (S.Q8_0, S.Q4_0, 2080, 320), (S.IQ4_XS, S.Q4_K, 256, 2560),
+                                                 (S.Q5_K, S.Q6_K, 2304, 512), (S.Q3_K, S.Q4_K, 512, 768), (S.Q2_K, S.Q2_K, 768, 256)])
+@pytest.mark.parametrize("m", [1, 2, 4, 5, 70])
+def test_ffn_edges(tgu, td, hidden, inter, m):
+    import torch
+    from oxillama_b200.device import DeviceWeights, check_device_status, ffn
+    ws = [S.gen_weight(q, r, c, seed=71, stream=i, d_range=(1e-3, 3e-3)) for i, (q, r, c) in
+          enumerate([(tgu, inter, hidden), (tgu, inter, hidden), (td, hidden, inter)])]
+    x = S.gen_acts(m, hidden, seed=71) * np.float32(0.25)
+    st, ref = O.ffn(tgu, ws[0], ws[1], td, ws[2], x, m, hidden, inter, hidden)
+    assert st == 0
+    dw = [DeviceWeights(tgu, ws[0], inter, hidden), DeviceWeights(tgu, ws[1], inter, hidden), DeviceWeights(td, ws[2], hidden, inter)]
+    y = torch.full((m, hidden), float("nan"), device="cuda")
+    ffn(*dw, torch.from_numpy(x).cuda(), y, m)
+    check_device_status()
+    half = any(q in TC_TYPES and m > (2 if q == S.Q6_K else 4) for q in (tgu, td))
+    # three chained products: each within 1e-3 of its largest value on fp16 operands, within 2e-5 in f32
+    assert np.abs(y.cpu().numpy() - ref).max() <= (3e-3 if half else 6e-5) * np.abs(ref).max()
+    for d in dw:
+        d.free()
+
+
+# Up to 16 tokens: every expert that is hit, on the decode kernels up to four tokens and on the tensor
+# cores beside them above; one expert takes all tokens, another none; also a shard that starts inside.
+@pytest.mark.parametrize("t", [S.Q4_K, S.Q8_0, S.Q6_K, S.IQ4_XS])
+@pytest.mark.parametrize("tokens,top_k", [(1, 1), (1, 3), (2, 2), (4, 2), (5, 1), (9, 3), (16, 2)])
+def test_moe_few_tokens(t, tokens, top_k):
+    import torch
+    from oxillama_b200 import moe
+    from oxillama_b200.device import check_device_status
+    hidden, inter, n = 512, 2304, 6
+    w = [[S.gen_weight(t, r, c, seed=81, stream=3 * e + k, d_range=(1e-3, 3e-3)) for e in range(n)]
+         for k, (r, c) in enumerate([(inter, hidden), (inter, hidden), (hidden, inter)])]
+    dq = [np.stack([O.dequant_matrix(t, a, r, c) for a in ws]) for ws, (r, c) in zip(w, [(inter, hidden), (inter, hidden), (hidden, inter)])]
+    x = S.gen_acts(tokens, hidden, seed=82) * np.float32(0.25)
+    logits = S.gen_acts(tokens, n, seed=83)
+    logits[:, 5], logits[:, 1] = -30.0, logits[:, 1] + 6.0
+    for b, e in ((0, n), (1, 4)):
+        ids, wts = O.moe_route(logits, top_k)
+        ref = np.zeros((tokens, hidden))
+        for i in range(tokens):
+            for s in range(top_k):
+                if b <= ids[i, s] < e:
+                    g, u, d = (q[ids[i, s]].astype(np.float64) for q in dq)
+                    hg = g @ x[i]
+                    ref[i] += wts[i, s] * (d @ (hg / (1 + np.exp(-hg)) * (u @ x[i])))
+        ex = moe.MoeExperts(t, w[0][b:e], w[1][b:e], w[2][b:e], hidden, inter, n, expert_begin=b)
+        y = torch.full((tokens, hidden), float("nan"), device="cuda")
+        ex.forward(torch.from_numpy(logits).cuda(), torch.from_numpy(x).cuda(), y, top_k)
+        check_device_status()
+        ex.free()
+        half = tokens > (2 if t == S.Q6_K else 4)  # an expert may then have more rows than the decode kernels take
+        assert np.abs(y.cpu().numpy() - ref).max() <= (3e-3 if half else 6e-5) * np.abs(ref).max()
+
+
+# Host buffers: x and y each go through a staging buffer of 256 KB or are copied, on both sides of it.
+@pytest.mark.parametrize("rows,cols,m", [(1, 256, 1), (14336, 512, 4), (16384, 512, 4), (16385, 512, 4), (64, 8192, 8), (64, 8448, 8),
+                                         (4096, 4096, 16), (4104, 4096, 17)])
+def test_host_call_around_the_staging_size(rows, cols, m):
+    from oxillama_b200.kernels import KernelDispatcher, QuantTensor
+    w, x = S.gen_weight(S.Q4_K, rows, cols, seed=91), S.gen_acts(m, cols, seed=91)
+    y = np.full((m, rows), np.nan, np.float32)
+    KernelDispatcher().get_kernel(S.Q4_K).gemm(QuantTensor(w, (rows, cols), S.Q4_K), x, y, m, rows, cols)
+    assert_product(y, x, O.dequant_matrix(S.Q4_K, w, rows, cols), m > 4)

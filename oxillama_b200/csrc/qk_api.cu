@@ -147,6 +147,7 @@ extern "C" int qk_shutdown(qk_ctx *c) {
   if (c->scratch) cudaFree(c->scratch);
   if (c->moe) cudaFree(c->moe);
   if (c->ffn) cudaFree(c->ffn);
+  if (c->up) cudaFree(c->up);
   cudaStreamDestroy(c->stream);
   delete c;
   return QK_OK;
@@ -202,18 +203,33 @@ static int upload_impl(qk_ctx *c, int type, const uint8_t *w, size_t n_cols, siz
     free_weights(h);
     return QK_CUDA_ERROR;
   }
-  uint8_t *raw = nullptr;
+  // The GGUF bytes pass through the context's upload buffer, whole 8-row chunks at a time (a device
+  // allocation and a release per call cost more than the repacking, and now and then many milliseconds);
+  // only rows of which it does not hold eight get a buffer of their own.
   int st = QK_OK;
+  uint8_t *raw = nullptr;
   do {
-    if ((e = cudaMemsetAsync(h->dev, 0, tiled, c->stream)) != cudaSuccess) break;
+    // every byte of a whole chunk is written by the repacking: clear only one with rows missing
+    const uint64_t whole = h->L.rows / QK_TILE_ROWS * h->L.chunk_bytes;
+    if (whole < tiled && (e = cudaMemsetAsync(h->dev + whole, 0, tiled - whole, c->stream)) != cudaSuccess) break;
     if (h->algo_bytes == 0) break;
-    if ((e = cudaMalloc(&raw, h->algo_bytes)) != cudaSuccess) break;
-    if ((e = cudaMemcpyAsync(raw, w + row_begin * row_bytes, h->algo_bytes, cudaMemcpyHostToDevice,
-                             c->stream)) != cudaSuccess)
-      break;
-    if ((e = qk_launch_repack(h->L, raw, h->dev, c->stream)) != cudaSuccess) break;
+    size_t step = QK_UPLOAD_STAGE / (QK_TILE_ROWS * row_bytes) * QK_TILE_ROWS;
+    if (step && !c->up && (e = cudaMalloc(&c->up, QK_UPLOAD_STAGE)) != cudaSuccess) break;
+    if (!step) {
+      step = QK_TILE_ROWS;
+      if ((e = cudaMalloc(&raw, step * row_bytes)) != cudaSuccess) break;
+    }
+    uint8_t *buf = raw ? raw : c->up;
+    for (size_t r = 0; r < h->L.rows && e == cudaSuccess; r += step) {
+      QkLayout part;
+      const size_t n = h->L.rows - r < step ? h->L.rows - r : step;
+      qk_make_layout(type, n, n_cols, &part);
+      e = cudaMemcpyAsync(buf, w + (row_begin + r) * row_bytes, n * row_bytes, cudaMemcpyHostToDevice, c->stream);
+      if (e == cudaSuccess) e = qk_launch_repack(part, buf, h->dev + r / QK_TILE_ROWS * h->L.chunk_bytes, c->stream);
+    }
   } while (0);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  else cudaStreamSynchronize(c->stream);
   if (raw) cudaFree(raw);
   if (e != cudaSuccess) {
     c->err = std::string("weights upload: ") + cudaGetErrorString(e);

@@ -502,6 +502,17 @@ __device__ __forceinline__ float silu_mul(float g, float u) {
   const float sg = __fdiv_rn(1.f, __fadd_rn(1.f, expf(-g)));
   return __fmul_rn(__fmul_rn(g, sg), u);
 }
+// Columns ka .. + 3 and kb .. + 3 of conv_load in the order in which they land at positions 8 c ..
+template <int T>
+__device__ __forceinline__ void conv_order(const float (&a)[4], const float (&b)[4], float (&v)[8]) {
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    uint32_t e;  // which of the eight values lands at position j
+    if (T == QK_T_Q4_K) e = (j & 4) + ((j & 3) == 1 ? 2 : (j & 3) == 2 ? 1 : (j & 3));
+    else e = WFmt<T>::src((uint32_t)j);
+    v[j] = e < 4 ? a[e & 3] : b[e & 3];
+  }
+}
 // The eight activations of positions 8 c .. 8 c + 7.
 template <int T, bool GLU>
 __device__ __forceinline__ void conv_load(const float *__restrict__ x, const float *__restrict__ x2, uint32_t c,
@@ -525,13 +536,7 @@ __device__ __forceinline__ void conv_load(const float *__restrict__ x, const flo
     }
   };
   quad(ka, a), quad(kb, b);
-#pragma unroll
-  for (int j = 0; j < 8; j++) {
-    uint32_t e;  // which of the eight loaded values lands at position j
-    if (T == QK_T_Q4_K) e = (j & 4) + ((j & 3) == 1 ? 2 : (j & 3) == 2 ? 1 : (j & 3));
-    else e = WFmt<T>::src((uint32_t)j);
-    v[j] = e < 4 ? a[e & 3] : b[e & 3];
-  }
+  conv_order<T>(a, b, v);
 }
 
 __device__ __forceinline__ float conv_scale(float amax) {
@@ -600,6 +605,56 @@ __global__ void __launch_bounds__(CT, CT == 256 ? 6 : 1) qk_x16_kernel(const Con
     float w[8];
     conv_load<T, GLU>(xr, ur, c, A.cols, vec, w);
     conv_store(orow, c, w, inv);
+  }
+}
+
+// silu(x) * x2 rows through shared memory: 512 threads of 40 registers and a row of 14336 columns leave room
+// for three CTAs on an SM, where the form above holds one (78 registers) that loads, computes and stores in
+// turn.  Up to one row per SM 1024 threads share it.  14336 columns by 512 rows: 27 -> 9 us.
+template <int T, int CT>
+__global__ void __launch_bounds__(CT, CT == 512 ? 3 : 1) qk_glu16_kernel(const ConvArgs A) {
+  extern __shared__ __align__(16) float glu_row[];
+  __shared__ float red[CT / 32];
+  pdl_launch_dependents();
+  pdl_wait();
+  if (blockIdx.x == 0)
+    for (uint32_t i = threadIdx.x; i < A.n_zero; i += CT) A.zero[i] = 0u;
+  const uint32_t t = blockIdx.x;
+  if (A.counts && t % A.cap >= (uint32_t)A.counts[t / A.cap]) return;  // rows past the live ones
+  const float *xr = A.x + (uint64_t)t * A.cols, *ur = A.x2 + (uint64_t)t * A.cols;
+  const bool vec = (A.cols & 3u) == 0 && (((uintptr_t)xr | (uintptr_t)ur) & 15u) == 0;
+  float amax = 0.f;
+#pragma unroll 2
+  for (uint32_t k = threadIdx.x * 4; k < A.Kp; k += CT * 4) {
+    float4 g = make_float4(0.f, 0.f, 0.f, 0.f), u = g;
+    if (vec && k < A.cols) {
+      g = __ldg(reinterpret_cast<const float4 *>(xr + k)), u = __ldg(reinterpret_cast<const float4 *>(ur + k));
+    } else {
+      if (k < A.cols) g.x = __ldg(xr + k), u.x = __ldg(ur + k);
+      if (k + 1 < A.cols) g.y = __ldg(xr + k + 1), u.y = __ldg(ur + k + 1);
+      if (k + 2 < A.cols) g.z = __ldg(xr + k + 2), u.z = __ldg(ur + k + 2);
+      if (k + 3 < A.cols) g.w = __ldg(xr + k + 3), u.w = __ldg(ur + k + 3);
+    }
+    const float4 h = make_float4(silu_mul(g.x, u.x), silu_mul(g.y, u.y), silu_mul(g.z, u.z), silu_mul(g.w, u.w));
+    amax = fmaxf(fmaxf(fmaxf(amax, fabsf(h.x)), fmaxf(fabsf(h.y), fabsf(h.z))), fabsf(h.w));
+    *reinterpret_cast<float4 *>(glu_row + k) = h;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
+  __syncthreads();
+  amax = red[threadIdx.x % (CT / 32)];
+#pragma unroll
+  for (int o = CT / 64; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  const float scale = conv_scale(amax), inv = 1.f / scale;  // a power of two: exact
+  if (threadIdx.x == 0) A.scales[t] = scale;
+  for (uint32_t c = threadIdx.x; c < A.Kp / 8; c += CT) {
+    const uint32_t ka = T == QK_T_Q4_K ? (c >> 3) * 64 + (c & 7u) * 4 : c * 8, kb = T == QK_T_Q4_K ? ka + 32 : ka + 4;
+    const float4 fa = *reinterpret_cast<const float4 *>(glu_row + ka), fb = *reinterpret_cast<const float4 *>(glu_row + kb);
+    const float a[4] = {fa.x, fa.y, fa.z, fa.w}, b[4] = {fb.x, fb.y, fb.z, fb.w};
+    float v[8];
+    conv_order<T>(a, b, v);
+    conv_store(A.out + (uint64_t)t * A.Kp, c, v, inv);
   }
 }
 
@@ -1099,6 +1154,7 @@ __global__ void __maxnreg__(REGS)
 }
 
 // ---------------------------------------------------------------- host side
+constexpr uint32_t GLU_SMEM = 110u * 1024u;    // two CTAs on an SM at least
 constexpr uint32_t SMEM_BUDGET = 225u * 1024u;  // leaves room for a CTA of the conversion
 
 struct TcPlan {
@@ -1159,8 +1215,22 @@ cudaError_t launch_fmt(const QkTcCall &c, unsigned *status, unsigned char *scrat
   cudaLaunchConfig_t c0 = {};
   c0.gridDim = dim3(c.counts || c.n_act > 1 ? c.n_act * c.xcap : c.m), c0.blockDim = dim3(beside ? 256 : 512), c0.stream = s, c0.attrs = &at, c0.numAttrs = 1;
   cudaError_t e;
-  if (beside) e = c.x2 ? cudaLaunchKernelEx(&c0, qk_x16_kernel<T, true, 256, 2>, C) : cudaLaunchKernelEx(&c0, qk_x16_kernel<T, false, 256, 2>, C);
-  else e = c.x2 ? cudaLaunchKernelEx(&c0, qk_x16_kernel<T, true, 512, 4>, C) : cudaLaunchKernelEx(&c0, qk_x16_kernel<T, false, 512, 4>, C);
+  if (c.x2 && !c.lists && Kp * 4 <= GLU_SMEM) {
+    static QkPerDevice attr_set;
+    if (attr_set.first()) {
+      e = cudaFuncSetAttribute(qk_glu16_kernel<T, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GLU_SMEM);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(qk_glu16_kernel<T, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GLU_SMEM);
+      if (e != cudaSuccess) return attr_set.reset(), e;
+    }
+    const bool few = !c.counts && c0.gridDim.x <= (uint32_t)sm_count;
+    c0.blockDim = dim3(few ? 1024 : 512), c0.dynamicSmemBytes = Kp * 4;
+    e = few ? cudaLaunchKernelEx(&c0, qk_glu16_kernel<T, 1024>, C) : cudaLaunchKernelEx(&c0, qk_glu16_kernel<T, 512>, C);
+  } else if (c.x2) {
+    c0.blockDim = dim3(512);
+    e = cudaLaunchKernelEx(&c0, qk_x16_kernel<T, true, 512, 4>, C);
+  } else {
+    e = beside ? cudaLaunchKernelEx(&c0, qk_x16_kernel<T, false, 256, 2>, C) : cudaLaunchKernelEx(&c0, qk_x16_kernel<T, false, 512, 4>, C);
+  }
   if (e != cudaSuccess) return e;
 
   TcArgs A;

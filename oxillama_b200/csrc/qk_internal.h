@@ -21,6 +21,8 @@ struct qk_weights {
 // or to pageable memory costs more than the memcpy (larger ones are left to the driver, which overlaps).
 #define QK_HOST_STAGE ((size_t)256 << 10)
 
+#define QK_UPLOAD_STAGE ((size_t)32 << 20)
+
 struct qk_ctx {
   int device;
   int sm_count;
@@ -42,6 +44,8 @@ struct qk_ctx {
   // pinned, device-mapped staging of those calls' activations and results (QK_HOST_STAGE bytes each,
   // made by the first such call)
   unsigned char *hx = nullptr, *hx_dev = nullptr, *hy = nullptr, *hy_dev = nullptr;
+  // device buffer through which weights are uploaded (QK_UPLOAD_STAGE bytes, made by the first upload)
+  uint8_t *up = nullptr;
   // weight cache for the host-pointer entry points
   typedef std::tuple<const void *, size_t, int, size_t, size_t, uint64_t> Key;
   std::map<Key, qk_weights *> cache;

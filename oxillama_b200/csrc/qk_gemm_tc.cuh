@@ -29,11 +29,13 @@
 //   warps 4-19  two sets of eight warps that take the super-blocks in turn, one thread per row and
 //               128 columns
 //   warps 20-23 epilogue: accumulator -> y (or the workspace of a split tile)
-// Tensor memory: two accumulator halves of up to 128 tokens in columns 0-255 and the expanded
-// weights of two super-blocks behind them; up to 64 tokens, halves of 64 in columns 0-127 and three
-// super-blocks.  A tile of up to 128 tokens uses one half, the halves alternating from tile to tile;
-// a wider tile uses both.  An SM stores 32 bytes a cycle, so writing out a half takes the time of
-// about 32 of its MMAs: at the ends of a wide tile the two super-blocks there are issued first half
+// Tensor memory, 512 columns: tiles of more than 128 tokens have two accumulator halves of up to 128
+// and two super-blocks of expanded weights; up to 128 tokens one accumulator and three super-blocks
+// (a second accumulator would only hide the writing out of one tile under the next one's MMAs, the third
+// super-block shortens every round of hand-overs: Q4_K 4096 x 4096 by 512 22.6 -> 21.6 us); up to 64 tokens two
+// accumulators of 64, alternating from tile to tile, and three super-blocks.  An SM stores 32 bytes a
+// cycle, so writing out a half takes the time of about 32 of its MMAs: at the ends of a wide tile the two
+// super-blocks there are issued first half
 // by first half, then second half by second half, so that one half is written out under the MMAs of
 // the other and the tensor pipe does not wait.
 //
@@ -737,9 +739,9 @@ __global__ void __maxnreg__(REGS)
   const uint32_t sbase = smem_u32(smem);
   const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t rank = CG == 1 ? 0u : blockIdx.x & 1u;  // in the pair; rank 0 issues the MMAs of both
-  // Tensor memory: two accumulator halves, then na buffers of 128 columns for the expanded weights.
-  const bool narrow = A.hn <= 64;
-  const uint32_t na = narrow ? 3u : 2u, d_step = narrow ? 64u : 128u, a_col = 2 * d_step;
+  // Tensor memory (see the top): accumulators, then na buffers of 128 columns for the expanded weights.
+  const bool narrow = A.hn <= 64, both = A.bn > 128;  // (both: a tile owns two accumulator halves)
+  const uint32_t na = both ? 2u : 3u, d_step = narrow ? 64u : 128u, a_col = both ? 256u : 128u, alt = narrow ? 1u : 0u;
 
   pdl_launch_dependents();
   if (threadIdx.x == 0) {
@@ -806,7 +808,6 @@ __global__ void __maxnreg__(REGS)
     q.n = left >= A.bn ? A.bn : ((left + 15u) & ~15u);
     return q;
   };
-  const bool both = A.bn > 128;  // a tile owns both accumulator halves
   // Token rows that an activation box brings: each CTA of a pair loads half of the n tokens.
   const uint32_t hq = A.hn / (4 * CG);
   auto box_rows = [&](uint32_t n) { return NG > 1 ? (n / CG + hq - 1) / hq * hq : A.hn / CG; };
@@ -866,7 +867,7 @@ __global__ void __maxnreg__(REGS)
       uint32_t begun = 0;      // halves whose accumulator this segment has taken over
       uint32_t ab1 = 0;        // (two super-blocks at a time) buffers are walked again under the second half
       const bool ok = walk_segment(s0, s1, wide, [&](uint32_t, uint32_t h, uint32_t k, bool last, bool end) {
-        const uint32_t n = h ? q.n - A.hn : wide ? A.hn : q.n, dh = both ? h : i & 1u;
+        const uint32_t n = h ? q.n - A.hn : wide ? A.hn : q.n, dh = both ? h : i & alt;
         const uint32_t step16 = box_rows(n) * 8u;  // a step of the activation stage, in units of 16 bytes
         const uint32_t idesc = (1u << 4) | ((n >> 3) << 17) | ((CG * BM >> 4) << 24), d = tmem + dh * d_step;
         uint32_t acc = 1u;
@@ -996,7 +997,7 @@ __global__ void __maxnreg__(REGS)
       const uint32_t slot = A.bn * BM;
       float *mine = A.part + (blockIdx.x * 2 + (i == sc.whole ? 0u : 1u)) * slot + r;
       for (uint32_t h = 0; h < (wide ? 2u : 1u); h++) {
-        const uint32_t dh = both ? h : i & 1u, hoff = h * A.hn;  // first token of the half inside the tile
+        const uint32_t dh = both ? h : i & alt, hoff = h * A.hn;  // first token of the half inside the tile
         const uint32_t n = h ? q.n - A.hn : wide ? A.hn : q.n;
         const uint32_t live = min(q.live - q.t0 - hoff, n);      // tokens to write
         if (!split) {

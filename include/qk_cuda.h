@@ -51,7 +51,7 @@ typedef enum qk_status {
 #define QK_TYPE_Q4_0 2
 #define QK_TYPE_Q8_0 8
 #define QK_TYPE_Q4_K 12
-#define QK_TYPE_Q5_K 13 /* Q5_K, Q2_K, Q3_K, Q8_K: generic kernels only so far (exact, not tuned) */
+#define QK_TYPE_Q5_K 13 /* Q5_K, Q2_K, Q3_K: decode kernels, larger batches in pieces; Q8_K: generic kernels only */
 #define QK_TYPE_Q2_K 10
 #define QK_TYPE_Q3_K 11
 #define QK_TYPE_Q8_K 15
@@ -184,10 +184,12 @@ int qk_gemm_dev(qk_ctx *ctx, const qk_weights *h, const float *x_dev, float *y_d
  * feed_forward does it as three QuantLinear::forward calls and swiglu_inplace,
  * crates/oxillama-arch/src/llama/model.rs:281-310, crates/oxillama-arch/src/common/swiglu.rs:15-21):
  *   y_dev[i][:] = down( silu(gate x_i) * (up x_i) ),  i < m,  x_dev [m x hidden], y_dev [m x down rows].
- * gate and up are [inter x hidden], down is [rows x inter].  For Q4_K gate / up and m <= 4 the
- * two projections run as one launch over both matrices (they share the split activations) and
- * silu(g) * u is formed where the dot products are reduced, so neither g nor u is ever
- * written out; otherwise the three matmuls and an element-wise pass are enqueued in turn.
+ * gate and up are [inter x hidden], down is [rows x inter].  For gate and up of one format (any
+ * but Q6_K) and rows that fit its decode kernel (m <= 4 at most) the two projections run as one
+ * launch over both matrices (they share the split activations) and silu(g) * u is formed where the
+ * dot products are reduced, so neither g nor u is ever written out; larger batches of one format
+ * run gate and up as one grouped matmul and form silu(g) * u in the conversion that precedes the
+ * down projection; otherwise the three matmuls and an element-wise pass are enqueued in turn.
  * Keeps its own scratch for the hidden activations, grown on first use. */
 int qk_ffn_dev(qk_ctx *ctx, const qk_weights *gate, const qk_weights *up, const qk_weights *down,
                const float *x_dev, float *y_dev, size_t m, void *stream);
@@ -217,11 +219,11 @@ int qk_moe_route_dev(qk_ctx *ctx, const float *logits_dev, size_t tokens, size_t
  * gate[e], up[e] are [inter x hidden] shards, down[e] is [hidden x inter].  With every
  * expert local this is MoeFfn::forward given the router's logits; an expert-sharded
  * layer sums the y of its ranks.  logits_dev is [tokens x n_exp], x_dev [tokens x hidden].
- * More than 16 tokens, at most 16 local experts of one format: every projection is one
- * grouped matmul launch over all local experts, the per-expert token counts stay on the
- * device and the call does not synchronise (a fixed sequence of launches on `stream`).
- * Otherwise (decode-sized calls) the experts run one after the other on the decode kernels
- * and the call synchronises `stream` once to read the counts that size them.  The context
+ * At most 16 local experts, equal formats: the call does not synchronise (a fixed sequence of
+ * launches on `stream`; the token counts stay on the device).  More than 16 tokens take one grouped
+ * matmul launch per projection, fewer one decode-kernel launch per projection over all experts
+ * that are hit.  Otherwise (mixed or other formats, more local experts, few tokens) the experts
+ * run one after the other and the call synchronises `stream` once to read the counts that size them.  The context
  * keeps the device scratch, grown (with a device synchronise) on first use of a larger size. */
 int qk_moe_ffn_dev(qk_ctx *ctx, const qk_weights *const *gate, const qk_weights *const *up,
                    const qk_weights *const *down, size_t n_local, size_t expert_begin, size_t n_exp,

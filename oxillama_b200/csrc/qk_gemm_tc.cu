@@ -117,7 +117,7 @@ bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
         if (k && bn < 32) break;
         if (cg == 1 && bn > 64) continue;
         const uint32_t tbr = (c.m + bn - 1) / bn, own = bn / cg;
-        const float sb = fmaxf(expand + (own > 16 ? 5.f * (own - 16) : 0.f), cg == 2 ? (1060.f + 6.1f * bn) * (bn <= 128 ? 0.82f : 1.f) : 0.f), out = bn * 19.f;
+        const float sb = fmaxf(expand + (own > 16 ? 5.f * (own - 16) : 0.f), cg == 2 ? (1060.f + 6.1f * bn) * (bn <= 128 ? 0.94f : 1.f) : 0.f), out = bn * 19.f;
         const uint64_t tiles = (uint64_t)c.n * rbs * tbr;
         for (uint32_t run = 1; run <= 16; run <<= 1) {
           const uint32_t R = (uint32_t)(tiles % units), total = R * p.nsb;

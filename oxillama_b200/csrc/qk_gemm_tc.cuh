@@ -43,7 +43,10 @@
 // equal runs of super-blocks over all CTAs (pairs).  A tile cut this way has several contributors: each
 // leaves its f32 partial in a workspace and counts itself in, and whoever comes last adds the
 // partials in a fixed order (so the result does not depend on who that is: the same bits on every
-// run) and writes y.  Nobody waits for another CTA.
+// run) and writes y.  Nobody waits for another CTA.  Where the tiles are so few that each can have a
+// cluster of four or eight CTAs, its CTAs take one run each and store their partials straight into the
+// shared memory of the CTA that adds up the token (Q4_K 1024 x 4096 by 8 tokens: 8.3 -> 6.6 us; the fence,
+// the counter and the loads of the other way cost 4).
 //
 // The activations are converted to fp16 once per call by qk_x16_kernel, the columns of every
 // 64-group in the order in which the packed words yield their weights (both operands use the same

@@ -14,7 +14,7 @@ from __future__ import annotations
 import numpy as np
 
 Q4_0, Q8_0, Q4_K, Q6_K, IQ4_XS = 2, 8, 12, 14, 23
-Q5_K, Q2_K, Q3_K, Q8_K = 13, 10, 11, 15  # served by the generic kernels; not among the benchmark's formats
+Q5_K, Q2_K, Q3_K, Q8_K = 13, 10, 11, 15  # not among the benchmark's formats
 BLOCK_SIZE = {Q4_0: 32, Q8_0: 32, Q4_K: 256, Q6_K: 256, IQ4_XS: 256, Q5_K: 256, Q2_K: 256, Q3_K: 256, Q8_K: 256}
 BLOCK_BYTES = {Q4_0: 18, Q8_0: 34, Q4_K: 144, Q6_K: 210, IQ4_XS: 136, Q5_K: 176, Q2_K: 84, Q3_K: 110, Q8_K: 292}
 NAMES = {Q4_0: "Q4_0", Q8_0: "Q8_0", Q4_K: "Q4_K", Q6_K: "Q6_K", IQ4_XS: "IQ4_XS", Q5_K: "Q5_K", Q2_K: "Q2_K", Q3_K: "Q3_K",

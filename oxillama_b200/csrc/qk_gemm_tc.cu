@@ -51,8 +51,8 @@ static bool plan_smem(uint32_t hn, uint32_t cg, uint32_t cs, uint32_t w_stage, u
   s.pre = off, off += (QK_MAX_GROUPS + 1) * 4;
   off = (off + 15u) & ~15u;
   s.scales = off, off += 4 * 512 + 16;  // a copy of a half's token scales per epilogue warp, and one word
-  off = (off + 127u) & ~127u;
-  s.lut = off, off += lut;
+  if (off > LUT_OFF) return false;
+  off = LUT_OFF + lut;
   s.red = off, off += cs > 1 ? cs * ((hn + cs - 1) / cs) * BM * 4 : 0;  // the cluster's partial sums of this CTA's tokens
   off = (off + 1023u) & ~1023u;
   s.w_stage = w_stage, s.b_stage = (hn / cg) * 512u;  // this CTA's tokens, a super-block's four steps

@@ -539,10 +539,12 @@ extern "C" int qk_moe_ffn_dev(qk_ctx *c, const qk_weights *const *gate, const qk
   }
 
   // A handful of tokens: the experts with up to QK_MOE_DEC_ROWS rows on the decode kernels (f32-grade
-  // sums, as a plain matmul of that many rows), any others on the tensor cores beside them.
+  // sums, as a plain matmul of that many rows), any others on the tensor cores beside them.  Where K is so
+  // long that a job holds one row only (Q8_0 from 12032 columns), nine experts and up can make more jobs
+  // than the list takes: such a call goes expert by expert.
   const uint32_t rg = grouped ? qk_moe_dec_rows(gate[0]->L) : 0, rd = grouped ? qk_moe_dec_rows(down[0]->L) : 0;
   const uint32_t per_job = rg < rd ? rg : rd;
-  if (grouped && per_job) {
+  if (grouped && per_job && qk_moe_dec_jobs(slots, n_local, per_job) <= QK_MOE_JOBS) {
     const bool big_too = tokens > QK_MOE_DEC_ROWS;
     const size_t ig = qk_moe_dec_image_bytes(gate[0]->L), id = qk_moe_dec_image_bytes(down[0]->L);
     const size_t o_jobs = 0, o_ids = al(sizeof(QkMoeJobs)), o_wts = o_ids + al(slots * 4), o_big = o_wts + al(slots * 4);

@@ -85,7 +85,7 @@ __global__ void __launch_bounds__((MAX_CW + 2) * 32, 1) qk_gemv_moe_kernel(const
   const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int nstage = A.nstage, nslot = A.nslot;
   MoeSeg *segs = reinterpret_cast<MoeSeg *>(smem + A.seg);
-  volatile uint32_t *meta = reinterpret_cast<volatile uint32_t *>(smem + A.seg + 2 * QK_MOE_MAX * sizeof(MoeSeg));  // segments, chunks
+  volatile uint32_t *meta = reinterpret_cast<volatile uint32_t *>(smem + A.seg + QK_MOE_JOBS * sizeof(MoeSeg));  // segments, chunks
 
   if (A.early) pdl_launch_dependents();
   if (threadIdx.x == 0) {
@@ -313,7 +313,7 @@ struct PlanMoe {
 // The decode kernel's plan for `rows` activation rows; the run table goes behind the ring.
 inline bool make_plan_moe(const QkLayout &L, uint32_t rows, uint32_t xsb, PlanMoe *p) {
   if (!make_plan_mma(L, rows, &p->P, xsb)) return false;
-  const uint32_t table = 2 * QK_MOE_MAX * sizeof(MoeSeg) + 16;
+  const uint32_t table = QK_MOE_JOBS * sizeof(MoeSeg) + 16;
   // (the plan leaves 1 KB of the budget unused; the table takes a stage's place where it does not fit)
   while (p->P.total + table > 227u * 1024u) {
     const int unit = p->P.groups * (int)L.ktiles;

@@ -119,12 +119,18 @@ cudaError_t qk_launch_gemv_fast(const QkLayout &L, const uint8_t *tiled, const f
 #define QK_MOE_MAX 16       // most local experts
 #define QK_MOE_DEC_TOKENS 16  // most tokens of such a call
 #define QK_MOE_DEC_ROWS 4   // experts with more rows than this go to the tensor cores
+#define QK_MOE_JOBS 32      // most jobs: a lane of the warp that deals them out holds one
 struct QkMoeJobs {
   uint32_t n, pad[3];
   struct {
     uint32_t expert, rows, slot[2];  // slots = token * top_k + k
-  } job[2 * QK_MOE_MAX];
+  } job[QK_MOE_JOBS];
 };
+// Most jobs that `slots` routed rows over n_local experts can make (QK_MOE_JOBS at most is served).
+static inline size_t qk_moe_dec_jobs(size_t slots, size_t n_local, uint32_t rows_per_job) {
+  const size_t all = n_local * ((QK_MOE_DEC_ROWS + rows_per_job - 1) / rows_per_job);
+  return slots < all ? slots : all;
+}
 uint32_t qk_moe_dec_rows(const QkLayout &L);  // rows a job may have: 2, 1, or 0 where the format or shape is not served
 size_t qk_moe_dec_image_bytes(const QkLayout &L);  // scratch per split activation row
 // plan != null: the same launch also makes the plan (qk_moe_plan.cuh): ids / wts as qk_launch_moe_route,

@@ -137,6 +137,44 @@ def test_moe_few_tokens(t, tokens, top_k):
         assert np.abs(y.cpu().numpy() - ref).max() <= (3e-3 if half else 6e-5) * np.abs(ref).max()
 
 
+# Long rows: a job of the decode kernels holds one row where two split activation rows do not fit beside
+# the tiles, so 16 experts of four rows each make 64 of them; also nine experts at the edge of the job list.
+@pytest.mark.parametrize("n,tokens,top_k", [(16, 16, 4), (9, 11, 3), (16, 16, 2), (8, 8, 4)])
+def test_moe_few_tokens_long_rows(n, tokens, top_k):
+    import torch
+    from oxillama_b200 import moe
+    from oxillama_b200.device import check_device_status
+    t, hidden, inter = S.Q8_0, 256, 12288
+    shapes = [(inter, hidden), (inter, hidden), (hidden, inter)]
+    w = [[S.gen_weight(t, r, c, seed=85, stream=3 * e + k, d_range=(1e-3, 3e-3)) for e in range(2)] for k, (r, c) in enumerate(shapes)]
+    dq = [[torch.from_numpy(O.dequant_matrix(t, a, r, c)).cuda().double() for a in ws] for ws, (r, c) in zip(w, shapes)]
+    x = S.gen_acts(tokens, hidden, seed=86) * np.float32(0.25)
+    logits = S.gen_acts(tokens, n, seed=87) * np.float32(0.1)
+    for i in range(tokens):  # every expert gets its share of the rows
+        for k in range(top_k):
+            logits[i, (i + k * (n // top_k)) % n] += 5.0
+    ids, wts = O.moe_route(logits, top_k)
+    xd = torch.from_numpy(x).cuda()
+    ref = torch.zeros(tokens, hidden, dtype=torch.float64, device="cuda")
+    for i in range(tokens):
+        for s in range(top_k):
+            g, u, d = (q[ids[i, s] % 2] for q in dq)
+            hg = g @ xd[i].double()
+            ref[i] += float(wts[i, s]) * (d @ (hg / (1 + torch.exp(-hg)) * (u @ xd[i].double())))
+    ex = moe.MoeExperts(t, *[[ws[e % 2] for e in range(n)] for ws in w], hidden, inter, n)
+    lg = torch.from_numpy(logits).cuda()
+    ys = []
+    for xi in (torch.zeros_like(xd), xd):  # rows that were left out would show what the first call left
+        ys.append(torch.full((tokens, hidden), float("nan"), device="cuda"))
+        ex.forward(lg, xi, ys[-1], top_k)
+        check_device_status()
+    ex.free()
+    assert torch.all(ys[0] == 0)
+    # up to four rows of an expert: gate and up f32-grade; the down projection of several such rows may
+    # take fp16 operands (its K is long)
+    assert float((ys[1] - ref).abs().max()) <= 1e-3 * float(ref.abs().max())
+
+
 # Host buffers: x and y each go through a staging buffer of 256 KB or are copied, on both sides of it.
 @pytest.mark.parametrize("rows,cols,m", [(1, 256, 1), (14336, 512, 4), (16384, 512, 4), (16385, 512, 4), (64, 8192, 8), (64, 8448, 8),
                                          (4096, 4096, 16), (4104, 4096, 17)])

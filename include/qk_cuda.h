@@ -19,6 +19,10 @@
  *    columns past n_cols contribute nothing.
  *  - One context drives one GPU (one process per GPU); a context may be used
  *    from any thread, one call at a time.
+ *  - Entry points that take a stream return without waiting, and most keep split or converted
+ *    activations in scratch of the context between their kernels: issue those of one context on one
+ *    stream, or on streams ordered by events.  Calls that overlap on the GPU race on that scratch.
+ *    The host-pointer entry points have scratch of their own and may follow at any time.
  *  - There is no CPU fallback: without a usable CUDA device every compute
  *    entry point fails with QK_CUDA_ERROR.
  */

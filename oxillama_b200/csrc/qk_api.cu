@@ -115,14 +115,14 @@ extern "C" int qk_init(int device, qk_ctx **out) {
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaHostAlloc((void **)&sh, sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess ||
       cudaHostGetDevicePointer((void **)&c->status_dev, sh, 0) != cudaSuccess ||
-      cudaMalloc(&c->scratch, (size_t)1 << 20) != cudaSuccess) {
+      cudaMalloc(&c->scratch.p, QK_MIN_SCRATCH) != cudaSuccess) {
     if (sh) cudaFreeHost(sh);
     delete c;
     return QK_CUDA_ERROR;
   }
   *sh = 0;
   c->status_host = sh;
-  c->scratch_cap = (size_t)1 << 20;
+  c->scratch.cap = QK_MIN_SCRATCH;
   const char *fs = qk_knob("QK_FORCE_SIMPLE");
   c->force_simple = fs && fs[0] == '1';
   *out = c;
@@ -144,7 +144,8 @@ extern "C" int qk_shutdown(qk_ctx *c) {
   if (c->sb) cudaFree(c->sb);
   cudaFreeHost((void *)c->status_host);
   if (c->hx) cudaFreeHost(c->hx);
-  if (c->scratch) cudaFree(c->scratch);
+  if (c->scratch.p) cudaFree(c->scratch.p);
+  if (c->host_scratch.p) cudaFree(c->host_scratch.p);
   if (c->moe) cudaFree(c->moe);
   if (c->ffn) cudaFree(c->ffn);
   if (c->up) cudaFree(c->up);
@@ -347,24 +348,27 @@ extern "C" int qk_weights_cache_evict(qk_ctx *c, const uint8_t *w) {
 }
 
 // ------------------------------------------------------------ device entry points
-static int ensure_scratch(qk_ctx *c, size_t need) {
-  if (need <= c->scratch_cap) return QK_OK;
-  CK(c, cudaDeviceSynchronize());
-  cudaFree(c->scratch);
-  c->scratch = nullptr, c->scratch_cap = 0;
-  CK(c, cudaMalloc(&c->scratch, need + need / 4));
-  c->scratch_cap = need + need / 4;
+int qk_ensure_scratch(qk_ctx *c, QkScratch &sc, size_t need) {
+  if (need <= sc.cap) return QK_OK;
+  if (sc.p) {
+    CK(c, cudaDeviceSynchronize());
+    cudaFree(sc.p);
+    sc.p = nullptr, sc.cap = 0;
+  }
+  const size_t want = need + need / 4 > QK_MIN_SCRATCH ? need + need / 4 : QK_MIN_SCRATCH;
+  CK(c, cudaMalloc(&sc.p, want));
+  sc.cap = want;
   return QK_OK;
 }
 
-static int tc_call(qk_ctx *c, const QkTcCall &call, cudaStream_t s) {
-  int st = ensure_scratch(c, qk_gemm_tc_scratch_bytes(call, c->sm_count));
+static int tc_call(qk_ctx *c, QkScratch &sc, const QkTcCall &call, cudaStream_t s) {
+  int st = qk_ensure_scratch(c, sc, qk_gemm_tc_scratch_bytes(call, c->sm_count));
   if (st) return st;
-  CK(c, qk_launch_gemm_tc(call, c->status_dev, c->scratch, c->sm_count, s));
+  CK(c, qk_launch_gemm_tc(call, c->status_dev, sc.p, c->sm_count, s));
   return QK_OK;
 }
 
-static int gemm_dispatch(qk_ctx *c, const qk_weights *h, const float *x, float *y, size_t m,
+static int gemm_dispatch(qk_ctx *c, QkScratch &sc, const qk_weights *h, const float *x, float *y, size_t m,
                          size_t ldy, cudaStream_t s) {
   if (h->L.rows == 0 || m == 0) return QK_OK;
   if (h->L.cols == 0) {  // empty dot products
@@ -378,11 +382,11 @@ static int gemm_dispatch(qk_ctx *c, const qk_weights *h, const float *x, float *
     size_t step = m < QK_GEMV_MAX_M ? m : QK_GEMV_MAX_M;
     while (step > 1 && !qk_gemv_fast_supported(h->L, (uint32_t)step)) step--;
     if (step == m || !qk_gemm_tc_supported(h->L, 1)) {
-      int st = ensure_scratch(c, qk_gemv_fast_scratch_bytes(h->L, (uint32_t)step));
+      int st = qk_ensure_scratch(c, sc, qk_gemv_fast_scratch_bytes(h->L, (uint32_t)step));
       if (st) return st;
       for (size_t i = 0; i < m; i += step) {
         const uint32_t k = (uint32_t)(m - i < step ? m - i : step);
-        CK(c, qk_launch_gemv_fast(h->L, h->dev, x + i * h->L.cols, y + i * ldy, k, ldy, c->status_dev, c->scratch, c->sm_count, s));
+        CK(c, qk_launch_gemv_fast(h->L, h->dev, x + i * h->L.cols, y + i * ldy, k, ldy, c->status_dev, sc.p, c->sm_count, s));
       }
       return QK_OK;
     }
@@ -398,7 +402,7 @@ static int gemm_dispatch(qk_ctx *c, const qk_weights *h, const float *x, float *
     QkTcCall call = {};
     call.L = &h->L, call.maps[0] = h->tmap, call.n = call.n_act = 1;
     call.x = x, call.m = (uint32_t)m, call.y = y, call.ldy = ldy;
-    return tc_call(c, call, s);
+    return tc_call(c, sc, call, s);
   }
   CK(c, qk_launch_gemm_simple(h->L, h->dev, x, y, (uint32_t)m, ldy, s));
   return QK_OK;
@@ -408,7 +412,7 @@ extern "C" int qk_gemv_dev(qk_ctx *c, const qk_weights *h, const float *x_dev, f
                            void *stream) {
   if (!c || !h || !x_dev || !y_dev) return QK_INVALID_ARGUMENT;
   if (h->device != c->device) return QK_INVALID_ARGUMENT;
-  return gemm_dispatch(c, h, x_dev, y_dev, 1, h->L.rows, (cudaStream_t)stream);
+  return gemm_dispatch(c, c->scratch, h, x_dev, y_dev, 1, h->L.rows, (cudaStream_t)stream);
 }
 
 extern "C" int qk_gemm_dev(qk_ctx *c, const qk_weights *h, const float *x_dev, float *y_dev,
@@ -416,7 +420,7 @@ extern "C" int qk_gemm_dev(qk_ctx *c, const qk_weights *h, const float *x_dev, f
   if (!c || !h || !x_dev || !y_dev) return QK_INVALID_ARGUMENT;
   if (h->device != c->device) return QK_INVALID_ARGUMENT;
   if (ldy < h->L.rows) return QK_DIMENSION_MISMATCH;
-  return gemm_dispatch(c, h, x_dev, y_dev, m, ldy, (cudaStream_t)stream);
+  return gemm_dispatch(c, c->scratch, h, x_dev, y_dev, m, ldy, (cudaStream_t)stream);
 }
 
 extern "C" int qk_moe_route_dev(qk_ctx *c, const float *logits_dev, size_t tokens, size_t n_exp,
@@ -504,19 +508,19 @@ extern "C" int qk_moe_ffn_dev(qk_ctx *c, const qk_weights *const *gate, const qk
     if (one_launch)
       for (size_t e = 0; e < n_local; e++) gu.maps[n_local + e] = up[e]->tmap;
     gu.n = (uint32_t)(one_launch ? 2 * n_local : n_local);
-    int st = tc_call(c, gu, s);
+    int st = tc_call(c, c->scratch, gu, s);
     if (st) return st;
     if (!one_launch) {
       for (size_t e = 0; e < n_local; e++) gu.maps[e] = up[e]->tmap;
       gu.y = u;
-      if ((st = tc_call(c, gu, s))) return st;
+      if ((st = tc_call(c, c->scratch, gu, s))) return st;
     }
     // silu(g) * u is formed where the down projection's activations are converted
     QkTcCall dn = {};
     dn.L = &down[0]->L, dn.n = dn.n_act = (uint32_t)n_local, dn.counts = cnt, dn.m = (uint32_t)tokens, dn.expect = gu.expect;
     dn.xcap = dn.ycap = (uint32_t)cap, dn.x = g, dn.x2 = u, dn.y = o, dn.ldy = hidden;
     for (size_t e = 0; e < n_local; e++) dn.maps[e] = down[e]->tmap;
-    return tc_call(c, dn, s);
+    return tc_call(c, c->scratch, dn, s);
   };
 
   if (grouped && tokens > QK_MOE_DEC_TOKENS) {
@@ -601,12 +605,12 @@ extern "C" int qk_moe_ffn_dev(qk_ctx *c, const qk_weights *const *gate, const qk
     if (m == 0) continue;
     const int *list = lists + e * slots;
     CK(c, qk_launch_moe_gather(x_dev, list, (uint32_t)m, (uint32_t)top_k, (uint32_t)hidden, xe, s));
-    int st = gemm_dispatch(c, gate[e], xe, g, m, inter, s);
+    int st = gemm_dispatch(c, c->scratch, gate[e], xe, g, m, inter, s);
     if (st) return st;
-    st = gemm_dispatch(c, up[e], xe, u, m, inter, s);
+    st = gemm_dispatch(c, c->scratch, up[e], xe, u, m, inter, s);
     if (st) return st;
     CK(c, qk_launch_moe_silu_mul(g, u, (uint64_t)m * inter, s));
-    st = gemm_dispatch(c, down[e], u, o, m, hidden, s);
+    st = gemm_dispatch(c, c->scratch, down[e], u, o, m, hidden, s);
     if (st) return st;
     CK(c, qk_launch_moe_scatter(o, list, wts, (uint32_t)m, (uint32_t)top_k, (uint32_t)hidden, y_dev, s));
   }
@@ -638,9 +642,9 @@ extern "C" int qk_ffn_dev(qk_ctx *c, const qk_weights *gate, const qk_weights *u
   const bool fused = !c->force_simple && gate->L.type == up->L.type && hidden > 0 && inter > 0 && m <= QK_GEMV_MAX_M && qk_gemv_dual_supported(gate->L, (uint32_t)m);
   if (fused) {
     // gate and up in one launch (they share the split activations), silu(g) * u in its reducer
-    int st = ensure_scratch(c, qk_gemv_fast_scratch_bytes(gate->L, (uint32_t)m));
+    int st = qk_ensure_scratch(c, c->scratch, qk_gemv_fast_scratch_bytes(gate->L, (uint32_t)m));
     if (st) return st;
-    CK(c, qk_launch_gemv_dual(gate->L, gate->dev, up->dev, x_dev, h, (uint32_t)m, inter, c->status_dev, c->scratch,
+    CK(c, qk_launch_gemv_dual(gate->L, gate->dev, up->dev, x_dev, h, (uint32_t)m, inter, c->status_dev, c->scratch.p,
                               c->sm_count, s));
   } else if (!c->force_simple && m > QK_GEMV_MAX_M && m < (1u << 30) && hidden > 0 && inter > 0 && gate->L.type == up->L.type &&
              qk_gemm_tc_supported(gate->L, (uint32_t)m) && qk_gemm_tc_supported(down->L, (uint32_t)m)) {
@@ -649,19 +653,19 @@ extern "C" int qk_ffn_dev(qk_ctx *c, const qk_weights *gate, const qk_weights *u
     QkTcCall gu = {};
     gu.L = &gate->L, gu.maps[0] = gate->tmap, gu.maps[1] = up->tmap, gu.n = 2, gu.n_act = 1;
     gu.x = x_dev, gu.m = (uint32_t)m, gu.xcap = gu.ycap = (uint32_t)m, gu.y = h, gu.ldy = inter;
-    int st = tc_call(c, gu, s);
+    int st = tc_call(c, c->scratch, gu, s);
     if (st) return st;
     QkTcCall dn = {};
     dn.L = &down->L, dn.maps[0] = down->tmap, dn.n = dn.n_act = 1;
     dn.x = h, dn.x2 = u, dn.m = (uint32_t)m, dn.y = y_dev, dn.ldy = down->L.rows;
-    return tc_call(c, dn, s);
+    return tc_call(c, c->scratch, dn, s);
   } else {
-    int st = gemm_dispatch(c, gate, x_dev, h, m, inter, s);
+    int st = gemm_dispatch(c, c->scratch, gate, x_dev, h, m, inter, s);
     if (st) return st;
-    if ((st = gemm_dispatch(c, up, x_dev, u, m, inter, s))) return st;
+    if ((st = gemm_dispatch(c, c->scratch, up, x_dev, u, m, inter, s))) return st;
     CK(c, qk_launch_swiglu(h, u, (uint64_t)m * inter, s));
   }
-  return gemm_dispatch(c, down, h, y_dev, m, down->L.rows, s);
+  return gemm_dispatch(c, c->scratch, down, h, y_dev, m, down->L.rows, s);
 }
 
 extern "C" int qk_dequant_dev(qk_ctx *c, const qk_weights *h, float *out_dev, void *stream) {
@@ -784,13 +788,13 @@ static int host_gemm(qk_ctx *c, int type, const uint8_t *w, size_t w_len, size_t
   }
   if (stage_x) memcpy(c->hx, x, xb);
   if (decode && stage_x) {
-    if ((st = ensure_scratch(c, qk_gemv_fast_scratch_bytes(h->L, (uint32_t)m)))) return st;
-    CK(c, qk_launch_gemv_fast(h->L, h->dev, (const float *)c->hx_dev, ydev, (uint32_t)m, n, c->status_dev, c->scratch,
-                              c->sm_count, c->stream, true));
+    if ((st = qk_ensure_scratch(c, c->host_scratch, qk_gemv_fast_scratch_bytes(h->L, (uint32_t)m)))) return st;
+    CK(c, qk_launch_gemv_fast(h->L, h->dev, (const float *)c->hx_dev, ydev, (uint32_t)m, n, c->status_dev,
+                              c->host_scratch.p, c->sm_count, c->stream, true));
   } else {
     if ((st = grow(c, &c->sa, &c->sa_cap, xb ? xb : 4))) return st;
     if (xb) CK(c, cudaMemcpyAsync(c->sa, stage_x ? (const void *)c->hx : x, xb, cudaMemcpyHostToDevice, c->stream));
-    if ((st = gemm_dispatch(c, h, (const float *)c->sa, ydev, m, n, c->stream))) return st;
+    if ((st = gemm_dispatch(c, c->host_scratch, h, (const float *)c->sa, ydev, m, n, c->stream))) return st;
   }
   const bool from_dev = ydev == (float *)c->sb;
   if (from_dev) CK(c, cudaMemcpyAsync(stage_y ? (void *)c->hy : y, c->sb, yb, cudaMemcpyDeviceToHost, c->stream));

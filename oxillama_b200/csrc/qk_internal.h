@@ -23,6 +23,13 @@ struct qk_weights {
 
 #define QK_UPLOAD_STAGE ((size_t)32 << 20)
 
+#define QK_MIN_SCRATCH ((size_t)1 << 20)
+
+struct QkScratch {
+  unsigned char *p = nullptr;
+  size_t cap = 0;
+};
+
 struct qk_ctx {
   int device;
   int sm_count;
@@ -32,10 +39,11 @@ struct qk_ctx {
   // it after a stream synchronise without another copy.
   unsigned *status_dev;                  // device-side address, passed to kernels
   volatile unsigned *status_host = nullptr;  // the same word as the host sees it
-  // device scratch of the *_dev entry points (split activations); grown on demand,
-  // which synchronises: size it once before capturing into a CUDA graph
-  unsigned char *scratch = nullptr;
-  size_t scratch_cap = 0;
+  // device scratch of the *_dev entry points (split or converted activations, partial tiles); grown on
+  // demand, which synchronises: size it once before capturing into a CUDA graph.  The host-pointer entry
+  // points have their own: they run on the context's stream, where nothing orders them behind *_dev calls
+  // that are still in flight on the caller's.
+  QkScratch scratch, host_scratch;
   std::string err;
   std::mutex mu;
   // scratch for the host-pointer entry points
@@ -59,3 +67,5 @@ struct qk_ctx {
   size_t ffn_cap = 0;
 };
 
+// Grows `sc` (with a device synchronise where it has to be replaced) to `need` bytes.
+int qk_ensure_scratch(qk_ctx *c, QkScratch &sc, size_t need);

@@ -184,3 +184,29 @@ def test_host_call_around_the_staging_size(rows, cols, m):
     y = np.full((m, rows), np.nan, np.float32)
     KernelDispatcher().get_kernel(S.Q4_K).gemm(QuantTensor(w, (rows, cols), S.Q4_K), x, y, m, rows, cols)
     assert_product(y, x, O.dequant_matrix(S.Q4_K, w, rows, cols), m > 4)
+
+
+# Host calls run on a stream of the context that nothing orders behind the caller's: they share no scratch
+# with device calls still in flight there (a matmul's converted activations and counters, split activations).
+@pytest.mark.parametrize("rows,cols,m", [(4096, 4096, 96), (512, 12288, 3)])
+def test_host_call_beside_device_calls(rows, cols, m):
+    import torch
+    from oxillama_b200.device import DeviceWeights, check_device_status
+    from oxillama_b200.kernels import KernelDispatcher, QuantTensor
+    w, wh = S.gen_weight(S.Q4_K, rows, cols, seed=95), S.gen_weight(S.Q4_K, 256, 4096, seed=96)
+    dw, x, xh = DeviceWeights(S.Q4_K, w, rows, cols), torch.from_numpy(S.gen_acts(m, cols, seed=95)).cuda(), S.gen_acts(1, 4096, seed=96)
+    kern, qt = KernelDispatcher().get_kernel(S.Q4_K), QuantTensor(wh, (256, 4096), S.Q4_K)
+    want, yh0, yh = torch.empty(m, rows, device="cuda"), np.empty((1, 256), np.float32), np.empty((1, 256), np.float32)
+    dw.gemm(x, want, m)
+    check_device_status()
+    kern.gemv(qt, xh, yh0)
+    side, ys = torch.cuda.Stream(), [torch.empty(m, rows, device="cuda") for _ in range(24)]
+    side.wait_stream(torch.cuda.current_stream())
+    for _ in range(4):
+        for y in ys:
+            dw.gemm(x, y, m, stream=side)
+        kern.gemv(qt, xh, yh)
+        side.synchronize()
+        assert np.array_equal(yh, yh0)
+        assert all(torch.equal(y, want) for y in ys)
+    dw.free()

@@ -115,14 +115,16 @@ extern "C" int qk_init(int device, qk_ctx **out) {
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaHostAlloc((void **)&sh, sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess ||
       cudaHostGetDevicePointer((void **)&c->status_dev, sh, 0) != cudaSuccess ||
-      cudaMalloc(&c->scratch.p, QK_MIN_SCRATCH) != cudaSuccess) {
+      cudaMalloc(&c->scratch.p, QK_MIN_SCRATCH) != cudaSuccess ||
+      cudaMalloc(&c->host_scratch.p, QK_MIN_SCRATCH) != cudaSuccess) {  // (here: the first host call would wait milliseconds for it)
     if (sh) cudaFreeHost(sh);
+    if (c->scratch.p) cudaFree(c->scratch.p);
     delete c;
     return QK_CUDA_ERROR;
   }
   *sh = 0;
   c->status_host = sh;
-  c->scratch.cap = QK_MIN_SCRATCH;
+  c->scratch.cap = c->host_scratch.cap = QK_MIN_SCRATCH;
   const char *fs = qk_knob("QK_FORCE_SIMPLE");
   c->force_simple = fs && fs[0] == '1';
   *out = c;

@@ -116,9 +116,11 @@ extern "C" int qk_init(int device, qk_ctx **out) {
       cudaHostAlloc((void **)&sh, sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess ||
       cudaHostGetDevicePointer((void **)&c->status_dev, sh, 0) != cudaSuccess ||
       cudaMalloc(&c->scratch.p, QK_MIN_SCRATCH) != cudaSuccess ||
-      cudaMalloc(&c->host_scratch.p, QK_MIN_SCRATCH) != cudaSuccess) {  // (here: the first host call would wait milliseconds for it)
+      cudaMalloc(&c->host_scratch.p, QK_MIN_SCRATCH) != cudaSuccess ||  // (here: the first host call would wait milliseconds for it)
+      cudaMalloc(&c->images, QK_IMAGES * QK_IMAGE_BYTES) != cudaSuccess) {
     if (sh) cudaFreeHost(sh);
     if (c->scratch.p) cudaFree(c->scratch.p);
+    if (c->host_scratch.p) cudaFree(c->host_scratch.p);
     delete c;
     return QK_CUDA_ERROR;
   }
@@ -148,6 +150,7 @@ extern "C" int qk_shutdown(qk_ctx *c) {
   if (c->hx) cudaFreeHost(c->hx);
   if (c->scratch.p) cudaFree(c->scratch.p);
   if (c->host_scratch.p) cudaFree(c->host_scratch.p);
+  cudaFree(c->images);
   if (c->moe) cudaFree(c->moe);
   if (c->ffn) cudaFree(c->ffn);
   if (c->up) cudaFree(c->up);
@@ -363,6 +366,32 @@ int qk_ensure_scratch(qk_ctx *c, QkScratch &sc, size_t need) {
   return QK_OK;
 }
 
+// Where a decode call of m rows leaves its split activations, if it has to.  Formats with a tensor-core
+// matmul share the context's scratch; the others, which have no other scratch, take a slot of the call's
+// stream, or none: in a capture (the graph may run beside the stream it was captured from) and when all
+// slots are taken.  (Without a slot every CTA splits: Q5_K 4096 x 14336, four rows 40.8 us against 33.4.)
+static int split_image(qk_ctx *c, QkScratch &sc, const QkLayout &L, size_t m, cudaStream_t s, unsigned char **img) {
+  *img = nullptr;
+  if (qk_gemm_tc_supported(L, 1) || &sc == &c->host_scratch) {
+    int st = qk_ensure_scratch(c, sc, qk_gemv_fast_scratch_bytes(L, (uint32_t)m));
+    *img = sc.p;
+    return st;
+  }
+  if (m * L.nb * L.bs <= QK_SPLIT_IN_CTA) return QK_OK;
+  cudaStreamCaptureStatus cap;
+  unsigned long long id;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone || cudaStreamGetId(s, &id) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return QK_OK;
+  }
+  int i = 0;
+  while (i < c->n_images && c->image_of[i] != id) i++;
+  if (i == QK_IMAGES) return QK_OK;
+  if (i == c->n_images) c->image_of[c->n_images++] = id;
+  *img = c->images + i * QK_IMAGE_BYTES;
+  return QK_OK;
+}
+
 static int tc_call(qk_ctx *c, QkScratch &sc, const QkTcCall &call, cudaStream_t s) {
   int st = qk_ensure_scratch(c, sc, qk_gemm_tc_scratch_bytes(call, c->sm_count));
   if (st) return st;
@@ -384,11 +413,12 @@ static int gemm_dispatch(qk_ctx *c, QkScratch &sc, const qk_weights *h, const fl
     size_t step = m < QK_GEMV_MAX_M ? m : QK_GEMV_MAX_M;
     while (step > 1 && !qk_gemv_fast_supported(h->L, (uint32_t)step)) step--;
     if (step == m || !qk_gemm_tc_supported(h->L, 1)) {
-      int st = qk_ensure_scratch(c, sc, qk_gemv_fast_scratch_bytes(h->L, (uint32_t)step));
+      unsigned char *img;
+      int st = split_image(c, sc, h->L, step, s, &img);
       if (st) return st;
       for (size_t i = 0; i < m; i += step) {
         const uint32_t k = (uint32_t)(m - i < step ? m - i : step);
-        CK(c, qk_launch_gemv_fast(h->L, h->dev, x + i * h->L.cols, y + i * ldy, k, ldy, c->status_dev, sc.p, c->sm_count, s));
+        CK(c, qk_launch_gemv_fast(h->L, h->dev, x + i * h->L.cols, y + i * ldy, k, ldy, c->status_dev, img, c->sm_count, s));
       }
       return QK_OK;
     }
@@ -644,9 +674,10 @@ extern "C" int qk_ffn_dev(qk_ctx *c, const qk_weights *gate, const qk_weights *u
   const bool fused = !c->force_simple && gate->L.type == up->L.type && hidden > 0 && inter > 0 && m <= QK_GEMV_MAX_M && qk_gemv_dual_supported(gate->L, (uint32_t)m);
   if (fused) {
     // gate and up in one launch (they share the split activations), silu(g) * u in its reducer
-    int st = qk_ensure_scratch(c, c->scratch, qk_gemv_fast_scratch_bytes(gate->L, (uint32_t)m));
+    unsigned char *img;
+    int st = split_image(c, c->scratch, gate->L, m, s, &img);
     if (st) return st;
-    CK(c, qk_launch_gemv_dual(gate->L, gate->dev, up->dev, x_dev, h, (uint32_t)m, inter, c->status_dev, c->scratch.p,
+    CK(c, qk_launch_gemv_dual(gate->L, gate->dev, up->dev, x_dev, h, (uint32_t)m, inter, c->status_dev, img,
                               c->sm_count, s));
   } else if (!c->force_simple && m > QK_GEMV_MAX_M && m < (1u << 30) && hidden > 0 && inter > 0 && gate->L.type == up->L.type &&
              qk_gemm_tc_supported(gate->L, (uint32_t)m) && qk_gemm_tc_supported(down->L, (uint32_t)m)) {

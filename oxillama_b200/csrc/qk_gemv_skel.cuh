@@ -772,7 +772,7 @@ inline bool split_in_cta(const PlanMma &P, uint32_t m) {
     force = e ? atoi(e) : -1;  // 0: always the split kernel, 1: always in-CTA
   }
   if (force >= 0) return force == 1;
-  return m * P.Kp <= 8192;
+  return m * P.Kp <= QK_SPLIT_IN_CTA;
 }
 
 template <class F, int M>
@@ -784,7 +784,7 @@ cudaError_t launch_mma_m(const QkLayout &L, const uint8_t *W, const float *x, fl
   // so the ring depth is a multiple of G * ktiles; P.groups was chosen to allow that.
   const bool peer = peers != nullptr;
 #define QK_LAUNCH1(CWV, GV, PV)                                                                               \
-  return !host_x && split_in_cta(P, M)                                                                                   \
+  return !host_x && (!ximg || split_in_cta(P, M))                                                             \
              ? launch_mma<F, M, true, CWV, GV, PV>(L, W, x, y, ldy, status, ximg, sm_count, P, s, peers, W2)  \
              : launch_mma<F, M, false, CWV, GV, PV>(L, W, x, y, ldy, status, ximg, sm_count, P, s, peers, W2)
 #define QK_LAUNCH(CWV, GV)                \

@@ -30,6 +30,12 @@ struct QkScratch {
   size_t cap = 0;
 };
 
+// Images of split activations, one per stream, for the formats whose calls may overlap on different
+// streams (Q5_K, Q3_K, Q2_K).  A slot belongs to the stream that first asked for it, by its id (which,
+// unlike a handle, is never used again), until the context ends.
+#define QK_IMAGES 16
+#define QK_IMAGE_BYTES ((size_t)256 << 10)  // above what fits a CTA's shared memory
+
 struct qk_ctx {
   int device;
   int sm_count;
@@ -44,6 +50,9 @@ struct qk_ctx {
   // points have their own: they run on the context's stream, where nothing orders them behind *_dev calls
   // that are still in flight on the caller's.
   QkScratch scratch, host_scratch;
+  unsigned char *images = nullptr;  // QK_IMAGES slots, made with the context
+  unsigned long long image_of[QK_IMAGES] = {};
+  int n_images = 0;
   std::string err;
   std::mutex mu;
   // scratch for the host-pointer entry points

@@ -80,6 +80,9 @@ struct QkPeers {
 
 // Bandwidth-bound decode path (m <= QK_GEMV_MAX_M): bulk-copied tiles, integer dot.
 #define QK_GEMV_MAX_M 4
+// Up to this many activations (rows x padded columns) every CTA of the decode kernel splits them itself;
+// above, a kernel of its own does it once into scratch -- if the call has any (scratch == null: in the CTAs).
+#define QK_SPLIT_IN_CTA 8192u
 bool qk_gemv_fast_supported(const QkLayout &L, uint32_t m);
 // Q4_K decode path on the integer tensor-core MMA (m16n8k32 u8 x s8).  `scratch`
 // is device memory of at least qk_gemv_mma_scratch_bytes(L, m) bytes, 16-byte

@@ -210,3 +210,34 @@ def test_host_call_beside_device_calls(rows, cols, m):
         assert np.array_equal(yh, yh0)
         assert all(torch.equal(y, want) for y in ys)
     dw.free()
+
+
+# Calls of the formats without a tensor-core matmul may overlap on different streams of one context: each
+# stream has its own place for split activations, and the calls of streams that found none left (20 streams),
+# like those of a captured graph, use none.
+@pytest.mark.parametrize("t", [S.Q5_K, S.Q3_K, S.Q2_K])
+def test_calls_on_many_streams(t):
+    import torch
+    from oxillama_b200.device import DeviceWeights, check_device_status
+    from oxillama_b200.kernels import Context
+    rows, cols, ctx = 1024, 12288, Context()
+    dw = DeviceWeights(t, S.gen_weight(t, rows, cols, seed=97), rows, cols, ctx=ctx)
+    xs = [torch.from_numpy(S.gen_acts(m, cols, seed=m)).cuda() for m in (1, 2)]
+    want = [torch.empty(len(x), rows, device="cuda") for x in xs]
+    for x, y in zip(xs, want):
+        dw.gemm(x, y, len(x))
+    streams = [torch.cuda.Stream() for _ in range(20)]
+    ys = [[torch.empty_like(w) for w in want] for _ in range(40)]
+    graph, yg = torch.cuda.CUDAGraph(), torch.empty_like(want[1])
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        dw.gemm(xs[1], yg, 2)
+    for i, pair in enumerate(ys):
+        for x, y in zip(xs, pair):
+            dw.gemm(x, y, len(x), stream=streams[i % 20])
+        graph.replay()
+    torch.cuda.synchronize()
+    check_device_status(ctx)
+    assert torch.equal(yg, want[1])
+    assert all(torch.equal(y, w) for pair in ys for y, w in zip(pair, want))
+    dw.free()

@@ -65,13 +65,12 @@ __global__ void __launch_bounds__(256)
   s4 += __shfl_xor_sync(0xffffffffu, s4, 1);
   s4 += __shfl_xor_sync(0xffffffffu, s4, 2);
   const float other = __shfl_xor_sync(0xffffffffu, s4, 4);
-  if (!(amax < 8.0e37f)) amax = 8.0e37f;  // as qk_xsplit_kernel
-  const float inv = amax > 0.f ? __fdividef(127.f, amax) : 0.f;
+  const float inv = digit_inv(amax);
   uint32_t w0, w1, w2;
   split_quad(v, inv, w0, w1, w2);
   unsigned char *row = img + (uint64_t)r * stride;
   F::store_digits(row, PS, e0, w0, w1, w2);
-  if ((threadIdx.x & 7) == 0) F::store_xs(row + 3 * PS, e0 / 32, amax * (1.f / 127.f), s4 + other, s4, other);
+  if ((threadIdx.x & 7) == 0) F::store_xs(row + 3 * PS, e0 / 32, digit_scale(amax, s4 + other), s4 + other, s4, other);
 }
 
 template <class F, bool DUAL, int G>

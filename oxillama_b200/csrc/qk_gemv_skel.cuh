@@ -34,6 +34,7 @@
 // mbarrier is bounded: when one runs out the warp stops, QK_DEV_TIMEOUT is
 // raised in the status word, and the other warps run into their own bounds.
 #pragma once
+#include <cfloat>
 #include <cstdlib>
 #include <type_traits>
 
@@ -129,7 +130,7 @@ __device__ __forceinline__ void mma_u8s8(float (&c)[4], uint32_t a0, uint32_t a1
 // packed word per digit plane: x ~ (amax / 127) (d0 + d1 / 254 + d2 / 254^2).  Adding
 // 1.5 * 2^23 rounds to the nearest integer and leaves it, as two's complement, in the low
 // mantissa byte; with |v| <= amax every digit lies in [-127, 127] without a clamp.  (Values
-// that are not finite give arbitrary digits: the product is meaningless for them anyway.)
+// that are not finite give arbitrary digits: digit_scale marks their block.)
 __device__ __forceinline__ void split_quad(const float (&v)[4], float inv, uint32_t &w0, uint32_t &w1,
                                            uint32_t &w2) {
   constexpr float MAGIC = 12582912.f;
@@ -146,6 +147,19 @@ __device__ __forceinline__ void split_quad(const float (&v)[4], float inv, uint3
   w0 = __byte_perm(__byte_perm(b0[0], b0[1], 0x0040), __byte_perm(b0[2], b0[3], 0x0040), 0x5410);
   w1 = __byte_perm(__byte_perm(b1[0], b1[1], 0x0040), __byte_perm(b1[2], b1[3], 0x0040), 0x5410);
   w2 = __byte_perm(__byte_perm(b2[0], b2[1], 0x0040), __byte_perm(b2[2], b2[3], 0x0040), 0x5410);
+}
+
+// 127 / amax, finite whatever the block holds: a block whose largest magnitude is below 1e-36 keeps the
+// grid of 1e-36 (last digit 1.2e-43), and up to FLT_MAX the divisor stays below the 2^126 from which
+// __fdividef gives 0.
+__device__ __forceinline__ float digit_inv(float &amax) {
+  amax = fmaxf(amax, 1e-36f);
+  return __fdividef(127.f / 16.f, amax * (1.f / 16.f));
+}
+// The scale that goes with it.  A block with an infinity or a NaN in it (s32: the sum of its columns) has
+// no digits: its scale is NaN, and so is every result that it is part of.
+__device__ __forceinline__ float digit_scale(float amax, float s32) {
+  return amax > FLT_MAX || s32 != s32 ? __int_as_float(0x7FFFFFFF) : amax * (1.f / 127.f);
 }
 
 // Activations e0 .. e0 + 3 of one row out of the tagged slots of a gathered buffer (columns
@@ -198,13 +212,12 @@ __global__ void __launch_bounds__(256)
   s4 += __shfl_xor_sync(0xffffffffu, s4, 1);
   s4 += __shfl_xor_sync(0xffffffffu, s4, 2);  // this thread's 16-column half
   const float other = __shfl_xor_sync(0xffffffffu, s4, 4);
-  if (!(amax < 8.0e37f)) amax = 8.0e37f;  // inf/nan/huge x: keep the scale finite (__fdividef: y < 2^126)
-  const float inv = amax > 0.f ? __fdividef(127.f, amax) : 0.f;
+  const float inv = digit_inv(amax);
   uint32_t w0, w1, w2;
   split_quad(v, inv, w0, w1, w2);
   F::store_digits(img + (size_t)m * 3 * PS, PS, e0, w0, w1, w2);
   if ((threadIdx.x & 7) == 0)
-    F::store_xs(img + xs_off, (size_t)m * (Kp / 32) + e0 / 32, amax * (1.f / 127.f), s4 + other, s4, other);
+    F::store_xs(img + xs_off, (size_t)m * (Kp / 32) + e0 / 32, digit_scale(amax, s4 + other), s4 + other, s4, other);
 }
 
 // ---------------------------------------------------------------- main kernel
@@ -267,14 +280,13 @@ __device__ void xsplit_in_cta(const float *__restrict__ x, uint32_t cols, uint32
       s4 += __shfl_xor_sync(0xffffffffu, s4, 1);
       s4 += __shfl_xor_sync(0xffffffffu, s4, 2);  // this thread's 16-column half
       const float other = __shfl_xor_sync(0xffffffffu, s4, 4);
-      if (!(amax < 8.0e37f)) amax = 8.0e37f;
       QK_STAMP(threadIdx.x == 0 && j == 0 && amax >= 0.f, 122);
-      const float inv = amax > 0.f ? __fdividef(127.f, amax) : 0.f;
+      const float inv = digit_inv(amax);
       uint32_t w0, w1, w2;
       split_quad(v[j], inv, w0, w1, w2);
       F::store_digits(img + (size_t)m * 3 * PS, PS, e0, w0, w1, w2);
       if ((threadIdx.x & 7) == 0)
-        F::store_xs(img + xs_off, (size_t)m * (Kp / 32) + e0 / 32, amax * (1.f / 127.f), s4 + other, s4, other);
+        F::store_xs(img + xs_off, (size_t)m * (Kp / 32) + e0 / 32, digit_scale(amax, s4 + other), s4 + other, s4, other);
     }
   }
 }

@@ -241,3 +241,41 @@ def test_calls_on_many_streams(t):
     assert torch.equal(yg, want[1])
     assert all(torch.equal(y, w) for pair in ys for y, w in zip(pair, want))
     dw.free()
+
+
+# Activations at the ends of the f32 range, on the kernels that split them into digits (in the CTAs and by
+# the kernel before: 512 and 9216 columns) and through a host call.  Tiny rows keep the f32-grade bound down
+# to 1e-36, below it on that value's grid; a row with an infinity or a NaN gives no finite number, and its
+# neighbour does not notice.
+@pytest.mark.parametrize("cols", [512, 9216])
+@pytest.mark.parametrize("t", TC_TYPES + [S.Q5_K, S.Q3_K, S.Q2_K])
+def test_decode_activation_range(t, cols):
+    import torch
+    from oxillama_b200.kernels import KernelDispatcher, QuantTensor
+    rows = 40
+    kern = KernelDispatcher().get_kernel(t)
+    big, small = (5e-3, 1e-2) if t == S.Q6_K else (2.0, 4.0), (1e-6, 1e-5)
+    for scale, d_range in ((1e-30, big), (1e-36, big), (3e-38, big), (1e36, small), (6e37, small)):
+        w = S.gen_weight(t, rows, cols, seed=98, d_range=d_range)  # (scales large: products of tiny rows stay normal numbers)
+        wd = O.dequant_matrix(t, w, rows, cols).astype(np.float64)
+        x = S.gen_acts(2, cols, seed=98).clip(-4, 4)
+        if scale > 1:  # one large value: the sums must not overflow
+            x[:, 1:] = 0
+            x[:, 0] = (4, -4)
+        x = (x * np.float64(scale)).astype(np.float32)
+        ref = x.astype(np.float64) @ wd.T
+        s = np.sqrt(np.maximum(block_max(x), 1e-36 if scale < 1 else 0) ** 2 @ (block_max(wd) ** 2).T)
+        bound = 7 * 2.0 ** -23 * (1 + np.sqrt(2 * cols / 32)) * s
+        ys = [device_product(t, w, x, rows, cols, 2), device_product(t, w, x[:1], rows, cols, 1), np.empty((2, rows), np.float32)]
+        kern.gemm(QuantTensor(w, (rows, cols), t), x, ys[2], 2, rows, cols)
+        for y in ys:
+            assert np.all(np.abs(y - ref[: len(y)]) <= bound[: len(y)]), (scale, float((np.abs(y - ref[: len(y)]) / bound[: len(y)]).max()))
+    w = S.gen_weight(t, rows, cols, seed=98)
+    x = S.gen_acts(2, cols, seed=99)
+    want = device_product(t, w, x, rows, cols, 2)
+    for bad in (np.nan, np.inf, -np.inf):
+        xb = x.copy()
+        xb[1, cols - 7] = bad
+        y = device_product(t, w, xb, rows, cols, 2)
+        assert not np.isfinite(y[1]).any() and np.array_equal(y[0], want[0])
+

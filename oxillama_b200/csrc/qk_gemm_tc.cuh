@@ -485,9 +485,9 @@ struct WFmt<QK_T_IQ4_XS> {  // super-block of 256: f16 d, scales_h, scales_l[4],
 
 // ---------------------------------------------------------------- activations -> fp16
 // X16[t][256 s + p] = x[t][256 s + src(p)] / scale[t] in fp16, where scale[t] is the power
-// of two that puts the row's largest magnitude in [512, 1024): the division is exact, no
-// activation overflows or falls into fp16's subnormals, and the epilogue multiplies the
-// row of results by scale[t] again (also exact).  Columns >= cols are zero.  One CTA per token
+// of two that puts the row's largest magnitude in [512, 1024) (2^-126 at least): the division is
+// exact, no activation overflows, only those below 2^-24 of the largest fall into fp16's subnormals, and the
+// epilogue multiplies the row of results by scale[t] again (also exact).  Columns >= cols are zero.  One CTA per token
 // row; a row of up to 16384 columns is read once and stays in registers between the maximum and
 // the conversion (a thread's eight positions come from two float4s whatever the format's order).
 // GLU: the row is silu(x) * x2, formed here (crates/oxillama-arch/src/common/swiglu.rs:15-21, each
@@ -553,7 +553,7 @@ __device__ __forceinline__ float conv_scale(float amax) {
   if (!(amax > 0.f && amax <= FLT_MAX)) return 1.f;  // zero, or not finite (a NaN row stays NaN)
   int e;
   frexpf(amax, &e);  // amax = f * 2^e, f in [0.5, 1)
-  return ldexpf(1.f, e - 10);
+  return ldexpf(1.f, max(e - 10, -126));  // (from -126 on the reciprocal is finite; a row below 2^-116 starts lower in fp16's range)
 }
 __device__ __forceinline__ void conv_store(__half *orow, uint32_t c, const float (&w)[8], float inv) {
   uint32_t h[4];

@@ -279,3 +279,42 @@ def test_decode_activation_range(t, cols):
         y = device_product(t, w, xb, rows, cols, 2)
         assert not np.isfinite(y[1]).any() and np.array_equal(y[0], want[0])
 
+
+
+# The conversion of activations to fp16 at the lower end of the f32 range, where the row's scale is a power
+# of two without a finite reciprocal (below 2^-118) or the row is subnormal, and at rows longer than it
+# keeps in registers (16384 columns).
+@pytest.mark.parametrize("rows,cols,m", [(96, 512, 5), (96, 512, 70), (40, 16640, 6)])
+@pytest.mark.parametrize("scale", [1.0, 1e-30, 1e-37, 1e-41])
+def test_conversion_of_small_rows(rows, cols, m, scale):
+    w = S.gen_weight(S.Q4_K, rows, cols, seed=101, d_range=(2.0, 4.0))
+    wd = O.dequant_matrix(S.Q4_K, w, rows, cols).astype(np.float64)
+    x = S.gen_acts(m, cols, seed=101)
+    x[1::2] = (x[1::2] * np.float64(scale)).astype(np.float32)  # every second row: a scale of its own
+    x[2] = 0
+    y = device_product(S.Q4_K, w, x, rows, cols, m)
+    ref = x.astype(np.float64) @ wd.T
+    s = np.sqrt(x.astype(np.float64) ** 2 @ (block_max(wd) ** 2).T)
+    assert np.all(np.abs(y - ref) <= 7 * 2.0 ** -11 * np.sqrt(4 / 3) * s + 2.0 ** -149)
+
+
+# silu(g) * u of tiny activations (products of about 1e-40), and of rows longer than the conversion keeps in
+# shared memory (28160 columns).
+@pytest.mark.parametrize("hidden,inter,m,scale", [(512, 768, 5, 1e-20), (512, 768, 70, 1e-20), (256, 28416, 5, 1.0), (256, 28416, 5, 1e-20)])
+def test_ffn_conversion(hidden, inter, m, scale):
+    import torch
+    from oxillama_b200.device import DeviceWeights, check_device_status, ffn
+    shapes = [(inter, hidden), (inter, hidden), (hidden, inter)]
+    ws = [S.gen_weight(S.Q4_K, r, c, seed=102, stream=i, d_range=(1e-3, 3e-3)) for i, (r, c) in enumerate(shapes)]
+    g, u, d = (O.dequant_matrix(S.Q4_K, w, r, c).astype(np.float64) for w, (r, c) in zip(ws, shapes))
+    x = (S.gen_acts(m, hidden, seed=102) * np.float64(scale)).astype(np.float32)
+    hg = x.astype(np.float64) @ g.T
+    ref = (hg / (1 + np.exp(-hg)) * (x.astype(np.float64) @ u.T)) @ d.T
+    dw = [DeviceWeights(S.Q4_K, w, r, c) for w, (r, c) in zip(ws, shapes)]
+    y = torch.full((m, hidden), float("nan"), device="cuda")
+    ffn(*dw, torch.from_numpy(x).cuda(), y, m)
+    check_device_status()
+    # three chained products, each within 1e-3 of its largest value (fp16 operands)
+    assert np.abs(y.cpu().numpy() - ref).max() <= 3e-3 * np.abs(ref).max()
+    for w in dw:
+        w.free()

@@ -112,11 +112,12 @@ extern "C" int qk_init(int device, qk_ctx **out) {
   }
   c->sm_count = prop.multiProcessorCount;
   unsigned *sh = nullptr;
+  const size_t scratch = QK_MIN_SCRATCH + qk_gemm_tc_part_bytes(c->sm_count);
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaHostAlloc((void **)&sh, sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess ||
       cudaHostGetDevicePointer((void **)&c->status_dev, sh, 0) != cudaSuccess ||
-      cudaMalloc(&c->scratch.p, QK_MIN_SCRATCH) != cudaSuccess ||
-      cudaMalloc(&c->host_scratch.p, QK_MIN_SCRATCH) != cudaSuccess ||  // (here: the first host call would wait milliseconds for it)
+      cudaMalloc(&c->scratch.p, scratch) != cudaSuccess ||
+      cudaMalloc(&c->host_scratch.p, scratch) != cudaSuccess ||  // (here: the first host call would wait milliseconds for it)
       cudaMalloc(&c->images, QK_IMAGES * QK_IMAGE_BYTES) != cudaSuccess) {
     if (sh) cudaFreeHost(sh);
     if (c->scratch.p) cudaFree(c->scratch.p);
@@ -126,7 +127,7 @@ extern "C" int qk_init(int device, qk_ctx **out) {
   }
   *sh = 0;
   c->status_host = sh;
-  c->scratch.cap = c->host_scratch.cap = QK_MIN_SCRATCH;
+  c->scratch.cap = c->host_scratch.cap = scratch;
   const char *fs = qk_knob("QK_FORCE_SIMPLE");
   c->force_simple = fs && fs[0] == '1';
   *out = c;
@@ -355,14 +356,11 @@ extern "C" int qk_weights_cache_evict(qk_ctx *c, const uint8_t *w) {
 // ------------------------------------------------------------ device entry points
 int qk_ensure_scratch(qk_ctx *c, QkScratch &sc, size_t need) {
   if (need <= sc.cap) return QK_OK;
-  if (sc.p) {
-    CK(c, cudaDeviceSynchronize());
-    cudaFree(sc.p);
-    sc.p = nullptr, sc.cap = 0;
-  }
-  const size_t want = need + need / 4 > QK_MIN_SCRATCH ? need + need / 4 : QK_MIN_SCRATCH;
-  CK(c, cudaMalloc(&sc.p, want));
-  sc.cap = want;
+  CK(c, cudaDeviceSynchronize());
+  cudaFree(sc.p);
+  sc.p = nullptr, sc.cap = 0;
+  CK(c, cudaMalloc(&sc.p, need * 2));
+  sc.cap = need * 2;
   return QK_OK;
 }
 

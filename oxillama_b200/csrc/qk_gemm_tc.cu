@@ -154,7 +154,7 @@ bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
   p.o_cnt = al(p.o_scale + (size_t)(p.xrows + MAX_BN) * 4);
   p.o_part = al(p.o_cnt + (size_t)sm_count * 2 * 4);
   p.grid *= p.cg;
-  p.bytes = p.o_part + (size_t)p.grid * 2 * p.bn * BM * 4;
+  p.bytes = p.o_part + qk_gemm_tc_part_bytes(sm_count);  // (whatever this plan uses of them)
   *P = p;
   return true;
 }
@@ -190,6 +190,8 @@ cudaError_t qk_gemm_tc_map(const QkLayout &L, uint8_t *tiled, void *map) {
   memcpy(map, &m, sizeof(m));
   return cudaSuccess;
 }
+
+size_t qk_gemm_tc_part_bytes(int sm_count) { return (size_t)sm_count * 2 * qktc::MAX_BN * qktc::BM * 4; }
 
 size_t qk_gemm_tc_scratch_bytes(const QkTcCall &c, int sm_count) {
   qktc::TcPlan P;

@@ -23,7 +23,10 @@ struct qk_weights {
 
 #define QK_UPLOAD_STAGE ((size_t)32 << 20)
 
-#define QK_MIN_SCRATCH ((size_t)1 << 20)
+// A context starts with scratch for this many bytes of converted activations beside the partial tiles of a
+// matmul (128 rows of 4096 columns and their rounding): calls up to there never grow it, so they may be
+// captured without a call before.
+#define QK_MIN_SCRATCH ((size_t)2 << 20)
 
 struct QkScratch {
   unsigned char *p = nullptr;
@@ -76,5 +79,5 @@ struct qk_ctx {
   size_t ffn_cap = 0;
 };
 
-// Grows `sc` (with a device synchronise where it has to be replaced) to `need` bytes.
+// Grows `sc` (with a device synchronise) to twice `need` bytes, if it is smaller than `need`.
 int qk_ensure_scratch(qk_ctx *c, QkScratch &sc, size_t need);

@@ -318,3 +318,26 @@ def test_ffn_conversion(hidden, inter, m, scale):
     assert np.abs(y.cpu().numpy() - ref).max() <= 3e-3 * np.abs(ref).max()
     for w in dw:
         w.free()
+
+
+# The first matmul of a context, captured: up to 128 rows of 4096 columns need no more scratch than the
+# context starts with, whichever tiles and K split the shape gets.
+@pytest.mark.parametrize("t,rows,cols,m", [(S.Q4_K, 4096, 4096, 8), (S.Q6_K, 300, 8192, 60), (S.Q8_0, 1024, 3840, 128),
+                                           (S.Q5_K, 512, 9216, 4), (S.IQ4_XS, 14336, 4096, 120)])
+def test_first_call_in_a_capture(t, rows, cols, m):
+    import torch
+    from oxillama_b200.device import DeviceWeights, check_device_status
+    from oxillama_b200.kernels import Context
+    w, x = S.gen_weight(t, rows, cols, seed=103), S.gen_acts(m, cols, seed=103)
+    want = device_product(t, w, x, rows, cols, m)
+    ctx = Context()
+    dw, xd, y = DeviceWeights(t, w, rows, cols, ctx=ctx), torch.from_numpy(x).cuda(), torch.zeros(m, rows, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        dw.gemm(xd, y, m)
+    graph.replay()
+    torch.cuda.synchronize()
+    check_device_status(ctx)
+    assert np.array_equal(y.cpu().numpy(), want)
+    dw.free()

@@ -992,7 +992,8 @@ __global__ void __maxnreg__(REGS)
     uint32_t dph = 0;
     pdl_wait();  // y, the scales and the workspace belong to the previous kernel until it has finished
     const uint64_t ldy = A.ldy;
-    for (uint32_t i = 0; i < sc.n_seg && !dead; i++) {
+    uint32_t i = 0;
+    for (; i < sc.n_seg && !dead; i++) {
       uint32_t tile, s0, s1;
       sc.get(i, tile, s0, s1);
       const TileAt q = at(tile);
@@ -1076,7 +1077,16 @@ __global__ void __maxnreg__(REGS)
       if (*told != i1 - i0) continue;
       if (warp == FIRST_EW && lane == 0) *last |= 1u << (i - sc.whole);  // all warps add them up, below
     }
-    if (dead && lane == 0) atomicOr(A.status, QK_DEV_TIMEOUT);
+    if (dead) {
+      // A warp whose wait ran out still comes to the barriers of the split tiles that are left: there the
+      // other three, if theirs did not, learn of it.
+      if (lane == 0) atomicOr(A.status, QK_DEV_TIMEOUT);
+      for (; i < sc.n_seg; i++) {
+        uint32_t tile, s0, s1;
+        sc.get(i, tile, s0, s1);
+        if ((s0 != 0 || s1 != sc.nsb) && !(CG == 1 && NG == 1 && A.cs > 1)) (void)any_of_128(true);
+      }
+    }
   } else if (warp >= FIRST_DW) {
     // ======================= expanding warps =======================
     // Set `set` takes every second super-block; in it, warp (hh, quarter) the columns [128 hh, + 128)

@@ -2,6 +2,7 @@
 // reference's order, the context (stream, scratch, weight cache), and the
 // choice of kernel for each shape.  Nothing here computes on the CPU: a call
 // that cannot reach the GPU returns QK_CUDA_ERROR.
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -397,6 +398,20 @@ static int tc_call(qk_ctx *c, QkScratch &sc, const QkTcCall &call, cudaStream_t 
   return QK_OK;
 }
 
+// Whether m > 4 rows of a format without a tensor-core matmul take less time as pieces of `step` rows on the
+// decode kernels than on the generic kernel, which decodes a weight once per eight rows in one launch: it wins
+// where the matrix is too small to repay a launch per piece (Q2_K 8 x 256 by 1024: 21 against 1440 us; Q5_K 1024 x
+// 4096 by 256: 1516 against 343).  Microseconds of both: over 222 shapes (8 x 256 .. 4096 x 4096, 5 .. 1024
+// rows) the choice takes 1.001 times the faster one's time in the mean, 1.16 at worst.
+static bool pieces_pay(const QkLayout &L, size_t m, size_t step) {
+  const double cols = L.cols, elems = cols * L.rows, eights = (double)((m + 7) / 8), pieces = (double)((m + step - 1) / step);
+  const double chain = 0.031 * cols * ceil(eights / 64), all = 1.1e-5 * elems * eights;  // a warp's row; all weights on all SMs
+  const double generic = 5 + (L.type == QK_TYPE_Q3_K ? 1.25 : 1.0) * (chain > all ? chain : all);
+  const double acts = step * cols;  // (Q5_K: the more there are, the fewer weight tiles fit beside them)
+  const double split = L.type == QK_TYPE_Q5_K ? (1e-4 + 1e-9 * acts) * acts : 1.8e-4 * acts;
+  return pieces * (3.2 + split + 2.5e-4 * L.rows + 1.9e-7 * elems) <= generic;
+}
+
 static int gemm_dispatch(qk_ctx *c, QkScratch &sc, const qk_weights *h, const float *x, float *y, size_t m,
                          size_t ldy, cudaStream_t s) {
   if (h->L.rows == 0 || m == 0) return QK_OK;
@@ -404,13 +419,14 @@ static int gemm_dispatch(qk_ctx *c, QkScratch &sc, const qk_weights *h, const fl
     CK(c, cudaMemset2DAsync(y, ldy * sizeof(float), 0, h->L.rows * sizeof(float), m, s));
     return QK_OK;
   }
-  // Formats without a tensor-core matmul (Q5_K, Q3_K, Q2_K) take a batch of any size on the decode
-  // kernels, as many rows at a time as these take: the weights are streamed once per four rows, where
-  // the generic kernel decodes them byte by byte once per eight.
-  if (!c->force_simple && qk_gemv_fast_supported(h->L, 1) && (m <= QK_GEMV_MAX_M || !qk_gemm_tc_supported(h->L, 1))) {
+  // Formats without a tensor-core matmul (Q5_K, Q3_K, Q2_K) take a batch on the decode kernels too, as many
+  // rows at a time as these take: the weights are streamed once per four rows (or two), where the generic
+  // kernel decodes them byte by byte once per eight.
+  const bool tc = qk_gemm_tc_supported(h->L, 1);
+  if (!c->force_simple && qk_gemv_fast_supported(h->L, 1) && (m <= QK_GEMV_MAX_M || !tc)) {
     size_t step = m < QK_GEMV_MAX_M ? m : QK_GEMV_MAX_M;
     while (step > 1 && !qk_gemv_fast_supported(h->L, (uint32_t)step)) step--;
-    if (step == m || !qk_gemm_tc_supported(h->L, 1)) {
+    if (step == m || (!tc && (m <= QK_GEMV_MAX_M || pieces_pay(h->L, m, step)))) {
       unsigned char *img;
       int st = split_image(c, sc, h->L, step, s, &img);
       if (st) return st;

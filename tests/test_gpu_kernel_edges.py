@@ -341,3 +341,23 @@ def test_first_call_in_a_capture(t, rows, cols, m):
     check_device_status(ctx)
     assert np.array_equal(y.cpu().numpy(), want)
     dw.free()
+
+
+# Batches of the formats without a tensor-core matmul: on the decode kernels in pieces of up to four rows, or,
+# where the matrix is too small for that many launches, in one launch of the generic kernel.
+@pytest.mark.parametrize("rows,cols,m,launches", [(8, 256, 300, 1), (64, 512, 70, 1), (256, 1024, 256, 1), (2048, 2048, 24, 24), (37, 14336, 6, 12)])
+@pytest.mark.parametrize("t", [S.Q5_K, S.Q3_K, S.Q2_K])
+def test_batches_without_tensor_cores(t, rows, cols, m, launches):
+    import torch
+    from cuda.bindings import runtime
+    from oxillama_b200.device import DeviceWeights
+    w, x = S.gen_weight(t, rows, cols, seed=104), S.gen_acts(m, cols, seed=104)
+    assert_product(device_product(t, w, x, rows, cols, m), x, O.dequant_matrix(t, w, rows, cols), False)
+    dw, xd, y = DeviceWeights(t, w, rows, cols), torch.from_numpy(x).cuda(), torch.empty(m, rows, device="cuda")
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        dw.gemm(xd, y, m)
+    err, _, n = runtime.cudaGraphGetNodes(graph.raw_cuda_graph())
+    assert int(err) == 0 and n <= launches
+    dw.free()

@@ -199,7 +199,7 @@ static int upload_impl(qk_ctx *c, int type, const uint8_t *w, size_t n_cols, siz
   }
   h->algo_bytes = need_bytes(type, rows, n_cols);
   size_t row_bytes = (size_t)h->L.nb * h->L.bb;
-  size_t tiled = h->L.total_bytes ? h->L.total_bytes : 16;
+  size_t tiled = h->L.total_bytes ? h->L.total_bytes + qk_gemm_tc_pad_bytes(h->L) : 16;
   cudaError_t e = cudaMalloc(&h->dev, tiled);
   if (e != cudaSuccess) {
     c->err = std::string("cudaMalloc(weights): ") + cudaGetErrorString(e);
@@ -217,7 +217,7 @@ static int upload_impl(qk_ctx *c, int type, const uint8_t *w, size_t n_cols, siz
   int st = QK_OK;
   uint8_t *raw = nullptr;
   do {
-    // every byte of a whole chunk is written by the repacking: clear only one with rows missing
+    // every byte of a whole chunk is written by the repacking: clear only one with rows missing and what lies behind
     const uint64_t whole = h->L.rows / QK_TILE_ROWS * h->L.chunk_bytes;
     if (whole < tiled && (e = cudaMemsetAsync(h->dev + whole, 0, tiled - whole, c->stream)) != cudaSuccess) break;
     if (h->algo_bytes == 0) break;

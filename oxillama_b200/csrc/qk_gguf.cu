@@ -283,7 +283,7 @@ extern "C" int qk_weights_upload_gguf(qk_ctx *c, const qk_gguf *g, const char *n
   h->device = c->device, h->dev = nullptr;
   qk_make_layout(type, rows, n_cols, &h->L);
   h->algo_bytes = nbytes;
-  const size_t tiled = h->L.total_bytes ? h->L.total_bytes : 16;
+  const size_t tiled = h->L.total_bytes ? h->L.total_bytes + qk_gemm_tc_pad_bytes(h->L) : 16;
   uint8_t *raw = nullptr, *stage[2] = {nullptr, nullptr};
   cudaEvent_t done[2] = {nullptr, nullptr};
   const size_t piece = (size_t)32 << 20;

@@ -166,7 +166,9 @@ struct QkTcCall {
   uint64_t ldy;
 };
 bool qk_gemm_tc_supported(const QkLayout &L, uint32_t m);
-// The tensor map (128 bytes, 64-byte aligned) through which the kernel fetches a matrix.
+// The tensor map (128 bytes, 64-byte aligned) through which the kernel fetches a matrix: L.total_bytes and
+// this many zeros behind them.
+uint64_t qk_gemm_tc_pad_bytes(const QkLayout &L);
 cudaError_t qk_gemm_tc_map(const QkLayout &L, uint8_t *tiled, void *map);
 // Scratch of a call: the fp16 activations, their scales and, at their most for every call, the partial
 // tiles of a K split (two per CTA; which plan a shape gets then does not change what it needs).

@@ -361,3 +361,21 @@ def test_batches_without_tensor_cores(t, rows, cols, m, launches):
     err, _, n = runtime.cudaGraphGetNodes(graph.raw_cuda_graph())
     assert int(err) == 0 and n <= launches
     dw.free()
+
+
+# Few rows: the last box of 128 rows ends in zeroed chunks behind the matrix (or, where those would be many
+# bytes, outside of it); a shard's end is not the matrix's.
+@pytest.mark.parametrize("t,rows,cols,m", [(S.Q8_0, 8, 1280, 600), (S.Q4_K, 1, 256, 300), (S.IQ4_XS, 120, 768, 70), (S.Q6_K, 129, 512, 40), (S.Q4_K, 8, 262144, 5)])
+def test_matmul_of_few_rows(t, rows, cols, m):
+    import torch
+    from oxillama_b200.device import DeviceWeights, check_device_status
+    w, x = S.gen_weight(t, rows, cols, seed=105), S.gen_acts(m, cols, seed=105)
+    wd = O.dequant_matrix(t, w, rows, cols)
+    assert_product(device_product(t, w, x, rows, cols, m), x, wd, True)
+    b, e = rows // 3, rows - rows // 4
+    dw = DeviceWeights(t, w, rows, cols, row_begin=b, row_end=e)
+    y = torch.full((m, e - b), float("nan"), device="cuda")
+    dw.gemm(torch.from_numpy(x).cuda(), y, m)
+    check_device_status()
+    dw.free()
+    assert_product(y.cpu().numpy(), x, wd[b:e], True)

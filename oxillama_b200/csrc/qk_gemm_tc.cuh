@@ -493,12 +493,13 @@ struct WFmt<QK_T_IQ4_XS> {  // super-block of 256: f16 d, scales_h, scales_l[4],
 // GLU: the row is silu(x) * x2, formed here (crates/oxillama-arch/src/common/swiglu.rs:15-21, each
 // step rounded), so the hidden activations of a feed-forward block are never written out in f32.
 //
-// CT threads keep CCH chunks of eight positions each.  512 threads are the faster conversion, but their
-// CTAs and those of the matmul (24 warps of 80 registers) do not fit on an SM together: the matmul's CTA
+// CT threads keep CCH chunks of eight positions each.  512 threads are the faster conversion of few rows, but
+// their CTAs and those of the matmul (24 warps of 80 registers) do not fit on an SM together: the matmul's CTA
 // there starts, sets itself up and fetches its first weights only when the conversion is over.  From 64 rows
-// of up to 4096 columns (so many CTAs that few SMs are without one) 256 threads of 40 registers run beside
-// a matmul of 72 registers.  Q4_K 4096 x 4096: 37 rows 11.1 (apart) against 11.5 us (beside), 64 rows 13.8
-// against 12.6, 128 rows 19.7 against 18.3.
+// of up to 4096 columns 256 threads of 40 registers run beside a matmul of 72 registers.  Q4_K 4096 x 4096
+// (where the crossing was measured): 37 rows 11.1 (apart) against 11.5 us (beside), 64 rows 13.8 against 12.6, 128
+// rows 19.7 against 18.3.  Short rows keep few of 512 threads busy, so the smaller CTAs pay for Q6_K as well, whose
+// matmul stays at 80 registers: 4096 x 4096 by 64 rows 15.6 -> 13.7 us, by 2048 66.8 -> 62.2, 300 x 256 by 4096 27.0 -> 16.9.
 struct ConvArgs {
   const float *x, *x2;
   __half *out;
@@ -1228,10 +1229,10 @@ cudaError_t launch_fmt(const QkTcCall &c, unsigned *status, unsigned char *scrat
   C.x = c.x, C.x2 = c.x2, C.out = x16, C.scales = scales, C.zero = cnt, C.n_zero = (uint32_t)sm_count * 2;
   C.counts = c.counts, C.lists = c.lists, C.m = c.m, C.cols = L.cols, C.Kp = Kp, C.cap = c.xcap;
   C.list_stride = c.list_stride, C.list_div = c.list_div ? c.list_div : 1u;
-  const bool beside = beside_of(T) && c.n == 1 && !c.counts && c.m >= 64 && Kp <= 4096;
+  const bool narrow = c.n == 1 && !c.counts && c.m >= 64 && Kp <= 4096, beside = beside_of(T) && narrow;
   cudaLaunchAttribute at = pdl_attr();
   cudaLaunchConfig_t c0 = {};
-  c0.gridDim = dim3(c.counts || c.n_act > 1 ? c.n_act * c.xcap : c.m), c0.blockDim = dim3(beside ? 256 : 512), c0.stream = s, c0.attrs = &at, c0.numAttrs = 1;
+  c0.gridDim = dim3(c.counts || c.n_act > 1 ? c.n_act * c.xcap : c.m), c0.blockDim = dim3(narrow ? 256 : 512), c0.stream = s, c0.attrs = &at, c0.numAttrs = 1;
   cudaError_t e;
   if (c.x2 && !c.lists && Kp * 4 <= GLU_SMEM) {
     static QkPerDevice attr_set;
@@ -1247,7 +1248,7 @@ cudaError_t launch_fmt(const QkTcCall &c, unsigned *status, unsigned char *scrat
     c0.blockDim = dim3(512);
     e = cudaLaunchKernelEx(&c0, qk_x16_kernel<T, true, 512, 4>, C);
   } else {
-    e = beside ? cudaLaunchKernelEx(&c0, qk_x16_kernel<T, false, 256, 2>, C) : cudaLaunchKernelEx(&c0, qk_x16_kernel<T, false, 512, 4>, C);
+    e = narrow ? cudaLaunchKernelEx(&c0, qk_x16_kernel<T, false, 256, 2>, C) : cudaLaunchKernelEx(&c0, qk_x16_kernel<T, false, 512, 4>, C);
   }
   if (e != cudaSuccess) return e;
 

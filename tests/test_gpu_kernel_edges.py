@@ -379,3 +379,12 @@ def test_matmul_of_few_rows(t, rows, cols, m):
     check_device_status()
     dw.free()
     assert_product(y.cpu().numpy(), x, wd[b:e], True)
+
+
+# Either form of the activations' conversion (up to 63 rows, from 64 rows of up to 4096 columns, longer ones).
+@pytest.mark.parametrize("cols,m", [(256, 63), (256, 64), (4096, 64), (4352, 64)])
+@pytest.mark.parametrize("t", TC_TYPES)
+def test_conversion_forms(t, cols, m):
+    rows = 100
+    w, x = S.gen_weight(t, rows, cols, seed=106), S.gen_acts(m, cols, seed=106)
+    assert_product(device_product(t, w, x, rows, cols, m), x, O.dequant_matrix(t, w, rows, cols), True)

@@ -689,7 +689,7 @@ struct Sched {
     whole = tiles / pairs;
     R = tiles - whole * pairs;
     const uint32_t total = R * nsb, runs = total / min_run;
-    const uint32_t n = runs < pairs ? (runs ? runs : 1u) : pairs;  // pairs that share the split part
+    const uint32_t n = min(max(max(runs, R), 1u), pairs);           // pairs that share the split part: never fewer than tiles
     base = total / n, rem = total - base * n;                             // the first `rem` runs are one longer
     b = e = first_tile = n_split = 0;
     if (R && me < n) {

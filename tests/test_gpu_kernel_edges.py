@@ -388,3 +388,30 @@ def test_conversion_forms(t, cols, m):
     rows = 100
     w, x = S.gen_weight(t, rows, cols, seed=106), S.gen_acts(m, cols, seed=106)
     assert_product(device_product(t, w, x, rows, cols, m), x, O.dequant_matrix(t, w, rows, cols), True)
+
+
+# Expert layers with one to three super-blocks a row (a tile each to a CTA pair, however few) and rows that the
+# conversion takes in either form, up to 4096 columns and above.
+@pytest.mark.parametrize("t,hidden,inter", [(S.Q4_K, 256, 256), (S.Q8_0, 768, 288), (S.Q6_K, 512, 4352)])
+@pytest.mark.parametrize("tokens", [17, 300])
+def test_moe_short_rows(t, hidden, inter, tokens):
+    import torch
+    from oxillama_b200 import moe
+    from oxillama_b200.device import check_device_status
+    n, top_k, shapes = 4, 2, [(inter, hidden), (inter, hidden), (hidden, inter)]
+    w = [[S.gen_weight(t, r, c, seed=107, stream=3 * e + k, d_range=(1e-3, 3e-3)) for e in range(n)] for k, (r, c) in enumerate(shapes)]
+    x, logits = S.gen_acts(tokens, hidden, seed=108) * np.float32(0.25), S.gen_acts(tokens, n, seed=109)
+    ids, wts = O.moe_route(logits, top_k)
+    ref = np.zeros((tokens, hidden))
+    for e in range(n):
+        g, u, d = (O.dequant_matrix(t, ws[e], r, c).astype(np.float64) for ws, (r, c) in zip(w, shapes))
+        at, slot = np.nonzero(ids == e)
+        hg = x[at] @ g.T
+        ref[at] += wts[at, slot][:, None] * ((hg / (1 + np.exp(-hg)) * (x[at] @ u.T)) @ d.T)
+    ex = moe.MoeExperts(t, *w, hidden, inter, n)
+    y = torch.full((tokens, hidden), float("nan"), device="cuda")
+    ex.forward(torch.from_numpy(logits).cuda(), torch.from_numpy(x).cuda(), y, top_k)
+    check_device_status()
+    ex.free()
+    # three chained products, each within 1e-3 of its largest value (fp16 operands)
+    assert np.abs(y.cpu().numpy() - ref).max() <= 3e-3 * np.abs(ref).max()

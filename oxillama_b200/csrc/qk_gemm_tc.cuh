@@ -499,7 +499,8 @@ struct WFmt<QK_T_IQ4_XS> {  // super-block of 256: f16 d, scales_h, scales_l[4],
 // of up to 4096 columns 256 threads of 40 registers run beside a matmul of 72 registers.  Q4_K 4096 x 4096
 // (where the crossing was measured): 37 rows 11.1 (apart) against 11.5 us (beside), 64 rows 13.8 against 12.6, 128
 // rows 19.7 against 18.3.  Short rows keep few of 512 threads busy, so the smaller CTAs pay for Q6_K as well, whose
-// matmul stays at 80 registers: 4096 x 4096 by 64 rows 15.6 -> 13.7 us, by 2048 66.8 -> 62.2, 300 x 256 by 4096 27.0 -> 16.9.
+// matmul stays at 80 registers: 4096 x 4096 by 64 rows 15.6 -> 13.7 us, by 2048 66.8 -> 62.2, 300 x 256 by 4096 27.0 -> 16.9.  And for
+// the experts of a mixture, whose rows are mostly not live: 16 experts of 1024 x 1024, 900 tokens top 2, 156 -> 129.
 struct ConvArgs {
   const float *x, *x2;
   __half *out;
@@ -1229,7 +1230,7 @@ cudaError_t launch_fmt(const QkTcCall &c, unsigned *status, unsigned char *scrat
   C.x = c.x, C.x2 = c.x2, C.out = x16, C.scales = scales, C.zero = cnt, C.n_zero = (uint32_t)sm_count * 2;
   C.counts = c.counts, C.lists = c.lists, C.m = c.m, C.cols = L.cols, C.Kp = Kp, C.cap = c.xcap;
   C.list_stride = c.list_stride, C.list_div = c.list_div ? c.list_div : 1u;
-  const bool narrow = c.n == 1 && !c.counts && c.m >= 64 && Kp <= 4096, beside = beside_of(T) && narrow;
+  const bool narrow = (c.counts || (c.n == 1 && c.m >= 64)) && Kp <= 4096, beside = beside_of(T) && narrow && !c.counts;
   cudaLaunchAttribute at = pdl_attr();
   cudaLaunchConfig_t c0 = {};
   c0.gridDim = dim3(c.counts || c.n_act > 1 ? c.n_act * c.xcap : c.m), c0.blockDim = dim3(narrow ? 256 : 512), c0.stream = s, c0.attrs = &at, c0.numAttrs = 1;

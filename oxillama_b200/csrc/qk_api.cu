@@ -437,11 +437,12 @@ static int gemm_dispatch(qk_ctx *c, QkScratch &sc, const qk_weights *h, const fl
       return QK_OK;
     }
   }
-  // The tensor-core path rounds its operands to fp16; batches the decode kernels take keep
-  // f32-grade activations.  Decode-sized calls the decode kernels cannot take (K not a
-  // multiple of 256, activations too long for shared memory) go to the generic kernel below.
-  // (Two to four rows of a format whose decode kernel stops below four rows for register
-  // reasons also go to the tensor cores.)
+  // The tensor-core path rounds its operands to fp16; what the decode kernels take keeps f32-grade
+  // activations.  Two to four rows that they do not take go to the tensor cores as well: three and four of
+  // Q6_K (registers), and rows whose split does not fit the shared memory beside the tiles (four of Q4_K and
+  // Q4_0 from 10240 columns, of IQ4_XS from 10496, of Q8_0 from 7680; two of Q8_0 from 12288, of Q6_K from 12544, of
+  // Q4_K and Q4_0 from 16640, of IQ4_XS from 17408).  One row too long for them, and a K that is not a multiple
+  // of 256, go to the generic kernel below.
   const bool tc_small = m <= QK_GEMV_MAX_M && m > 1 && qk_gemv_fast_supported(h->L, 1);
   if (!c->force_simple && (m > QK_GEMV_MAX_M || tc_small) && m < (1u << 30) &&
       qk_gemm_tc_supported(h->L, (uint32_t)m)) {

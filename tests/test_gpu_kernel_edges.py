@@ -76,7 +76,10 @@ def test_tensor_core_matmul_edges(t, rows, cols, m):
 def test_decode_kernel_edges(t, m, rows, cols):
     w, x = S.gen_weight(t, rows, cols, seed=rows + m), S.gen_acts(m, cols, seed=rows + m)
     # (more than one row of 14336 columns may not fit the shared memory beside the tiles: tensor cores)
-    half = t in TC_TYPES and (m > (2 if t == S.Q6_K else 4) or (m > 1 and cols > 8192))
+    # the tensor cores (fp16 operands) take what the decode kernels do not: at 14336 columns those have room beside
+    # the tiles for one split row of Q8_0 and Q6_K, for two of the others
+    most = {S.Q8_0: 1, S.Q6_K: 1}.get(t, 2) if cols == 14336 else 2 if t == S.Q6_K else 4
+    half = t in TC_TYPES and m > most
     assert_product(device_product(t, w, x, rows, cols, m), x, O.dequant_matrix(t, w, rows, cols), half)
 
 
@@ -104,8 +107,9 @@ def test_ffn_edges(tgu, td, hidden, inter, m):
         d.free()
 
 
-# Up to 16 tokens: every expert that is hit, on the decode kernels up to four tokens and on the tensor
-# cores beside them above; one expert takes all tokens, another none; also a shard that starts inside.
+# Up to 16 tokens: every expert that is hit, on the decode kernels up to four rows and on the tensor cores
+# beside them above; one expert takes all tokens, another none; also shards that start inside, with that
+# expert and without.  A token whose experts here have up to four rows each keeps the f32-grade bound.
 @pytest.mark.parametrize("t", [S.Q4_K, S.Q8_0, S.Q6_K, S.IQ4_XS])
 @pytest.mark.parametrize("tokens,top_k", [(1, 1), (1, 3), (2, 2), (4, 2), (5, 1), (9, 3), (16, 2)])
 def test_moe_few_tokens(t, tokens, top_k):
@@ -119,7 +123,7 @@ def test_moe_few_tokens(t, tokens, top_k):
     x = S.gen_acts(tokens, hidden, seed=82) * np.float32(0.25)
     logits = S.gen_acts(tokens, n, seed=83)
     logits[:, 5], logits[:, 1] = -30.0, logits[:, 1] + 6.0
-    for b, e in ((0, n), (1, 4)):
+    for b, e in ((0, n), (1, 4), (2, 6)):
         ids, wts = O.moe_route(logits, top_k)
         ref = np.zeros((tokens, hidden))
         for i in range(tokens):
@@ -133,8 +137,45 @@ def test_moe_few_tokens(t, tokens, top_k):
         ex.forward(torch.from_numpy(logits).cuda(), torch.from_numpy(x).cuda(), y, top_k)
         check_device_status()
         ex.free()
-        half = tokens > (2 if t == S.Q6_K else 4)  # an expert may then have more rows than the decode kernels take
-        assert np.abs(y.cpu().numpy() - ref).max() <= (3e-3 if half else 6e-5) * np.abs(ref).max()
+        check_moe(y.cpu().numpy(), ref, ids, b, e)
+
+
+def check_moe(y, ref, ids, b, e):
+    # three chained products, each within 1e-3 of its largest value on fp16 operands, within 2e-5 in f32
+    local = (ids >= b) & (ids < e)
+    many = local & (np.bincount(ids[ids >= 0], minlength=e)[ids] > 4)
+    bound = np.where(many.any(axis=1), 3e-3, 6e-5)[:, None] * np.abs(ref).max()
+    assert np.all(np.abs(y - ref) <= bound)
+
+
+# The same with a down projection of another format and hidden rows of several k-tiles.
+@pytest.mark.parametrize("t,td,hidden,inter", [(S.Q4_K, S.Q6_K, 512, 4608), (S.IQ4_XS, S.Q8_0, 256, 6400), (S.Q4_0, S.Q4_K, 4352, 512)])
+@pytest.mark.parametrize("tokens", [1, 3, 9])
+def test_moe_few_tokens_mixed(t, td, hidden, inter, tokens):
+    import torch
+    from oxillama_b200 import moe
+    from oxillama_b200.device import DeviceWeights, check_device_status
+    n, top_k = 4, 2
+    shapes = [(t, inter, hidden), (t, inter, hidden), (td, hidden, inter)]
+    w = [[S.gen_weight(q, r, c, seed=83, stream=3 * e + k, d_range=(1e-3, 3e-3)) for e in range(n)] for k, (q, r, c) in enumerate(shapes)]
+    x, logits = S.gen_acts(tokens, hidden, seed=84) * np.float32(0.25), S.gen_acts(tokens, n, seed=84)
+    ids, wts = O.moe_route(logits, top_k)
+    ref = np.zeros((tokens, hidden))
+    for e in range(n):
+        g, u, d = (O.dequant_matrix(q, ws[e], r, c).astype(np.float64) for ws, (q, r, c) in zip(w, shapes))
+        at, slot = np.nonzero(ids == e)
+        hg = x[at] @ g.T
+        ref[at] += wts[at, slot][:, None] * ((hg / (1 + np.exp(-hg)) * (x[at] @ u.T)) @ d.T)
+    dn = [DeviceWeights(td, ws, hidden, inter) for ws in w[2]]
+    ex = moe.MoeExperts(t, w[0], w[1], [S.gen_weight(t, hidden, inter)] * n, hidden, inter, n)
+    ex._d = type(ex._d)(*[d.handle for d in dn])  # (the class uploads one format)
+    y = torch.full((tokens, hidden), float("nan"), device="cuda")
+    ex.forward(torch.from_numpy(logits).cuda(), torch.from_numpy(x).cuda(), y, top_k)
+    check_device_status()
+    check_moe(y.cpu().numpy(), ref, ids, 0, n)
+    ex.free()
+    for d in dn:
+        d.free()
 
 
 # Long rows: a job of the decode kernels holds one row where two split activation rows do not fit beside

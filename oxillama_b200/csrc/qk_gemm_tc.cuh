@@ -252,7 +252,7 @@ __device__ __forceinline__ float4 ldcg4(const float *p) { return __ldcg(reinterp
 // (one weight row x 128 columns: half hh) from the staged super-block and expands them, 32 columns
 // at a time.  Each format expands in the order its packed words yield values; src(p) names the
 // column (inside the super-block) that lands at position p, and the activations are laid out in the
-// same order, so the contraction is unchanged.
+// same order, so the contraction is unchanged.  (Q4_K, whose order spans 64 columns: conv_order.)
 //
 //   BB, BPS   bytes of a block of one row; blocks per super-block.  A staged super-block is
 //             [16 chunks][BPS blocks][8 rows x BB bytes], block-major as in HBM
@@ -301,10 +301,6 @@ struct WFmt<QK_T_Q4_K> {  // d, dmin, 12 bytes of 6-bit scales / mins, 128 bytes
   __device__ static void fill_lut(unsigned char *, uint32_t, uint32_t) {}
   // position 8 i + j of a 64-group <- column 4 i + {0,2,1,3}[j & 3] + 32 (j >> 2): byte 4 i + b of
   // the group's 32 holds column 4 i + b (low nibble) and 32 + 4 i + b (high nibble)
-  __host__ __device__ static uint32_t src(uint32_t p) {
-    const uint32_t g = p >> 6, i = (p >> 3) & 7u, j = p & 7u, jj = j & 3u;
-    return 64 * g + 4 * i + (jj == 1 ? 2 : jj == 2 ? 1 : jj) + 32 * (j >> 2);
-  }
   struct Hd { uint32_t scw, mnw, d; };  // the half's four 6-bit scales and minima, one per byte; d and dmin
   struct Qt { uint4 q; };
   // [8 rows x 16 header | 4 groups x 8 rows x 32 nibble bytes]
@@ -484,7 +480,7 @@ struct WFmt<QK_T_IQ4_XS> {  // super-block of 256: f16 d, scales_h, scales_l[4],
 };
 
 // ---------------------------------------------------------------- activations -> fp16
-// X16[t][256 s + p] = x[t][256 s + src(p)] / scale[t] in fp16, where scale[t] is the power
+// X16[t][256 s + p] = x[t][256 s + (its format's src of p)] / scale[t] in fp16, where scale[t] is the power
 // of two that puts the row's largest magnitude in [512, 1024) (2^-126 at least): the division is
 // exact, no activation overflows, only those below 2^-24 of the largest fall into fp16's subnormals, and the
 // epilogue multiplies the row of results by scale[t] again (also exact).  Columns >= cols are zero.  One CTA per token
@@ -520,7 +516,7 @@ __device__ __forceinline__ void conv_order(const float (&a)[4], const float (&b)
 #pragma unroll
   for (int j = 0; j < 8; j++) {
     uint32_t e;  // which of the eight values lands at position j
-    if (T == QK_T_Q4_K) e = (j & 4) + ((j & 3) == 1 ? 2 : (j & 3) == 2 ? 1 : (j & 3));
+    if constexpr (T == QK_T_Q4_K) e = (j & 4) + ((j & 3) == 1 ? 2 : (j & 3) == 2 ? 1 : (j & 3));
     else e = WFmt<T>::src((uint32_t)j);
     v[j] = e < 4 ? a[e & 3] : b[e & 3];
   }

@@ -746,7 +746,7 @@ cudaError_t launch_mma(const QkLayout &L, const uint8_t *W, const float *x, floa
                                        peers ? peers->wait_epoch : nullptr, peers ? peers->wait_ld : (uint64_t)0, status);
     if (e != cudaSuccess) return e;
   }
-  static int ctas = -1;  // developer knob: persistent CTAs per SM (they must fit: see QK_CW, QK_NSTAGE)
+  static int ctas = -1;  // developer knob: persistent CTAs per SM (they must fit: see QK_NSTAGE)
   if (ctas < 0) {
     const char *e = qk_knob("QK_CTAS");
     ctas = (e && atoi(e) == 2) ? 2 : 1;

@@ -23,6 +23,7 @@
  *    activations in scratch of the context between their kernels: issue those of one context on one
  *    stream, or on streams ordered by events.  Calls that overlap on the GPU race on that scratch.
  *    The host-pointer entry points have scratch of their own and may follow at any time.
+ *  - An activation row with an infinity or a NaN in it yields no finite result.
  *  - There is no CPU fallback: without a usable CUDA device every compute
  *    entry point fails with QK_CUDA_ERROR.
  */
@@ -55,7 +56,7 @@ typedef enum qk_status {
 #define QK_TYPE_Q4_0 2
 #define QK_TYPE_Q8_0 8
 #define QK_TYPE_Q4_K 12
-#define QK_TYPE_Q5_K 13 /* Q5_K, Q2_K, Q3_K: decode kernels, larger batches in pieces; Q8_K: generic kernels only */
+#define QK_TYPE_Q5_K 13 /* Q5_K, Q2_K, Q3_K: decode kernels, larger batches in pieces (small matrices: generic kernel); Q8_K: generic kernels only */
 #define QK_TYPE_Q2_K 10
 #define QK_TYPE_Q3_K 11
 #define QK_TYPE_Q8_K 15
@@ -66,6 +67,7 @@ typedef struct qk_ctx qk_ctx;         /* one GPU + its stream and scratch */
 typedef struct qk_weights qk_weights; /* one weight matrix (or row shard) resident in HBM */
 
 /* ---- context: stands where KernelDispatcher::new() stands (dispatch.rs:128-131) ---- */
+/* Holds about 86 MB of the GPU's memory from the start (scratch of device and of host calls). */
 int qk_init(int device, qk_ctx **out);
 int qk_shutdown(qk_ctx *ctx);
 /* Copies the text of the last error raised on this context (empty if none). */
@@ -226,7 +228,8 @@ int qk_moe_route_dev(qk_ctx *ctx, const float *logits_dev, size_t tokens, size_t
  * At most 16 local experts, equal formats: the call does not synchronise (a fixed sequence of
  * launches on `stream`; the token counts stay on the device).  More than 16 tokens take one grouped
  * matmul launch per projection, fewer one decode-kernel launch per projection over all experts
- * that are hit.  Otherwise (mixed or other formats, more local experts, few tokens) the experts
+ * that are hit.  Otherwise (mixed or other formats, more local experts; few tokens whose K is
+ * so long that the decode kernels do not take it, or one row at a time with more than 32 rows routed) the experts
  * run one after the other and the call synchronises `stream` once to read the counts that size them.  The context
  * keeps the device scratch, grown (with a device synchronise) on first use of a larger size. */
 int qk_moe_ffn_dev(qk_ctx *ctx, const qk_weights *const *gate, const qk_weights *const *up,

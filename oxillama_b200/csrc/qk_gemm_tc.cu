@@ -76,7 +76,7 @@ static uint32_t round_up(uint32_t v, uint32_t to) { return (v + to - 1) / to * t
 // Form of the kernel, token-tile width and K split by predicted time: cycles of the slowest CTA.  The
 // constants are a fit to 46 shapes (300 x 8192 .. 14336 x 4096, 8 .. 2048 tokens, Q4_K, Q6_K, Q8_0, Q4_0), each
 // timed with every tile width and split: the prediction is 10 % off (rms), the form it picks 0.8 % slower than
-// the fastest (mean).  A super-block takes as long as its expansion, which loads of wider activations slow down,
+// the fastest (mean).  (IQ4_XS takes Q4_K's: its times are within 5 % of Q4_K's but at 128 tokens.)  A super-block takes as long as its expansion, which loads of wider activations slow down,
 // or in a pair the round of hand-overs (expanding warps -> issuer -> tensor pipe -> back).  A tile whose
 // partials go through the workspace costs some 8000 cycles and 58 per token (writing them out, the fence, the
 // counter, reading them back); through the cluster 5300, whatever its width.

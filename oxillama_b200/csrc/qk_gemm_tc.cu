@@ -83,13 +83,9 @@ static uint32_t round_up(uint32_t v, uint32_t to) { return (v + to - 1) / to * t
 bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
   const QkLayout &L = *c.L;
   const uint32_t w_stage = 16u * 8u * L.bb * (256u / L.bs), lut = L.type == QK_T_IQ4_XS ? WFmt<QK_T_IQ4_XS>::LUT : 0u;
-  const bool many = c.n > 1 || c.counts;
   TcPlan p;
   p.nsb = (L.cols + 255u) / 256u, p.cs = 1;
-  auto half_of = [&](uint32_t bn, uint32_t cg) {
-    const uint32_t h = bn <= 128 ? bn : round_up((bn + 1) / 2, 16);
-    return many ? round_up(h, 32 * cg) : h;  // groups: boxes come in quarters of whole 8-row swizzle atoms per CTA
-  };
+  auto half_of = [&](uint32_t bn) { return bn <= 128 ? bn : round_up((bn + 1) / 2, 16); };
   if (c.counts) {
     // Counts on the device: tiles wide enough for a group somewhat above the average, so that most
     // groups take one (the MMA covers only a tile's live tokens, rounded up to 16).
@@ -146,7 +142,7 @@ bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
       }
     }
   }
-  p.hn = half_of(p.bn, p.cg);
+  p.hn = half_of(p.bn);
   if (!plan_smem(p.hn, p.cg, p.cs, w_stage, lut, &p.S, &p.smem)) return false;
   p.xrows = c.counts || c.n_act > 1 ? c.n_act * c.xcap : p.tok_blocks * p.bn;
   const size_t Kp = (size_t)p.nsb * 256u;

@@ -59,6 +59,7 @@
 #pragma once
 #include <cuda.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <cstdlib>
@@ -108,8 +109,10 @@ struct TcArgs {
   const int *counts;               // device: live rows per activation group, or null (m rows each)
 };
 // Tensor maps: the matrices, and the fp16 activations as boxes of 64 columns x h tokens x the steps of
-// a stage: h = hn, or one of the quarters of it where the live tokens of a group are known on the
-// device only.
+// a stage: h = this CTA's share of hn, or one to four times box_unit where the live tokens of a group are
+// known on the device only (whole atoms of 8 rows, and never more than the share, so that a stage is no
+// larger than the tile: hn rounded up to four boxes of whole atoms had left tiles of 96 tokens two weight stages).
+__host__ __device__ constexpr uint32_t box_unit(uint32_t own) { return (own / 4 + 7) / 8 * 8; }
 template <int NG>
 struct TcMaps {
   CUtensorMap x[NG > 1 ? 4 : 1];
@@ -125,6 +128,15 @@ __device__ __forceinline__ bool elect_one() {
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) {
   if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity));
+}
+// Whether the phase is over, without waiting.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(ok)
+               : "r"(bar), "r"(parity)
+               : "memory");
+  return ok != 0;
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
@@ -285,10 +297,24 @@ __device__ __forceinline__ uint32_t word(const uint4 &v, int i) { return i == 0 
 // Four nibble pairs of one packed word -> 8 halves: low nibbles q become 1024 + q
 // (0x6400 | q), high nibbles 64 + q (0x5400 | q << 4, no shift needed); values come out
 // as pairs (byte 0, byte 2), (byte 1, byte 3) of the low nibbles, then of the high ones.
-__device__ __forceinline__ void nibbles_to_magic(uint32_t w, uint32_t e[4]) {
+// The exponents come from registers: an instruction takes one constant of 32 bits, and with two of them the
+// compiler makes two of every mask-and-or (157 -> 99 integer instructions a thread and super-block).
+struct NibbleMagic { uint32_t lo, hi; };
+__device__ __forceinline__ NibbleMagic nibble_magic() {
+  NibbleMagic k;
+  asm volatile("mov.b32 %0, 0x64006400;" : "=r"(k.lo));
+  asm volatile("mov.b32 %0, 0x54005400;" : "=r"(k.hi));
+  return k;
+}
+__device__ __forceinline__ uint32_t and_or(uint32_t w, uint32_t mask, uint32_t v) {
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(w), "r"(mask), "r"(v));
+  return d;
+}
+__device__ __forceinline__ void nibbles_to_magic(uint32_t w, const NibbleMagic &k, uint32_t e[4]) {
   const uint32_t wj = w >> 8;
-  e[0] = (w & 0x000F000Fu) | 0x64006400u, e[1] = (wj & 0x000F000Fu) | 0x64006400u;
-  e[2] = (w & 0x00F000F0u) | 0x54005400u, e[3] = (wj & 0x00F000F0u) | 0x54005400u;
+  e[0] = and_or(w, 0x000F000Fu, k.lo), e[1] = and_or(wj, 0x000F000Fu, k.lo);
+  e[2] = and_or(w, 0x00F000F0u, k.hi), e[3] = and_or(wj, 0x00F000F0u, k.hi);
 }
 // Four unsigned bytes -> halves 1024 + b, in byte order.
 __device__ __forceinline__ void bytes_to_magic(uint32_t w, uint32_t &lo, uint32_t &hi) {
@@ -323,10 +349,11 @@ struct WFmt<QK_T_Q4_K> {  // d, dmin, 12 bytes of 6-bit scales / mins, 128 bytes
     const __half2 s_hi = __hmul2(__hsub2(bits_h2(prmt(c.scw, 0x64646464u, hi)), k1024), d);
     const __half2 m_lo = __hmul2(__hsub2(bits_h2(prmt(c.mnw, 0x64646464u, lo)), k1024), m);
     const __half2 m_hi = __hmul2(__hsub2(bits_h2(prmt(c.mnw, 0x64646464u, hi)), k1024), m);
+    const NibbleMagic km = nibble_magic();
 #pragma unroll
     for (int i = 0; i < 4; i++) {
       uint32_t e[4];
-      nibbles_to_magic(word(t.q, i), e);
+      nibbles_to_magic(word(t.q, i), km, e);
       o[4 * i + 0] = h2_bits(__hfma2(__hsub2(bits_h2(e[0]), k1024), s_lo, m_lo));
       o[4 * i + 1] = h2_bits(__hfma2(__hsub2(bits_h2(e[1]), k1024), s_lo, m_lo));
       o[4 * i + 2] = h2_bits(__hfma2(__hsub2(bits_h2(e[2]), k_hi), s_hi, m_hi));
@@ -383,10 +410,11 @@ struct WFmt<QK_T_Q4_0> {  // block of 32: f16 d, 16 bytes; byte j = elements 2 j
   __device__ static void expand(const Qt &t, const Hd &, uint32_t, uint32_t (&o)[16], uint32_t) {
     const __half2 off_lo = __float2half2_rn(1032.f), off_hi = __float2half2_rn(72.f);  // (K + q) - (K + 8) = q - 8, exact
     const __half2 d = __low2half2(bits_h2(t.d));
+    const NibbleMagic km = nibble_magic();
 #pragma unroll
     for (int i = 0; i < 4; i++) {
       uint32_t e[4];
-      nibbles_to_magic(word(t.q, i), e);
+      nibbles_to_magic(word(t.q, i), km, e);
       o[4 * i + 0] = h2_bits(__hmul2(__hsub2(bits_h2(e[0]), off_lo), d));
       o[4 * i + 1] = h2_bits(__hmul2(__hsub2(bits_h2(e[1]), off_lo), d));
       o[4 * i + 2] = h2_bits(__hmul2(__hsub2(bits_h2(e[2]), off_hi), d));
@@ -718,14 +746,16 @@ struct TileAt {
 
 // The super-blocks of a segment in the order the MMAs take them: one at a time (`half` 0, then 1),
 // but at either end of a wide tile two at a time (both under half 0, then both under half 1).
-// Calls step(sb, half, which of the two, last use of the super-block's weights, end of the segment) -> false to stop.
-template <class Step>
-__device__ __forceinline__ bool walk_segment(uint32_t s0, uint32_t s1, bool wide, Step &&step) {
+// Calls step(sb, half, which of the two, last use of the super-block's weights, end of the segment) -> false to stop,
+// and after every one or two super-blocks next(how many).
+template <class Step, class Next>
+__device__ __forceinline__ bool walk_segment(uint32_t s0, uint32_t s1, bool wide, Step &&step, Next &&next) {
   for (uint32_t sb = s0; sb < s1;) {
     const uint32_t two = wide && s1 - sb >= 2 && (sb == s0 || s1 - sb == 2) ? 2u : 1u;
     for (uint32_t h = 0; h < (wide ? 2u : 1u); h++)
       for (uint32_t k = 0; k < two; k++)
         if (!step(sb + k, h, k, h == (wide ? 1u : 0u), sb + k + 1 == s1)) return false;
+    next(two);
     sb += two;
   }
   return true;
@@ -815,8 +845,9 @@ __global__ void __maxnreg__(REGS)
     return q;
   };
   // Token rows that an activation box brings: each CTA of a pair loads half of the n tokens.
-  const uint32_t hq = A.hn / (4 * CG);
-  auto box_rows = [&](uint32_t n) { return NG > 1 ? (n / CG + hq - 1) / hq * hq : A.hn / CG; };
+  const uint32_t hq = box_unit(A.hn / CG);
+  auto box_of = [&](uint32_t n) { return NG > 1 ? (n / CG + hq - 1) / hq : 1u; };  // the how-manieth box (from 1)
+  auto box_rows = [&](uint32_t n) { return NG > 1 ? min(box_of(n) * hq, A.hn / CG) : A.hn / CG; };
 
   // The last contributor of a split tile adds the partials up, in the order of their K runs: a warp four
   // tokens at a time, a lane four rows.
@@ -863,53 +894,84 @@ __global__ void __maxnreg__(REGS)
   bool dead = false;
   if (warp == 0 && rank == 0) {
     // ======================= MMA issuer =======================
+    // Narrow tiles are bound by this loop unless it is short: beside its 16 MMAs (14 cycles each) a step has room
+    // for some 500 cycles before it takes longer than the expansion.  So what a segment does not change is worked
+    // out ahead of its steps, and the next step's barriers are looked at (without waiting) behind the commits.  (As
+    // one general step per super-block and half, worked out anew each time: 1250 cycles at 8 to 128 tokens.)
     const uint32_t lead = elect_one() ? 1u : 0u;
+    const uint32_t a_full = sbase + S.a_full, a_empty = sbase + S.a_empty, b_full = sbase + S.b_full, b_empty = sbase + S.b_empty;
+    const uint32_t nbs = S.b_stages, stage16 = S.b_stage >> 4, bd0 = umma_desc_lo(sbase + S.b), a0 = tmem + a_col;
     uint32_t bs = 0, bph = 0, ab = 0, aph = 0, dph = 0;  // dph bit h: parity of the next wait for half h; bit 2 + h: it was used before
+    bool ready = false;                                  // (this lane) the next step's operands were there when last looked at
+    auto take_half = [&](uint32_t dh) {                  // a segment's first MMA into an accumulator
+      if ((dph >> (2 + dh)) & 1u) {
+        if (!warp_wait(sbase + S.d_empty + dh * 8, (dph >> dh) & 1u)) return false;
+        dph ^= 1u << dh;
+      }
+      dph |= 4u << dh;
+      return true;
+    };
+    auto issue16 = [&](uint32_t d, uint32_t a, uint32_t bd, uint32_t step16, uint32_t idesc, uint32_t acc) {
+#pragma unroll
+      for (uint32_t g = 0; g < 4; g++)
+#pragma unroll
+        for (uint32_t j = 0; j < 4; j++) umma_f16_ta<CG>(d, a + g * 32 + j * 8, bd + g * step16 + j * 2, idesc, g || j ? 1u : acc, lead);
+    };
     for (uint32_t i = 0; i < sc.n_seg && !dead; i++) {
       uint32_t tile, s0, s1;
       sc.get(i, tile, s0, s1);
       const TileAt q = at(tile);
-      const bool wide = q.n > A.hn;
-      uint32_t begun = 0;      // halves whose accumulator this segment has taken over
-      uint32_t ab1 = 0;        // (two super-blocks at a time) buffers are walked again under the second half
-      const bool ok = walk_segment(s0, s1, wide, [&](uint32_t, uint32_t h, uint32_t k, bool last, bool end) {
-        const uint32_t n = h ? q.n - A.hn : wide ? A.hn : q.n, dh = both ? h : i & alt;
-        const uint32_t step16 = box_rows(n) * 8u;  // a step of the activation stage, in units of 16 bytes
-        const uint32_t idesc = (1u << 4) | ((n >> 3) << 17) | ((CG * BM >> 4) << 24), d = tmem + dh * d_step;
-        uint32_t acc = 1u;
-        if (!(begun & (1u << h))) {
-          begun |= 1u << h, acc = 0u;
-          if ((dph >> (2 + dh)) & 1u) {
-            if (!warp_wait(sbase + S.d_empty + dh * 8, (dph >> dh) & 1u)) return false;
-            dph ^= 1u << dh;
+      const bool wide = CG == 2 && q.n > A.hn;
+      const uint32_t n0 = wide ? A.hn : q.n, idesc0 = (1u << 4) | ((n0 >> 3) << 17) | ((CG * BM >> 4) << 24);
+      const uint32_t step0 = box_rows(n0) * 8u;  // a step of the activation stage, in units of 16 bytes
+      if (!wide) {
+        const uint32_t dh = both ? 0u : i & alt, d = tmem + dh * d_step;
+        if (!take_half(dh)) {
+          dead = true;
+          break;
+        }
+        uint32_t acc = 0u;
+        for (uint32_t sb = s0; sb < s1; sb++) {
+          if (!__all_sync(0xffffffffu, ready) && !(warp_wait(a_full + ab * 8, aph) && warp_wait(b_full + bs * 8, bph))) {
+            dead = true;
+            break;
           }
-          dph |= 4u << dh;
-        }
-        if (h == 0) {
-          if (k == 0) ab1 = ab;
-          if (!warp_wait(sbase + S.a_full + ab * 8, aph)) return false;
           tc_fence_after();
-        } else if (k == 0) {
-          ab = ab1;
+          issue16(d, a0 + ab * 128u, bd0 + bs * stage16, step0, idesc0, acc);
+          umma_commit<CG>(b_empty + bs * 8, lead);
+          umma_commit<CG>(a_empty + ab * 8, lead);
+          acc = 1u;
+          if (++bs == nbs) bs = 0, bph ^= 1u;
+          if (++ab == na) ab = 0, aph ^= 1u;
+          ready = mbar_test(a_full + ab * 8, aph) & mbar_test(b_full + bs * 8, bph);
         }
-        const uint32_t a = tmem + a_col + ab * 128u;
-        if (!warp_wait(sbase + S.b_full + bs * 8, bph)) return false;
-        const uint32_t bd = umma_desc_lo(sbase + S.b + bs * S.b_stage);
-#pragma unroll
-        for (uint32_t g = 0; g < 4; g++)
-#pragma unroll
-          for (uint32_t j = 0; j < 4; j++) umma_f16_ta<CG>(d, a + g * 32 + j * 8, bd + g * step16 + j * 2, idesc, g || j ? 1u : acc, lead);
-        umma_commit<CG>(sbase + S.b_empty + bs * 8, lead);
-        if (++bs == S.b_stages) bs = 0, bph ^= 1u;
-        if (last) umma_commit<CG>(sbase + S.a_empty + ab * 8, lead);
-        if (end) umma_commit<CG>(sbase + S.d_full + dh * 8, lead);
-        if (++ab == na) {
-          ab = 0;
-          if (h == 0) aph ^= 1u;
-        }
-        return true;
-      });
-      if (!ok) dead = true;
+        if (!dead) umma_commit<CG>(sbase + S.d_full + dh * 8, lead);
+      } else {
+        // Two accumulator halves: one super-block at a time under half 0, then half 1, but at either end of the
+        // segment two at a time (walk_segment); the buffers are walked again under the second half.
+        const uint32_t n1 = q.n - A.hn, idesc1 = (1u << 4) | ((n1 >> 3) << 17) | ((CG * BM >> 4) << 24), step1 = box_rows(n1) * 8u;
+        ready = false;
+        if (!walk_segment(s0, s1, true, [&](uint32_t sb, uint32_t h, uint32_t k, bool last, bool end) {
+              if (sb == s0 && !take_half(h)) return false;
+              uint32_t abk = ab + k, ph = aph;
+              if (abk >= na) abk -= na, ph ^= 1u;
+              if (h == 0) {
+                if (!warp_wait(a_full + abk * 8, ph)) return false;
+                tc_fence_after();
+              }
+              if (!warp_wait(b_full + bs * 8, bph)) return false;
+              issue16(tmem + h * d_step, a0 + abk * 128u, bd0 + bs * stage16, h ? step1 : step0, h ? idesc1 : idesc0, sb == s0 ? 0u : 1u);
+              umma_commit<CG>(b_empty + bs * 8, lead);
+              if (last) umma_commit<CG>(a_empty + abk * 8, lead);
+              if (end) umma_commit<CG>(sbase + S.d_full + h * 8, lead);
+              if (++bs == nbs) bs = 0, bph ^= 1u;
+              return true;
+            }, [&](uint32_t two) {
+              ab += two;
+              if (ab >= na) ab -= na, aph ^= 1u;
+            }))
+          dead = true;
+      }
     }
     if (dead) {  // let what was issued retire before the CTA gives its memory back
       if (lead) atomicOr(A.status, QK_DEV_TIMEOUT);
@@ -927,20 +989,20 @@ __global__ void __maxnreg__(REGS)
       uint32_t tile, s0, s1;
       sc.get(i, tile, s0, s1);
       const TileAt q = at(tile);
-      const bool wide = q.n > A.hn;
+      const bool wide = CG == 2 && q.n > A.hn;
+      const uint32_t n0 = wide ? A.hn : q.n, n1 = wide ? q.n - A.hn : 0u, rows0 = box_rows(n0), rows1 = box_rows(n1);
       const uint32_t row0 = (NG > 1 ? (q.g % A.n_act) * A.xcap : 0u) + q.t0;
+      const int r0 = (int)(row0 + (rank ? n0 / 2 : 0u)), r1 = (int)(row0 + A.hn + (rank ? n1 / 2 : 0u));
+      const CUtensorMap *map0 = &M.x[box_of(n0) - 1], *map1 = &M.x[wide ? box_of(n1) - 1 : 0];
       const bool ok = walk_segment(s0, s1, wide, [&](uint32_t sb, uint32_t h, uint32_t, bool, bool) {
-        const uint32_t n = h ? q.n - A.hn : wide ? A.hn : q.n, rows = box_rows(n);
-        const uint32_t r0 = row0 + (h ? A.hn : 0u) + (rank ? n / 2 : 0u);
-        const CUtensorMap *map = &M.x[NG > 1 ? rows / hq - 1 : 0];
         if (rounds && !warp_wait(bar + to_empty, bph ^ 1u)) return false;
         // the halves of both CTAs land on the barrier of rank 0, which alone announces them
-        if (rank == 0) expect_tx(bar, rows * 512u * CG, lead);
-        tma_load_3d<CG>(dst, map, 0, (int)r0, (int)(sb * 4), full, lead);
+        if (rank == 0) expect_tx(bar, (h ? rows1 : rows0) * 512u * CG, lead);
+        tma_load_3d<CG>(dst, h ? map1 : map0, 0, h ? r1 : r0, (int)(sb * 4), full, lead);
         bs++, bar += 8, full += 8, dst += stage;
         if (bs == nst) bs = 0, bph ^= 1u, rounds = 1, bar = sbase + S.b_full, full = full0, dst = sbase + S.b;
         return true;
-      });
+      }, [](uint32_t) {});
       if (!ok) dead = true;
     }
     if (dead) {
@@ -1199,7 +1261,7 @@ cudaError_t launch_main(const TcPlan &P, const TcArgs &A, __half *x16, const QkT
   }
   TcMaps<NG> M;
   for (uint32_t k = 0; k < (NG > 1 ? 4u : 1u); k++)
-    if (!x_map(&M.x[k], x16, P.xrows, P.nsb * 256u, NG > 1 ? P.hn / (4 * CG) * (k + 1) : P.hn / CG)) return cudaErrorInvalidValue;
+    if (!x_map(&M.x[k], x16, P.xrows, P.nsb * 256u, NG > 1 ? std::min(box_unit(P.hn / CG) * (k + 1), P.hn / CG) : P.hn / CG)) return cudaErrorInvalidValue;
   for (uint32_t g = 0; g < (NG == 1 ? 1u : c.n); g++) memcpy(&M.w[g], c.maps[g], sizeof(CUtensorMap));
   cudaLaunchAttribute at[2] = {pdl_attr(), {}};
   at[1].id = cudaLaunchAttributeClusterDimension;

@@ -456,3 +456,34 @@ def test_moe_short_rows(t, hidden, inter, tokens):
     ex.free()
     # three chained products, each within 1e-3 of its largest value (fp16 operands)
     assert np.abs(y.cpu().numpy() - ref).max() <= 3e-3 * np.abs(ref).max()
+
+
+# Groups of every size around the activation boxes (one to four of whole 8-row atoms): tiles of 64 tokens in one CTA
+# and of 96 and 160 in a pair.  The bound: three chained products, each within 1e-3 of its largest value.
+@pytest.mark.parametrize("counts", [[1, 15, 16, 17, 47, 48, 49, 64, 65, 0], [96, 97, 64, 65, 81, 80, 1, 33, 95, 20],
+                                    [160, 161, 128, 127, 40, 41, 79, 300, 2, 0]])
+@pytest.mark.parametrize("t", [S.Q4_K, S.IQ4_XS])
+def test_moe_group_sizes(t, counts):
+    import torch
+    from oxillama_b200 import moe
+    from oxillama_b200.device import check_device_status
+    n, hidden, inter = len(counts), 512, 768
+    shapes = [(inter, hidden), (inter, hidden), (hidden, inter)]
+    w = [[S.gen_weight(t, r, c, seed=111, stream=3 * e + k, d_range=(1e-3, 3e-3)) for e in range(n)] for k, (r, c) in enumerate(shapes)]
+    which = np.random.default_rng(112).permutation(np.repeat(np.arange(n), counts))
+    tokens = len(which)
+    x = S.gen_acts(tokens, hidden, seed=113) * np.float32(0.25)
+    logits = np.zeros((tokens, n), np.float32)
+    logits[np.arange(tokens), which] = 9.0
+    ref = np.zeros((tokens, hidden))
+    for e in range(n):
+        g, u, d = (O.dequant_matrix(t, ws[e], r, c).astype(np.float64) for ws, (r, c) in zip(w, shapes))
+        at = which == e
+        hg = x[at] @ g.T
+        ref[at] = (hg / (1 + np.exp(-hg)) * (x[at] @ u.T)) @ d.T
+    ex = moe.MoeExperts(t, *w, hidden, inter, n)
+    y = torch.full((tokens, hidden), float("nan"), device="cuda")
+    ex.forward(torch.from_numpy(logits).cuda(), torch.from_numpy(x).cuda(), y, 1)
+    check_device_status()
+    ex.free()
+    assert np.abs(y.cpu().numpy() - ref).max() <= 3e-3 * np.abs(ref).max()

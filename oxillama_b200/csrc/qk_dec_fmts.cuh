@@ -97,6 +97,7 @@ struct DecQ80 {
   static constexpr int MAX_M = 4;
   static constexpr bool HAS_DUAL = true, HAS_PEER = true;
   static constexpr bool SPLIT_PRODUCER = true;  // the tile producer as a warp of its own (measured per format)
+  static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (make_plan_mma)
   // digit order inside a 32-column block: the lane's 8 bytes are columns 4 tig .. + 3 and
   // 16 + 4 tig .. + 3, the two 4-byte pieces of its A fragment (bytes 4 tig of both 16-byte granules)
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
@@ -168,6 +169,7 @@ struct DecQ40 {
   static constexpr int MAX_M = 4;
   static constexpr bool HAS_DUAL = true, HAS_PEER = true;
   static constexpr bool SPLIT_PRODUCER = true;  // the tile producer as a warp of its own (measured per format)
+  static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (make_plan_mma)
   // The lane's word (bytes 4 tig .. + 3 of the block) holds elements 8 tig .. + 7: low
   // nibbles the even ones, high nibbles the odd ones.  Digits go evens first, then odds,
   // inside every group of 8 columns.
@@ -249,6 +251,7 @@ struct DecIQ4XS {
   static constexpr int MAX_M = 4;
   static constexpr bool HAS_DUAL = true, HAS_PEER = true;
   static constexpr bool SPLIT_PRODUCER = true;  // the tile producer as a warp of its own (measured per format)
+  static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (make_plan_mma)
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
                                                       uint32_t w1, uint32_t w2) {
     store_digits_natural(row_img, PS, e0, w0, w1, w2);
@@ -344,10 +347,17 @@ struct DecQ6K {
   static constexpr uint32_t COLB = 1680, XSB = 16;
   static constexpr bool HAS_DUAL = false, HAS_PEER = true;
   static constexpr bool SPLIT_PRODUCER = false;  // the tile producer as a warp of its own (measured per format)
+  static constexpr bool ANY_DEPTH = true;  // ring depths that are no multiple of the groups (make_plan_mma)
   static constexpr int MAX_M = 2;  // three rows and up spill heavily (twelve weight words and sixteen fragments per column)
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
                                                       uint32_t w1, uint32_t w2) {
-    store_digits_natural(row_img, PS, e0, w0, w1, w2);
+    // a span's 256 bytes of a plane: [blocks 0-3, 4-7][strip][word of the strip][block]: a lane's words of four
+    // blocks are one 128-bit load
+    const uint32_t i = (e0 >> 5) & 7u;
+    unsigned char *p = row_img + (e0 & ~255u) + (i >> 2) * 128 + ((e0 >> 2) & 7u) * 16 + (i & 3u) * 4;
+    *reinterpret_cast<uint32_t *>(p) = w0;
+    *reinterpret_cast<uint32_t *>(p + PS) = w1;
+    *reinterpret_cast<uint32_t *>(p + 2 * PS) = w2;
   }
   // (sx, sum over the 32 columns, sums over its two 16-column strips)
   __device__ static __forceinline__ void store_xs(unsigned char *tab, size_t blk, float sx, float s32, float s16a,
@@ -360,11 +370,11 @@ struct DecQ6K {
     uint32_t qh[4];  // [G * 2 + is]
     uint32_t sc, dd; // scales 4 tig .. + 3 of row g (int8 x 4), f16 d
     float4 xs[M][2]; // scale table entries of 32-column blocks 2 tig, 2 tig + 1
-    uint32_t b[M][8];  // [G * 4 + k]: the lane's four digits of its strip of block 4 G + k
+    uint4 b[M][2];     // [G], word k: the lane's four digits of its strip of block 4 G + k
   };
   struct Lane {
     float kD;
-    uint32_t wl0, sl0, dl, xl, xsl, xm, xsm, m0, m1;
+    uint32_t wl0, sl0, dl, xl, xsl, xm, xsm;
     __device__ __forceinline__ void init(uint32_t lane, uint32_t wl, uint32_t ximg, uint32_t PS, uint32_t xs_off,
                                          uint32_t Kp) {
       const uint32_t g = lane >> 2, tig = lane & 3;
@@ -372,12 +382,11 @@ struct DecQ6K {
       wl0 = wl * COLB + g * 16 + tig * 4;
       sl0 = wl * COLB + 1536 + g * 16 + tig * 4;
       dl = wl * COLB + 1664 + 2 * g;
-      // B column g: digit g / 2 of strip g & 1 (columns 6, 7 unused): four bytes of the natural-order plane
-      const uint32_t b_off = (g < 6 ? (g >> 1) : 2u) * PS + (g & 1u) * 16u + tig * 4;
+      // B column g: digit g / 2 of strip g & 1 (columns 6, 7 unused)
+      const uint32_t b_off = (g < 6 ? (g >> 1) : 2u) * PS + (g & 1u) * 64u + tig * 16;
       xl = ximg + b_off + wl * 256;
       xsl = ximg + xs_off + (wl * 8 + 2 * tig) * 16;
       xm = 3 * PS, xsm = (Kp / 32) * 16;
-      m0 = (g & 1u) ? 0u : 0xFFFFFFFFu, m1 = ~m0;  // an even column is zero in k-slots 16-31, an odd one in 0-15
     }
   };
   struct Base {
@@ -404,10 +413,7 @@ struct DecQ6K {
       D.xs[m][0] = lds128fo<J * WG * 128>(B.xs + m * LN.xsm);
       D.xs[m][1] = lds128fo<J * WG * 128 + 16>(B.xs + m * LN.xsm);
       const uint32_t xb = B.x + m * LN.xm;
-      static_for<0, 8>([&](auto iq) {
-        constexpr int I = decltype(iq)::value;  // G * 4 + k: columns 128 G + 32 k
-        D.b[m][I] = lds32o<J * WG * 256 + I * 32>(xb);
-      });
+      D.b[m][0] = lds128o<J * WG * 256>(xb), D.b[m][1] = lds128o<J * WG * 256 + 128>(xb);
     }
   }
   template <int M>
@@ -417,7 +423,9 @@ struct DecQ6K {
     float ds[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) ds[j] = d * (float)(int)(signed char)((D.sc >> (8 * j)) & 0xFFu);
-    // the A fragments: strip is = 0 in k-slots 0-15 (a[.][0]), is = 1 in slots 16-31 (a[.][1])
+    // the A fragments, k = 16 of the MMA being one strip: rows 0-7 are the weight rows' strip 0 (a[.][0]), rows
+    // 8-15 their strip 1 (a[.][1]), so an even column meets strip 0 in c[0] and an odd one strip 1 in c[3].  (With
+    // k = 32 as strip 0 | strip 1 every B word had to be masked for either half.)
     uint32_t a[8][2];
 #pragma unroll
     for (int G = 0; G < 2; G++)
@@ -441,7 +449,7 @@ struct DecQ6K {
       float c[8][4];
 #pragma unroll
       for (int i = 0; i < 8; i++)
-        mma_u8s8(c[i], a[i][0], 0u, a[i][1], 0u, D.b[m][i] & LN.m0, D.b[m][i] & LN.m1);
+        mma_u8s8_k16(c[i], a[i][0], a[i][1], word(D.b[m][i >> 2], i & 3));
 #pragma unroll
       for (int G = 0; G < 2; G++)
 #pragma unroll
@@ -451,7 +459,7 @@ struct DecQ6K {
           const float ta = __shfl_sync(0xffffffffu, t[2 * (k & 1)], src, 4);
           const float tb = __shfl_sync(0xffffffffu, t[2 * (k & 1) + 1], src, 4);
           acc[m][0] = fmaf(ta, c[G * 4 + k][0] - MMA_BIAS, acc[m][0]);
-          acc[m][1] = fmaf(tb, c[G * 4 + k][1] - MMA_BIAS, acc[m][1]);
+          acc[m][1] = fmaf(tb, c[G * 4 + k][3] - MMA_BIAS, acc[m][1]);
         }
     }
   }

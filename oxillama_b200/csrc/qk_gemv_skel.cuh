@@ -70,6 +70,7 @@ constexpr int MAX_SLOT = MAX_STAGE + 1;
 struct SmemMma {
   uint32_t full, redfull, xbar;  // mbarriers (8 B each)
   uint32_t prog;                 // chunks the reducer warp has read so far (one word, polled by the producer warp)
+                                 // and behind it the tiles issued so far (polled by the compute warps)
   uint32_t red, ximg, stage;
   uint32_t PS;         // digit plane stride, bytes
   uint32_t xs_off;     // offset of the (sx, Sx) table inside the x image
@@ -126,6 +127,16 @@ __device__ __forceinline__ void mma_u8s8(float (&c)[4], uint32_t a0, uint32_t a1
   for (int i = 0; i < 4; i++) c[i] = __int_as_float(r[i]);
 }
 
+__device__ __forceinline__ void mma_u8s8_k16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+  int r[4];
+  asm("mma.sync.aligned.m16n8k16.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+      : "r"(a0), "r"(a1), "r"(b0), "r"(0x4B400000));
+#pragma unroll
+  for (int i = 0; i < 4; i++) c[i] = __int_as_float(r[i]);
+}
+__device__ __forceinline__ uint32_t word(const uint4 &v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+
 // Four activations of one 32-column block -> their three balanced base-254 digits, one
 // packed word per digit plane: x ~ (amax / 127) (d0 + d1 / 254 + d2 / 254^2).  Adding
 // 1.5 * 2^23 rounds to the nearest integer and leaves it, as two's complement, in the low
@@ -160,6 +171,25 @@ __device__ __forceinline__ float digit_inv(float &amax) {
 // no digits: its scale is NaN, and so is every result that it is part of.
 __device__ __forceinline__ float digit_scale(float amax, float s32) {
   return amax > FLT_MAX || s32 != s32 ? __int_as_float(0x7FFFFFFF) : amax * (1.f / 127.f);
+}
+
+// Waits (bounded) until more than `item` tiles have been issued: from then on the barrier of the item's stage
+// is in the item's phase.  A stage goes from group to group of the compute warps, so a group could come to it
+// while the tile before, another group's, is still on its way, two phases back, and take that barrier for its
+// own.  `seen`: the count as last read.
+__device__ __forceinline__ bool wait_issued(uint32_t word_addr, uint32_t item, uint32_t &seen) {
+  if (seen > item) return true;
+  unsigned long long t0 = 0;
+  for (uint32_t polls = 1;; polls++) {
+    asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(seen) : "r"(word_addr) : "memory");
+    if (seen > item) return true;
+    if ((polls & 1023u) == 0) {
+      unsigned long long t;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+      if (!t0) t0 = t;
+      if (t - t0 > 250000000ull) return false;
+    }
+  }
 }
 
 // Activations e0 .. e0 + 3 of one row out of the tagged slots of a gathered buffer (columns
@@ -362,7 +392,7 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
     for (int s = 0; s < nstage; s++) mbar_init(sbase + S.full + s * 8, 1);
     for (int s = 0; s < nslot; s++) mbar_init(sbase + S.redfull + s * 8, WG);
     mbar_init(sbase + S.xbar, 1);
-    *reinterpret_cast<volatile uint32_t *>(smem + S.prog) = 0u;
+    *reinterpret_cast<volatile uint32_t *>(smem + S.prog) = 0u, *reinterpret_cast<volatile uint32_t *>(smem + S.prog + 4) = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -384,7 +414,11 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
   uint32_t item = 0;  // items issued so far; kept in step by every lane
   auto issue_upto = [&](uint32_t limit) {
     const uint32_t end = limit < my_items ? limit : my_items;
-    for (; item < end; item++) issue();
+    for (; item < end;) {
+      issue();
+      item++;
+      if (F::ANY_DEPTH && lead) *reinterpret_cast<volatile uint32_t *>(smem + S.prog + 4) = item;
+    }
   };
   if (SPLIT && warp == CW + 1) {
     lead = elect_lead();
@@ -593,7 +627,7 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
 
   QK_STAMP(warp == 0, 1);
   // loop state kept as counters: no integer division on the critical path
-  uint32_t st = 0, fph = 0, slot = 0;
+  uint32_t st = 0, fph = 0, slot = 0, seen = 0;
   auto advance_stage = [&](uint32_t n) {
     st += n;
     while (st >= (uint32_t)nstage) st -= nstage, fph ^= 1;
@@ -605,7 +639,9 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
     for (uint32_t kt = 0; kt < L.ktiles; kt++) {
       const uint32_t nbt = qk_tile_nb(L, kt) * L.bs / 256u;  // 256-column spans in this tile
       const uint32_t tile = sbase + S.stage + st * stage_bytes;
-      if (!mbar_wait_bounded(sbase + S.full + st * 8, fph)) {
+      // (in the ring's first round there is no tile before)
+      const uint32_t it = c * L.ktiles + kt;
+      if ((F::ANY_DEPTH && it >= (uint32_t)nstage && !wait_issued(sbase + S.prog + 4, it, seen)) || !mbar_wait_bounded(sbase + S.full + st * 8, fph)) {
         dead = true;
         break;
       }
@@ -665,8 +701,8 @@ struct PlanMma {
   int nstage, nslot, groups;
 };
 
-// xsb: bytes per 32-column block in the activation scale table (F::XSB).
-inline bool make_plan_mma(const QkLayout &L, uint32_t m, PlanMma *P, uint32_t xsb) {
+// xsb: bytes per 32-column block in the activation scale table (F::XSB).  any_depth: see below.
+inline bool make_plan_mma(const QkLayout &L, uint32_t m, PlanMma *P, uint32_t xsb, bool any_depth = false) {
   if (L.nb == 0 || L.chunks == 0) return false;  // nothing to stream: the callers handle empty shapes
   uint32_t Kp = L.nb * L.bs;
   if (Kp % 256u) return false;  // the kernels walk K in spans of 256 columns
@@ -699,15 +735,19 @@ inline bool make_plan_mma(const QkLayout &L, uint32_t m, PlanMma *P, uint32_t xs
   // a chunk's stages are refilled only once the whole chunk is reduced: its k-tiles
   // must all fit in the ring with room to prefetch the next chunk
   if ((uint32_t)nstage < L.ktiles + 1) return false;
-  // largest group count whose G * ktiles divides a ring depth we can afford
+  // Largest group count whose G * ktiles the ring holds.  A stage must always be consumed by the same group (a
+  // waiter on an mbarrier may be at most one phase ahead of it), so the depth is rounded down to a multiple of
+  // G * ktiles -- but for formats with F::ANY_DEPTH, which take every stage there is and count the tiles issued
+  // (wait_issued).  Measured both ways: Q6_K, four or seven stages at 4096 columns, 128256 x 4096 76.3 -> 66.5 us
+  // (with the k = 16 MMA); Q4_K, eight or eleven, 14336 x 4096 7.5 -> 8.2.
   int groups = 1;
   const char *ge = qk_knob("QK_GROUPS");
   const int gmax = ge ? atoi(ge) : 4;
   for (int gtry = 4; gtry >= 2; gtry >>= 1) {
     const int unit = gtry * (int)L.ktiles;
-    if (gtry <= gmax && nstage / unit >= 1 && (nstage / unit) * unit >= (int)L.ktiles + 1) {
+    if (gtry <= gmax && nstage >= unit && (any_depth || (nstage / unit) * unit >= (int)L.ktiles + 1)) {
       groups = gtry;
-      nstage = (nstage / unit) * unit;
+      if (!any_depth) nstage = (nstage / unit) * unit;
       break;
     }
   }
@@ -791,9 +831,7 @@ template <class F, int M>
 cudaError_t launch_mma_m(const QkLayout &L, const uint8_t *W, const float *x, float *y,
                          uint64_t ldy, unsigned *status, unsigned char *ximg, int sm_count,
                          const PlanMma &P, cudaStream_t s, const QkPeers *peers, const uint8_t *W2, bool host_x) {
-  // Warp groups: a group owns every G-th chunk.  A stage must always be consumed by
-  // the same group (a waiter on an mbarrier may be at most one phase ahead of it),
-  // so the ring depth is a multiple of G * ktiles; P.groups was chosen to allow that.
+  // Warp groups: a group owns every G-th chunk (P.groups was chosen with the ring's depth, see make_plan_mma).
   const bool peer = peers != nullptr;
 #define QK_LAUNCH1(CWV, GV, PV)                                                                               \
   return !host_x && (!ximg || split_in_cta(P, M))                                                             \
@@ -831,13 +869,13 @@ template <class F>
 bool supported(const QkLayout &L, uint32_t m) {
   if (m < 1 || m > (uint32_t)F::MAX_M) return false;
   PlanMma P;
-  return make_plan_mma(L, m, &P, F::XSB);
+  return make_plan_mma(L, m, &P, F::XSB, F::ANY_DEPTH);
 }
 
 template <class F>
 size_t scratch_bytes(const QkLayout &L, uint32_t m) {
   PlanMma P;
-  return make_plan_mma(L, m, &P, F::XSB) ? P.S.ximg_bytes : 0;
+  return make_plan_mma(L, m, &P, F::XSB, F::ANY_DEPTH) ? P.S.ximg_bytes : 0;
 }
 
 // tiled2 != nullptr: the two-matrix (feed-forward gate and up) mode, formats with F::HAS_DUAL only.
@@ -846,7 +884,7 @@ cudaError_t launch(const QkLayout &L, const uint8_t *tiled, const float *x, floa
                    unsigned *status, unsigned char *scratch, int sm_count, cudaStream_t s, const QkPeers *peers,
                    const uint8_t *tiled2 = nullptr, bool host_x = false) {
   PlanMma P;
-  if (!make_plan_mma(L, m, &P, F::XSB)) return cudaErrorInvalidConfiguration;
+  if (!make_plan_mma(L, m, &P, F::XSB, F::ANY_DEPTH)) return cudaErrorInvalidConfiguration;
   if (m < 1 || m > (uint32_t)F::MAX_M) return cudaErrorInvalidConfiguration;
   if ((tiled2 && (!F::HAS_DUAL || peers)) || (peers && !F::HAS_PEER)) return cudaErrorInvalidConfiguration;
   if (m == 1) return launch_mma_m<F, 1>(L, tiled, x, y, ldy, status, scratch, sm_count, P, s, peers, tiled2, host_x);

@@ -33,9 +33,9 @@ namespace qktc {
 // a stage then always belongs to the same set of expanding warps, which is never more than one phase
 // ahead of its barrier (with an odd number a set could find the barrier of a stage that the other set
 // has not been given yet, two phases back, and take that for its own).  Narrow tiles are bound by the
-// weight stream and give it what they can; wide ones need four activation stages first (a stage is
-// refilled only after the MMAs that read it have retired).
-static bool plan_smem(uint32_t hn, uint32_t cg, uint32_t cs, uint32_t w_stage, uint32_t lut, TcSmem *S, uint32_t *total) {
+// weight stream and give it what they can; tiles of more than 128 tokens need four activation stages first (a
+// stage is refilled only after the MMAs that read it have retired).
+static bool plan_smem(uint32_t bn, uint32_t hn, uint32_t cg, uint32_t cs, uint32_t w_stage, uint32_t lut, TcSmem *S, uint32_t *total) {
   TcSmem s;
   uint32_t off = 0;
   s.w_full = off, off += MAX_WST * 8;
@@ -60,8 +60,8 @@ static bool plan_smem(uint32_t hn, uint32_t cg, uint32_t cs, uint32_t w_stage, u
   auto fits = [&](uint32_t w, uint32_t b) { return w * s.w_stage + b * s.b_stage <= room; };
   if (!fits(2, 2)) return false;
   uint32_t nb = 2, nw = 2;
-  const uint32_t enough = hn <= 64 ? 3u : 4u;
-  while (nb < enough && fits(hn <= 64 ? 4 : 2, nb + 1)) nb++;
+  const uint32_t enough = bn <= 128 ? 3u : 4u;
+  while (nb < enough && fits(bn <= 128 ? 4 : 2, nb + 1)) nb++;
   while (nw < (uint32_t)MAX_WST && fits(nw + 2, nb)) nw += 2;
   while (nb < (uint32_t)MAX_BST && hn > 64 && fits(nw, nb + 1)) nb++;
   s.b_stages = nb, s.w_stages = nw;
@@ -74,12 +74,13 @@ static bool plan_smem(uint32_t hn, uint32_t cg, uint32_t cs, uint32_t w_stage, u
 static uint32_t round_up(uint32_t v, uint32_t to) { return (v + to - 1) / to * to; }
 
 // Form of the kernel, token-tile width and K split by predicted time: cycles of the slowest CTA.  The
-// constants are a fit to 46 shapes (300 x 8192 .. 14336 x 4096, 8 .. 2048 tokens, Q4_K, Q6_K, Q8_0, Q4_0), each
-// timed with every tile width and split: the prediction is 10 % off (rms), the form it picks 0.8 % slower than
-// the fastest (mean).  (IQ4_XS takes Q4_K's: its times are within 5 % of Q4_K's but at 128 tokens.)  A super-block takes as long as its expansion, which loads of wider activations slow down,
-// or in a pair the round of hand-overs (expanding warps -> issuer -> tensor pipe -> back).  A tile whose
-// partials go through the workspace costs some 8000 cycles and 58 per token (writing them out, the fence, the
-// counter, reading them back); through the cluster 5300, whatever its width.
+// constants are a fit to 96 shapes (256 x 12288 .. 28672 x 4096, 8 .. 2048 tokens, Q4_K, Q6_K, Q8_0, IQ4_XS; Q4_0
+// takes Q4_K's), each timed with every tile width and split: the prediction is 12 % off (rms, plans within 1.6 times
+// the fastest), the form it picks 1.0 % slower than the fastest (mean; 2.7 % with the constants of the kernel before
+// its MMA loop was shortened).  A super-block takes as long as its expansion or its MMAs, or
+// in a pair the round of hand-overs (expanding warps -> issuer -> tensor pipe -> back).  A tile whose
+// partials go through the workspace costs some 7000 cycles and 40 per token (writing them out, the fence, the
+// counter, reading them back); through the cluster 4600, whatever its width.
 bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
   const QkLayout &L = *c.L;
   const uint32_t w_stage = 16u * 8u * L.bb * (256u / L.bs), lut = L.type == QK_T_IQ4_XS ? WFmt<QK_T_IQ4_XS>::LUT : 0u;
@@ -99,12 +100,14 @@ bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
     p.row_blocks = (L.rows + p.cg * BM - 1) / (p.cg * BM);
     p.grid = (uint32_t)sm_count / p.cg;
   } else {
-    const float expand = L.type == QK_T_Q6_K ? 1440.f : 1110.f;
+    const float expand = L.type == QK_T_Q6_K ? 1170.f : L.type == QK_T_IQ4_XS ? 1000.f : L.type == QK_T_Q8_0 ? 980.f : 930.f;
     float best = FLT_MAX;
     auto take = [&](float t, uint32_t cg, uint32_t cs, uint32_t bn, uint32_t tbr, uint32_t rbs, uint32_t run, uint32_t grid) {
       if (t < best) best = t, p.cg = cg, p.cs = cs, p.bn = bn, p.tok_blocks = tbr, p.row_blocks = rbs, p.min_run = run, p.grid = grid;
     };
     const uint32_t tb0 = (c.m + MAX_BN - 1) / MAX_BN;
+    // Every token block reads the weights again, from L2 at best: 1.5 % for twice as many blocks as needed (gate and up
+    // 14336 x 4096 by 512 tokens: 96.3 us in three blocks, 95.5 in two, but 3 us more where the weights come from HBM).
     // (A pair only where its second CTA has rows: Q4_0 64 x 1280 by 2048 tokens 26.4 -> 14.0 us.)
     for (uint32_t cg = 1; cg <= (L.rows > BM ? 2u : 1u); cg++) {
       const uint32_t units = (uint32_t)sm_count / cg, rbs = (L.rows + cg * BM - 1) / (cg * BM);
@@ -113,12 +116,12 @@ bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
         const uint32_t bn = round_up((c.m + tbk - 1) / tbk, 16);
         if (k && bn < 32) break;
         if (cg == 1 && bn > 64) continue;
-        const uint32_t tbr = (c.m + bn - 1) / bn, own = bn / cg;
-        const float sb = fmaxf(expand + (own > 16 ? 5.f * (own - 16) : 0.f), cg == 2 ? (1060.f + 6.1f * bn) * (bn <= 128 ? 0.94f : 1.f) : 0.f), out = bn * 19.f;
+        const uint32_t tbr = (c.m + bn - 1) / bn;
+        const float sb = cg == 1 ? expand : fmaxf(fmaxf(expand + 125.f, 980.f + 2.f * bn), 9.f * bn), out = bn * 59.f;
         const uint64_t tiles = (uint64_t)c.n * rbs * tbr;
         for (uint32_t run = 1; run <= 16; run <<= 1) {
           const uint32_t R = (uint32_t)(tiles % units), total = R * p.nsb;
-          float t = (float)(tiles / units) * (p.nsb * sb + (bn > 128 ? 7000.f : 100.f)) + out;
+          float t = (float)(tiles / units) * (p.nsb * sb + (bn > 128 ? 9000.f : 70.f + 38.f * bn)) + out;
           uint32_t grid = units;
           if (R) {
             uint32_t sk = total / run;
@@ -129,8 +132,9 @@ bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
             }
             const float len = (float)((total + sk - 1) / sk), contrib = (float)sk / R;
             t += len * sb;
-            if (contrib > 1.01f) t += 7800.f + bn * (58.f + 5.f * contrib);
+            if (contrib > 1.01f) t += 7200.f + bn * (36.f + 3.5f * contrib);
           }
+          if (tb0 > 1) t *= 1.f + 0.015f * log2f((float)tbr / tb0);
           take(t, cg, 1, bn, tbr, rbs, run, grid);
         }
         // One tile per cluster of cs CTAs.  At most as many as fit at a time: 32 clusters of four, 14 of eight on
@@ -138,12 +142,12 @@ bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
         if (cg == 1 && c.n == 1)
           for (uint32_t cs = 4; cs <= 8 && cs <= p.nsb; cs <<= 1)
             if (tiles * cs <= (uint32_t)sm_count * (cs == 4 ? 14u : 12u) / 16u)
-              take((float)((p.nsb + cs - 1) / cs) * sb + 5300.f + out, 1, cs, bn, tbr, rbs, 1, (uint32_t)tiles * cs);
+              take((float)((p.nsb + cs - 1) / cs) * sb + 4600.f + out, 1, cs, bn, tbr, rbs, 1, (uint32_t)tiles * cs);
       }
     }
   }
   p.hn = half_of(p.bn);
-  if (!plan_smem(p.hn, p.cg, p.cs, w_stage, lut, &p.S, &p.smem)) return false;
+  if (!plan_smem(p.bn, p.hn, p.cg, p.cs, w_stage, lut, &p.S, &p.smem)) return false;
   p.xrows = c.counts || c.n_act > 1 ? c.n_act * c.xcap : p.tok_blocks * p.bn;
   const size_t Kp = (size_t)p.nsb * 256u;
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };

@@ -106,6 +106,7 @@ struct TcArgs {
   uint32_t xcap, ycap;             // rows reserved per group in the activation and output arrays
   uint32_t cs;                     // CTAs of a cluster that share a tile along K (CG = 1, one segment each); 1 = see Sched
   uint32_t once;                   // weights are read once: evict-first in L2
+  uint32_t ahead;                  // super-blocks of weights asked for before the CTA sets itself up (two at most; not with counts)
   const int *counts;               // device: live rows per activation group, or null (m rows each)
 };
 // Tensor maps: the matrices, and the fp16 activations as boxes of 64 columns x h tokens x the steps of
@@ -746,16 +747,14 @@ struct TileAt {
 
 // The super-blocks of a segment in the order the MMAs take them: one at a time (`half` 0, then 1),
 // but at either end of a wide tile two at a time (both under half 0, then both under half 1).
-// Calls step(sb, half, which of the two, last use of the super-block's weights, end of the segment) -> false to stop,
-// and after every one or two super-blocks next(how many).
-template <class Step, class Next>
-__device__ __forceinline__ bool walk_segment(uint32_t s0, uint32_t s1, bool wide, Step &&step, Next &&next) {
+// Calls step(sb, half) -> false to stop.
+template <class Step>
+__device__ __forceinline__ bool walk_segment(uint32_t s0, uint32_t s1, bool wide, Step &&step) {
   for (uint32_t sb = s0; sb < s1;) {
     const uint32_t two = wide && s1 - sb >= 2 && (sb == s0 || s1 - sb == 2) ? 2u : 1u;
     for (uint32_t h = 0; h < (wide ? 2u : 1u); h++)
       for (uint32_t k = 0; k < two; k++)
-        if (!step(sb + k, h, k, h == (wide ? 1u : 0u), sb + k + 1 == s1)) return false;
-    next(two);
+        if (!step(sb + k, h)) return false;
     sb += two;
   }
   return true;
@@ -780,51 +779,13 @@ __global__ void __maxnreg__(REGS)
   const uint32_t na = both ? 2u : 3u, d_step = narrow ? 64u : 128u, a_col = both ? 256u : 128u, alt = narrow ? 1u : 0u;
 
   pdl_launch_dependents();
-  if (threadIdx.x == 0) {
-    for (uint32_t s = 0; s < S.w_stages; s++) mbar_init(sbase + S.w_full + s * 8, 1), mbar_init(sbase + S.w_empty + s * 8, 8);
-    for (uint32_t s = 0; s < S.b_stages; s++) mbar_init(sbase + S.b_full + s * 8, 1), mbar_init(sbase + S.b_empty + s * 8, 1);
-    for (uint32_t s = 0; s < 3; s++) mbar_init(sbase + S.a_full + s * 8, CG * 8), mbar_init(sbase + S.a_empty + s * 8, 1);
-    for (uint32_t s = 0; s < 2; s++) mbar_init(sbase + S.d_full + s * 8, 1), mbar_init(sbase + S.d_empty + s * 8, CG * 4);
-    mbar_init(sbase + S.drain, 1);
-    *reinterpret_cast<volatile uint32_t *>(smem + S.scales + 2052) = 0u;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  }
-  if (threadIdx.x == 32) asm volatile("prefetch.tensormap [%0];" ::"l"(&M.x[0]) : "memory");
-  if (threadIdx.x == 64 && NG == 1) asm volatile("prefetch.tensormap [%0];" ::"l"(&M.w[0]) : "memory");
-  if (F::LUT) F::fill_lut(smem + LUT_OFF, threadIdx.x, NTHREADS);
-  if (warp == 3) {
-    if (CG == 1) {
-      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + S.tmem_slot), "r"(512u) : "memory");
-      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    } else {
-      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + S.tmem_slot), "r"(512u) : "memory");
-      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-    }
-  }
-  uint32_t *pre = reinterpret_cast<uint32_t *>(smem + S.pre);  // tiles before group g (device-counted groups)
   const bool counted = NG > 1 && A.counts;
-  if (counted) {
-    pdl_wait();  // the counts are the work of an earlier kernel
-    if (threadIdx.x == 0) {
-      uint32_t s = 0;
-      for (uint32_t g = 0; g < A.n; g++) {
-        pre[g] = s;
-        s += A.row_blocks * (((uint32_t)A.counts[g % A.n_act] + A.bn - 1) / A.bn);
-      }
-      pre[A.n] = s;
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  const bool clustered = CG == 2 || (NG == 1 && A.cs > 1);
-  if (clustered) cluster_sync();  // the other CTAs run, their barriers are initialised, their tensor memory is there
-  tc_fence_after();
-  const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(smem + S.tmem_slot);
-
   Sched sc{};
-  if (CG == 1 && NG == 1 && A.cs > 1) sc.init_cluster((A.L.cols + 255u) / 256u, A.cs);
-  else sc.template init<CG>(counted ? pre[A.n] : A.n * A.row_blocks * A.tok_blocks, (A.L.cols + 255u) / 256u, A.min_run);
+  auto make_schedule = [&](uint32_t tiles) {
+    if (CG == 1 && NG == 1 && A.cs > 1) sc.init_cluster((A.L.cols + 255u) / 256u, A.cs);
+    else sc.template init<CG>(tiles, (A.L.cols + 255u) / 256u, A.min_run);
+  };
+  uint32_t *pre = reinterpret_cast<uint32_t *>(smem + S.pre);  // tiles before group g (device-counted groups)
   auto at = [&](uint32_t tile) {
     TileAt q;
     uint32_t tb;
@@ -844,6 +805,74 @@ __global__ void __maxnreg__(REGS)
     q.n = left >= A.bn ? A.bn : ((left + 15u) & ~15u);
     return q;
   };
+  if (!counted) make_schedule(A.n * A.row_blocks * A.tok_blocks);
+  // Where A.ahead says so the first weights are asked for before anything else: a CTA that starts when the
+  // previous one on its SM has ended gets them 1.9 us later, and the rest of its setting up takes 1.3.
+  uint32_t ws = 0, w_ahead = 0;    // (warp 2) ring stage of the next super-block; super-blocks asked for here
+  uint32_t w_lead = 0;
+  uint64_t policy = 0;
+  if (warp == 2) {
+    w_lead = elect_one() ? 1u : 0u;
+    if (w_lead) {
+      for (uint32_t s = 0; s < S.w_stages; s++) mbar_init(sbase + S.w_full + s * 8, 1), mbar_init(sbase + S.w_empty + s * 8, 8);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncwarp();
+    if (A.once) policy = stream_policy();
+    else asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(policy));
+    if (A.ahead && sc.n_seg) {  // of the first segment
+      uint32_t tile, s0, s1;
+      sc.get(0, tile, s0, s1);
+      const TileAt q = at(tile);
+      for (uint32_t sb = s0; sb < s1 && ws < A.ahead; sb++, ws++) {
+        expect_tx(sbase + S.w_full + ws * 8, S.w_stage, w_lead);
+        tma_load_3d_hint(sbase + S.w + ws * S.w_stage, &M.w[NG > 1 ? q.g : 0], 0, (int)(sb * F::BPS), (int)(q.rb * (16 * CG) + rank * 16),
+                         sbase + S.w_full + ws * 8, policy, w_lead);
+      }
+      w_ahead = ws;
+    }
+  }
+  if (threadIdx.x == 0) {
+    for (uint32_t s = 0; s < S.b_stages; s++) mbar_init(sbase + S.b_full + s * 8, 1), mbar_init(sbase + S.b_empty + s * 8, 1);
+    for (uint32_t s = 0; s < 3; s++) mbar_init(sbase + S.a_full + s * 8, CG * 8), mbar_init(sbase + S.a_empty + s * 8, 1);
+    for (uint32_t s = 0; s < 2; s++) mbar_init(sbase + S.d_full + s * 8, 1), mbar_init(sbase + S.d_empty + s * 8, CG * 4);
+    mbar_init(sbase + S.drain, 1);
+    *reinterpret_cast<volatile uint32_t *>(smem + S.scales + 2052) = 0u;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (threadIdx.x == 32) asm volatile("prefetch.tensormap [%0];" ::"l"(&M.x[0]) : "memory");
+  if (F::LUT) F::fill_lut(smem + LUT_OFF, threadIdx.x, NTHREADS);
+  if (warp == 3) {
+    if (CG == 1) {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + S.tmem_slot), "r"(512u) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + S.tmem_slot), "r"(512u) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+  }
+  if (counted) {
+    pdl_wait();  // the counts are the work of an earlier kernel
+    if (threadIdx.x == 0) {
+      uint32_t s = 0;
+      for (uint32_t g = 0; g < A.n; g++) {
+        pre[g] = s;
+        s += A.row_blocks * (((uint32_t)A.counts[g % A.n_act] + A.bn - 1) / A.bn);
+      }
+      pre[A.n] = s;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  const bool shared = CG == 1 && NG == 1 && A.cs > 1;  // a tile's K runs in the CTAs of a cluster
+  if (CG == 2) cluster_sync();  // the other CTA runs, its barriers are initialised, its tensor memory is there
+  if (shared) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // (waited for ahead of the stores into other CTAs)
+  tc_fence_after();
+  const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(smem + S.tmem_slot);
+
+  if (counted) make_schedule(pre[A.n]);
   // Token rows that an activation box brings: each CTA of a pair loads half of the n tokens.
   const uint32_t hq = box_unit(A.hn / CG);
   auto box_of = [&](uint32_t n) { return NG > 1 ? (n / CG + hq - 1) / hq : 1u; };  // the how-manieth box (from 1)
@@ -948,29 +977,44 @@ __global__ void __maxnreg__(REGS)
         if (!dead) umma_commit<CG>(sbase + S.d_full + dh * 8, lead);
       } else {
         // Two accumulator halves: one super-block at a time under half 0, then half 1, but at either end of the
-        // segment two at a time (walk_segment); the buffers are walked again under the second half.
+        // segment two at a time (walk_segment); the buffers are walked again under the second half.  (Written out: as one
+        // step for either half, gate and up of 14336 x 4096 by 512 took 111.6 us under ncu instead of 103.3.)
         const uint32_t n1 = q.n - A.hn, idesc1 = (1u << 4) | ((n1 >> 3) << 17) | ((CG * BM >> 4) << 24), step1 = box_rows(n1) * 8u;
+        bool ok = take_half(0);
         ready = false;
-        if (!walk_segment(s0, s1, true, [&](uint32_t sb, uint32_t h, uint32_t k, bool last, bool end) {
-              if (sb == s0 && !take_half(h)) return false;
-              uint32_t abk = ab + k, ph = aph;
-              if (abk >= na) abk -= na, ph ^= 1u;
-              if (h == 0) {
-                if (!warp_wait(a_full + abk * 8, ph)) return false;
-                tc_fence_after();
-              }
-              if (!warp_wait(b_full + bs * 8, bph)) return false;
-              issue16(tmem + h * d_step, a0 + abk * 128u, bd0 + bs * stage16, h ? step1 : step0, h ? idesc1 : idesc0, sb == s0 ? 0u : 1u);
-              umma_commit<CG>(b_empty + bs * 8, lead);
-              if (last) umma_commit<CG>(a_empty + abk * 8, lead);
-              if (end) umma_commit<CG>(sbase + S.d_full + h * 8, lead);
-              if (++bs == nbs) bs = 0, bph ^= 1u;
-              return true;
-            }, [&](uint32_t two) {
-              ab += two;
-              if (ab >= na) ab -= na, aph ^= 1u;
-            }))
-          dead = true;
+        uint32_t acc0 = 0u, acc1 = 0u;
+        for (uint32_t sb = s0; sb < s1 && ok;) {
+          const uint32_t two = s1 - sb >= 2 && (sb == s0 || s1 - sb == 2) ? 2u : 1u;
+          uint32_t abk = ab, ph = aph;
+          for (uint32_t k = 0; k < two && ok; k++) {
+            ok = __all_sync(0xffffffffu, ready) || (warp_wait(a_full + abk * 8, ph) && warp_wait(b_full + bs * 8, bph));
+            if (!ok) break;
+            tc_fence_after();
+            issue16(tmem, a0 + abk * 128u, bd0 + bs * stage16, step0, idesc0, acc0);
+            umma_commit<CG>(b_empty + bs * 8, lead);
+            acc0 = 1u;
+            if (++bs == nbs) bs = 0, bph ^= 1u;
+            if (++abk == na) abk = 0, ph ^= 1u;
+            ready = k + 1 < two && (mbar_test(a_full + abk * 8, ph) & mbar_test(b_full + bs * 8, bph));
+          }
+          if (sb + two == s1 && ok) umma_commit<CG>(sbase + S.d_full, lead);
+          if (!acc1 && ok) ok = take_half(1);
+          abk = ab;
+          for (uint32_t k = 0; k < two && ok; k++) {
+            if (!(ok = warp_wait(b_full + bs * 8, bph))) break;
+            issue16(tmem + d_step, a0 + abk * 128u, bd0 + bs * stage16, step1, idesc1, acc1);
+            umma_commit<CG>(b_empty + bs * 8, lead);
+            umma_commit<CG>(a_empty + abk * 8, lead);
+            acc1 = 1u;
+            if (++bs == nbs) bs = 0, bph ^= 1u;
+            if (++abk == na) abk = 0;
+          }
+          if (sb + two == s1 && ok) umma_commit<CG>(sbase + S.d_full + 8, lead);
+          ab = abk, aph = ph;
+          sb += two;
+          ready = mbar_test(a_full + ab * 8, aph) & mbar_test(b_full + bs * 8, bph);
+        }
+        if (!ok) dead = true;
       }
     }
     if (dead) {  // let what was issued retire before the CTA gives its memory back
@@ -994,7 +1038,7 @@ __global__ void __maxnreg__(REGS)
       const uint32_t row0 = (NG > 1 ? (q.g % A.n_act) * A.xcap : 0u) + q.t0;
       const int r0 = (int)(row0 + (rank ? n0 / 2 : 0u)), r1 = (int)(row0 + A.hn + (rank ? n1 / 2 : 0u));
       const CUtensorMap *map0 = &M.x[box_of(n0) - 1], *map1 = &M.x[wide ? box_of(n1) - 1 : 0];
-      const bool ok = walk_segment(s0, s1, wide, [&](uint32_t sb, uint32_t h, uint32_t, bool, bool) {
+      const bool ok = walk_segment(s0, s1, wide, [&](uint32_t sb, uint32_t h) {
         if (rounds && !warp_wait(bar + to_empty, bph ^ 1u)) return false;
         // the halves of both CTAs land on the barrier of rank 0, which alone announces them
         if (rank == 0) expect_tx(bar, (h ? rows1 : rows0) * 512u * CG, lead);
@@ -1002,7 +1046,7 @@ __global__ void __maxnreg__(REGS)
         bs++, bar += 8, full += 8, dst += stage;
         if (bs == nst) bs = 0, bph ^= 1u, rounds = 1, bar = sbase + S.b_full, full = full0, dst = sbase + S.b;
         return true;
-      }, [](uint32_t) {});
+      });
       if (!ok) dead = true;
     }
     if (dead) {
@@ -1014,18 +1058,16 @@ __global__ void __maxnreg__(REGS)
   } else if (warp == 2) {
     // ======================= weight producer =======================
     // The weights are immutable: their stream starts before the previous kernel has ended.
-    const uint32_t lead = elect_one() ? 1u : 0u;
-    uint64_t policy;
-    if (A.once) policy = stream_policy();
-    else asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(policy));
-    uint32_t ws = 0, wph = 0, rounds = 0, bar = sbase + S.w_full, dst = sbase + S.w;
-    const uint32_t to_empty = S.w_empty - S.w_full, nst = S.w_stages, stage = S.w_stage;
+    const uint32_t lead = w_lead, to_empty = S.w_empty - S.w_full, nst = S.w_stages, stage = S.w_stage;
+    uint32_t wph = 0, rounds = 0;
+    if (ws == nst) ws = 0, wph = 1u, rounds = 1;
+    uint32_t bar = sbase + S.w_full + ws * 8, dst = sbase + S.w + ws * stage;
     for (uint32_t i = 0; i < sc.n_seg && !dead; i++) {
       uint32_t tile, s0, s1;
       sc.get(i, tile, s0, s1);
       const TileAt q = at(tile);
       const CUtensorMap *map = &M.w[NG > 1 ? q.g : 0];
-      for (uint32_t sb = s0; sb < s1; sb++) {
+      for (uint32_t sb = s0 + (i == 0 ? w_ahead : 0u); sb < s1; sb++) {
         if (rounds && !warp_wait(bar + to_empty, wph ^ 1u)) {
           dead = true;
           break;
@@ -1048,6 +1090,7 @@ __global__ void __maxnreg__(REGS)
     const uint32_t tlane = tmem + ((32 * quarter) << 16);
     const uint32_t d_empty = in_first<CG>(sbase + S.d_empty);
     float *scales = reinterpret_cast<float *>(smem + S.scales) + quarter * 128;  // this warp's copy of a half's token scales
+    if (shared) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // the other CTAs run
     volatile uint32_t *told = reinterpret_cast<volatile uint32_t *>(smem + S.scales + 2048);
     uint32_t dph = 0;
     pdl_wait();  // y, the scales and the workspace belong to the previous kernel until it has finished
@@ -1091,13 +1134,13 @@ __global__ void __maxnreg__(REGS)
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(d_empty + dh * 8);
           }
-          if (CG == 1 && NG == 1 && A.cs > 1) {
+          if (shared) {
             // to the CTA of the cluster that adds up the token
-            const uint32_t own = (q.n + A.cs - 1) / A.cs, at = sbase + S.red + (blockIdx.x % A.cs * own * BM + r) * 4;
+            const uint32_t own = (live + A.cs - 1) / A.cs, at = sbase + S.red + (blockIdx.x % A.cs * own * BM + r) * 4;
             uint32_t to = c / own, t = c % own;
 #pragma unroll
             for (uint32_t j = 0; j < 16; j++) {
-              st_cluster(at + t * (BM * 4), to, __uint_as_float(v[j]));
+              if (c + j < live) st_cluster(at + t * (BM * 4), to, __uint_as_float(v[j]));
               if (++t == own) t = 0, to++;
             }
           } else if (split) {
@@ -1123,7 +1166,7 @@ __global__ void __maxnreg__(REGS)
         }
       }
       if (!split) continue;
-      if (CG == 1 && NG == 1 && A.cs > 1) break;  // see below
+      if (shared) break;  // see below
       // Count in, once both halves are in the workspace (the accumulators are free by now); the last
       // contributor adds the partials up, in the order of their K runs.
       const uint32_t i0 = sc.owner_of(tile * sc.nsb), i1 = sc.owner_of((tile + 1) * sc.nsb - 1);
@@ -1144,7 +1187,7 @@ __global__ void __maxnreg__(REGS)
       for (; i < sc.n_seg; i++) {
         uint32_t tile, s0, s1;
         sc.get(i, tile, s0, s1);
-        if ((s0 != 0 || s1 != sc.nsb) && !(CG == 1 && NG == 1 && A.cs > 1)) (void)any_of_128(true);
+        if ((s0 != 0 || s1 != sc.nsb) && !shared) (void)any_of_128(true);
       }
     }
   } else if (warp >= FIRST_DW) {
@@ -1206,22 +1249,42 @@ __global__ void __maxnreg__(REGS)
 
   // common exit: the tensor memory is always returned
   tc_fence_before();
+  if (shared && warp < FIRST_EW) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // (the epilogue warps have)
   __syncthreads();
-  if (clustered) cluster_sync();  // neither CTA leaves while the other may still arrive on its barriers or read its operands
-  tc_fence_after();
-  if (CG == 1 && NG == 1 && A.cs > 1 && warp >= FIRST_EW) {
-    // The partial sums of this CTA's tokens have arrived: add them up in the order of their K runs.
+  if (shared) {
+    // The partial sums of this CTA's tokens, by the epilogue warps (they alone have waited for the kernels before;
+    // for another warp that takes 0.3 us even when it is long over): a lane four rows of one token at a time, the
+    // first scale fetched ahead of the meeting.  Added up in the order of the K runs.
+    const bool adds = warp >= FIRST_EW;
     const TileAt q = at(sc.first_tile);
-    const uint32_t own = (q.n + A.cs - 1) / A.cs, k = blockIdx.x % A.cs, r = 32 * (warp & 3u) + lane, row = q.rb * BM + r;
-    const float *red = reinterpret_cast<const float *>(smem + S.red) + r;
-    const uint32_t left = q.live - q.t0, t1 = min((k + 1) * own, min(left, q.n));
-    if (row < A.L.rows)
-      for (uint32_t t = k * own; t < t1; t++) {
-        float v = 0.f;
-        for (uint32_t p = 0; p < A.cs; p++) v += red[(p * own + t - k * own) * BM];
-        A.y[(uint64_t)(q.t0 + t) * A.ldy + row] = v * __ldg(A.xscale + q.t0 + t);
+    const uint32_t live = min(q.live - q.t0, q.n), own = (live + A.cs - 1) / A.cs, t0 = blockIdx.x % A.cs * own, t1 = min(t0 + own, live);
+    const uint32_t first = t0 + warp - FIRST_EW, r = 4 * lane, row = q.rb * BM + r;
+    const float *sp = A.xscale + q.t0;
+    float f = adds && first < t1 ? __ldg(sp + first) : 0.f;
+    cluster_sync();  // all partial sums are here; nobody leaves while another may still store into its memory
+    const bool vec = q.rb * BM + BM <= A.L.rows && (A.ldy & 3u) == 0 && ((uintptr_t)A.y & 15u) == 0;
+    for (uint32_t t = first; adds && t < t1; t += 4) {
+      const float *red = reinterpret_cast<const float *>(smem + S.red) + (t - t0) * BM + r;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (uint32_t p = 0; p < A.cs; p++) {
+        const float4 o = *reinterpret_cast<const float4 *>(red + p * own * BM);
+        v.x += o.x, v.y += o.y, v.z += o.z, v.w += o.w;
       }
+      if (t != first) f = __ldg(sp + t);
+      float *yp = A.y + (uint64_t)(q.t0 + t) * A.ldy + row;
+      v.x *= f, v.y *= f, v.z *= f, v.w *= f;
+      if (vec) {
+        *reinterpret_cast<float4 *>(yp) = v;
+      } else {
+        if (row < A.L.rows) yp[0] = v.x;
+        if (row + 1 < A.L.rows) yp[1] = v.y;
+        if (row + 2 < A.L.rows) yp[2] = v.z;
+        if (row + 3 < A.L.rows) yp[3] = v.w;
+      }
+    }
   }
+  if (CG == 2) cluster_sync();  // neither CTA leaves while the other may still arrive on its barriers or read its operands
+  tc_fence_after();
   if (warp == 3) {
     if (CG == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
     else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
@@ -1315,6 +1378,10 @@ cudaError_t launch_fmt(const QkTcCall &c, unsigned *status, unsigned char *scrat
   A.L = L, A.S = P.S, A.xscale = scales, A.y = c.y, A.part = reinterpret_cast<float *>(scratch + P.o_part), A.cnt = cnt;
   A.status = status, A.ldy = c.ldy, A.m = c.m, A.bn = P.bn, A.hn = P.hn, A.tok_blocks = P.tok_blocks, A.row_blocks = P.row_blocks;
   A.cs = P.cs, A.min_run = P.min_run, A.n = c.n, A.n_act = c.n_act, A.xcap = c.xcap, A.ycap = c.ycap, A.once = P.tok_blocks == 1, A.counts = c.counts;
+  // Early weights get in the way of the conversion's loads where that has many rows (Q8_0 4096 x 4096 by 509 22.7 -> 23.4
+  // us), and clusters gain nothing (Q4_K 4096 x 4096 by 8 8.2 -> 8.4); else 14336 x 4096 by 8 13.8 -> 13.1, IQ4_XS by 37
+  // 16.7 -> 15.9.
+  A.ahead = P.cg == 1 && !c.counts && P.cs == 1 && c.m < 64 ? 2u : 0u;
   if (c.n == 1 && !c.counts) {
     if constexpr (beside_of(T))
       if (beside) return P.cg == 1 ? launch_main<T, 1, 1, 72>(P, A, x16, c, s) : launch_main<T, 2, 1, 72>(P, A, x16, c, s);

@@ -487,3 +487,16 @@ def test_moe_group_sizes(t, counts):
     check_device_status()
     ex.free()
     assert np.abs(y.cpu().numpy() - ref).max() <= 3e-3 * np.abs(ref).max()
+
+
+# Chunks through the ring of weight tiles: fewer than groups of warps, several rounds of the ring, one to three k-tiles
+# a chunk with the last one whole, one span and half.
+@pytest.mark.parametrize("rows,cols", [(5, 8448), (1190, 12288), (9480, 4096), (5003, 8448)])
+@pytest.mark.parametrize("m", [1, 2, 3])
+@pytest.mark.parametrize("t", [S.Q6_K, S.Q4_K, S.Q8_0])
+def test_decode_ring(t, m, rows, cols):
+    w = S.gen_weight(t, rows, cols, seed=121)
+    x = S.gen_acts(m, cols, seed=122)
+    y = device_product(t, w, x, rows, cols, m)
+    # (three rows of Q6_K, and of Q8_0 two of 12288 columns or three, go to the tensor cores: fp16 operands)
+    assert_product(y, x, O.dequant_matrix(t, w, rows, cols), half=m > {S.Q6_K: 2, S.Q8_0: 1}.get(t, 4))

@@ -148,7 +148,9 @@ bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
   }
   p.hn = half_of(p.bn);
   if (!plan_smem(p.bn, p.hn, p.cg, p.cs, w_stage, lut, &p.S, &p.smem)) return false;
-  p.xrows = c.counts || c.n_act > 1 ? c.n_act * c.xcap : p.tok_blocks * p.bn;
+  // The rows that the MMAs cover, whatever the tiles: a wider box of the last token block ends outside the tensor map,
+  // and the copy unit fills it with zeros (381 calls whose tiles cover more rows, timed both ways: no difference).
+  p.xrows = c.counts || c.n_act > 1 ? c.n_act * c.xcap : round_up(c.m, 16);
   const size_t Kp = (size_t)p.nsb * 256u;
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
   p.o_scale = al((size_t)p.xrows * Kp * 2);

@@ -170,8 +170,8 @@ bool qk_gemm_tc_supported(const QkLayout &L, uint32_t m);
 // this many zeros behind them.
 uint64_t qk_gemm_tc_pad_bytes(const QkLayout &L);
 cudaError_t qk_gemm_tc_map(const QkLayout &L, uint8_t *tiled, void *map);
-// Scratch of a call: the fp16 activations, their scales and, at their most for every call, the partial
-// tiles of a K split (two per CTA; which plan a shape gets then does not change what it needs).
+// Scratch of a call: the fp16 activations (rows in sixteens), their scales and, at their most for every call, the
+// partial tiles of a K split (two per CTA): which plan a shape gets does not change what it needs.
 size_t qk_gemm_tc_part_bytes(int sm_count);
 size_t qk_gemm_tc_scratch_bytes(const QkTcCall &c, int sm_count);
 cudaError_t qk_launch_gemm_tc(const QkTcCall &c, unsigned *status, unsigned char *scratch, int sm_count, cudaStream_t s);

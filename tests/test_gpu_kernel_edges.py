@@ -362,9 +362,11 @@ def test_ffn_conversion(hidden, inter, m, scale):
 
 
 # The first matmul of a context, captured: up to 128 rows of 4096 columns need no more scratch than the
-# context starts with, whichever tiles and K split the shape gets.
+# context starts with, whichever tiles and K split the shape gets (the last two: tiles that cover more rows
+# than the scratch would hold, of which only the sixteens with activations count).
 @pytest.mark.parametrize("t,rows,cols,m", [(S.Q4_K, 4096, 4096, 8), (S.Q6_K, 300, 8192, 60), (S.Q8_0, 1024, 3840, 128),
-                                           (S.Q5_K, 512, 9216, 4), (S.IQ4_XS, 14336, 4096, 120)])
+                                           (S.Q5_K, 512, 9216, 4), (S.IQ4_XS, 14336, 4096, 120), (S.Q4_K, 4096, 8192, 107),
+                                           (S.Q4_0, 2396, 12288, 74)])
 def test_first_call_in_a_capture(t, rows, cols, m):
     import torch
     from oxillama_b200.device import DeviceWeights, check_device_status

@@ -27,7 +27,7 @@ struct DecQ5K {
   static constexpr int MAX_M = 4;
   static constexpr bool HAS_DUAL = true, HAS_PEER = false;
   static constexpr bool SPLIT_PRODUCER = true;
-  static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (make_plan_mma)
+  static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
                                                       uint32_t w1, uint32_t w2) {
     store_digits_natural(row_img, PS, e0, w0, w1, w2);
@@ -166,7 +166,7 @@ struct DecQ3K {
   static constexpr int MAX_M = 2;  // three rows and up spill, as with Q6_K
   static constexpr bool HAS_DUAL = true, HAS_PEER = false;
   static constexpr bool SPLIT_PRODUCER = true;
-  static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (make_plan_mma)
+  static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
                                                       uint32_t w1, uint32_t w2) {
     store_digits_natural(row_img, PS, e0, w0, w1, w2);
@@ -245,7 +245,7 @@ struct DecQ2K {
   static constexpr int MAX_M = 2;  // as Q3_K
   static constexpr bool HAS_DUAL = true, HAS_PEER = false;
   static constexpr bool SPLIT_PRODUCER = true;
-  static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (make_plan_mma)
+  static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
                                                       uint32_t w1, uint32_t w2) {
     store_digits_natural(row_img, PS, e0, w0, w1, w2);

@@ -30,7 +30,7 @@ struct DecQ4K {
   static constexpr int MAX_M = 4;
   static constexpr bool HAS_DUAL = true, HAS_PEER = true;
   static constexpr bool SPLIT_PRODUCER = true;  // the tile producer as a warp of its own (measured per format)
-  static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (make_plan_mma)
+  static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
 
   // digit planes in natural column order
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,

@@ -363,7 +363,8 @@ __device__ __forceinline__ void unpack_slots(const QkPeers &peers, unsigned uwan
 // 8 i ..), both see the same split activations, and the reducer writes
 // silu(gate) * up (crates/oxillama-arch/src/common/swiglu.rs:15-21) where a plain matvec
 // writes its dot products.
-template <class F, int M, bool INCTA, int CW, int G, int MODE>
+// DEEP: the ring has every stage that fits, not a multiple of the groups' (see make_plan_mma).
+template <class F, int M, bool INCTA, int CW, int G, int MODE, bool DEEP>
 __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE == 1 ? 1 : 0)) * 32, 1)
     qk_gemv_imma_kernel(QkLayout L, const uint8_t *__restrict__ W, const uint8_t *__restrict__ W2,
                            const float *__restrict__ x,
@@ -417,7 +418,7 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
     for (; item < end;) {
       issue();
       item++;
-      if (F::ANY_DEPTH && lead) *reinterpret_cast<volatile uint32_t *>(smem + S.prog + 4) = item;
+      if (DEEP && lead) *reinterpret_cast<volatile uint32_t *>(smem + S.prog + 4) = item;
     }
   };
   if (SPLIT && warp == CW + 1) {
@@ -641,7 +642,7 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
       const uint32_t tile = sbase + S.stage + st * stage_bytes;
       // (in the ring's first round there is no tile before)
       const uint32_t it = c * L.ktiles + kt;
-      if ((F::ANY_DEPTH && it >= (uint32_t)nstage && !wait_issued(sbase + S.prog + 4, it, seen)) || !mbar_wait_bounded(sbase + S.full + st * 8, fph)) {
+      if ((DEEP && it >= (uint32_t)nstage && !wait_issued(sbase + S.prog + 4, it, seen)) || !mbar_wait_bounded(sbase + S.full + st * 8, fph)) {
         dead = true;
         break;
       }
@@ -699,10 +700,11 @@ struct PlanMma {
   SmemMma S;
   uint32_t Kp, stage_bytes, total;
   int nstage, nslot, groups;
+  int deep;  // stages that fit
 };
 
-// xsb: bytes per 32-column block in the activation scale table (F::XSB).  any_depth: see below.
-inline bool make_plan_mma(const QkLayout &L, uint32_t m, PlanMma *P, uint32_t xsb, bool any_depth = false) {
+// xsb: bytes per 32-column block in the activation scale table (F::XSB).
+inline bool make_plan_mma(const QkLayout &L, uint32_t m, PlanMma *P, uint32_t xsb) {
   if (L.nb == 0 || L.chunks == 0) return false;  // nothing to stream: the callers handle empty shapes
   uint32_t Kp = L.nb * L.bs;
   if (Kp % 256u) return false;  // the kernels walk K in spans of 256 columns
@@ -735,32 +737,43 @@ inline bool make_plan_mma(const QkLayout &L, uint32_t m, PlanMma *P, uint32_t xs
   // a chunk's stages are refilled only once the whole chunk is reduced: its k-tiles
   // must all fit in the ring with room to prefetch the next chunk
   if ((uint32_t)nstage < L.ktiles + 1) return false;
-  // Largest group count whose G * ktiles the ring holds.  A stage must always be consumed by the same group (a
-  // waiter on an mbarrier may be at most one phase ahead of it), so the depth is rounded down to a multiple of
-  // G * ktiles -- but for formats with F::ANY_DEPTH, which take every stage there is and count the tiles issued
-  // (wait_issued).  Measured both ways: Q6_K, four or seven stages at 4096 columns, 128256 x 4096 76.3 -> 66.5 us
-  // (with the k = 16 MMA); Q4_K, eight or eleven, 14336 x 4096 7.5 -> 8.2.
+  // Largest group count whose G * ktiles divides a ring depth we can afford.  A stage must always be consumed by
+  // the same group (a waiter on an mbarrier may be at most one phase ahead of it), so the depth is a multiple of
+  // G * ktiles -- but where ring_is_deep says so.
+  const int deep = nstage;
   int groups = 1;
   const char *ge = qk_knob("QK_GROUPS");
   const int gmax = ge ? atoi(ge) : 4;
   for (int gtry = 4; gtry >= 2; gtry >>= 1) {
     const int unit = gtry * (int)L.ktiles;
-    if (gtry <= gmax && nstage >= unit && (any_depth || (nstage / unit) * unit >= (int)L.ktiles + 1)) {
+    if (gtry <= gmax && (nstage / unit) * unit >= (int)L.ktiles + 1) {
       groups = gtry;
-      if (!any_depth) nstage = (nstage / unit) * unit;
+      nstage = (nstage / unit) * unit;
       break;
     }
   }
   P->S = S, P->Kp = Kp, P->stage_bytes = stage_bytes, P->nstage = nstage, P->nslot = nstage + 1, P->groups = groups;
+  P->deep = deep;
   P->total = off + nstage * stage_bytes;
   return true;
 }
 
-template <class F, int M, bool INCTA, int CW, int G, int MODE = 0>
+// Whether a launch takes every stage that fits and counts the tiles issued (wait_issued): formats with F::ANY_DEPTH,
+// where a CTA has more tiles than the multiple holds.  Q6_K, four or seven stages at 4096 columns (us, graph):
+// 32000 rows 22.6 -> 19.3, 14336 11.2 -> 10.2, 8192 (seven tiles) 7.8 -> 7.2; but 4096 (four) 5.1 -> 5.4,
+// 1024 (one) 3.4 -> 3.55: the further stages stay empty and the count costs.  Q4_K, eight or eleven, 14336 rows
+// 7.5 -> 8.2.
+template <class F>
+inline bool ring_is_deep(const QkLayout &L, const PlanMma &P, int sm_count, bool dual) {
+  const uint32_t grid = L.chunks < (uint32_t)sm_count ? L.chunks : (uint32_t)sm_count;
+  return F::ANY_DEPTH && P.deep > P.nstage && (L.chunks + grid - 1) / grid * L.ktiles * (dual ? 2u : 1u) > (uint32_t)P.nstage;
+}
+
+template <class F, int M, bool INCTA, int CW, int G, int MODE = 0, bool DEEP = false>
 cudaError_t launch_mma(const QkLayout &L, const uint8_t *W, const float *x, float *y, uint64_t ldy,
                        unsigned *status, unsigned char *ximg, int sm_count, const PlanMma &P,
                        cudaStream_t s, const QkPeers *peers = nullptr, const uint8_t *W2 = nullptr) {
-  auto kern = qk_gemv_imma_kernel<F, M, INCTA, CW, G, MODE>;
+  auto kern = qk_gemv_imma_kernel<F, M, INCTA, CW, G, MODE, DEEP>;
   static QkPerDevice attr_set;
   if (attr_set.first()) {
     cudaError_t e =
@@ -793,9 +806,10 @@ cudaError_t launch_mma(const QkLayout &L, const uint8_t *W, const float *x, floa
   }
   uint32_t grid = (uint32_t)sm_count * (uint32_t)ctas;  // persistent
   if (grid > L.chunks) grid = L.chunks;
+  const int nstage = DEEP ? P.deep : P.nstage;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid), cfg.blockDim = dim3((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + ((MODE == 1 && peers && peers->unpack_n) ? 1 : 0)) * 32);
-  cfg.dynamicSmemBytes = P.total, cfg.stream = s;
+  cfg.dynamicSmemBytes = P.total + (uint32_t)(nstage - P.nstage) * P.stage_bytes, cfg.stream = s;
   cfg.attrs = at, cfg.numAttrs = use_pdl ? 1 : 0;
   QkPeers pv = {};
   if (peers) pv = *peers;
@@ -810,9 +824,9 @@ cudaError_t launch_mma(const QkLayout &L, const uint8_t *W, const float *x, floa
     npre_env = e ? atoi(e) : 0;
   }
   int npre = npre_env > 0 ? npre_env : (M == 1 ? 2 : 1);
-  if (npre > P.nstage) npre = P.nstage;
+  if (npre > nstage) npre = nstage;
   return cudaLaunchKernelEx(&cfg, kern, L, W, W2, x, (const unsigned char *)ximg, y, ldy, status,
-                            P.nstage, P.nslot, P.stage_bytes, P.S, P.Kp, pv, npre);
+                            nstage, nstage + 1, P.stage_bytes, P.S, P.Kp, pv, npre);
 }
 
 // Every CTA redoing the split costs ~M*K/512 quads per thread; past this size the
@@ -832,11 +846,20 @@ cudaError_t launch_mma_m(const QkLayout &L, const uint8_t *W, const float *x, fl
                          uint64_t ldy, unsigned *status, unsigned char *ximg, int sm_count,
                          const PlanMma &P, cudaStream_t s, const QkPeers *peers, const uint8_t *W2, bool host_x) {
   // Warp groups: a group owns every G-th chunk (P.groups was chosen with the ring's depth, see make_plan_mma).
-  const bool peer = peers != nullptr;
-#define QK_LAUNCH1(CWV, GV, PV)                                                                               \
-  return !host_x && (!ximg || split_in_cta(P, M))                                                             \
-             ? launch_mma<F, M, true, CWV, GV, PV>(L, W, x, y, ldy, status, ximg, sm_count, P, s, peers, W2)  \
-             : launch_mma<F, M, false, CWV, GV, PV>(L, W, x, y, ldy, status, ximg, sm_count, P, s, peers, W2)
+  const bool peer = peers != nullptr, deep = ring_is_deep<F>(L, P, sm_count, W2 != nullptr);
+#define QK_LAUNCH2(CWV, GV, PV, DV)                                                                               \
+  return !host_x && (!ximg || split_in_cta(P, M))                                                                 \
+             ? launch_mma<F, M, true, CWV, GV, PV, DV>(L, W, x, y, ldy, status, ximg, sm_count, P, s, peers, W2)  \
+             : launch_mma<F, M, false, CWV, GV, PV, DV>(L, W, x, y, ldy, status, ximg, sm_count, P, s, peers, W2)
+#define QK_LAUNCH1(CWV, GV, PV)                            \
+  do {                                                     \
+    if constexpr (F::ANY_DEPTH && GV > 1) {                \
+      if (deep) {                                          \
+        QK_LAUNCH2(CWV, GV, PV, true);                     \
+      }                                                    \
+    }                                                      \
+    QK_LAUNCH2(CWV, GV, PV, false);                        \
+  } while (0)
 #define QK_LAUNCH(CWV, GV)                \
   do {                                    \
     if constexpr (F::HAS_DUAL) {          \
@@ -859,6 +882,7 @@ cudaError_t launch_mma_m(const QkLayout &L, const uint8_t *W, const float *x, fl
     default:
       QK_LAUNCH(MAX_CW, 1);
   }
+#undef QK_LAUNCH2
 #undef QK_LAUNCH1
 #undef QK_LAUNCH
 }
@@ -869,13 +893,13 @@ template <class F>
 bool supported(const QkLayout &L, uint32_t m) {
   if (m < 1 || m > (uint32_t)F::MAX_M) return false;
   PlanMma P;
-  return make_plan_mma(L, m, &P, F::XSB, F::ANY_DEPTH);
+  return make_plan_mma(L, m, &P, F::XSB);
 }
 
 template <class F>
 size_t scratch_bytes(const QkLayout &L, uint32_t m) {
   PlanMma P;
-  return make_plan_mma(L, m, &P, F::XSB, F::ANY_DEPTH) ? P.S.ximg_bytes : 0;
+  return make_plan_mma(L, m, &P, F::XSB) ? P.S.ximg_bytes : 0;
 }
 
 // tiled2 != nullptr: the two-matrix (feed-forward gate and up) mode, formats with F::HAS_DUAL only.
@@ -884,7 +908,7 @@ cudaError_t launch(const QkLayout &L, const uint8_t *tiled, const float *x, floa
                    unsigned *status, unsigned char *scratch, int sm_count, cudaStream_t s, const QkPeers *peers,
                    const uint8_t *tiled2 = nullptr, bool host_x = false) {
   PlanMma P;
-  if (!make_plan_mma(L, m, &P, F::XSB, F::ANY_DEPTH)) return cudaErrorInvalidConfiguration;
+  if (!make_plan_mma(L, m, &P, F::XSB)) return cudaErrorInvalidConfiguration;
   if (m < 1 || m > (uint32_t)F::MAX_M) return cudaErrorInvalidConfiguration;
   if ((tiled2 && (!F::HAS_DUAL || peers)) || (peers && !F::HAS_PEER)) return cudaErrorInvalidConfiguration;
   if (m == 1) return launch_mma_m<F, 1>(L, tiled, x, y, ldy, status, scratch, sm_count, P, s, peers, tiled2, host_x);

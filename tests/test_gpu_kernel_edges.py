@@ -491,14 +491,19 @@ def test_moe_group_sizes(t, counts):
     assert np.abs(y.cpu().numpy() - ref).max() <= 3e-3 * np.abs(ref).max()
 
 
-# Chunks through the ring of weight tiles: fewer than groups of warps, several rounds of the ring, one to three k-tiles
-# a chunk with the last one whole, one span and half.
-@pytest.mark.parametrize("rows,cols", [(5, 8448), (1190, 12288), (9480, 4096), (5003, 8448)])
+# Chunks through the ring of weight tiles: fewer than groups of warps, one more or fewer than the stages, several rounds
+# of the ring, one to three k-tiles a chunk with the last one whole, half and one span.  (Q6_K takes further stages where
+# a CTA has more tiles than a multiple of the groups holds: at 4096 columns up to 4736 rows four, above them seven.)
+RING_SHAPES = [(5, 8448), (1190, 12288), (9480, 4096), (5003, 8448), (5003, 6144), (5003, 8192)]
+
+
+@pytest.mark.parametrize("t,rows,cols", [(t, *s) for t in (S.Q6_K, S.Q4_K, S.Q8_0) for s in RING_SHAPES] +
+                         [(S.Q6_K, 4736, 4096), (S.Q6_K, 4737, 4096), (S.Q6_K, 24100, 4096)])
 @pytest.mark.parametrize("m", [1, 2, 3])
-@pytest.mark.parametrize("t", [S.Q6_K, S.Q4_K, S.Q8_0])
 def test_decode_ring(t, m, rows, cols):
     w = S.gen_weight(t, rows, cols, seed=121)
     x = S.gen_acts(m, cols, seed=122)
     y = device_product(t, w, x, rows, cols, m)
-    # (three rows of Q6_K, and of Q8_0 two of 12288 columns or three, go to the tensor cores: fp16 operands)
-    assert_product(y, x, O.dequant_matrix(t, w, rows, cols), half=m > {S.Q6_K: 2, S.Q8_0: 1}.get(t, 4))
+    # (three rows of Q6_K, and of Q8_0 two of 12288 columns or three of 8448, go to the tensor cores: fp16 operands)
+    most = 2 if t == S.Q6_K else {12288: 1, 8448: 2}.get(cols, 3) if t == S.Q8_0 else 3
+    assert_product(y, x, O.dequant_matrix(t, w, rows, cols), half=m > most)

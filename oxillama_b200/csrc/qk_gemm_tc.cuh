@@ -935,6 +935,7 @@ __global__ void __maxnreg__(REGS)
     auto take_half = [&](uint32_t dh) {                  // a segment's first MMA into an accumulator
       if ((dph >> (2 + dh)) & 1u) {
         if (!warp_wait(sbase + S.d_empty + dh * 8, (dph >> dh) & 1u)) return false;
+        tc_fence_after();  // its former contents have been read by other warps
         dph ^= 1u << dh;
       }
       dph |= 4u << dh;

@@ -107,6 +107,28 @@ def test_ffn_edges(tgu, td, hidden, inter, m):
         d.free()
 
 
+# Gate and up as a prompt has them: pairs of CTAs, tiles of one and of two accumulator halves, equal and not (160 to 240
+# tokens), several tiles a pair, a ragged last token block, segments of one to a few super-blocks.
+@pytest.mark.parametrize("t,hidden,inter", [(S.Q6_K, 512, 14336), (S.Q4_K, 256, 14336), (S.Q6_K, 1024, 4736), (S.IQ4_XS, 768, 9472)])
+@pytest.mark.parametrize("m", [129, 150, 200, 300, 512, 700, 801])
+def test_ffn_of_a_prompt(t, hidden, inter, m):
+    import torch
+    from oxillama_b200.device import DeviceWeights, check_device_status, ffn
+    shapes = [(inter, hidden), (inter, hidden), (hidden, inter)]
+    ws = [S.gen_weight(t, r, c, seed=72, stream=i, d_range=(1e-3, 3e-3)) for i, (r, c) in enumerate(shapes)]
+    x = torch.from_numpy(S.gen_acts(m, hidden, seed=72) * np.float32(0.25)).cuda()
+    g, u, d = (torch.from_numpy(O.dequant_matrix(t, w, r, c)).cuda().double() for w, (r, c) in zip(ws, shapes))
+    ref = (torch.nn.functional.silu(x.double() @ g.T) * (x.double() @ u.T)) @ d.T
+    dw = [DeviceWeights(t, w, r, c) for w, (r, c) in zip(ws, shapes)]
+    y = torch.full((m, hidden), float("nan"), device="cuda")
+    ffn(*dw, x, y, m)
+    check_device_status()
+    # three chained products, each within 1e-3 of its largest value (fp16 operands)
+    assert float((y.double() - ref).abs().max()) <= 3e-3 * float(ref.abs().max())
+    for w in dw:
+        w.free()
+
+
 # Up to 16 tokens: every expert that is hit, on the decode kernels up to four rows and on the tensor cores
 # beside them above; one expert takes all tokens, another none; also shards that start inside, with that
 # expert and without.  A token whose experts here have up to four rows each keeps the f32-grade bound.
@@ -461,7 +483,7 @@ def test_moe_short_rows(t, hidden, inter, tokens):
 
 
 # Groups of every size around the activation boxes (one to four of whole 8-row atoms): tiles of 64 tokens in one CTA
-# and of 96 and 160 in a pair.  The bound: three chained products, each within 1e-3 of its largest value.
+# and of 96 and 256 in a pair.  The bound: three chained products, each within 1e-3 of its largest value.
 @pytest.mark.parametrize("counts", [[1, 15, 16, 17, 47, 48, 49, 64, 65, 0], [96, 97, 64, 65, 81, 80, 1, 33, 95, 20],
                                     [160, 161, 128, 127, 40, 41, 79, 300, 2, 0]])
 @pytest.mark.parametrize("t", [S.Q4_K, S.IQ4_XS])

@@ -70,7 +70,7 @@ constexpr int MAX_SLOT = MAX_STAGE + 1;
 struct SmemMma {
   uint32_t full, redfull, xbar;  // mbarriers (8 B each)
   uint32_t prog;                 // chunks the reducer warp has read so far (one word, polled by the producer warp)
-                                 // and behind it the tiles issued so far (polled by the compute warps)
+  uint32_t issued;               // DEEP: tiles issued so far (one word, polled by the compute warps)
   uint32_t red, ximg, stage;
   uint32_t PS;         // digit plane stride, bytes
   uint32_t xs_off;     // offset of the (sx, Sx) table inside the x image
@@ -176,12 +176,13 @@ __device__ __forceinline__ float digit_scale(float amax, float s32) {
 // Waits (bounded) until more than `item` tiles have been issued: from then on the barrier of the item's stage
 // is in the item's phase.  A stage goes from group to group of the compute warps, so a group could come to it
 // while the tile before, another group's, is still on its way, two phases back, and take that barrier for its
-// own.  `seen`: the count as last read.
+// own.  That the phases before are over reaches this group through the count alone: published with a release
+// behind the waits that saw it, read with an acquire.  `seen`: the count as last read.
 __device__ __forceinline__ bool wait_issued(uint32_t word_addr, uint32_t item, uint32_t &seen) {
   if (seen > item) return true;
   unsigned long long t0 = 0;
   for (uint32_t polls = 1;; polls++) {
-    asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(seen) : "r"(word_addr) : "memory");
+    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(seen) : "r"(word_addr) : "memory");
     if (seen > item) return true;
     if ((polls & 1023u) == 0) {
       unsigned long long t;
@@ -190,6 +191,10 @@ __device__ __forceinline__ bool wait_issued(uint32_t word_addr, uint32_t item, u
       if (t - t0 > 250000000ull) return false;
     }
   }
+}
+
+__device__ __forceinline__ void tell_issued(uint32_t word_addr, uint32_t items) {
+  asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(word_addr), "r"(items) : "memory");
 }
 
 // Activations e0 .. e0 + 3 of one row out of the tagged slots of a gathered buffer (columns
@@ -393,7 +398,7 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
     for (int s = 0; s < nstage; s++) mbar_init(sbase + S.full + s * 8, 1);
     for (int s = 0; s < nslot; s++) mbar_init(sbase + S.redfull + s * 8, WG);
     mbar_init(sbase + S.xbar, 1);
-    *reinterpret_cast<volatile uint32_t *>(smem + S.prog) = 0u, *reinterpret_cast<volatile uint32_t *>(smem + S.prog + 4) = 0u;
+    *reinterpret_cast<volatile uint32_t *>(smem + S.prog) = 0u, *reinterpret_cast<volatile uint32_t *>(smem + S.issued) = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -418,7 +423,7 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
     for (; item < end;) {
       issue();
       item++;
-      if (DEEP && lead) *reinterpret_cast<volatile uint32_t *>(smem + S.prog + 4) = item;
+      if (DEEP && lead) tell_issued(sbase + S.issued, item);
     }
   };
   if (SPLIT && warp == CW + 1) {
@@ -642,7 +647,7 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
       const uint32_t tile = sbase + S.stage + st * stage_bytes;
       // (in the ring's first round there is no tile before)
       const uint32_t it = c * L.ktiles + kt;
-      if ((DEEP && it >= (uint32_t)nstage && !wait_issued(sbase + S.prog + 4, it, seen)) || !mbar_wait_bounded(sbase + S.full + st * 8, fph)) {
+      if ((DEEP && it >= (uint32_t)nstage && !wait_issued(sbase + S.issued, it, seen)) || !mbar_wait_bounded(sbase + S.full + st * 8, fph)) {
         dead = true;
         break;
       }
@@ -716,7 +721,8 @@ inline bool make_plan_mma(const QkLayout &L, uint32_t m, PlanMma *P, uint32_t xs
   S.full = off, off += MAX_STAGE * 8;
   S.redfull = off, off += MAX_SLOT * 8;
   S.xbar = off, off += 8;
-  S.prog = off, off += 8;
+  S.prog = off, off += 4;
+  S.issued = off, off += 4;
   off = (off + 127u) & ~127u;
   S.red = off, off += MAX_SLOT * MAX_CW * m * 8 * 4;
   off = (off + 127u) & ~127u;

@@ -745,13 +745,17 @@ struct TileAt {
   uint32_t g, rb, t0, live, n;  // n: tokens the MMA covers, a multiple of 16
 };
 
-// The super-blocks of a segment in the order the MMAs take them: one at a time (`half` 0, then 1),
-// but at either end of a wide tile two at a time (both under half 0, then both under half 1).
-// Calls step(sb, half) -> false to stop.
+// The order in which a segment's super-blocks are taken, for the producer of the activations and the issuer of the
+// MMAs, who meet only at the ring's stages and must agree: one at a time (under half 0, then half 1), but at either
+// end of a wide segment two at a time (both under half 0, then both under half 1).
+__device__ __forceinline__ uint32_t taken_together(uint32_t sb, uint32_t s0, uint32_t s1) {
+  return s1 - sb >= 2 && (sb == s0 || s1 - sb == 2) ? 2u : 1u;
+}
+// Calls step(sb, half) in that order -> false to stop.
 template <class Step>
 __device__ __forceinline__ bool walk_segment(uint32_t s0, uint32_t s1, bool wide, Step &&step) {
   for (uint32_t sb = s0; sb < s1;) {
-    const uint32_t two = wide && s1 - sb >= 2 && (sb == s0 || s1 - sb == 2) ? 2u : 1u;
+    const uint32_t two = wide ? taken_together(sb, s0, s1) : 1u;
     for (uint32_t h = 0; h < (wide ? 2u : 1u); h++)
       for (uint32_t k = 0; k < two; k++)
         if (!step(sb + k, h)) return false;
@@ -977,15 +981,15 @@ __global__ void __maxnreg__(REGS)
         }
         if (!dead) umma_commit<CG>(sbase + S.d_full + dh * 8, lead);
       } else {
-        // Two accumulator halves: one super-block at a time under half 0, then half 1, but at either end of the
-        // segment two at a time (walk_segment); the buffers are walked again under the second half.  (Written out: as one
-        // step for either half, gate and up of 14336 x 4096 by 512 took 111.6 us under ncu instead of 103.3.)
+        // Two accumulator halves, in the order of walk_segment; the buffers are walked again under the second half.
+        // (Written out: as one step for either half, gate and up of 14336 x 4096 by 512 took 111.6 us under ncu instead of
+        // 103.3.)
         const uint32_t n1 = q.n - A.hn, idesc1 = (1u << 4) | ((n1 >> 3) << 17) | ((CG * BM >> 4) << 24), step1 = box_rows(n1) * 8u;
         bool ok = take_half(0);
         ready = false;
         uint32_t acc0 = 0u, acc1 = 0u;
         for (uint32_t sb = s0; sb < s1 && ok;) {
-          const uint32_t two = s1 - sb >= 2 && (sb == s0 || s1 - sb == 2) ? 2u : 1u;
+          const uint32_t two = taken_together(sb, s0, s1);
           uint32_t abk = ab, ph = aph;
           for (uint32_t k = 0; k < two && ok; k++) {
             ok = __all_sync(0xffffffffu, ready) || (warp_wait(a_full + abk * 8, ph) && warp_wait(b_full + bs * 8, bph));

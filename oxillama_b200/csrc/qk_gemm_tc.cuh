@@ -768,7 +768,10 @@ __device__ __forceinline__ bool walk_segment(uint32_t s0, uint32_t s1, bool wide
 // T: weight format.  CG: CTAs per tile (see the top).  NG: 1 = one matrix; otherwise up to NG matrices
 // of one shape and format (the projections of a feed-forward block, the experts of a mixture), each
 // multiplying its own group of activation rows.
-// REGS: registers per thread: 80, or 72 to leave room for CTAs of the conversion beside it.
+// REGS: registers per thread: 80, or 72 to leave room for CTAs of the conversion beside it, and for the pairs of one
+// matrix: since the wide loop is written out, their build of 80 spills more than that of 72 and is the slower one
+// (us, before the wide loop / with 80 / with 72: IQ4_XS 2048 x 5632 by 160 20.1 / 21.4 / 20.2, 5120 x 5120 by 160
+// 22.8 / 23.8 / 22.4, Q6_K 4096 x 14336 by 256 50.1 / 44.8 / 43.5, 14336 x 4096 by 512 66.2 / 67.0 / 63.7).
 template <int T, int CG, int NG, int REGS>
 __global__ void __maxnreg__(REGS)
     qk_gemm_tc_kernel(const __grid_constant__ TcArgs A, const __grid_constant__ TcMaps<NG> M) {
@@ -1340,7 +1343,7 @@ cudaError_t launch_main(const TcPlan &P, const TcArgs &A, __half *x16, const QkT
   return cudaLaunchKernelEx(&cfg, kern, A, M);
 }
 
-// Formats whose expansion runs as fast on 72 registers (Q6_K does not: 4096 x 14336 by 512 66.0 against 63.0 us).
+// Formats whose single CTAs take 72 registers beside the conversion.
 constexpr bool beside_of(int t) { return t != QK_T_Q6_K; }
 
 template <int T>
@@ -1388,9 +1391,10 @@ cudaError_t launch_fmt(const QkTcCall &c, unsigned *status, unsigned char *scrat
   // 16.7 -> 15.9.
   A.ahead = P.cg == 1 && !c.counts && P.cs == 1 && c.m < 64 ? 2u : 0u;
   if (c.n == 1 && !c.counts) {
+    if (P.cg == 2) return launch_main<T, 2, 1, 72>(P, A, x16, c, s);
     if constexpr (beside_of(T))
-      if (beside) return P.cg == 1 ? launch_main<T, 1, 1, 72>(P, A, x16, c, s) : launch_main<T, 2, 1, 72>(P, A, x16, c, s);
-    return P.cg == 1 ? launch_main<T, 1, 1>(P, A, x16, c, s) : launch_main<T, 2, 1>(P, A, x16, c, s);
+      if (beside) return launch_main<T, 1, 1, 72>(P, A, x16, c, s);
+    return launch_main<T, 1, 1>(P, A, x16, c, s);
   }
   return P.cg == 1 ? launch_main<T, 1, QK_MAX_GROUPS>(P, A, x16, c, s) : launch_main<T, 2, QK_MAX_GROUPS>(P, A, x16, c, s);
 }

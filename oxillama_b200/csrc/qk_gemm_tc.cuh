@@ -1343,9 +1343,6 @@ cudaError_t launch_main(const TcPlan &P, const TcArgs &A, __half *x16, const QkT
   return cudaLaunchKernelEx(&cfg, kern, A, M);
 }
 
-// Formats whose single CTAs take 72 registers beside the conversion.
-constexpr bool beside_of(int t) { return t != QK_T_Q6_K; }
-
 template <int T>
 cudaError_t launch_fmt(const QkTcCall &c, unsigned *status, unsigned char *scratch, int sm_count, cudaStream_t s) {
   const QkLayout &L = *c.L;
@@ -1359,7 +1356,11 @@ cudaError_t launch_fmt(const QkTcCall &c, unsigned *status, unsigned char *scrat
   C.x = c.x, C.x2 = c.x2, C.out = x16, C.scales = scales, C.zero = cnt, C.n_zero = (uint32_t)sm_count * 2;
   C.counts = c.counts, C.lists = c.lists, C.m = c.m, C.cols = L.cols, C.Kp = Kp, C.cap = c.xcap;
   C.list_stride = c.list_stride, C.list_div = c.list_div ? c.list_div : 1u;
-  const bool narrow = (c.counts || (c.n == 1 && c.m >= 64)) && Kp <= 4096, beside = beside_of(T) && narrow && !c.counts;
+  const bool narrow = (c.counts || (c.n == 1 && c.m >= 64)) && Kp <= 4096;
+  // Single CTAs beside the conversion (72 registers).  Q6_K only where the conversion has more rows than a tile: its
+  // expansion wants the 80 (us, 80 / 72 registers: 4096 x 4096 by 80 16.5 / 14.4, by 160 17.1 / 15.4; 14336 x 4096 by
+  // 64 16.1 / 16.9).
+  const bool beside = narrow && !c.counts && (T != QK_T_Q6_K || c.m > 64);
   cudaLaunchAttribute at = pdl_attr();
   cudaLaunchConfig_t c0 = {};
   c0.gridDim = dim3(c.counts || c.n_act > 1 ? c.n_act * c.xcap : c.m), c0.blockDim = dim3(narrow ? 256 : 512), c0.stream = s, c0.attrs = &at, c0.numAttrs = 1;
@@ -1392,9 +1393,7 @@ cudaError_t launch_fmt(const QkTcCall &c, unsigned *status, unsigned char *scrat
   A.ahead = P.cg == 1 && !c.counts && P.cs == 1 && c.m < 64 ? 2u : 0u;
   if (c.n == 1 && !c.counts) {
     if (P.cg == 2) return launch_main<T, 2, 1, 72>(P, A, x16, c, s);
-    if constexpr (beside_of(T))
-      if (beside) return launch_main<T, 1, 1, 72>(P, A, x16, c, s);
-    return launch_main<T, 1, 1>(P, A, x16, c, s);
+    return beside ? launch_main<T, 1, 1, 72>(P, A, x16, c, s) : launch_main<T, 1, 1>(P, A, x16, c, s);
   }
   return P.cg == 1 ? launch_main<T, 1, QK_MAX_GROUPS>(P, A, x16, c, s) : launch_main<T, 2, QK_MAX_GROUPS>(P, A, x16, c, s);
 }

@@ -49,6 +49,7 @@ static bool plan_smem(uint32_t bn, uint32_t hn, uint32_t cg, uint32_t cs, uint32
   s.drain = off, off += 8;
   s.tmem_slot = off, off += 8;
   s.pre = off, off += (QK_MAX_GROUPS + 1) * 4;
+  s.sched = off, off += (uint32_t)sizeof(Sched);
   off = (off + 15u) & ~15u;
   s.scales = off, off += 4 * 512 + 16;  // a copy of a half's token scales per epilogue warp, and one word
   if (off > LUT_OFF) return false;

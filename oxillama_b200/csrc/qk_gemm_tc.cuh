@@ -78,10 +78,10 @@ constexpr int NDW = 16;            // expanding warps: two sets of eight (three 
 constexpr int FIRST_EW = FIRST_DW + NDW, NTHREADS = (FIRST_EW + 4) * 32;
 constexpr uint32_t MAX_BN = 256;   // most tokens per tile: two accumulator halves of 128
 constexpr int MAX_WST = 12, MAX_BST = 6;
-constexpr uint32_t LUT_OFF = 2560;  // of a format's look-up table in shared memory, behind the barriers and scales
+constexpr uint32_t LUT_OFF = 2688;  // of a format's look-up table in shared memory, behind the barriers and scales
 
 struct TcSmem {
-  uint32_t w_full, w_empty, b_full, b_empty, a_full, a_empty, d_full, d_empty, drain, tmem_slot, pre, scales, red;
+  uint32_t w_full, w_empty, b_full, b_empty, a_full, a_empty, d_full, d_empty, drain, tmem_slot, pre, sched, scales, red;
   uint32_t w, b;                   // ring bases
   uint32_t w_stage, b_stage;       // bytes per stage
   uint32_t w_stages, b_stages;
@@ -769,9 +769,8 @@ __device__ __forceinline__ bool walk_segment(uint32_t s0, uint32_t s1, bool wide
 // of one shape and format (the projections of a feed-forward block, the experts of a mixture), each
 // multiplying its own group of activation rows.
 // REGS: registers per thread: 80, or 72 to leave room for CTAs of the conversion beside it, and for the pairs of one
-// matrix: since the wide loop is written out, their build of 80 spills more than that of 72 and is the slower one
-// (us, before the wide loop / with 80 / with 72: IQ4_XS 2048 x 5632 by 160 20.1 / 21.4 / 20.2, 5120 x 5120 by 160
-// 22.8 / 23.8 / 22.4, Q6_K 4096 x 14336 by 256 50.1 / 44.8 / 43.5, 14336 x 4096 by 512 66.2 / 67.0 / 63.7).
+// matrix at every K (72 / 80, neither of them spilling, us: Q8_0 5120 x 5120 by 160 20.0 / 20.7, Q6_K 4096 x 14336 by 80
+// 22.6 / 23.4; 0.7 % over 191 calls).
 template <int T, int CG, int NG, int REGS>
 __global__ void __maxnreg__(REGS)
     qk_gemm_tc_kernel(const __grid_constant__ TcArgs A, const __grid_constant__ TcMaps<NG> M) {
@@ -787,10 +786,19 @@ __global__ void __maxnreg__(REGS)
 
   pdl_launch_dependents();
   const bool counted = NG > 1 && A.counts;
-  Sched sc{};
+  // The schedule of a pair of one matrix lies in shared memory, and a role takes its own copy: in registers from the start
+  // its twelve words were live in every role, and the pairs spilled (us, so / now: Q8_0 5120 x 5120 by 80 17.0 / 15.9, Q6_K
+  // 4096 x 14336 by 80 24.5 / 22.6, Q4_K 5120 x 5120 by 256 25.8 / 24.4).  Single CTAs do not spill and are up to 12 %
+  // slower without it in registers; of the pairs of several matrices some are faster, some slower (8 Q4_K experts, 512
+  // tokens 461 / 480).
+  constexpr bool SHARED_SCHED = CG == 2 && NG == 1;
+  Sched own{};
+  Sched &sched = SHARED_SCHED ? *reinterpret_cast<Sched *>(smem + S.sched) : own;
   auto make_schedule = [&](uint32_t tiles) {
-    if (CG == 1 && NG == 1 && A.cs > 1) sc.init_cluster((A.L.cols + 255u) / 256u, A.cs);
-    else sc.template init<CG>(tiles, (A.L.cols + 255u) / 256u, A.min_run);
+    Sched t{};
+    if (CG == 1 && NG == 1 && A.cs > 1) t.init_cluster((A.L.cols + 255u) / 256u, A.cs);
+    else t.template init<CG>(tiles, (A.L.cols + 255u) / 256u, A.min_run);
+    sched = t;
   };
   uint32_t *pre = reinterpret_cast<uint32_t *>(smem + S.pre);  // tiles before group g (device-counted groups)
   auto at = [&](uint32_t tile) {
@@ -812,7 +820,7 @@ __global__ void __maxnreg__(REGS)
     q.n = left >= A.bn ? A.bn : ((left + 15u) & ~15u);
     return q;
   };
-  if (!counted) make_schedule(A.n * A.row_blocks * A.tok_blocks);
+  if (!counted && (!SHARED_SCHED || threadIdx.x == FIRST_DW * 32)) make_schedule(A.n * A.row_blocks * A.tok_blocks);
   // Where A.ahead says so the first weights are asked for before anything else: a CTA that starts when the
   // previous one on its SM has ended gets them 1.9 us later, and the rest of its setting up takes 1.3.
   uint32_t ws = 0, w_ahead = 0;    // (warp 2) ring stage of the next super-block; super-blocks asked for here
@@ -828,9 +836,9 @@ __global__ void __maxnreg__(REGS)
     __syncwarp();
     if (A.once) policy = stream_policy();
     else asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(policy));
-    if (A.ahead && sc.n_seg) {  // of the first segment
+    if (CG == 1 && A.ahead && sched.n_seg) {  // of the first segment
       uint32_t tile, s0, s1;
-      sc.get(0, tile, s0, s1);
+      sched.get(0, tile, s0, s1);
       const TileAt q = at(tile);
       for (uint32_t sb = s0; sb < s1 && ws < A.ahead; sb++, ws++) {
         expect_tx(sbase + S.w_full + ws * 8, S.w_stage, w_lead);
@@ -889,6 +897,7 @@ __global__ void __maxnreg__(REGS)
   // tokens at a time, a lane four rows.
   auto add_up = [&](uint32_t tile) {
     __threadfence();
+    const Sched sc = sched;
     const TileAt q = at(tile);
     const uint32_t i0 = sc.owner_of(tile * sc.nsb), i1 = sc.owner_of((tile + 1) * sc.nsb - 1), slot = A.bn * BM;
     const uint32_t live = min(q.live - q.t0, q.n), row0 = (q.rb * CG + rank) * BM, rw = row0 + 4 * lane;
@@ -934,6 +943,7 @@ __global__ void __maxnreg__(REGS)
     // for some 500 cycles before it takes longer than the expansion.  So what a segment does not change is worked
     // out ahead of its steps, and the next step's barriers are looked at (without waiting) behind the commits.  (As
     // one general step per super-block and half, worked out anew each time: 1250 cycles at 8 to 128 tokens.)
+    const Sched sc = sched;
     const uint32_t lead = elect_one() ? 1u : 0u;
     const uint32_t a_full = sbase + S.a_full, a_empty = sbase + S.a_empty, b_full = sbase + S.b_full, b_empty = sbase + S.b_empty;
     const uint32_t nbs = S.b_stages, stage16 = S.b_stage >> 4, bd0 = umma_desc_lo(sbase + S.b), a0 = tmem + a_col;
@@ -1032,6 +1042,7 @@ __global__ void __maxnreg__(REGS)
     }
   } else if (warp == 1) {
     // ======================= activation producer =======================
+    const Sched sc = sched;
     const uint32_t lead = elect_one() ? 1u : 0u;
     pdl_wait();  // X16 belongs to the previous kernel until it has finished
     const uint32_t full0 = in_first<CG>(sbase + S.b_full);
@@ -1066,6 +1077,7 @@ __global__ void __maxnreg__(REGS)
   } else if (warp == 2) {
     // ======================= weight producer =======================
     // The weights are immutable: their stream starts before the previous kernel has ended.
+    const Sched sc = sched;
     const uint32_t lead = w_lead, to_empty = S.w_empty - S.w_full, nst = S.w_stages, stage = S.w_stage;
     uint32_t wph = 0, rounds = 0;
     if (ws == nst) ws = 0, wph = 1u, rounds = 1;
@@ -1094,6 +1106,7 @@ __global__ void __maxnreg__(REGS)
   } else if (warp >= FIRST_EW) {
     // ======================= epilogue warps =======================
     // Warp `quarter` owns accumulator lanes (weight rows) 32 quarter .. + 32 of every half.
+    const Sched sc = sched;
     const uint32_t quarter = warp & 3u, r = 32 * quarter + lane;
     const uint32_t tlane = tmem + ((32 * quarter) << 16);
     const uint32_t d_empty = in_first<CG>(sbase + S.d_empty);
@@ -1206,9 +1219,9 @@ __global__ void __maxnreg__(REGS)
     const uint32_t r = 32 * quarter + lane, rr = r & 7u;               // weight row inside the tile, inside its chunk
     constexpr uint32_t CHB = 8 * F::BB * F::BPS;                       // a chunk's bytes of one super-block
     uint32_t n_sb = 0;
-    for (uint32_t i = 0; i < sc.n_seg; i++) {
+    for (uint32_t i = 0; i < sched.n_seg; i++) {
       uint32_t tile, s0, s1;
-      sc.get(i, tile, s0, s1);
+      sched.get(i, tile, s0, s1);
       n_sb += s1 - s0;
     }
     const uint32_t w_bytes = S.w_stage, nst = S.w_stages, w0 = sbase + S.w + (r >> 3) * CHB;
@@ -1264,7 +1277,7 @@ __global__ void __maxnreg__(REGS)
     // for another warp that takes 0.3 us even when it is long over): a lane four rows of one token at a time, the
     // first scale fetched ahead of the meeting.  Added up in the order of the K runs.
     const bool adds = warp >= FIRST_EW;
-    const TileAt q = at(sc.first_tile);
+    const TileAt q = at(sched.first_tile);
     const uint32_t live = min(q.live - q.t0, q.n), own = (live + A.cs - 1) / A.cs, t0 = blockIdx.x % A.cs * own, t1 = min(t0 + own, live);
     const uint32_t first = t0 + warp - FIRST_EW, r = 4 * lane, row = q.rb * BM + r;
     const float *sp = A.xscale + q.t0;
@@ -1298,8 +1311,8 @@ __global__ void __maxnreg__(REGS)
     else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
   }
   if (*last)
-    for (uint32_t i = 0; i < sc.n_split; i++)
-      if (*last >> i & 1u) add_up(sc.first_tile + i);
+    for (uint32_t i = 0; i < sched.n_split; i++)
+      if (*last >> i & 1u) add_up(sched.first_tile + i);
 }
 
 // ---------------------------------------------------------------- host side

@@ -74,14 +74,16 @@ static bool plan_smem(uint32_t bn, uint32_t hn, uint32_t cg, uint32_t cs, uint32
 
 static uint32_t round_up(uint32_t v, uint32_t to) { return (v + to - 1) / to * to; }
 
-// Form of the kernel, token-tile width and K split by predicted time: cycles of the slowest CTA.  The
-// constants are a fit to 96 shapes (256 x 12288 .. 28672 x 4096, 8 .. 2048 tokens, Q4_K, Q6_K, Q8_0, IQ4_XS; Q4_0
-// takes Q4_K's), each timed with every tile width and split: the prediction is 12 % off (rms, plans within 1.6 times
-// the fastest), the form it picks 1.0 % slower than the fastest (mean; 2.7 % with the constants of the kernel before
-// its MMA loop was shortened).  A super-block takes as long as its expansion or its MMAs, or
-// in a pair the round of hand-overs (expanding warps -> issuer -> tensor pipe -> back).  A tile whose
-// partials go through the workspace costs some 7000 cycles and 40 per token (writing them out, the fence, the
-// counter, reading them back); through the cluster 4600, whatever its width.
+// Form of the kernel, token-tile width and K split by predicted time: cycles of the slowest CTA.  The constants are a
+// fit to 96 shapes (256 x 12288 .. 28672 x 4096, 8 .. 2048 tokens, Q4_K, Q6_K, Q8_0, IQ4_XS), each timed with every tile
+// width and split; the expansion's (one for all but Q6_K), the cluster's and the one for Q8_0 were then fitted to 1076
+// calls with the weights from HBM (16 shapes 1024 x 1024 .. 28672 x 4096, 300 x 8192 .. 4096 x 14336, the same tokens and
+// formats; rows of gate and up together are such shapes too): the form it picks is 1.1 % slower than the fastest in the
+// mean, 19 % at worst; 1.3 % and 22 % before.  A super-block takes as long as its expansion or its MMAs, or in a pair the
+// round of hand-overs (expanding warps -> issuer -> tensor pipe -> back).  A tile whose partials go through the
+// workspace costs some 7000 cycles and 40 per token (writing them out, the fence, the counter, reading them back);
+// through the cluster 4300 and 17 per token (with 4600 for any width IQ4_XS 2048 x 2048 by 64 took 9.5 us in clusters, 8.1
+// without).
 bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
   const QkLayout &L = *c.L;
   const uint32_t w_stage = 16u * 8u * L.bb * (256u / L.bs), lut = L.type == QK_T_IQ4_XS ? WFmt<QK_T_IQ4_XS>::LUT : 0u;
@@ -101,14 +103,15 @@ bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
     p.row_blocks = (L.rows + p.cg * BM - 1) / (p.cg * BM);
     p.grid = (uint32_t)sm_count / p.cg;
   } else {
-    const float expand = L.type == QK_T_Q6_K ? 1170.f : L.type == QK_T_IQ4_XS ? 1000.f : L.type == QK_T_Q8_0 ? 980.f : 930.f;
+    const float expand = L.type == QK_T_Q6_K ? 1170.f : 1000.f;
     float best = FLT_MAX;
     auto take = [&](float t, uint32_t cg, uint32_t cs, uint32_t bn, uint32_t tbr, uint32_t rbs, uint32_t run, uint32_t grid) {
       if (t < best) best = t, p.cg = cg, p.cs = cs, p.bn = bn, p.tok_blocks = tbr, p.row_blocks = rbs, p.min_run = run, p.grid = grid;
     };
     const uint32_t tb0 = (c.m + MAX_BN - 1) / MAX_BN;
-    // Every token block reads the weights again, from L2 at best: 1.5 % for twice as many blocks as needed (gate and up
-    // 14336 x 4096 by 512 tokens: 96.3 us in three blocks, 95.5 in two, but 3 us more where the weights come from HBM).
+    // Every token block reads the weights again, from L2 at best: 1.5 % for twice as many blocks as needed.  (Three blocks
+    // instead of two can still be the faster form, from HBM too: Q4_K 28672 x 4096 by 512 108 against 120 us, 112 row
+    // blocks being 3.03 rounds of 74 pairs in two and 4.54 in three; 14336 x 4096 by 512 65.5 against 59.4.)
     // (A pair only where its second CTA has rows: Q4_0 64 x 1280 by 2048 tokens 26.4 -> 14.0 us.)
     for (uint32_t cg = 1; cg <= (L.rows > BM ? 2u : 1u); cg++) {
       const uint32_t units = (uint32_t)sm_count / cg, rbs = (L.rows + cg * BM - 1) / (cg * BM);
@@ -118,7 +121,11 @@ bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
         if (k && bn < 32) break;
         if (cg == 1 && bn > 64) continue;
         const uint32_t tbr = (c.m + bn - 1) / bn;
-        const float sb = cg == 1 ? expand : fmaxf(fmaxf(expand + 125.f, 980.f + 2.f * bn), 9.f * bn), out = bn * 59.f;
+        float sb = cg == 1 ? expand : fmaxf(fmaxf(expand + 125.f, 980.f + 2.f * bn), 9.f * bn);
+        const float out = bn * 59.f;
+        // Beside Q8_0's four stages of weights there is room for two of such a tile's activations (plan_smem): 4096 x
+        // 14336 by 512 76.6 us in tiles of 128, 71.2 of 176.
+        if (L.type == QK_T_Q8_0 && bn > 112 && bn <= 128) sb += 60.f;
         const uint64_t tiles = (uint64_t)c.n * rbs * tbr;
         for (uint32_t run = 1; run <= 16; run <<= 1) {
           const uint32_t R = (uint32_t)(tiles % units), total = R * p.nsb;
@@ -143,7 +150,7 @@ bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
         if (cg == 1 && c.n == 1)
           for (uint32_t cs = 4; cs <= 8 && cs <= p.nsb; cs <<= 1)
             if (tiles * cs <= (uint32_t)sm_count * (cs == 4 ? 14u : 12u) / 16u)
-              take((float)((p.nsb + cs - 1) / cs) * sb + 4600.f + out, 1, cs, bn, tbr, rbs, 1, (uint32_t)tiles * cs);
+              take((float)((p.nsb + cs - 1) / cs) * sb + 4300.f + 17.f * bn + out, 1, cs, bn, tbr, rbs, 1, (uint32_t)tiles * cs);
       }
     }
   }

@@ -1,7 +1,7 @@
 // Q8_0, Q4_0, IQ4_XS and Q6_K policies of the decode kernel (qk_gemv_skel.cuh).
 //
 // All four use the MMA the way the Q4_K policy does: k = 32 of one
-// mma.sync.m16n8k32 is one group of 32 weights that share a scale, the even B columns
+// mma.sync.m16n8k32 (Q6_K: k = 16 of m16n8k16) is one group of weights that share a scale, the even B columns
 // carry the three activation digits of one group and the odd columns those of a second
 // group, and every lane of an MMA quad (g = lane / 4 = weight row, tig = lane % 4 = digit)
 // keeps fixed registers.  They differ in what the two groups of an MMA are:
@@ -10,10 +10,10 @@
 //                        2p, A rows 8-15 = the same rows of block 2p + 1; wanted are
 //                        C[r][2j] (block 2p, digit j) and C[8 + r][2j + 1] (block 2p + 1).
 //   Q6_K                 its scales cover 16 columns, so the two groups are the two
-//                        16-column strips of one 32-column block: k-slots 0-15 hold strip
-//                        0, slots 16-31 strip 1, the even B columns are zero in slots
-//                        16-31 and the odd ones zero in slots 0-15; A rows 8-15 are zero.
-//                        Wanted are C[r][2j] (strip 0) and C[r][2j + 1] (strip 1).
+//                        16-column strips of one 32-column block: A rows 0-7 are the
+//                        weight rows' strip 0, A rows 8-15 their strip 1, the even B columns
+//                        carry the digits of strip 0, the odd ones those of strip 1.
+//                        Wanted are C[r][2j] (strip 0) and C[8 + r][2j + 1] (strip 1).
 //
 // Zero points (Q4_0: q - 8, Q6_K: q - 32) are not subtracted from the weights: the
 // unsigned fields go into the MMA and  zero * scale * (sum of x over the group)  comes off

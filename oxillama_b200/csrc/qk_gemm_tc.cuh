@@ -298,8 +298,7 @@ __device__ __forceinline__ uint32_t word(const uint4 &v, int i) { return i == 0 
 // Four nibble pairs of one packed word -> 8 halves: low nibbles q become 1024 + q
 // (0x6400 | q), high nibbles 64 + q (0x5400 | q << 4, no shift needed); values come out
 // as pairs (byte 0, byte 2), (byte 1, byte 3) of the low nibbles, then of the high ones.
-// The exponents come from registers: an instruction takes one constant of 32 bits, and with two of them the
-// compiler makes two of every mask-and-or (157 -> 99 integer instructions for a thread's half super-block).
+// The exponents come from registers, so that a mask-and-or has one constant of 32 bits, as many as an instruction takes.
 struct NibbleMagic { uint32_t lo, hi; };
 __device__ __forceinline__ NibbleMagic nibble_magic() {
   NibbleMagic k;

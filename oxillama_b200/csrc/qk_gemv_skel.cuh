@@ -379,7 +379,7 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
   constexpr int WG = CW / G;  // warps per group; a group owns every G-th chunk
   // The tile producer as a warp of its own (F::SPLIT_PRODUCER) or as a second job of the reducer
   // warp: measured per format (IQ4_XS 14336 x 4096: 11.3 -> 10.95 us with its own warp; Q6_K
-  // 128256 x 4096: 88.8 -> 91.4 us a call, with its former MMA of k = 32).
+  // 128256 x 4096: 88.8 -> 91.4 us a call, with its former MMA of k = 32 and ring of four stages).
   constexpr bool SPLIT = F::SPLIT_PRODUCER;
   constexpr int XW = CW + 1 + (SPLIT ? 1 : 0);  // first warp behind the compute, reducer and producer warps
   constexpr bool PEER = MODE == 1, DUAL = MODE == 2;

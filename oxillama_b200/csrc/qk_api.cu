@@ -547,6 +547,7 @@ extern "C" int qk_moe_ffn_dev(qk_ctx *c, const qk_weights *const *gate, const qk
     QkTcCall gu = {};
     gu.L = &gate[0]->L, gu.n_act = (uint32_t)n_local, gu.counts = cnt, gu.m = (uint32_t)tokens;
     gu.expect = (uint32_t)((slots + n_exp - 1) / n_exp), gu.xcap = gu.ycap = (uint32_t)cap;
+    gu.live = (uint32_t)slots;
     gu.x = x_dev, gu.lists = lists, gu.list_stride = (uint32_t)slots, gu.list_div = (uint32_t)top_k;
     gu.y = g, gu.ldy = inter;
     // gate and up as 2 n groups over n activation groups (groups n .. 2 n - 1 write u, behind g)
@@ -564,7 +565,7 @@ extern "C" int qk_moe_ffn_dev(qk_ctx *c, const qk_weights *const *gate, const qk
     }
     // silu(g) * u is formed where the down projection's activations are converted
     QkTcCall dn = {};
-    dn.L = &down[0]->L, dn.n = dn.n_act = (uint32_t)n_local, dn.counts = cnt, dn.m = (uint32_t)tokens, dn.expect = gu.expect;
+    dn.L = &down[0]->L, dn.n = dn.n_act = (uint32_t)n_local, dn.counts = cnt, dn.m = (uint32_t)tokens, dn.expect = gu.expect, dn.live = gu.live;
     dn.xcap = dn.ycap = (uint32_t)cap, dn.x = g, dn.x2 = u, dn.y = o, dn.ldy = hidden;
     for (size_t e = 0; e < n_local; e++) dn.maps[e] = down[e]->tmap;
     return tc_call(c, c->scratch, dn, s);
@@ -580,9 +581,8 @@ extern "C" int qk_moe_ffn_dev(qk_ctx *c, const qk_weights *const *gate, const qk
     int *ids = (int *)(base + o_ids), *cnt = (int *)(base + o_cnt), *lists = (int *)(base + o_lists);
     int *pos = (int *)(base + o_pos);
     float *wts = (float *)(base + o_wts), *g = (float *)(base + o_g), *o = (float *)(base + o_o);
-    CK(c, qk_launch_moe_route(logits_dev, (uint32_t)tokens, (uint32_t)n_exp, (uint32_t)top_k, ids, wts, s));
-    CK(c, qk_launch_moe_lists(ids, (uint32_t)tokens, (uint32_t)top_k, (uint32_t)expert_begin, (uint32_t)n_local,
-                              cnt, lists, pos, s));
+    CK(c, qk_launch_moe_group_plan(logits_dev, (uint32_t)tokens, (uint32_t)n_exp, (uint32_t)top_k, (uint32_t)expert_begin,
+                                   (uint32_t)n_local, ids, wts, cnt, lists, pos, s));
     if ((st = on_tensor_cores(cnt, lists, g, o))) return st;
     CK(c, qk_launch_moe_combine(o, nullptr, nullptr, ids, pos, wts, (uint32_t)tokens, (uint32_t)top_k, (uint32_t)expert_begin,
                                 (uint32_t)n_local, (uint32_t)cap, (uint32_t)hidden, y_dev, s));

@@ -531,8 +531,28 @@ struct ConvArgs {
   float *scales;
   unsigned *zero;                 // arrival counters of the matmul that follows, cleared here
   const int *counts, *lists;      // grouped: live rows per group; rows to gather (row t of group e = x[lists[e][t] / list_div])
-  uint32_t m, cols, Kp, n_zero, cap, list_stride, list_div;
+  uint32_t m, cols, Kp, n_zero, cap, list_stride, list_div, n_act;
 };
+// Which row a conversion CTA takes, as group * cap + place in the group: without counts the CTA's own number, with them the
+// blockIdx.x-th live one.  (A CTA per reserved row, most of which left at once, held up the live ones, for which silu(g) * u
+// has three places on an SM: 16 experts of 1024 x 2048 by 300 tokens, top 2, 94.6 -> 78.7 us, of it some 4 from
+// qk_moe_group_plan_kernel.)
+__device__ __forceinline__ bool conv_row(const ConvArgs &A, uint32_t &t) {
+  t = blockIdx.x;
+  if (!A.counts) return true;
+  const uint32_t lane = threadIdx.x & 31, c = lane < A.n_act ? min((uint32_t)__ldg(A.counts + lane), A.cap) : 0u;
+  uint32_t end = c;
+#pragma unroll
+  for (int o = 1; o < QK_MAX_GROUPS; o <<= 1) {
+    const uint32_t v = __shfl_up_sync(0xffffffffu, end, o);
+    if (lane >= (uint32_t)o) end += v;
+  }
+  const uint32_t mine = __ballot_sync(0xffffffffu, lane < A.n_act && blockIdx.x < end);
+  if (!mine) return false;
+  const uint32_t e = __ffs(mine) - 1;
+  t = e * A.cap + blockIdx.x - __shfl_sync(0xffffffffu, end - c, e);
+  return true;
+}
 
 __device__ __forceinline__ float silu_mul(float g, float u) {
   const float sg = __fdiv_rn(1.f, __fadd_rn(1.f, expf(-g)));
@@ -595,13 +615,10 @@ __global__ void __launch_bounds__(CT, CT == 256 ? 6 : 1) qk_x16_kernel(const Con
   pdl_wait();
   if (blockIdx.x == 0)
     for (uint32_t i = threadIdx.x; i < A.n_zero; i += CT) A.zero[i] = 0u;
-  const uint32_t t = blockIdx.x;
+  uint32_t t;
+  if (!conv_row(A, t)) return;  // (rows past the live ones: never stored, their values do not matter)
   const float *xr = A.x + (uint64_t)t * A.cols, *ur = A.x2 + (uint64_t)t * A.cols;
-  if (A.counts) {
-    const uint32_t e = t / A.cap, tl = t % A.cap;
-    if (tl >= (uint32_t)A.counts[e]) return;  // rows past the live ones: never stored, their values do not matter
-    if (A.lists) xr = A.x + (uint64_t)(A.lists[(uint64_t)e * A.list_stride + tl] / (int)A.list_div) * A.cols;
-  }
+  if (A.lists) xr = A.x + (uint64_t)(A.lists[(uint64_t)(t / A.cap) * A.list_stride + t % A.cap] / (int)A.list_div) * A.cols;
   const bool vec = (A.cols & 3u) == 0 && (((uintptr_t)xr | (GLU ? (uintptr_t)ur : 0u)) & 15u) == 0;
   const uint32_t nch = A.Kp / 8;
   float v[CCH][8];
@@ -655,8 +672,8 @@ __global__ void __launch_bounds__(CT, CT == 512 ? 3 : 1) qk_glu16_kernel(const C
   pdl_wait();
   if (blockIdx.x == 0)
     for (uint32_t i = threadIdx.x; i < A.n_zero; i += CT) A.zero[i] = 0u;
-  const uint32_t t = blockIdx.x;
-  if (A.counts && t % A.cap >= (uint32_t)A.counts[t / A.cap]) return;  // rows past the live ones
+  uint32_t t;
+  if (!conv_row(A, t)) return;
   const float *xr = A.x + (uint64_t)t * A.cols, *ur = A.x2 + (uint64_t)t * A.cols;
   const bool vec = (A.cols & 3u) == 0 && (((uintptr_t)xr | (uintptr_t)ur) & 15u) == 0;
   float amax = 0.f;
@@ -1367,7 +1384,7 @@ cudaError_t launch_fmt(const QkTcCall &c, unsigned *status, unsigned char *scrat
   ConvArgs C = {};
   C.x = c.x, C.x2 = c.x2, C.out = x16, C.scales = scales, C.zero = cnt, C.n_zero = (uint32_t)sm_count * 2;
   C.counts = c.counts, C.lists = c.lists, C.m = c.m, C.cols = L.cols, C.Kp = Kp, C.cap = c.xcap;
-  C.list_stride = c.list_stride, C.list_div = c.list_div ? c.list_div : 1u;
+  C.list_stride = c.list_stride, C.list_div = c.list_div ? c.list_div : 1u, C.n_act = c.n_act;
   const bool narrow = (c.counts || (c.n == 1 && c.m >= 64)) && Kp <= 4096;
   // Single CTAs beside the conversion (72 registers).  Q6_K only where the conversion has more rows than a tile: its
   // expansion wants the 80 (us, 80 / 72 registers: 4096 x 4096 by 80 16.5 / 14.4, by 160 17.1 / 15.4; 14336 x 4096 by
@@ -1375,7 +1392,8 @@ cudaError_t launch_fmt(const QkTcCall &c, unsigned *status, unsigned char *scrat
   const bool beside = narrow && !c.counts && (T != QK_T_Q6_K || c.m > 64);
   cudaLaunchAttribute at = pdl_attr();
   cudaLaunchConfig_t c0 = {};
-  c0.gridDim = dim3(c.counts || c.n_act > 1 ? c.n_act * c.xcap : c.m), c0.blockDim = dim3(narrow ? 256 : 512), c0.stream = s, c0.attrs = &at, c0.numAttrs = 1;
+  const uint32_t all_rows = c.counts || c.n_act > 1 ? c.n_act * c.xcap : c.m;
+  c0.gridDim = dim3(c.counts && c.live < all_rows ? c.live : all_rows), c0.blockDim = dim3(narrow ? 256 : 512), c0.stream = s, c0.attrs = &at, c0.numAttrs = 1;
   cudaError_t e;
   if (c.x2 && !c.lists && Kp * 4 <= GLU_SMEM) {
     static QkPerDevice attr_set;

@@ -162,6 +162,7 @@ struct QkTcCall {
   // m rows per group, or (counts != null, on the device) counts[e] of at most m; `expect`: the rows of an average group
   const int *counts;
   uint32_t m, expect, xcap, ycap;
+  uint32_t live;                     // with counts: most rows that all groups have together
   float *y;                          // output row i of matrix e: y + (e * ycap + i) * ldy
   uint64_t ldy;
 };
@@ -179,6 +180,11 @@ cudaError_t qk_launch_gemm_tc(const QkTcCall &c, unsigned *status, unsigned char
 // Mixture-of-experts glue (routing, token lists, gather, silu * up, weighted scatter-add).
 cudaError_t qk_launch_moe_route(const float *logits, uint32_t tokens, uint32_t n_exp, uint32_t top_k,
                                 int *ids, float *wts, cudaStream_t s);
+// Both for a call whose experts go together, in one launch where the pairs are few enough.
+#define QK_MOE_PLAN_SLOTS 16384u
+cudaError_t qk_launch_moe_group_plan(const float *logits, uint32_t tokens, uint32_t n_exp, uint32_t top_k,
+                                     uint32_t expert_begin, uint32_t n_local, int *ids, float *wts, int *counts,
+                                     int *lists, int *pos, cudaStream_t s);
 cudaError_t qk_launch_moe_lists(const int *ids, uint32_t tokens, uint32_t top_k, uint32_t expert_begin,
                                 uint32_t n_local, int *counts, int *lists, int *pos, cudaStream_t s);
 // y[token] = sum in slot order of wts * output row; the rows of expert e lie at o + e * cap (position

@@ -75,6 +75,47 @@ __device__ __forceinline__ void route_token_warp(const float *__restrict__ logit
   for (uint32_t k = ek + lane; k < top_k; k += 32) ids[(uint64_t)t * top_k + k] = -1, wts[(uint64_t)t * top_k + k] = 0.f;
 }
 
+// The same by one thread that holds the logits and probabilities of up to E experts in registers: the same sums in
+// the same order, without the loads and the second exponentials of route_token.  Calls store(k, id, weight).
+template <int E, class Store>
+__device__ __forceinline__ void route_token_regs(const float *__restrict__ logits, uint32_t t, uint32_t n_exp, uint32_t top_k, Store &&store) {
+  const float *l = logits + (uint64_t)t * n_exp;
+  const uint32_t ek = top_k < n_exp ? top_k : n_exp;
+  float p[E], mx = -INFINITY, es = 0.f;
+#pragma unroll
+  for (int i = 0; i < E; i++) p[i] = i < (int)n_exp ? __ldg(l + i) : -INFINITY;
+#pragma unroll
+  for (int i = 0; i < E; i++) mx = fmaxf(mx, p[i]);
+#pragma unroll
+  for (int i = 0; i < E; i++) {
+    p[i] = expf(__fsub_rn(p[i], mx));
+    if (i < (int)n_exp) es = __fadd_rn(es, p[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < E; i++) p[i] = es > 0.f ? __fdiv_rn(p[i], es) : __fdiv_rn(1.f, (float)n_exp);
+  // the largest not yet taken, ties to the lower expert (every p compares: where a logit is NaN or infinite, es is NaN and
+  // all are 1 / n_exp)
+  uint32_t taken = n_exp < 32 ? ~0u << n_exp : 0u;
+  auto next = [&](float &best) {
+    uint32_t bi = 0;
+    best = -1.f;
+#pragma unroll
+    for (int i = 0; i < E; i++)
+      if (!(taken >> i & 1u) && p[i] > best) best = p[i], bi = (uint32_t)i;
+    taken |= 1u << bi;
+    return bi;
+  };
+  const uint32_t all = taken;
+  float ssum = 0.f, best;
+  for (uint32_t k = 0; k < ek; k++) next(best), ssum = __fadd_rn(ssum, best);
+  taken = all;
+  for (uint32_t k = 0; k < ek; k++) {
+    const uint32_t id = next(best);
+    store(k, (int)id, ssum > 1e-9f ? __fdiv_rn(best, ssum) : __fdiv_rn(1.f, (float)ek));
+  }
+  for (uint32_t k = ek; k < top_k; k++) store(k, -1, 0.f);
+}
+
 // Everything the projections of a handful of tokens need to know, by one block of 256 threads: ids and
 // weights, the lists of the experts with many rows, the job list of the others.
 struct PlanArgs {

@@ -529,3 +529,36 @@ def test_decode_ring(t, m, rows, cols):
     # (three rows of Q6_K, and of Q8_0 two of 12288 columns or three of 8448, go to the tensor cores: fp16 operands)
     most = 2 if t == S.Q6_K else {12288: 1, 8448: 2}.get(cols, 3) if t == S.Q8_0 else 3
     assert_product(y, x, O.dequant_matrix(t, w, rows, cols), half=m > most)
+
+
+# Routing and lists of a grouped call: one round of 1024 (token, slot) pairs and several, up to eight experts and up to 32, a
+# shard of them, the last size that one block plans and the first that it does not.  Equal logits go to the lower experts, and
+# so do those of a token with a NaN among them.  Routing as the stand-alone entry point gives it (tested against the
+# oracle); the bound is test_moe_short_rows'.
+@pytest.mark.parametrize("n,top_k,tokens,begin,local", [(8, 2, 512, 0, 8), (8, 3, 683, 0, 8), (9, 2, 40, 3, 5), (32, 3, 400, 8, 16),
+                                                        (4, 4, 4096, 0, 4), (4, 4, 4097, 0, 4), (3, 1, 18, 0, 1)])
+def test_moe_group_plan(n, top_k, tokens, begin, local):
+    import torch
+    from oxillama_b200 import moe
+    from oxillama_b200.device import check_device_status
+    hidden, inter = 256, 256
+    shapes = [(inter, hidden), (inter, hidden), (hidden, inter)]
+    w = [[S.gen_weight(S.Q8_0, r, c, seed=131, stream=3 * e + k, d_range=(1e-3, 3e-3)) for e in range(local)] for k, (r, c) in enumerate(shapes)]
+    x, logits = S.gen_acts(tokens, hidden, seed=132) * np.float32(0.25), S.gen_acts(tokens, n, seed=133)
+    logits[7] = 0.5
+    logits[11] = np.nan
+    logits[tokens - 1, n - 1] = np.nan
+    ids, wts = (v.cpu().numpy() for v in moe.route(torch.from_numpy(logits).cuda(), top_k))
+    assert all(np.array_equal(ids[t], np.arange(top_k)) for t in (7, 11, tokens - 1))
+    ref = np.zeros((tokens, hidden))
+    for e in range(local):
+        g, u, d = (O.dequant_matrix(S.Q8_0, ws[e], r, c).astype(np.float64) for ws, (r, c) in zip(w, shapes))
+        at, slot = np.nonzero(ids == begin + e)
+        hg = x[at] @ g.T
+        np.add.at(ref, at, wts[at, slot][:, None] * ((hg / (1 + np.exp(-hg)) * (x[at] @ u.T)) @ d.T))
+    ex = moe.MoeExperts(S.Q8_0, *w, hidden, inter, n, expert_begin=begin)
+    y = torch.full((tokens, hidden), float("nan"), device="cuda")
+    ex.forward(torch.from_numpy(logits).cuda(), torch.from_numpy(x).cuda(), y, top_k)
+    check_device_status()
+    ex.free()
+    assert np.abs(y.cpu().numpy() - ref).max() <= 3e-3 * np.abs(ref).max()

@@ -96,8 +96,8 @@ struct DecQ80 {
   static constexpr uint32_t COLB = 8 * 272, XSB = 8;
   static constexpr int MAX_M = 4;
   static constexpr bool HAS_DUAL = true, HAS_PEER = true;
-  static constexpr bool SPLIT_PRODUCER = true;  // the tile producer as a warp of its own (measured per format)
   static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
+  static constexpr uint32_t PAIR_COLS = 14336;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
   // digit order inside a 32-column block: the lane's 8 bytes are columns 4 tig .. + 3 and
   // 16 + 4 tig .. + 3, the two 4-byte pieces of its A fragment (bytes 4 tig of both 16-byte granules)
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
@@ -168,8 +168,8 @@ struct DecQ40 {
   static constexpr uint32_t COLB = 8 * 144, XSB = 8;
   static constexpr int MAX_M = 4;
   static constexpr bool HAS_DUAL = true, HAS_PEER = true;
-  static constexpr bool SPLIT_PRODUCER = true;  // the tile producer as a warp of its own (measured per format)
   static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
+  static constexpr uint32_t PAIR_COLS = 0;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
   // The lane's word (bytes 4 tig .. + 3 of the block) holds elements 8 tig .. + 7: low
   // nibbles the even ones, high nibbles the odd ones.  Digits go evens first, then odds,
   // inside every group of 8 columns.
@@ -250,8 +250,8 @@ struct DecIQ4XS {
   static constexpr uint32_t COLB = 1088, XSB = 8;
   static constexpr int MAX_M = 4;
   static constexpr bool HAS_DUAL = true, HAS_PEER = true;
-  static constexpr bool SPLIT_PRODUCER = true;  // the tile producer as a warp of its own (measured per format)
   static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
+  static constexpr uint32_t PAIR_COLS = 8704;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
                                                       uint32_t w1, uint32_t w2) {
     store_digits_natural(row_img, PS, e0, w0, w1, w2);
@@ -346,8 +346,8 @@ struct DecIQ4XS {
 struct DecQ6K {
   static constexpr uint32_t COLB = 1680, XSB = 16;
   static constexpr bool HAS_DUAL = false, HAS_PEER = true;
-  static constexpr bool SPLIT_PRODUCER = false;  // the tile producer as a warp of its own (measured per format)
   static constexpr bool ANY_DEPTH = true;  // ring depths that are no multiple of the groups (ring_is_deep)
+  static constexpr uint32_t PAIR_COLS = 11008;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
   static constexpr int MAX_M = 2;  // three rows and up spill heavily (twelve weight words and sixteen fragments per column)
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
                                                       uint32_t w1, uint32_t w2) {

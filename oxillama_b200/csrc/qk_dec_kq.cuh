@@ -26,8 +26,8 @@ struct DecQ5K {
   static constexpr uint32_t COLB = 1408, XSB = 8;
   static constexpr int MAX_M = 4;
   static constexpr bool HAS_DUAL = true, HAS_PEER = false;
-  static constexpr bool SPLIT_PRODUCER = true;
   static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
+  static constexpr uint32_t PAIR_COLS = 8704;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
                                                       uint32_t w1, uint32_t w2) {
     store_digits_natural(row_img, PS, e0, w0, w1, w2);
@@ -165,8 +165,8 @@ struct DecQ3K {
   static constexpr uint32_t COLB = 880, XSB = 16;
   static constexpr int MAX_M = 2;  // three rows and up spill, as with Q6_K
   static constexpr bool HAS_DUAL = true, HAS_PEER = false;
-  static constexpr bool SPLIT_PRODUCER = true;
   static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
+  static constexpr uint32_t PAIR_COLS = 11008;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
                                                       uint32_t w1, uint32_t w2) {
     store_digits_natural(row_img, PS, e0, w0, w1, w2);
@@ -244,8 +244,8 @@ struct DecQ2K {
   static constexpr uint32_t COLB = 672, XSB = 16;
   static constexpr int MAX_M = 2;  // as Q3_K
   static constexpr bool HAS_DUAL = true, HAS_PEER = false;
-  static constexpr bool SPLIT_PRODUCER = true;
   static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
+  static constexpr uint32_t PAIR_COLS = 0;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
                                                       uint32_t w1, uint32_t w2) {
     store_digits_natural(row_img, PS, e0, w0, w1, w2);

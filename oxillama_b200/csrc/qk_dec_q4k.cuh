@@ -29,8 +29,8 @@ struct DecQ4K {
   static constexpr uint32_t XSB = 8;      // (sx, Sx) per 32-column block
   static constexpr int MAX_M = 4;
   static constexpr bool HAS_DUAL = true, HAS_PEER = true;
-  static constexpr bool SPLIT_PRODUCER = true;  // the tile producer as a warp of its own (measured per format)
   static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
+  static constexpr uint32_t PAIR_COLS = 0;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
 
   // digit planes in natural column order
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,

@@ -66,11 +66,13 @@ constexpr int MAX_CW = 16;                      // compute warps (+ one or two p
 constexpr uint32_t NBT = QK_TILE_ELEMS / 256;   // super-blocks per full k-tile (16)
 constexpr int MAX_STAGE = 12;
 constexpr int MAX_SLOT = MAX_STAGE + 1;
+constexpr uint32_t PAIR_CHUNKS = 32;            // most chunks of a pair of CTAs
 
 struct SmemMma {
   uint32_t full, redfull, xbar;  // mbarriers (8 B each)
   uint32_t prog;                 // chunks the reducer warp has read so far (one word, polled by the producer warp)
   uint32_t issued;               // DEEP: tiles issued so far (one word, polled by the compute warps)
+  uint32_t pbar, pair;           // PAIR: per chunk, the mbarrier and the 8 x M sums that the other CTA sends
   uint32_t red, ximg, stage;
   uint32_t PS;         // digit plane stride, bytes
   uint32_t xs_off;     // offset of the (sx, Sx) table inside the x image
@@ -211,6 +213,18 @@ __device__ __forceinline__ bool load_quad_slots(const unsigned long long *row, u
   return ok;
 }
 
+// A float into the same place of the other CTA's shared memory, counted by the mbarrier there.
+__device__ __forceinline__ void st_async_other(uint32_t addr, uint32_t bar, uint32_t rank, float v) {
+  asm volatile(
+      "{\n\t.reg .b32 a, b;\n\tmapa.shared::cluster.u32 a, %0, %2;\n\tmapa.shared::cluster.u32 b, %1, %2;\n\t"
+      "st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [a], %3, [b];\n\t}" ::"r"(addr),
+      "r"(bar), "r"(rank), "r"(__float_as_uint(v))
+      : "memory");
+}
+__device__ __forceinline__ float lds32f(uint32_t addr) { return __uint_as_float(lds32(addr)); }
+// Blocks of a row in its first half: whole spans of 256 columns, the longer half where they are odd.
+__host__ __device__ __forceinline__ uint32_t half_blocks(const QkLayout &L) { return (L.nb * L.bs / 256u + 1u) / 2u * (256u / L.bs); }
+
 // ---------------------------------------------------------------- x image
 // [M][3 digit planes of PS bytes, columns in the format's order F::store_digits][M][Kp/32] scale entries
 // of F::XSB bytes: (sx, sum over the 32 columns) and, for formats with 16-column scales, the two half sums
@@ -259,8 +273,9 @@ __global__ void __launch_bounds__(256)
 // The same split as qk_xsplit_kernel, done by the compute warps straight into the
 // CTA's shared-memory x image (used when x is small enough that every CTA
 // redoing it is cheaper than a second kernel and a copy).
-template <class F, int M, int CW, bool PEER>
-__device__ void xsplit_in_cta(const float *__restrict__ x, uint32_t cols, uint32_t Kp,
+// x: M rows of `cols` columns, ldx apart (PAIR: a CTA's half of the columns).
+template <class F, int M, int CW, bool PEER, bool PAIR>
+__device__ void xsplit_in_cta(const float *__restrict__ x, uint32_t cols, uint32_t ldx, uint32_t Kp,
                               unsigned char *img, uint32_t PS, uint32_t xs_off, bool tell_producer,
                               const QkPeers &peers, unsigned *status) {
   constexpr int CT = CW * 32;  // compute threads
@@ -269,11 +284,11 @@ __device__ void xsplit_in_cta(const float *__restrict__ x, uint32_t cols, uint32
   // a different 32-column block (whole blocks, so the 8 threads of a block stay together)
   // to spread the requests over the L2 slices, and loads 16 bytes at a time when it can.
   const uint32_t rot = (blockIdx.x * 40u) % total;  // a multiple of 8 quads
-  const bool vec = (cols & 3u) == 0 && ((uintptr_t)x & 15u) == 0;
+  const bool vec = (ldx & 3u) == 0 && ((uintptr_t)x & 15u) == 0;
   const bool from_slots = PEER && peers.wait_slots != nullptr;
   const unsigned want = from_slots ? *peers.wait_epoch : 0u;
   bool arrived = true;  // false once a slot has failed to arrive in time: this thread waits no more
-  constexpr int U = (M * 4096 / 4 + CT - 1) / CT < 4 ? (M * 4096 / 4 + CT - 1) / CT : 4;  // quads in flight per thread
+  constexpr int U = !PAIR && (M * 4096 / 4 + CT - 1) / CT < 4 ? (M * 4096 / 4 + CT - 1) / CT : 4;  // quads in flight per thread
   for (uint32_t base = 0; base < total; base += CT * U) {
     float v[U][4];
     uint32_t qidx[U];
@@ -292,12 +307,12 @@ __device__ void xsplit_in_cta(const float *__restrict__ x, uint32_t cols, uint32
           atomicOr(status, QK_DEV_TIMEOUT);
         }
       } else if (it0 < total && vec && e0 + 4 <= cols) {
-        const float4 q = __ldg(reinterpret_cast<const float4 *>(x + (uint64_t)m * cols + e0));
+        const float4 q = __ldg(reinterpret_cast<const float4 *>(x + (uint64_t)m * ldx + e0));
         v[j][0] = q.x, v[j][1] = q.y, v[j][2] = q.z, v[j][3] = q.w;
       } else {
 #pragma unroll
         for (int i = 0; i < 4; i++)
-          v[j][i] = (it0 < total && e0 + i < cols) ? __ldg(x + (uint64_t)m * cols + e0 + i) : 0.f;
+          v[j][i] = (it0 < total && e0 + i < cols) ? __ldg(x + (uint64_t)m * ldx + e0 + i) : 0.f;
       }
     }
     // This thread's first activation loads are on their way: the producer may send the rest
@@ -368,29 +383,31 @@ __device__ __forceinline__ void unpack_slots(const QkPeers &peers, unsigned uwan
 // 8 i ..), both see the same split activations, and the reducer writes
 // silu(gate) * up (crates/oxillama-arch/src/common/swiglu.rs:15-21) where a plain matvec
 // writes its dot products.
+// 3 = one matrix, each chunk by the two CTAs of a cluster, either half of K (see pair_pays); the reducer of the CTA that
+// does not own the chunk (they take turns) sends its sums into the other's shared memory.
 // DEEP: the ring has every stage that fits, not a multiple of the groups' (see make_plan_mma).
 template <class F, int M, bool INCTA, int CW, int G, int MODE, bool DEEP>
-__global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE == 1 ? 1 : 0)) * 32, 1)
+__global__ void __launch_bounds__((CW + 2 + (MODE == 1 ? 1 : 0)) * 32, 1)
     qk_gemv_imma_kernel(QkLayout L, const uint8_t *__restrict__ W, const uint8_t *__restrict__ W2,
                            const float *__restrict__ x,
                            const unsigned char *__restrict__ ximg_g, float *__restrict__ y,
                            uint64_t ldy, unsigned *status, int nstage, int nslot,
                            uint32_t stage_bytes, SmemMma S, uint32_t Kp, QkPeers peers, int npre) {
   constexpr int WG = CW / G;  // warps per group; a group owns every G-th chunk
-  // The tile producer as a warp of its own (F::SPLIT_PRODUCER) or as a second job of the reducer
-  // warp: measured per format (IQ4_XS 14336 x 4096: 11.3 -> 10.95 us with its own warp; Q6_K
-  // 128256 x 4096: 88.8 -> 91.4 us a call, with its former MMA of k = 32 and ring of four stages).
-  constexpr bool SPLIT = F::SPLIT_PRODUCER;
-  constexpr int XW = CW + 1 + (SPLIT ? 1 : 0);  // first warp behind the compute, reducer and producer warps
-  constexpr bool PEER = MODE == 1, DUAL = MODE == 2;
+  constexpr int XW = CW + 2;  // first warp behind the compute, reducer and producer warps
+  constexpr bool PEER = MODE == 1, DUAL = MODE == 2, PAIR = MODE == 3;
   extern __shared__ __align__(128) unsigned char smem[];
   const uint32_t sbase = smem_u32(smem);
   const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
-  // chunks of this CTA, in the order it takes them; with two matrices every 8-row group counts twice
-  const uint32_t my_chunks =
-      (blockIdx.x < L.chunks ? (L.chunks - blockIdx.x + gridDim.x - 1) / gridDim.x : 0) * (DUAL ? 2u : 1u);
-  const uint32_t my_items = my_chunks * L.ktiles;
+  // chunks of this CTA (pair), in the order it takes them; with two matrices every 8-row group counts twice
+  const uint32_t rank = PAIR ? blockIdx.x & 1u : 0u, first = PAIR ? blockIdx.x >> 1 : blockIdx.x, step = PAIR ? gridDim.x >> 1 : gridDim.x;
+  const uint32_t my_chunks = (first < L.chunks ? (L.chunks - first + step - 1) / step : 0) * (DUAL ? 2u : 1u);
+  // its blocks of a row: from block b0 on, nb of them
+  const uint32_t nb0 = PAIR ? half_blocks(L) : 0u, b0 = rank ? nb0 : 0u, nb = !PAIR ? L.nb : rank ? L.nb - nb0 : nb0;
+  const uint32_t ktiles = PAIR ? (nb + L.nbt - 1) / L.nbt : L.ktiles;
+  auto tile_blocks = [&](uint32_t kt) { return min(nb - kt * L.nbt, L.nbt); };
+  const uint32_t my_items = my_chunks * ktiles;
 
   QK_STAMP(warp == 0, 0);
   pdl_launch_dependents();
@@ -402,19 +419,27 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  if (PAIR && warp == 1 && lane < my_chunks && (lane & 1u) == rank) {  // (PAIR_CHUNKS = 32: a lane each)
+    mbar_init(sbase + S.pbar + lane * 8, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    mbar_expect_tx(sbase + S.pbar + lane * 8, 8 * M * 4);
+  }
   __syncthreads();
+  if (PAIR) asm volatile("barrier.cluster.arrive.release;" ::: "memory");  // (the reducers wait for it, and alone come to the second one)
 
   // tile issue state and helpers of whichever warp streams the tiles
   uint32_t pc = 0, pkt = 0, pst = 0;  // chunk ordinal, k-tile and stage of the next item
   const uint64_t policy = stream_policy();
   uint32_t lead = 0;                  // the lane that issues, in the warp that does
   auto issue = [&]() {                // the whole warp
-    const uint32_t chunk = blockIdx.x + (DUAL ? pc >> 1 : pc) * gridDim.x;
+    const uint32_t chunk = first + (DUAL ? pc >> 1 : pc) * step;
     const uint8_t *Wc = (DUAL && (pc & 1u)) ? W2 : W;
-    const uint32_t bytes = QK_TILE_ROWS * qk_tile_nb(L, pkt) * L.bb;
+    const uint32_t bytes = QK_TILE_ROWS * tile_blocks(pkt) * L.bb;
     const uint32_t bar = sbase + S.full + pst * 8;
-    stream_tile(sbase + S.stage + pst * stage_bytes, Wc + qk_tile_offset(L, chunk, pkt), bytes, bar, policy, lead);
-    if (++pkt == L.ktiles) pkt = 0, pc++;
+    // (a chunk is its blocks one after the other, eight rows each)
+    const uint64_t at = qk_tile_offset(L, chunk, pkt) + (PAIR ? QK_TILE_ROWS * b0 * L.bb : 0u);
+    stream_tile(sbase + S.stage + pst * stage_bytes, Wc + at, bytes, bar, policy, lead);
+    if (++pkt == ktiles) pkt = 0, pc++;
     if (++pst == (uint32_t)nstage) pst = 0;
   };
   uint32_t item = 0;  // items issued so far; kept in step by every lane
@@ -426,7 +451,7 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
       if (DEEP && lead) tell_issued(sbase + S.issued, item);
     }
   };
-  if (SPLIT && warp == CW + 1) {
+  if (warp == CW + 1) {
     lead = elect_lead();
     // ================= producer warp =================
     // It streams the tiles: the first ring fill, then the k-tiles of chunk c + (ring depth)
@@ -434,7 +459,8 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
     // then).  A warp of its own, because a copy instruction does not return until the copy
     // unit has room for it -- a third of a microsecond and more under a saturated stream --
     // and behind the reducer's sums the refills went out up to 1.7 us late, leaving the
-    // stream idle between the first ring fill and the refills.  The producer stays at most
+    // stream idle between the first ring fill and the refills (IQ4_XS 14336 x 4096: 11.3 -> 10.95 us;
+    // Q6_K 4096 x 4096 5.13 -> 4.99, 14336 x 4096 10.21 -> 9.95).  The producer stays at most
     // one chunk ahead of the reducer (S.prog), which is what makes the ring of `nslot`
     // partial buffers safe: chunk c + nslot cannot be computed, let alone handed over,
     // before the reducer has read chunk c.
@@ -476,27 +502,18 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
         if (lane == 0) atomicOr(status, QK_DEV_TIMEOUT);
         break;
       }
-      issue_upto(item + L.ktiles);
+      issue_upto(item + ktiles);
       if (++slot == (uint32_t)nslot) slot = 0, sph ^= 1;
     }
     return;
   }
 
   if (warp == CW) {
-    // ================= reducer warp (and, without a producer warp, the tile producer) =================
+    // ================= reducer warp =================
     // When a chunk's partials are complete the warp sums them and writes the 8 x M outputs
-    // (or stores them into every rank's slots), then says so in S.prog.  Where it also streams
-    // the tiles (!SPLIT) it refills the chunk's stages first: gating the refills on the
-    // reduction bounds how far the compute warps can run ahead, which is what makes the ring
-    // of `nslot` partial buffers safe without a second handshake.
-    if (!SPLIT) lead = elect_lead();
-    if (!SPLIT) issue_upto((uint32_t)npre);  // weights are immutable: their prefetch need not wait for the previous kernel
+    // (or stores them into every rank's slots), then says so in S.prog.
     pdl_wait();  // the x image and y belong to the previous kernel until it has finished
     QK_STAMP(true, 120);
-    if (!SPLIT && !INCTA && lane == 0) {
-      mbar_expect_tx(sbase + S.xbar, S.ximg_bytes);
-      bulk_g2s(sbase + S.ximg, ximg_g, S.ximg_bytes, sbase + S.xbar);
-    }
     // Sharded output: this call's tag is the object's call count + 1.  Lane 0 reads the
     // count, then counts this CTA in (the add carries a dependency on the value read, so it
     // cannot overtake the read); the CTA that is counted in last knows that every CTA of the
@@ -514,11 +531,6 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
         *reinterpret_cast<volatile unsigned *>(peers.epoch) = e_count + 1u;
       }
     }
-    if (!SPLIT && npre < nstage) {
-      // the rest of the first ring fill, once the activation loads are out (see the producer warp)
-      if (INCTA) asm volatile("bar.sync 2, %0;" ::"n"((CW + 1) * 32) : "memory");
-      issue_upto((uint32_t)nstage);
-    }
     const unsigned tag = (PEER && peers.n) ? __shfl_sync(0xffffffffu, e_count, 0) + 1u : 0u;
     // this lane's two destination ranks (lane / 8 and lane / 8 + 4), held in registers: an
     // indexed read of the kernel parameters per chunk costs a constant-cache miss each time
@@ -535,16 +547,16 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
     // plain buffer -- by a warp of its own when the launch has one (see below), else here,
     // where this warp has nothing else to do until the first chunk is reduced.
     if (PEER && peers.unpack_n && blockDim.x == XW * 32) unpack_slots(peers, uwant, lane, status);
+    if (PAIR) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");  // the other CTA runs, its barriers are initialised
     uint32_t slot = 0, sph = 0;
+    bool dead = false;   // (a lane's) a wait for the other CTA's sums ran out
     float gate_v = 0.f;  // two matrices: the gate chunk's sum, kept until the up chunk's arrives
     for (uint32_t c = 0; c < my_chunks; c++) {
       if (!mbar_wait_bounded(sbase + S.redfull + slot * 8, sph)) {
         if (lane == 0) atomicOr(status, QK_DEV_TIMEOUT);
+        dead = true;
         break;
       }
-      // (!SPLIT) every warp of the owning group released the chunk's stages before it posted its
-      // partials: refill them first, the sums and stores below follow the copies out
-      if (!SPLIT) issue_upto(item + L.ktiles);
       const float *red = reinterpret_cast<const float *>(smem + S.red) + slot * (WG * M * 8);
       float v = 0.f;
       if (PEER && M == 1 && peers.n) {
@@ -563,8 +575,17 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
         const uint32_t m = lane >> 3, r = lane & 7u;
 #pragma unroll
         for (int wv = 0; wv < WG; wv++) v += red[(wv * M + m) * 8 + r];
-        const uint32_t row = (blockIdx.x + (DUAL ? c >> 1 : c) * gridDim.x) * 8 + r;
-        if (DUAL) {
+        const uint32_t row = (first + (DUAL ? c >> 1 : c) * step) * 8 + r;
+        if (PAIR) {
+          const uint32_t at = sbase + S.pair + (c * 8 * M + lane) * 4, bar = sbase + S.pbar + c * 8;
+          if ((c & 1u) != rank) {
+            st_async_other(at, bar, rank ^ 1u, v);
+          } else if (!mbar_wait_bounded(bar, 0)) {
+            dead = true;
+          } else if (row < L.rows) {
+            y[(uint64_t)m * ldy + row] = v + lds32f(at);
+          }
+        } else if (DUAL) {
           if ((c & 1u) == 0) {
             gate_v = v;
           } else if (row < L.rows) {
@@ -589,11 +610,17 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
           }
         }
       }
+      if (PAIR && __any_sync(0xffffffffu, dead)) {
+        if (lane == 0) atomicOr(status, QK_DEV_TIMEOUT);
+        break;
+      }
       __syncwarp();
-      if (SPLIT && lane == 0) *reinterpret_cast<volatile uint32_t *>(smem + S.prog) = c + 1u;  // read: its slot may be written again
+      if (lane == 0) *reinterpret_cast<volatile uint32_t *>(smem + S.prog) = c + 1u;  // read: its slot may be written again
       QK_STAMP(c < 30, 64 + c);
       if (++slot == (uint32_t)nslot) slot = 0, sph ^= 1;
     }
+    // No CTA ends while the other may still send into its memory: the reducers meet (threads that have ended do not count).
+    if (PAIR) asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
     return;
   }
 
@@ -620,7 +647,9 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
   QK_STAMP(warp == 0, 121);
   bool dead = false;
   if (INCTA) {
-    xsplit_in_cta<F, M, CW, PEER>(x, L.cols, Kp, smem + S.ximg, S.PS, S.xs_off, npre < nstage, peers, status);
+    const uint32_t c0 = b0 * L.bs;  // (PAIR: the second half begins inside the row)
+    xsplit_in_cta<F, M, CW, PEER, PAIR>(x + c0, PAIR && !rank ? min(nb0 * L.bs, L.cols) : L.cols - c0, L.cols, Kp, smem + S.ximg, S.PS, S.xs_off,
+                                        npre < nstage, peers, status);
     QK_STAMP(warp == 0, 123);
     asm volatile("bar.sync 1, %0;" ::"n"(CW * 32) : "memory");  // compute warps only
   } else if (!mbar_wait_bounded(sbase + S.xbar, 0)) {
@@ -638,15 +667,15 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
     st += n;
     while (st >= (uint32_t)nstage) st -= nstage, fph ^= 1;
   };
-  advance_stage(group * L.ktiles);
+  advance_stage(group * ktiles);
   slot = group % nslot;
   uint32_t tstamp = 0;
   for (uint32_t c = group; c < my_chunks && !dead; c += G) {
-    for (uint32_t kt = 0; kt < L.ktiles; kt++) {
-      const uint32_t nbt = qk_tile_nb(L, kt) * L.bs / 256u;  // 256-column spans in this tile
+    for (uint32_t kt = 0; kt < ktiles; kt++) {
+      const uint32_t nbt = tile_blocks(kt) * L.bs / 256u;  // 256-column spans in this tile
       const uint32_t tile = sbase + S.stage + st * stage_bytes;
       // (in the ring's first round there is no tile before)
-      const uint32_t it = c * L.ktiles + kt;
+      const uint32_t it = c * ktiles + kt;
       if ((DEEP && it >= (uint32_t)nstage && !wait_issued(sbase + S.issued, it, seen)) || !mbar_wait_bounded(sbase + S.full + st * 8, fph)) {
         dead = true;
         break;
@@ -695,7 +724,7 @@ __global__ void __launch_bounds__((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + (MODE 
     if (lane == 0) mbar_arrive(sbase + S.redfull + slot * 8);
     slot += G;
     while (slot >= (uint32_t)nslot) slot -= nslot;
-    advance_stage((G - 1) * L.ktiles);
+    advance_stage((G - 1) * ktiles);
   }
   if (dead) atomicOr(status, QK_DEV_TIMEOUT);  // a bounded wait ran out: results are invalid
   QK_STAMP(warp == 0, 100);
@@ -708,11 +737,18 @@ struct PlanMma {
   int deep;  // stages that fit
 };
 
-// xsb: bytes per 32-column block in the activation scale table (F::XSB).
-inline bool make_plan_mma(const QkLayout &L, uint32_t m, PlanMma *P, uint32_t xsb) {
-  if (L.nb == 0 || L.chunks == 0) return false;  // nothing to stream: the callers handle empty shapes
+// xsb: bytes per 32-column block in the activation scale table (F::XSB).  pair: for CTAs that take half of K each.
+inline bool make_plan_mma(const QkLayout &full, uint32_t m, PlanMma *P, uint32_t xsb, bool pair = false) {
+  if (full.nb == 0 || full.chunks == 0) return false;  // nothing to stream: the callers handle empty shapes
+  if (full.nb * full.bs % 256u) return false;          // the kernels walk K in spans of 256 columns
+  QkLayout L = full;
+  if (pair) {
+    L.nb = half_blocks(full);
+    L.ktiles = (L.nb + L.nbt - 1) / L.nbt;
+    // (both halves in as many tiles: the ring's depth is a multiple of theirs)
+    if (L.nb == full.nb || (full.nb - L.nb + L.nbt - 1) / L.nbt != L.ktiles) return false;
+  }
   uint32_t Kp = L.nb * L.bs;
-  if (Kp % 256u) return false;  // the kernels walk K in spans of 256 columns
   uint32_t nbt_max = L.nb < L.nbt ? L.nb : L.nbt;
   uint32_t stage_bytes = QK_TILE_ROWS * nbt_max * L.bb;
   stage_bytes = (stage_bytes + 127u) & ~127u;
@@ -723,6 +759,8 @@ inline bool make_plan_mma(const QkLayout &L, uint32_t m, PlanMma *P, uint32_t xs
   S.xbar = off, off += 8;
   S.prog = off, off += 4;
   S.issued = off, off += 4;
+  S.pbar = S.pair = off;
+  if (pair) off += PAIR_CHUNKS * 8, S.pair = off, off += PAIR_CHUNKS * 8 * m * 4;
   off = (off + 127u) & ~127u;
   S.red = off, off += MAX_SLOT * MAX_CW * m * 8 * 4;
   off = (off + 127u) & ~127u;
@@ -770,9 +808,10 @@ inline bool make_plan_mma(const QkLayout &L, uint32_t m, PlanMma *P, uint32_t xs
 // 1024 (one) 3.4 -> 3.55: the further stages stay empty and the count costs.  Q4_K, eight or eleven, 14336 rows
 // 7.5 -> 8.2.
 template <class F>
-inline bool ring_is_deep(const QkLayout &L, const PlanMma &P, int sm_count, bool dual) {
-  const uint32_t grid = L.chunks < (uint32_t)sm_count ? L.chunks : (uint32_t)sm_count;
-  return F::ANY_DEPTH && P.deep > P.nstage && (L.chunks + grid - 1) / grid * L.ktiles * (dual ? 2u : 1u) > (uint32_t)P.nstage;
+inline bool ring_is_deep(const QkLayout &L, const PlanMma &P, int sm_count, bool dual, bool pair = false) {
+  const uint32_t most = (uint32_t)sm_count / (pair ? 2u : 1u), grid = L.chunks < most ? L.chunks : most;
+  const uint32_t ktiles = pair ? (half_blocks(L) + L.nbt - 1) / L.nbt : L.ktiles;
+  return F::ANY_DEPTH && P.deep > P.nstage && (L.chunks + grid - 1) / grid * ktiles * (dual ? 2u : 1u) > (uint32_t)P.nstage;
 }
 
 template <class F, int M, bool INCTA, int CW, int G, int MODE = 0, bool DEEP = false>
@@ -791,9 +830,11 @@ cudaError_t launch_mma(const QkLayout &L, const uint8_t *W, const float *x, floa
     const char *e = qk_knob("QK_PDL");
     use_pdl = (e && e[0] == '0') ? 0 : 1;
   }
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = 2, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
 
   if (!INCTA) {
     const uint32_t quads = (uint32_t)M * P.Kp / 4;
@@ -811,12 +852,14 @@ cudaError_t launch_mma(const QkLayout &L, const uint8_t *W, const float *x, floa
     ctas = (e && atoi(e) == 2) ? 2 : 1;
   }
   uint32_t grid = (uint32_t)sm_count * (uint32_t)ctas;  // persistent
+  if (MODE == 3) grid = (uint32_t)sm_count / 2;         // pairs
   if (grid > L.chunks) grid = L.chunks;
+  if (MODE == 3) grid *= 2;
   const int nstage = DEEP ? P.deep : P.nstage;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid), cfg.blockDim = dim3((CW + 1 + (F::SPLIT_PRODUCER ? 1 : 0) + ((MODE == 1 && peers && peers->unpack_n) ? 1 : 0)) * 32);
+  cfg.gridDim = dim3(grid), cfg.blockDim = dim3((CW + 2 + ((MODE == 1 && peers && peers->unpack_n) ? 1 : 0)) * 32);
   cfg.dynamicSmemBytes = P.total + (uint32_t)(nstage - P.nstage) * P.stage_bytes, cfg.stream = s;
-  cfg.attrs = at, cfg.numAttrs = use_pdl ? 1 : 0;
+  cfg.attrs = at, cfg.numAttrs = MODE == 3 ? 2 : use_pdl ? 1 : 0;
   QkPeers pv = {};
   if (peers) pv = *peers;
   // Weight tiles issued before the wait on the previous kernel; the rest of the ring follows
@@ -847,12 +890,42 @@ inline bool split_in_cta(const PlanMma &P, uint32_t m) {
   return m * P.Kp <= QK_SPLIT_IN_CTA;
 }
 
+// Whether one row's matvec goes to pairs of CTAs, each streaming half of a chunk's K and splitting that half of the
+// activations itself: where the SMs' shares of chunks are so uneven that half chunks are a shorter longest share, and K so
+// long (F::PAIR_COLS; 0: never) that what drops out is worth the meeting of the pair: the launch that splits the activations,
+// and an image of them that leaves the ring few stages.  us, whole chunks / halves, 4096 rows (4 chunks / 7 halves a CTA):
+// Q6_K 14336 columns 14.4 / 12.6, 11008 11.5 / 10.9, 10240 10.1 / 10.1; Q8_0 14336 15.0 / 14.0, 12288 12.0 / 12.6; IQ4_XS
+// 14336 15.4 / 13.7, 9728 11.9 / 10.9; Q5_K 13.9 / 11.8, 10.9 / 9.3; Q3_K 16.0 / 13.6, 12288 12.8 / 12.3, 9728 11.1 / 11.1;
+// Q4_K 10.3 / 10.2, Q4_0 10.25 / 10.25 (their rings are long enough).  Even shares gain little or lose: Q6_K 1024 rows
+// (one chunk / two halves) 6.1 / 6.7, 4736 (4 / 8) 14.9 / 14.5.  Two rows and more mostly lose (Q4_K 1024 x 14336 6.2 / 8.5).
+template <class F>
+inline bool pair_pays(const QkLayout &L, int sm_count, PlanMma *P) {
+  const uint32_t sms = (uint32_t)sm_count, pairs = sms / 2;
+  return L.nb * L.bs >= F::PAIR_COLS && L.chunks <= PAIR_CHUNKS * pairs && 2 * ((L.chunks + sms - 1) / sms) > (L.chunks + pairs - 1) / pairs &&
+         make_plan_mma(L, 1, P, F::XSB, true);
+}
+
 template <class F, int M>
 cudaError_t launch_mma_m(const QkLayout &L, const uint8_t *W, const float *x, float *y,
                          uint64_t ldy, unsigned *status, unsigned char *ximg, int sm_count,
                          const PlanMma &P, cudaStream_t s, const QkPeers *peers, const uint8_t *W2, bool host_x) {
   // Warp groups: a group owns every G-th chunk (P.groups was chosen with the ring's depth, see make_plan_mma).
   const bool peer = peers != nullptr, deep = ring_is_deep<F>(L, P, sm_count, W2 != nullptr);
+  if constexpr (M == 1 && F::PAIR_COLS != 0) {
+    PlanMma H;
+    if (!peer && !W2 && !host_x && pair_pays<F>(L, sm_count, &H)) {
+#define QK_PAIR(GV, DV) return launch_mma<F, M, true, MAX_CW, GV, 3, DV>(L, W, x, y, ldy, status, ximg, sm_count, H, s)
+      if constexpr (F::ANY_DEPTH)
+        if (ring_is_deep<F>(L, H, sm_count, false, true)) {
+          if (H.groups == 4) QK_PAIR(4, true);
+          if (H.groups == 2) QK_PAIR(2, true);
+        }
+      if (H.groups == 4) QK_PAIR(4, false);
+      if (H.groups == 2) QK_PAIR(2, false);
+      QK_PAIR(1, false);
+#undef QK_PAIR
+    }
+  }
 #define QK_LAUNCH2(CWV, GV, PV, DV)                                                                               \
   return !host_x && (!ximg || split_in_cta(P, M))                                                                 \
              ? launch_mma<F, M, true, CWV, GV, PV, DV>(L, W, x, y, ldy, status, ximg, sm_count, P, s, peers, W2)  \

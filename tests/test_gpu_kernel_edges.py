@@ -562,3 +562,17 @@ def test_moe_group_plan(n, top_k, tokens, begin, local):
     check_device_status()
     ex.free()
     assert np.abs(y.cpu().numpy() - ref).max() <= 3e-3 * np.abs(ref).max()
+
+
+# One row by pairs of CTAs, half of K each (148 SMs: where 2 ceil(chunks / 148) > ceil(chunks / 74)): a single chunk, one and
+# two chunks for some pairs, the most chunks that a pair takes; halves of equal and of unequal length, the last block ragged;
+# and neighbours that stay with whole chunks (even shares, halves of 17 and 16 spans).
+@pytest.mark.parametrize("t,rows,cols", [(t, *s) for t in (S.Q6_K, S.Q5_K) for s in [
+    (3, 14336), (592, 11520), (593, 11300), (1190, 12288), (1777, 16128), (18352, 11008), (18353, 11008), (1184, 14336), (600, 8448)]] + [
+    (S.IQ4_XS, 4096, 8704), (S.Q3_K, 600, 11264), (S.Q8_0, 1200, 14336), (S.Q8_0, 600, 14581)])
+def test_decode_pairs(t, rows, cols):
+    w = S.gen_weight(t, rows, cols, seed=141)
+    x = S.gen_acts(1, cols, seed=142)
+    y = device_product(t, w, x, rows, cols, 1)
+    assert_product(y, x, O.dequant_matrix(t, w, rows, cols), half=False)
+    assert np.array_equal(y, device_product(t, w, x, rows, cols, 1))  # the same bits on every run

@@ -78,8 +78,10 @@ static uint32_t round_up(uint32_t v, uint32_t to) { return (v + to - 1) / to * t
 // fit to 96 shapes (256 x 12288 .. 28672 x 4096, 8 .. 2048 tokens, Q4_K, Q6_K, Q8_0, IQ4_XS), each timed with every tile
 // width and split; the expansion's (one for all but Q6_K), the cluster's and the one for Q8_0 were then fitted to 1076
 // calls with the weights from HBM (16 shapes 1024 x 1024 .. 28672 x 4096, 300 x 8192 .. 4096 x 14336, the same tokens and
-// formats; rows of gate and up together are such shapes too): the form it picks is 1.1 % slower than the fastest in the
-// mean, 19 % at worst; 1.3 % and 22 % before.  A super-block takes as long as its expansion or its MMAs, or in a pair the
+// formats; rows of gate and up together are such shapes too): the form it picks was 1.1 % slower than the fastest in the
+// mean, 19 % at worst.  Q4_K and Q6_K since expand faster (WFmt): with 870 and 1130 for 1000 and 1170 the 315 and 52 calls of
+// another sweep (15 and 4 shapes, 5 .. 1024 tokens) take 0.995 and 0.997 of the time in the mean (8192 x 4096 by 8 to 24
+// 13.4 -> 10.7 us; 5120 x 5120 by 80 15.4 -> 16.3); 900 and 930 gained less.  A super-block takes as long as its expansion or its MMAs, or in a pair the
 // round of hand-overs (expanding warps -> issuer -> tensor pipe -> back).  A tile whose partials go through the
 // workspace costs some 7000 cycles and 40 per token (writing them out, the fence, the counter, reading them back);
 // through the cluster 4300 and 17 per token (with 4600 for any width IQ4_XS 2048 x 2048 by 64 took 9.5 us in clusters, 8.1
@@ -103,7 +105,7 @@ bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
     p.row_blocks = (L.rows + p.cg * BM - 1) / (p.cg * BM);
     p.grid = (uint32_t)sm_count / p.cg;
   } else {
-    const float expand = L.type == QK_T_Q6_K ? 1170.f : 1000.f;
+    const float expand = L.type == QK_T_Q6_K ? 1130.f : L.type == QK_T_Q4_K ? 870.f : 1000.f;
     float best = FLT_MAX;
     auto take = [&](float t, uint32_t cg, uint32_t cs, uint32_t bn, uint32_t tbr, uint32_t rbs, uint32_t run, uint32_t grid) {
       if (t < best) best = t, p.cg = cg, p.cs = cs, p.bn = bn, p.tok_blocks = tbr, p.row_blocks = rbs, p.min_run = run, p.grid = grid;
@@ -209,6 +211,45 @@ cudaError_t qk_gemm_tc_map(const QkLayout &L, uint8_t *tiled, void *map) {
     return cudaErrorInvalidValue;
   memcpy(map, &m, sizeof(m));
   return cudaSuccess;
+}
+
+size_t qk_gemm_tc_factor_bytes(const QkLayout &L) {
+  return L.type == QK_T_Q4_K || L.type == QK_T_Q6_K ? (size_t)L.chunks * QK_TILE_ROWS * sizeof(float) : 0;
+}
+
+namespace {
+// A warp per row.  With b = the largest |scale| of the row's weights (Q4_K: 63 |d|, and |dmin|; Q6_K: 128 |d|) the factor is
+// the power of two over which 2^24 b is at most 0.998 of 2^16, about fp16's largest (2^-6 at least: 2^30 is what the kernel
+// takes).  Scales that are not finite do not count
+// (their blocks stay not finite), a row of zeros has factor 1.
+__global__ void __launch_bounds__(256) qk_row_factor_kernel(QkLayout L, const uint8_t *__restrict__ tiled, float *__restrict__ rows) {
+  const uint32_t row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= L.chunks * QK_TILE_ROWS) return;
+  const int dp = L.type == QK_T_Q4_K ? 0 : (int)L.nplanes - 1;  // the plane that (begins with) d
+  const float times = L.type == QK_T_Q4_K ? 63.f : 128.f;
+  float b = 0.f;
+  if (row < L.rows)
+    for (uint32_t k = lane; k < L.nb; k += 32) {
+      const uint32_t w = *reinterpret_cast<const uint16_t *>(tiled + qk_byte_offset(L, row, k, dp, 0));
+      const float d = fabsf(__half2float(__ushort_as_half((unsigned short)w))) * times;
+      if (d <= FLT_MAX) b = fmaxf(b, d);
+      if (L.type == QK_T_Q4_K) {
+        const float m = fabsf(__half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(tiled + qk_byte_offset(L, row, k, dp, 2)))));
+        if (m <= FLT_MAX) b = fmaxf(b, m);
+      }
+    }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) b = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, o));
+  int e = 0;
+  const float f = frexpf(b, &e);  // b = f * 2^e, f in [0.5, 1)
+  if (lane == 0) rows[row] = b > 0.f ? ldexpf(1.f, max(e + 8 + (f > 0.998f ? 1 : 0), -6)) : 1.f;
+}
+}  // namespace
+
+cudaError_t qk_gemm_tc_factors(const QkLayout &L, const uint8_t *tiled, float *rows, cudaStream_t s) {
+  if (!qk_gemm_tc_factor_bytes(L)) return cudaSuccess;
+  qk_row_factor_kernel<<<L.chunks, 256, 0, s>>>(L, tiled, rows);
+  return cudaGetLastError();
 }
 
 size_t qk_gemm_tc_part_bytes(int sm_count) { return (size_t)sm_count * 2 * qktc::MAX_BN * qktc::BM * 4; }

@@ -118,6 +118,7 @@ template <int NG>
 struct TcMaps {
   CUtensorMap x[NG > 1 ? 4 : 1];
   CUtensorMap w[NG];
+  const float *rows[NG];  // the rows' factors, powers of two (SCALED)
 };
 
 __device__ __forceinline__ bool elect_one() {
@@ -267,9 +268,20 @@ __device__ __forceinline__ float4 ldcg4(const float *p) { return __ldcg(reinterp
 // column (inside the super-block) that lands at position p, and the activations are laid out in the
 // same order, so the contraction is unchanged.  (Q4_K, whose order spans 64 columns: conv_order.)
 //
+// Q4_K and Q6_K expand their fields as fp16 subnormals: masked out of its word, q is the half q 2^-24 (2^-20 for a high
+// nibble), exact, and one fused multiply-add with scale 2^24 and offset gives the weight, rounded once.  (With an exponent
+// or-ed in and subtracted again it is two packed operations per pair, and the expansion is bound by issue.  us, before /
+// now: Q4_K 14336 x 4096 by 8 tokens 13.1 / 11.6, by 37 14.4 / 12.6, 4096 x 14336 by 8 15.5 / 14.3, 4096 x 4096 by 128 14.9 /
+// 13.1; Q6_K 4096 x 14336 by 8 16.65 / 16.2, 4096 x 4096 by 37 10.8 / 10.5.  Q8_0 and Q4_0, whose scales change with every 32
+// columns, gained nothing: 4096 x 4096 by 8 9.06 / 9.12, 8.31 / 8.33.)  scale 2^24 fits a half because the weights of a row
+// are expanded over a power of two of the row's own, its factor; the epilogue multiplies the row's results by it again.  Both
+// are exact: the weights are those of before over a power of two, but for the ones below 2^-10 of the row's largest (Q6_K
+// 2^-11), which fall among the subnormals and keep 2^-21 of it (2^-22).
+//
+//   SCALED    whether that is how the format is expanded and its rows have factors (qk_gemm_tc_factors)
 //   BB, BPS   bytes of a block of one row; blocks per super-block.  A staged super-block is
 //             [16 chunks][BPS blocks][8 rows x BB bytes], block-major as in HBM
-//   Hd        what the four quarters share (scales), head() fetches it (p: the row's chunk)
+//   Hd        what the four quarters share (scales), head() fetches it (p: the row's chunk, rf: see above)
 //   Qt        the packed bytes of quarter k (32 columns); quarter() fetches them
 //   expand    quarter k -> sixteen half2
 // (The four quarters are unrolled; as a rolled loop of a quarter of the code they take the same time,
@@ -316,6 +328,22 @@ __device__ __forceinline__ void nibbles_to_magic(uint32_t w, const NibbleMagic &
   e[0] = and_or(w, 0x000F000Fu, k.lo), e[1] = and_or(wj, 0x000F000Fu, k.lo);
   e[2] = and_or(w, 0x00F000F0u, k.hi), e[3] = and_or(wj, 0x00F000F0u, k.hi);
 }
+// The nibbles of one packed word -> 8 halves: low nibbles become q 2^-24, high ones q 2^-20; values come out
+// as pairs (byte 0, byte 2), (byte 1, byte 3) of the low nibbles, then of the high ones.
+__device__ __forceinline__ void nibbles_to_halves(uint32_t w, __half2 (&e)[4]) {
+  const uint32_t wj = w >> 8;
+  e[0] = bits_h2(w & 0x000F000Fu), e[1] = bits_h2(wj & 0x000F000Fu);
+  e[2] = bits_h2(w & 0x00F000F0u), e[3] = bits_h2(wj & 0x00F000F0u);
+}
+// rf as the product of two halves, since it may be up to 2^30 (all that it is multiplied with stays exact on the way).
+struct RowScale {
+  uint32_t a, b;
+  __device__ __forceinline__ void set(float factor) {  // 2^24 / factor
+    const int e = 24 + 127 - (int)(__float_as_uint(factor) >> 23), ea = max(min(e, 15), -14);
+    a = (uint32_t)(15 + ea) * 0x04000400u, b = (uint32_t)(15 + e - ea) * 0x04000400u;
+  }
+  __device__ __forceinline__ __half2 times(__half2 v) const { return __hmul2(__hmul2(v, bits_h2(a)), bits_h2(b)); }
+};
 // Four unsigned bytes -> halves 1024 + b, in byte order.
 __device__ __forceinline__ void bytes_to_magic(uint32_t w, uint32_t &lo, uint32_t &hi) {
   lo = prmt(w, 0x64646464u, 0x4140), hi = prmt(w, 0x64646464u, 0x4342);
@@ -324,40 +352,38 @@ __device__ __forceinline__ void bytes_to_magic(uint32_t w, uint32_t &lo, uint32_
 template <>
 struct WFmt<QK_T_Q4_K> {  // d, dmin, 12 bytes of 6-bit scales / mins, 128 bytes of nibbles (reference/q4_k.rs:27-102)
   static constexpr uint32_t BB = 144, BPS = 1, LUT = 0;
+  static constexpr bool SCALED = true;
   __device__ static void fill_lut(unsigned char *, uint32_t, uint32_t) {}
   // position 8 i + j of a 64-group <- column 4 i + {0,2,1,3}[j & 3] + 32 (j >> 2): byte 4 i + b of
   // the group's 32 holds column 4 i + b (low nibble) and 32 + 4 i + b (high nibble)
-  struct Hd { uint32_t scw, mnw, d; };  // the half's four 6-bit scales and minima, one per byte; d and dmin
+  struct Hd { uint32_t scw, mnw, d; };  // the half's four 6-bit scales and minima, one per byte; d rf and dmin rf
   struct Qt { uint4 q; };
   // [8 rows x 16 header | 4 groups x 8 rows x 32 nibble bytes]
-  __device__ static void head(Hd &c, uint32_t p, uint32_t rr, uint32_t hh) {
+  __device__ static void head(Hd &c, uint32_t p, uint32_t rr, uint32_t hh, RowScale rf) {
     const uint4 h = lds128(p + rr * 16);
     c.scw = hh ? ((h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u)) : (h.y & 0x3F3F3F3Fu);
     c.mnw = hh ? (((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u)) : (h.z & 0x3F3F3F3Fu);
-    c.d = h.x;
+    c.d = h2_bits(rf.times(bits_h2(h.x)));
   }
   __device__ static void quarter(Qt &t, uint32_t p, uint32_t rr, uint32_t hh, uint32_t k) {
     t.q = lds128(p + 128 + hh * 512 + rr * 32 + (k >> 1) * 256 + (k & 1u) * 16);
   }
   // d * sc and dmin * mn have 17 bits at most, so the fp16 products are the f32 ones rounded once.
-  // q is exact after the subtraction, then one fused q * scale - min.
+  // 6-bit fields as halves: sc exactly (1024 + sc less 1024), sc / 16 for the high nibbles, mn as mn 2^-24.
   __device__ static void expand(const Qt &t, const Hd &c, uint32_t k, uint32_t (&o)[16], uint32_t) {
-    const __half2 k1024 = __float2half2_rn(1024.f), k_hi = __float2half2_rn(64.f);
     const __half2 d = __low2half2(bits_h2(c.d)), m = __hneg2(__high2half2(bits_h2(c.d)));
     const uint32_t lo = 0x4040u + (k >> 1) * 0x0202u, hi = lo + 0x0101u;  // the 64-group's two sub-blocks
-    const __half2 s_lo = __hmul2(__hsub2(bits_h2(prmt(c.scw, 0x64646464u, lo)), k1024), d);
-    const __half2 s_hi = __hmul2(__hsub2(bits_h2(prmt(c.scw, 0x64646464u, hi)), k1024), d);
-    const __half2 m_lo = __hmul2(__hsub2(bits_h2(prmt(c.mnw, 0x64646464u, lo)), k1024), m);
-    const __half2 m_hi = __hmul2(__hsub2(bits_h2(prmt(c.mnw, 0x64646464u, hi)), k1024), m);
-    const NibbleMagic km = nibble_magic();
+    const __half2 s_lo = __hmul2(__hsub2(bits_h2(prmt(c.scw, 0x64646464u, lo)), __float2half2_rn(1024.f)), d);
+    const __half2 s_hi = __hmul2(__hsub2(bits_h2(prmt(c.scw, 0x54545454u, hi)), __float2half2_rn(64.f)), d);
+    const __half2 m_lo = __hmul2(bits_h2(prmt(c.mnw, 0u, lo)), m), m_hi = __hmul2(bits_h2(prmt(c.mnw, 0u, hi)), m);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-      uint32_t e[4];
-      nibbles_to_magic(word(t.q, i), km, e);
-      o[4 * i + 0] = h2_bits(__hfma2(__hsub2(bits_h2(e[0]), k1024), s_lo, m_lo));
-      o[4 * i + 1] = h2_bits(__hfma2(__hsub2(bits_h2(e[1]), k1024), s_lo, m_lo));
-      o[4 * i + 2] = h2_bits(__hfma2(__hsub2(bits_h2(e[2]), k_hi), s_hi, m_hi));
-      o[4 * i + 3] = h2_bits(__hfma2(__hsub2(bits_h2(e[3]), k_hi), s_hi, m_hi));
+      __half2 e[4];
+      nibbles_to_halves(word(t.q, i), e);
+      o[4 * i + 0] = h2_bits(__hfma2(e[0], s_lo, m_lo));
+      o[4 * i + 1] = h2_bits(__hfma2(e[1], s_lo, m_lo));
+      o[4 * i + 2] = h2_bits(__hfma2(e[2], s_hi, m_hi));
+      o[4 * i + 3] = h2_bits(__hfma2(e[3], s_hi, m_hi));
     }
   }
 };
@@ -365,11 +391,12 @@ struct WFmt<QK_T_Q4_K> {  // d, dmin, 12 bytes of 6-bit scales / mins, 128 bytes
 template <>
 struct WFmt<QK_T_Q8_0> {  // block of 32: f16 d, 32 int8 (reference/q8_0.rs)
   static constexpr uint32_t BB = 34, BPS = 8, LUT = 0;
+  static constexpr bool SCALED = false;
   __device__ static void fill_lut(unsigned char *, uint32_t, uint32_t) {}
   __host__ __device__ static uint32_t src(uint32_t p) { return p; }
   struct Hd {};
   struct Qt { uint4 q[2]; uint32_t d; };
-  __device__ static void head(Hd &, uint32_t, uint32_t, uint32_t) {}
+  __device__ static void head(Hd &, uint32_t, uint32_t, uint32_t, RowScale) {}
   // A block's 8 rows: [2 granules x 8 rows x 16 int8][8 x d].  Blocks past the end of the row
   // are zero-filled by the copy: d = 0.
   __device__ static void quarter(Qt &t, uint32_t p, uint32_t rr, uint32_t hh, uint32_t k) {
@@ -392,6 +419,7 @@ struct WFmt<QK_T_Q8_0> {  // block of 32: f16 d, 32 int8 (reference/q8_0.rs)
 template <>
 struct WFmt<QK_T_Q4_0> {  // block of 32: f16 d, 16 bytes; byte j = elements 2 j (low nibble) and 2 j + 1 (high) (reference/q4_0.rs:36-46)
   static constexpr uint32_t BB = 18, BPS = 8, LUT = 0;
+  static constexpr bool SCALED = false;
   __device__ static void fill_lut(unsigned char *, uint32_t, uint32_t) {}
   // a word yields its eight elements as (byte 0, byte 2), (byte 1, byte 3) low nibbles, then the
   // same of the high nibbles
@@ -401,7 +429,7 @@ struct WFmt<QK_T_Q4_0> {  // block of 32: f16 d, 16 bytes; byte j = elements 2 j
   }
   struct Hd {};
   struct Qt { uint4 q; uint32_t d; };
-  __device__ static void head(Hd &, uint32_t, uint32_t, uint32_t) {}
+  __device__ static void head(Hd &, uint32_t, uint32_t, uint32_t, RowScale) {}
   // A block's 8 rows: [8 rows x 16 nibble bytes][8 x d].
   __device__ static void quarter(Qt &t, uint32_t p, uint32_t rr, uint32_t hh, uint32_t k) {
     p += (hh * 4 + k) * 144;
@@ -426,37 +454,37 @@ struct WFmt<QK_T_Q4_0> {  // block of 32: f16 d, 16 bytes; byte j = elements 2 j
 template <>
 struct WFmt<QK_T_Q6_K> {  // super-block of 256: ql 128, qh 64, 16 int8 scales, f16 d (reference/q6_k.rs)
   static constexpr uint32_t BB = 210, BPS = 1, LUT = 0;
+  static constexpr bool SCALED = true;
   __device__ static void fill_lut(unsigned char *, uint32_t, uint32_t) {}
   // half hh = ql[64 hh ..], qh[32 hh ..]; its quarter k (columns 32 k ..) = nibble k >> 1 of ql bytes
   // 32 (k & 1) + l and bit pair 2 k of qh byte l
   __host__ __device__ static uint32_t src(uint32_t p) { return p; }
-  struct Hd { uint4 qh[2]; uint2 sc; float d; };
+  struct Hd { uint4 qh[2]; uint2 sc; __half2 d; };  // sc: the half's scales + 128; d rf
   struct Qt { uint4 ql[2]; };
   // A block's 8 rows: [12 granules x 8 rows x 16 bytes of ql+qh][8 rows x 16 scales][8 x d].
-  __device__ static void head(Hd &c, uint32_t p, uint32_t rr, uint32_t hh) {
+  __device__ static void head(Hd &c, uint32_t p, uint32_t rr, uint32_t hh, RowScale rf) {
     const uint32_t q = p + rr * 16;
     c.qh[0] = lds128(q + (8 + 2 * hh) * 128), c.qh[1] = lds128(q + (9 + 2 * hh) * 128);
     c.sc = lds64(q + 1536 + 8 * hh);
-    c.d = h2f_bits(lds16(p + 1664 + 2 * rr));
+    c.sc.x ^= 0x80808080u, c.sc.y ^= 0x80808080u;
+    c.d = rf.times(__low2half2(bits_h2(lds16(p + 1664 + 2 * rr))));
   }
   __device__ static void quarter(Qt &t, uint32_t p, uint32_t rr, uint32_t hh, uint32_t k) {
     const uint32_t q = p + rr * 16 + (4 * hh + 2 * (k & 1u)) * 128;
     t.ql[0] = lds128(q), t.ql[1] = lds128(q + 128);
   }
   __device__ static void expand(const Qt &t, const Hd &c, uint32_t k, uint32_t (&o)[16], uint32_t) {
-    const __half2 off = __float2half2_rn(1056.f);  // (1024 + q) - 1056 = q - 32, exact; then one rounding in the product
-    const uint32_t scw = ((k >> 1) ? c.sc.y : c.sc.x) >> (16 * (k & 1u)), nib = 4 * (k >> 1), rot = (4 - 2 * k) & 31u;
-    __half2 s[2];  // 16 columns per scale
-#pragma unroll
-    for (int i = 0; i < 2; i++) s[i] = __float2half2_rn(c.d * (float)(int)(signed char)((scw >> (8 * i)) & 0xFF));
+    const uint32_t scw = (k >> 1) ? c.sc.y : c.sc.x, pair = (k & 1u) ? 0x4342 : 0x4140, nib = 4 * (k >> 1), rot = (4 - 2 * k) & 31u;
+    // 16 columns per scale: 1024 + (sc + 128) less 1152; d * sc has 19 bits at most and is rounded once; q - 32
+    const __half2 sp = __hmul2(__hsub2(bits_h2(prmt(scw, 0x64646464u, pair)), __float2half2_rn(1152.f)), c.d);
+    const __half2 op = __hmul2(sp, __float2half2_rn(-0x1p-19f));
+    const __half2 s[2] = {__low2half2(sp), __high2half2(sp)}, off[2] = {__low2half2(op), __high2half2(op)};
 #pragma unroll
     for (int i = 0; i < 8; i++) {
       const uint32_t lw = word(t.ql[i >> 2], i & 3) >> nib, hw = word(c.qh[i >> 2], i & 3);
       const uint32_t q6 = (lw & 0x0F0F0F0Fu) | (__funnelshift_l(hw, hw, rot) & 0x30303030u);
-      uint32_t a, b2;
-      bytes_to_magic(q6, a, b2);
-      o[2 * i] = h2_bits(__hmul2(__hsub2(bits_h2(a), off), s[i >> 2]));
-      o[2 * i + 1] = h2_bits(__hmul2(__hsub2(bits_h2(b2), off), s[i >> 2]));
+      o[2 * i] = h2_bits(__hfma2(bits_h2(prmt(q6, 0u, 0x4140)), s[i >> 2], off[i >> 2]));  // bytes as halves b 2^-24
+      o[2 * i + 1] = h2_bits(__hfma2(bits_h2(prmt(q6, 0u, 0x4342)), s[i >> 2], off[i >> 2]));
     }
   }
 };
@@ -468,6 +496,7 @@ struct WFmt<QK_T_IQ4_XS> {  // super-block of 256: f16 d, scales_h, scales_l[4],
   // maps a byte straight to the half2 (K[low], K[high]) of its two adjacent elements; every lane has
   // a copy of its own in its own bank (32 KB), so the look-ups of a warp never conflict.
   static constexpr uint32_t BB = 136, BPS = 1, LUT = 32768;
+  static constexpr bool SCALED = false;  // (the table holds whole numbers as they are: one product)
   __host__ __device__ static uint32_t src(uint32_t p) { return p; }
   __device__ static void fill_lut(unsigned char *lut, uint32_t tid, uint32_t nthreads) {
     constexpr uint32_t K0 = 0xBFAD9881u, K1 = 0xF6EADDCFu, K2 = 0x26190D01u, K3 = 0x71594535u;  // K[0..15] as bytes
@@ -481,7 +510,7 @@ struct WFmt<QK_T_IQ4_XS> {  // super-block of 256: f16 d, scales_h, scales_l[4],
   struct Hd { float d; uint32_t ls; };  // ls: the half's four 6-bit scales, one per byte
   struct Qt { uint4 q; };
   // A block's 8 rows: [8 granules x 8 rows x 16 nibble bytes][8 rows x 8 header bytes].
-  __device__ static void head(Hd &c, uint32_t p, uint32_t rr, uint32_t hh) {
+  __device__ static void head(Hd &c, uint32_t p, uint32_t rr, uint32_t hh, RowScale) {
     const uint2 h = lds64(p + 1024 + rr * 8);
     c.d = h2f_bits(h.x);
     const uint32_t sl = hh ? h.y >> 16 : h.y, sh = h.x >> (16 + 8 * hh);
@@ -909,6 +938,10 @@ __global__ void __maxnreg__(REGS)
   auto box_of = [&](uint32_t n) { return NG > 1 ? (n / CG + hq - 1) / hq : 1u; };  // the how-manieth box (from 1)
   auto box_rows = [&](uint32_t n) { return NG > 1 ? min(box_of(n) * hq, A.hn / CG) : A.hn / CG; };
 
+  // The factors of four rows (a multiple of 4 the first; the table has whole chunks of 8)
+  auto factors4 = [&](uint32_t g, uint32_t row) {
+    return F::SCALED && row < A.L.rows ? __ldg(reinterpret_cast<const float4 *>(M.rows[g] + row)) : make_float4(1.f, 1.f, 1.f, 1.f);
+  };
   // The last contributor of a split tile adds the partials up, in the order of their K runs: a warp four
   // tokens at a time, a lane four rows.
   auto add_up = [&](uint32_t tile) {
@@ -920,6 +953,7 @@ __global__ void __maxnreg__(REGS)
     const float *sp = A.xscale + (NG > 1 ? (q.g % A.n_act) * A.xcap : 0u) + q.t0;
     float *yt = A.y + (uint64_t)((NG > 1 ? q.g * A.ycap : 0u) + q.t0) * A.ldy;
     const bool vec = row0 + BM <= A.L.rows && (A.ldy & 3u) == 0 && ((uintptr_t)A.y & 15u) == 0;
+    const float4 rk = factors4(NG > 1 ? q.g : 0, rw);
     for (uint32_t c = 4 * warp; c < live; c += NTHREADS / 8) {
       float4 s[4];
 #pragma unroll
@@ -938,7 +972,7 @@ __global__ void __maxnreg__(REGS)
       for (uint32_t j = 0; j < 4; j++, yp += A.ldy) {
         if (c + j >= live) break;
         const float f = __ldg(sp + c + j);
-        const float4 v = make_float4(s[j].x * f, s[j].y * f, s[j].z * f, s[j].w * f);
+        const float4 v = make_float4(s[j].x * rk.x * f, s[j].y * rk.y * f, s[j].z * rk.z * f, s[j].w * rk.w * f);
         if (vec) {
           *reinterpret_cast<float4 *>(yp) = v;
         } else {
@@ -1142,6 +1176,7 @@ __global__ void __maxnreg__(REGS)
       const uint32_t row0 = (q.rb * CG + rank) * BM, row = row0 + r;
       const float *sp = A.xscale + (NG > 1 ? (q.g % A.n_act) * A.xcap : 0u) + q.t0;
       float *yt = A.y + (uint64_t)((NG > 1 ? q.g * A.ycap : 0u) + q.t0) * ldy;  // the tile's first token
+      const float rk = F::SCALED && !split && row < A.L.rows ? __ldg(M.rows[NG > 1 ? q.g : 0] + row) : 1.f;
       // partial tiles: [slot][token][128 rows]
       const uint32_t slot = A.bn * BM;
       float *mine = A.part + (blockIdx.x * 2 + (i == sc.whole ? 0u : 1u)) * slot + r;
@@ -1189,15 +1224,15 @@ __global__ void __maxnreg__(REGS)
 #pragma unroll
               for (uint32_t j4 = 0; j4 < 4; j4++) {
                 const float4 f = f4[j4];
-                *yp = __uint_as_float(v[4 * j4]) * f.x, yp += ldy;
-                *yp = __uint_as_float(v[4 * j4 + 1]) * f.y, yp += ldy;
-                *yp = __uint_as_float(v[4 * j4 + 2]) * f.z, yp += ldy;
-                *yp = __uint_as_float(v[4 * j4 + 3]) * f.w, yp += ldy;
+                *yp = __uint_as_float(v[4 * j4]) * rk * f.x, yp += ldy;
+                *yp = __uint_as_float(v[4 * j4 + 1]) * rk * f.y, yp += ldy;
+                *yp = __uint_as_float(v[4 * j4 + 2]) * rk * f.z, yp += ldy;
+                *yp = __uint_as_float(v[4 * j4 + 3]) * rk * f.w, yp += ldy;
               }
             } else {
 #pragma unroll
               for (uint32_t j = 0; j < 16; j++, yp += ldy)
-                if (row < A.L.rows && c + j < live) *yp = __uint_as_float(v[j]) * scales[c + j];
+                if (row < A.L.rows && c + j < live) *yp = __uint_as_float(v[j]) * rk * scales[c + j];
             }
           }
         }
@@ -1240,11 +1275,31 @@ __global__ void __maxnreg__(REGS)
       sched.get(i, tile, s0, s1);
       n_sb += s1 - s0;
     }
+    // The factor of this thread's row in the segment that holds super-block j, and in the one behind it
+    uint32_t seg = 0, seg_end = 0;
+    auto row_of = [&](uint32_t i) {
+      if (i >= sched.n_seg) return 1.f;
+      uint32_t tile, s0, s1;
+      sched.get(i, tile, s0, s1);
+      const TileAt q = at(tile);
+      const uint32_t row = (q.rb * CG + rank) * BM + r;
+      return row < A.L.rows ? __ldg(M.rows[NG > 1 ? q.g : 0] + row) : 1.f;
+    };
+    auto seg_len = [&](uint32_t i) {
+      uint32_t tile, s0, s1;
+      sched.get(i, tile, s0, s1);
+      return s1 - s0;
+    };
+    RowScale rf = {};
+    float next_factor = 1.f;
+    if (F::SCALED && n_sb) rf.set(row_of(0)), next_factor = row_of(1), seg_end = seg_len(0);
     const uint32_t w_bytes = S.w_stage, nst = S.w_stages, w0 = sbase + S.w + (r >> 3) * CHB;
     const uint32_t ta0 = tmem + ((32 * quarter) << 16) + a_col + hh * 64u, a_full0 = in_first<CG>(sbase + S.a_full);
     uint32_t ws = set, wph = 0;      // ring stage and parity of this set's next super-block
     uint32_t ab = set, auses = 0;                       // its buffer, and how often that has been used (set < na)
     for (uint32_t j = set; j < n_sb; j += 2) {
+      if (F::SCALED)
+        while (j >= seg_end) rf.set(next_factor), next_factor = row_of(++seg + 1), seg_end += seg_len(seg);
       if (!warp_wait(sbase + S.w_full + ws * 8, wph)) {
         dead = true;  // warp-uniform: these warps execute .aligned tcgen05 instructions
         break;
@@ -1253,7 +1308,7 @@ __global__ void __maxnreg__(REGS)
       typename F::Hd hd;
       typename F::Qt qt;
       F::quarter(qt, p, rr, hh, 0);
-      F::head(hd, p, rr, hh);
+      F::head(hd, p, rr, hh, rf);
       // the MMAs that read this buffer's previous contents must have retired
       if (auses && !warp_wait(sbase + S.a_empty + ab * 8, (auses - 1) & 1u)) {
         dead = true;
@@ -1298,6 +1353,7 @@ __global__ void __maxnreg__(REGS)
     const uint32_t first = t0 + warp - FIRST_EW, r = 4 * lane, row = q.rb * BM + r;
     const float *sp = A.xscale + q.t0;
     float f = adds && first < t1 ? __ldg(sp + first) : 0.f;
+    const float4 rk = adds ? factors4(0, row) : make_float4(1.f, 1.f, 1.f, 1.f);
     cluster_sync();  // all partial sums are here; nobody leaves while another may still store into its memory
     const bool vec = q.rb * BM + BM <= A.L.rows && (A.ldy & 3u) == 0 && ((uintptr_t)A.y & 15u) == 0;
     for (uint32_t t = first; adds && t < t1; t += 4) {
@@ -1309,7 +1365,7 @@ __global__ void __maxnreg__(REGS)
       }
       if (t != first) f = __ldg(sp + t);
       float *yp = A.y + (uint64_t)(q.t0 + t) * A.ldy + row;
-      v.x *= f, v.y *= f, v.z *= f, v.w *= f;
+      v.x = v.x * rk.x * f, v.y = v.y * rk.y * f, v.z = v.z * rk.z * f, v.w = v.w * rk.w * f;
       if (vec) {
         *reinterpret_cast<float4 *>(yp) = v;
       } else {
@@ -1362,7 +1418,7 @@ cudaError_t launch_main(const TcPlan &P, const TcArgs &A, __half *x16, const QkT
   TcMaps<NG> M;
   for (uint32_t k = 0; k < (NG > 1 ? 4u : 1u); k++)
     if (!x_map(&M.x[k], x16, P.xrows, P.nsb * 256u, NG > 1 ? std::min(box_unit(P.hn / CG) * (k + 1), P.hn / CG) : P.hn / CG)) return cudaErrorInvalidValue;
-  for (uint32_t g = 0; g < (NG == 1 ? 1u : c.n); g++) memcpy(&M.w[g], c.maps[g], sizeof(CUtensorMap));
+  for (uint32_t g = 0; g < (NG == 1 ? 1u : c.n); g++) memcpy(&M.w[g], c.maps[g], sizeof(CUtensorMap)), M.rows[g] = c.rows[g];
   cudaLaunchAttribute at[2] = {pdl_attr(), {}};
   at[1].id = cudaLaunchAttributeClusterDimension;
   at[1].val.clusterDim.x = CG == 2 ? 2 : P.cs, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;

@@ -287,7 +287,8 @@ extern "C" int qk_weights_upload_gguf(qk_ctx *c, const qk_gguf *g, const char *n
   uint8_t *raw = nullptr, *stage[2] = {nullptr, nullptr};
   cudaEvent_t done[2] = {nullptr, nullptr};
   const size_t piece = (size_t)32 << 20;
-  cudaError_t e = cudaMalloc(&h->dev, tiled);
+  cudaError_t e = cudaMalloc(&h->dev, tiled + qk_gemm_tc_factor_bytes(h->L));
+  h->rows = (float *)(h->dev + tiled);
   int st = QK_OK;
   do {
     if (e != cudaSuccess) break;
@@ -320,6 +321,7 @@ extern "C" int qk_weights_upload_gguf(qk_ctx *c, const qk_gguf *g, const char *n
     }
     if (st != QK_OK || e != cudaSuccess) break;
     e = qk_launch_repack(h->L, raw, h->dev, c->stream);
+    if (e == cudaSuccess) e = qk_gemm_tc_factors(h->L, h->dev, h->rows, c->stream);
   } while (0);
   cudaError_t e2 = cudaStreamSynchronize(c->stream);
   if (e == cudaSuccess) e = e2;

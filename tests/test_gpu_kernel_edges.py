@@ -576,3 +576,33 @@ def test_decode_pairs(t, rows, cols):
     y = device_product(t, w, x, rows, cols, 1)
     assert_product(y, x, O.dequant_matrix(t, w, rows, cols), half=False)
     assert np.array_equal(y, device_product(t, w, x, rows, cols, 1))  # the same bits on every run
+
+
+# Rows whose scales lie anywhere in fp16's range (each row is expanded over a power of two of its own): rows of subnormal
+# scales, of the largest, and of both kinds of blocks in one row; a row of zeros; all ways of writing out (whole tiles in one
+# CTA and in pairs, clusters, partials through the workspace).  Weights of up to 65504 * 63 * 15 stay within f32 sums.
+# The bound is assert_product's, whose weights are the largest of their block: what falls among fp16's subnormals is below
+# 2^-10 of the row's largest weight, and keeps 2^-21 of that.
+@pytest.mark.parametrize("t", [S.Q4_K, S.Q6_K])
+@pytest.mark.parametrize("rows,cols,m", [(200, 512, 9), (4096, 2048, 33), (600, 1024, 130), (130, 8192, 300), (40, 256, 5)])
+def test_matmul_row_scales(t, rows, cols, m):
+    bb, nb = S.BLOCK_BYTES[t], cols // 256
+    w = S.gen_weight(t, rows, cols, seed=151).reshape(rows, nb, bb).copy()
+    at = [0, 2] if t == S.Q4_K else [208]
+    top = 900.0 if t == S.Q4_K else 440.0  # 63 d, 128 d: weights up to fp16's largest, as before
+    r, k = np.arange(rows)[:, None], np.arange(nb)[None, :]
+    d = 2.0 ** np.array([-24, -20, -14, -10, -4, 0, 6, 9])[r % 8] * np.where(r % 3 == 0, 2.0 ** -(k % 5), 1.0)
+    for o in at:
+        w[:, :, o:o + 2] = np.minimum(d, top).astype(np.float16)[:, :, None].view(np.uint8)
+    w[17:18] = 0
+    w = w.reshape(-1)
+    x = S.gen_acts(m, cols, seed=152)
+    wd = O.dequant_matrix(t, w, rows, cols)
+    y = device_product(t, w, x, rows, cols, m)
+    ref = x.astype(np.float64) @ wd.astype(np.float64).T
+    # 2^-11 for the activations, 2^-11 for the weights, and 2^-21 of the row's largest weight
+    sq = (x.astype(np.float64) ** 2) @ (wd.astype(np.float64) ** 2).T
+    low = (x.astype(np.float64) ** 2).sum(1)[:, None] * (np.abs(wd).max(1)[None, :].astype(np.float64) * 2.0 ** -21) ** 2
+    assert np.all(np.isfinite(y))
+    assert np.all(np.abs(y - ref) <= 7 * (2.0 ** -11 * np.sqrt(2 * sq) + np.sqrt(low)) + 1e-30)
+    assert np.all(y[:, 17] == 0)

@@ -70,6 +70,7 @@ constexpr uint32_t PAIR_CHUNKS = 32;            // most chunks of a pair of CTAs
 
 struct SmemMma {
   uint32_t full, redfull, xbar;  // mbarriers (8 B each)
+  uint32_t empty;                // chunks of several k-tiles: a stage's tile has been used (one arrival per warp of the group)
   uint32_t prog;                 // chunks the reducer warp has read so far (one word, polled by the producer warp)
   uint32_t issued;               // DEEP: tiles issued so far (one word, polled by the compute warps)
   uint32_t pbar, pair;           // PAIR: per chunk, the mbarrier and the 8 x M sums that the other CTA sends
@@ -193,6 +194,20 @@ __device__ __forceinline__ bool wait_issued(uint32_t word_addr, uint32_t item, u
       if (t - t0 > 250000000ull) return false;
     }
   }
+}
+
+// Waits (bounded) until the reducer has read `chunks` chunks.
+__device__ __forceinline__ bool wait_read(const volatile uint32_t *prog, uint32_t chunks) {
+  unsigned long long t0 = 0;
+  for (uint32_t polls = 1; *prog < chunks; polls++) {
+    if ((polls & 1023u) == 0) {
+      unsigned long long t;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+      if (!t0) t0 = t;
+      if (t - t0 > 250000000ull) return false;
+    }
+  }
+  return true;
 }
 
 __device__ __forceinline__ void tell_issued(uint32_t word_addr, uint32_t items) {
@@ -408,6 +423,7 @@ __global__ void __launch_bounds__((CW + 2 + (MODE == 1 ? 1 : 0)) * 32, 1)
   const uint32_t ktiles = PAIR ? (nb + L.nbt - 1) / L.nbt : L.ktiles;
   auto tile_blocks = [&](uint32_t kt) { return min(nb - kt * L.nbt, L.nbt); };
   const uint32_t my_items = my_chunks * ktiles;
+  const bool by_tile = M <= (int)F::BY_TILE_M && ktiles > 1 && my_items > (uint32_t)nstage;  // stages are handed back one by one (see the producer)
 
   QK_STAMP(warp == 0, 0);
   pdl_launch_dependents();
@@ -418,6 +434,10 @@ __global__ void __launch_bounds__((CW + 2 + (MODE == 1 ? 1 : 0)) * 32, 1)
     *reinterpret_cast<volatile uint32_t *>(smem + S.prog) = 0u, *reinterpret_cast<volatile uint32_t *>(smem + S.issued) = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (by_tile && warp == 2 && lane < (uint32_t)nstage) {
+    mbar_init(sbase + S.empty + lane * 8, WG);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (PAIR && warp == 1 && lane < my_chunks && (lane & 1u) == rank) {  // (PAIR_CHUNKS = 32: a lane each)
     mbar_init(sbase + S.pbar + lane * 8, 1);
@@ -477,34 +497,30 @@ __global__ void __launch_bounds__((CW + 2 + (MODE == 1 ? 1 : 0)) * 32, 1)
       if (INCTA) asm volatile("bar.sync 2, %0;" ::"n"((CW + 1) * 32) : "memory");
       issue_upto((uint32_t)nstage);
     }
-    uint32_t slot = 0, sph = 0;
     const volatile uint32_t *prog = reinterpret_cast<const volatile uint32_t *>(smem + S.prog);
-    for (uint32_t c = 0; c < my_chunks && item < my_items; c++) {
-      if (!mbar_wait_bounded(sbase + S.redfull + slot * 8, sph)) {  // chunk c handed over
-        if (lane == 0) atomicOr(status, QK_DEV_TIMEOUT);
-        break;
+    bool alive = true;
+    if (!by_tile) {
+      uint32_t slot = 0, sph = 0;
+      for (uint32_t c = 0; c < my_chunks && item < my_items; c++) {
+        alive = mbar_wait_bounded(sbase + S.redfull + slot * 8, sph)  // chunk c handed over
+                && wait_read(prog, c);                                // the reducer has read the chunks before c
+        if (!alive) break;
+        issue_upto(item + ktiles);
+        if (++slot == (uint32_t)nslot) slot = 0, sph ^= 1;
       }
-      unsigned long long t0 = 0;
-      uint32_t polls = 0;
-      bool dead = false;
-      while (*prog < c) {  // the reducer has read the chunks before c
-        if ((++polls & 1023u) == 0) {
-          unsigned long long t;
-          asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-          if (!t0) t0 = t;
-          if (t - t0 > 250000000ull) {
-            dead = true;
-            break;
-          }
-        }
+    } else {
+      // Chunks of several k-tiles: a stage is filled again as soon as its own tile has been used, not when the whole chunk
+      // has been handed over (us: Q4_K 4096 x 14336 by one 10.4 -> 9.7, by two 14.3 -> 12.8, 8192 x 14336 17.1 -> 14.3; Q6_K
+      // 16384 x 12288 32.9 -> 27.6; Q5_K 4096 x 14336 by four 41.5 -> 34.9); the first tile of a chunk once the reducer has read the one whose slot it takes.
+      uint32_t est = 0, eph = 0;
+      while (alive && item < my_items) {
+        alive = mbar_wait_bounded(sbase + S.empty + est * 8, eph) && (pkt || pc < (uint32_t)nslot || wait_read(prog, pc + 1 - nslot));
+        if (!alive) break;
+        issue_upto(item + 1);
+        if (++est == (uint32_t)nstage) est = 0, eph ^= 1;
       }
-      if (dead) {
-        if (lane == 0) atomicOr(status, QK_DEV_TIMEOUT);
-        break;
-      }
-      issue_upto(item + ktiles);
-      if (++slot == (uint32_t)nslot) slot = 0, sph ^= 1;
     }
+    if (!alive && lane == 0) atomicOr(status, QK_DEV_TIMEOUT);
     return;
   }
 
@@ -707,6 +723,10 @@ __global__ void __launch_bounds__((CW + 2 + (MODE == 1 ? 1 : 0)) * 32, 1)
         tile_body(std::false_type{});
       QK_STAMP(warp == 0 && tstamp < 30, 3 + 2 * tstamp);
       tstamp++;
+      if (by_tile) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(sbase + S.empty + st * 8);
+      }
       advance_stage(1);
     }
     if (dead) break;
@@ -755,6 +775,7 @@ inline bool make_plan_mma(const QkLayout &full, uint32_t m, PlanMma *P, uint32_t
   SmemMma S;
   uint32_t off = 0;
   S.full = off, off += MAX_STAGE * 8;
+  S.empty = off, off += MAX_STAGE * 8;
   S.redfull = off, off += MAX_SLOT * 8;
   S.xbar = off, off += 8;
   S.prog = off, off += 4;
@@ -893,11 +914,12 @@ inline bool split_in_cta(const PlanMma &P, uint32_t m) {
 // Whether one row's matvec goes to pairs of CTAs, each streaming half of a chunk's K and splitting that half of the
 // activations itself: where the SMs' shares of chunks are so uneven that half chunks are a shorter longest share, and K so
 // long (F::PAIR_COLS; 0: never) that what drops out is worth the meeting of the pair: the launch that splits the activations,
-// and an image of them that leaves the ring few stages.  us, whole chunks / halves, 4096 rows (4 chunks / 7 halves a CTA):
-// Q6_K 14336 columns 14.4 / 12.6, 11008 11.5 / 10.9, 10240 10.1 / 10.1; Q8_0 14336 15.0 / 14.0, 12288 12.0 / 12.6; IQ4_XS
-// 14336 15.4 / 13.7, 9728 11.9 / 10.9; Q5_K 13.9 / 11.8, 10.9 / 9.3; Q3_K 16.0 / 13.6, 12288 12.8 / 12.3, 9728 11.1 / 11.1;
-// Q4_K 10.3 / 10.2, Q4_0 10.25 / 10.25 (their rings are long enough).  Even shares gain little or lose: Q6_K 1024 rows
-// (one chunk / two halves) 6.1 / 6.7, 4736 (4 / 8) 14.9 / 14.5.  Two rows and more mostly lose (Q4_K 1024 x 14336 6.2 / 8.5).
+// and an image of them that leaves the ring few stages.  us, whole chunks / halves, a feed-forward block with this matrix last
+// (4096 rows: 4 chunks / 7 halves a CTA): Q6_K 14336 columns 27.4 / 26.1, 12288 23.1 / 23.4, 11008 22.0 / 22.4; Q5_K 26.0 /
+// 24.9, 12288 22.0 / 22.0, 11008 20.5 / 21.0; Q3_K 27.4 / 26.4, 11008 23.4 / 22.6; IQ4_XS 34.0 / 34.2, with 5120 rows of
+// 13824 40.8 / 39.3; Q8_0 33.8 / 33.7.  The matvec alone: Q6_K 13.0 / 12.9, Q5_K 13.1 / 11.2, Q3_K 14.6 / 12.7, IQ4_XS 13.3 /
+// 12.9.  Q4_K and Q4_0 have rings that are long enough; even shares gain little or lose (Q6_K, 1024 rows: one chunk or two
+// halves, 6.1 / 6.7), two rows and more mostly lose (Q4_K 1024 x 14336 6.2 / 8.5).
 template <class F>
 inline bool pair_pays(const QkLayout &L, int sm_count, PlanMma *P) {
   const uint32_t sms = (uint32_t)sm_count, pairs = sms / 2;

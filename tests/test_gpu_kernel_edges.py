@@ -566,10 +566,10 @@ def test_moe_group_plan(n, top_k, tokens, begin, local):
 
 # One row by pairs of CTAs, half of K each (148 SMs: where 2 ceil(chunks / 148) > ceil(chunks / 74)): a single chunk, one and
 # two chunks for some pairs, the most chunks that a pair takes; halves of equal and of unequal length, the last block ragged;
-# and neighbours that stay with whole chunks (even shares, halves of 17 and 16 spans).
+# and neighbours that stay with whole chunks (even shares, halves of 33 and 32 spans).
 @pytest.mark.parametrize("t,rows,cols", [(t, *s) for t in (S.Q6_K, S.Q5_K) for s in [
-    (3, 14336), (592, 11520), (593, 11300), (1190, 12288), (1777, 16128), (18352, 11008), (18353, 11008), (1184, 14336), (600, 8448)]] + [
-    (S.IQ4_XS, 4096, 8704), (S.Q3_K, 600, 11264), (S.Q8_0, 1200, 14336), (S.Q8_0, 600, 14581)])
+    (3, 14336), (592, 13568), (593, 13500), (1190, 14592), (1777, 16128), (18352, 13312), (18353, 13312), (1184, 14336), (600, 16640)]] + [
+    (S.IQ4_XS, 4096, 13312), (S.Q3_K, 600, 11264)])
 def test_decode_pairs(t, rows, cols):
     w = S.gen_weight(t, rows, cols, seed=141)
     x = S.gen_acts(1, cols, seed=142)
@@ -606,3 +606,16 @@ def test_matmul_row_scales(t, rows, cols, m):
     assert np.all(np.isfinite(y))
     assert np.all(np.abs(y - ref) <= 7 * (2.0 ** -11 * np.sqrt(2 * sq) + np.sqrt(low)) + 1e-30)
     assert np.all(y[:, 17] == 0)
+
+
+# Chunks of several k-tiles through a ring that hands its stages back one by one: as many tiles as stages, one more, and many
+# rounds, with one, two and four groups of warps.
+@pytest.mark.parametrize("t,m,rows,cols", [(S.Q4_K, 1, 1184, 16384), (S.Q4_K, 1, 1200, 16384), (S.Q4_K, 2, 9600, 14336), (S.Q4_K, 4, 5000, 8448),
+                                           (S.Q8_0, 1, 9480, 12288), (S.Q6_K, 1, 9481, 8192), (S.Q6_K, 2, 4800, 12032), (S.Q4_0, 3, 4736, 8192),
+                                           (S.IQ4_XS, 1, 9480, 8448), (S.Q5_K, 4, 2400, 12288), (S.Q2_K, 2, 2400, 12288)])
+def test_decode_ring_by_tile(t, m, rows, cols):
+    w = S.gen_weight(t, rows, cols, seed=161)
+    x = S.gen_acts(m, cols, seed=162)
+    y = device_product(t, w, x, rows, cols, m)
+    assert_product(y, x, O.dequant_matrix(t, w, rows, cols), half=False)
+    assert np.array_equal(y, device_product(t, w, x, rows, cols, m))

@@ -12,6 +12,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_obj")
 LIB = os.path.join(HERE, "libqk_cuda.so")
+EXT = os.path.join(HERE, "_qk_torch.so")  # Python extension over torch's C++ objects (csrc/qk_torch.cpp)
 SOURCES = ["qk_api.cu", "qk_simple.cu", "qk_gemv_mma.cu", "qk_gemv_imma.cu", "qk_dec_q80.cu", "qk_dec_q40.cu",
            "qk_dec_iq4xs.cu", "qk_dec_q6k.cu", "qk_dec_q5k.cu", "qk_dec_q3k.cu", "qk_dec_q2k.cu", "qk_noalloc.cu", "qk_gemm_tc.cu", "qk_tc_q4k.cu", "qk_tc_q80.cu", "qk_tc_q40.cu", "qk_tc_q6k.cu", "qk_tc_iq4xs.cu", "qk_moe.cu", "qk_moe_q4k.cu", "qk_moe_q80.cu", "qk_moe_q40.cu", "qk_moe_iq4xs.cu", "qk_moe_q6k.cu", "qk_gather.cu", "qk_gguf.cu"]
 NVCC_FLAGS = [
@@ -25,6 +26,18 @@ def _newer(src_list, target):
         return True
     t = os.path.getmtime(target)
     return any(os.path.getmtime(s) > t for s in src_list)
+
+
+def _ext_command(src):
+    import sysconfig
+    import torch
+    base = os.path.dirname(torch.__file__)
+    inc = [sysconfig.get_paths()["include"], os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
+           os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")]
+    lib = os.path.join(base, "lib")
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{i}" for i in inc), src, "-o", EXT,
+            f"-L{lib}", f"-Wl,-rpath,{lib}", "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
 
 
 def build(verbose: bool = False, force: bool = False) -> str:
@@ -43,6 +56,9 @@ def build(verbose: bool = False, force: bool = False) -> str:
                 cmd.insert(1, "-Xptxas=-v")
                 print(" ".join(cmd), flush=True)
             jobs.append(cmd)
+    ext_src = os.path.join(CSRC, "qk_torch.cpp")
+    if force or _newer([ext_src], EXT):
+        jobs.append(_ext_command(ext_src))
     if jobs:  # the translation units are independent: compile them side by side
         from concurrent.futures import ThreadPoolExecutor
         with ThreadPoolExecutor(max_workers=min(len(jobs), os.cpu_count() or 1)) as pool:

@@ -10,7 +10,13 @@ import ctypes as C
 import numpy as np
 import torch
 
+from . import _lib
 from .kernels import Context, QuantError, default_context
+
+try:
+    from . import _qk_torch as _native  # what a call needs, without ctypes (csrc/qk_torch.cpp)
+except ImportError:  # not built, or for another torch: the same calls through Python
+    _native = None
 
 
 _F32 = torch.float32
@@ -29,6 +35,19 @@ def _stream_ptr(stream=None) -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
+_bound = None
+
+
+def _bound_lib():
+    """The library whose entry points the extension calls: the one that the package has loaded."""
+    global _bound
+    if _bound is None and _native is not None:
+        lib = _lib.load()
+        _native.bind(*(C.cast(f, C.c_void_p).value for f in (lib.qk_gemv_dev, lib.qk_gemm_dev)))
+        _bound = lib
+    return _bound
+
+
 class DeviceWeights:
     """Rows [row_begin, row_end) of a [n_rows x n_cols] GGUF-layout matrix, resident in HBM."""
 
@@ -42,7 +61,7 @@ class DeviceWeights:
         self.ctx.check(self.ctx.lib.qk_weights_upload(
             self.ctx.handle, tensor_type, C.c_void_p(data.ctypes.data), data.size, n_rows, n_cols,
             row_begin, row_end, C.byref(h)))
-        self.handle = h
+        self._own(h)
         self.rows, self.cols = row_end - row_begin, n_cols
         t, r, c, b = C.c_int(), C.c_size_t(), C.c_size_t(), C.c_size_t()
         self.ctx.lib.qk_weights_info(h, C.byref(t), C.byref(r), C.byref(c), C.byref(b))
@@ -61,14 +80,20 @@ class DeviceWeights:
         h = C.c_void_p()
         self.ctx.check(self.ctx.lib.qk_weights_upload_gguf(self.ctx.handle, gguf.handle, name.encode(), row_begin,
                                                            row_end, C.byref(h)))
-        self.handle, self.tensor_type = h, info.tensor_type
+        self._own(h)
+        self.tensor_type = info.tensor_type
         t, r, c, b = C.c_int(), C.c_size_t(), C.c_size_t(), C.c_size_t()
         self.ctx.lib.qk_weights_info(h, C.byref(t), C.byref(r), C.byref(c), C.byref(b))
         self.rows, self.cols, self.algo_bytes = r.value, c.value, b.value
         return self
 
+    def _own(self, handle):
+        self.handle, self._addr = handle, handle.value  # (_addr: 0 once freed)
+        self._call = _native if self.ctx.lib is _bound_lib() else None
+
     def free(self):
         if self.handle:
+            self._addr = 0
             self.ctx.lib.qk_weights_free(self.ctx.handle, self.handle)
             self.handle = None
 
@@ -87,6 +112,12 @@ class DeviceWeights:
 
     def gemv(self, x: torch.Tensor, y: torch.Tensor, stream=None) -> None:
         """y[0:rows] = W x (overwrites)."""
+        if self._call is not None:
+            st = self._call.gemv(self.ctx.addr, self._addr, self.cols, self.rows, x, y, stream)
+            if st == 0:
+                return
+            if st is not None:
+                self.ctx.check(st)
         if not (x.is_cuda and x.dtype is _F32 and x.is_contiguous() and x.numel() >= self.cols
                 and y.is_cuda and y.dtype is _F32 and y.is_contiguous() and y.numel() >= self.rows):
             self._chk(x, _F32, self.cols, "input")
@@ -100,6 +131,12 @@ class DeviceWeights:
              col_offset: int = 0, stream=None) -> None:
         """y[i, col_offset + j] = dot(W row j, x row i); y has row pitch ldy (default rows)."""
         ldy = self.rows if ldy is None else ldy
+        if self._call is not None:
+            st = self._call.gemm(self.ctx.addr, self._addr, self.cols, self.rows, x, y, m, ldy, col_offset, stream)
+            if st == 0:
+                return
+            if st is not None:
+                self.ctx.check(st)
         self._chk(x, _F32, m * self.cols, "input")
         self._chk(y, _F32, (m - 1) * ldy + col_offset + self.rows if m else 0, "output")
         ctx = self.ctx

@@ -77,10 +77,12 @@ class Context:
         if st != 0:
             raise QuantError(st, f"qk_init(device={device}) failed: no usable sm_100 CUDA device")
         self.handle = h
+        self.addr = h.value  # the handle as a number, 0 once closed
         self.device = device
 
     def close(self):
         if self.handle:
+            self.addr = 0
             self.lib.qk_shutdown(self.handle)
             self.handle = None
 

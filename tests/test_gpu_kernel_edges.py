@@ -619,3 +619,60 @@ def test_decode_ring_by_tile(t, m, rows, cols):
     y = device_product(t, w, x, rows, cols, m)
     assert_product(y, x, O.dequant_matrix(t, w, rows, cols), half=False)
     assert np.array_equal(y, device_product(t, w, x, rows, cols, m))
+
+
+# What DeviceWeights.gemv / .gemm take and refuse is the same with the extension and without it.
+@pytest.mark.parametrize("native", [True, False])
+def test_device_call_arguments(native, monkeypatch):
+    import torch
+    from oxillama_b200 import device
+    from oxillama_b200.kernels import QuantError
+    assert device._native is not None, "the extension is not built"
+    rows, cols = 64, 512
+    w = S.gen_weight(S.Q4_K, rows, cols, seed=171)
+    dw = device.DeviceWeights(S.Q4_K, w, rows, cols)
+    if not native:
+        dw._call = None
+    xn = S.gen_acts(3, cols, seed=172)
+    wd = O.dequant_matrix(S.Q4_K, w, rows, cols)
+    x = torch.from_numpy(xn).cuda()
+
+    class Sub(torch.Tensor):
+        pass
+
+    side = torch.cuda.Stream()
+    for xs, stream in ((x, None), (x.clone().requires_grad_(), None), (torch.nn.Parameter(x.clone()), None), (x.clone().as_subclass(Sub), None),
+                       (x, side)):
+        y = torch.full((3, rows), float("nan"), device="cuda")
+        torch.cuda.synchronize()
+        dw.gemv(xs[0].detach() if xs.requires_grad else xs[0], y[0], stream=stream)
+        torch.cuda.synchronize()
+        assert_product(y[:1].cpu().numpy(), xn[:1], wd, half=False)
+        dw.gemm(xs, y, 3, stream=stream)
+        torch.cuda.synchronize()
+        assert_product(y.cpu().numpy(), xn, wd, half=False)
+    wide = torch.full((3, 200), 7.0, device="cuda")  # a block of columns of a wider result; sizes as numpy gives them
+    dw.gemm(x, wide, np.int64(3), ldy=np.int32(200), col_offset=100)
+    got = wide.cpu().numpy()
+    assert_product(got[:, 100:164], xn, wd, half=False)
+    assert np.all(got[:, :100] == 7) and np.all(got[:, 164:] == 7)
+    y = torch.empty(3, rows, device="cuda")
+    for bad in (x.double(), x.cpu(), x.t(), x[:, ::2], x.half()):
+        with pytest.raises(TypeError):
+            dw.gemv(bad, y)
+        with pytest.raises(TypeError):
+            dw.gemm(bad, y, 3)
+    with pytest.raises(TypeError):
+        dw.gemv(x, y.t())
+    with pytest.raises(QuantError):
+        dw.gemv(x[0, :500].contiguous(), y)
+    with pytest.raises(QuantError):
+        dw.gemm(x, y, 4)
+    with pytest.raises(QuantError):
+        dw.gemm(x, y, 3, ldy=rows - 1)
+    with pytest.raises(AttributeError):
+        dw.gemv(xn, y)
+    dw.gemm(x, y, 0)
+    dw.free()
+    with pytest.raises(QuantError):
+        dw.gemv(x, y)

@@ -99,6 +99,8 @@ struct DecQ80 {
   static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
   static constexpr uint32_t PAIR_COLS = 0;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
   static constexpr uint32_t BY_TILE_M = 4;  // most rows with which the stages of long chunks are handed back one by one
+  static constexpr uint32_t XCH = 0;       // shared memory per compute warp for what its lanes exchange
+  static constexpr bool HAS_ONE = false;   // a variant of the policy for one row
   // digit order inside a 32-column block: the lane's 8 bytes are columns 4 tig .. + 3 and
   // 16 + 4 tig .. + 3, the two 4-byte pieces of its A fragment (bytes 4 tig of both 16-byte granules)
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
@@ -172,6 +174,8 @@ struct DecQ40 {
   static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
   static constexpr uint32_t PAIR_COLS = 0;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
   static constexpr uint32_t BY_TILE_M = 4;  // most rows with which the stages of long chunks are handed back one by one
+  static constexpr uint32_t XCH = 0;       // shared memory per compute warp for what its lanes exchange
+  static constexpr bool HAS_ONE = false;   // a variant of the policy for one row
   // The lane's word (bytes 4 tig .. + 3 of the block) holds elements 8 tig .. + 7: low
   // nibbles the even ones, high nibbles the odd ones.  Digits go evens first, then odds,
   // inside every group of 8 columns.
@@ -255,6 +259,8 @@ struct DecIQ4XS {
   static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
   static constexpr uint32_t PAIR_COLS = 13312;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
   static constexpr uint32_t BY_TILE_M = 1;  // the same (two rows, bound by issue: 4096 x 14336 16.2 -> 16.6 us, a layer of experts 156 -> 160)
+  static constexpr uint32_t XCH = 0;       // shared memory per compute warp for what its lanes exchange
+  static constexpr bool HAS_ONE = false;   // a variant of the policy for one row
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
                                                       uint32_t w1, uint32_t w2) {
     store_digits_natural(row_img, PS, e0, w0, w1, w2);
@@ -346,12 +352,16 @@ struct DecIQ4XS {
 // reference/q6_k.rs:77-172.  Element (half G, strip k, l) of a super-block: column
 // 128 G + 32 k + l, q = (ql[64 G + 32 (k & 1) + l] nibble (k >> 1)) | (qh[32 G + l] bits 2k, 2k+1) << 4,
 // value d sc[8 G + 2 k + l / 16] (q - 32).
+struct DecQ6KOne;
 struct DecQ6K {
   static constexpr uint32_t COLB = 1680, XSB = 16;
   static constexpr bool HAS_DUAL = false, HAS_PEER = true;
   static constexpr bool ANY_DEPTH = true;  // ring depths that are no multiple of the groups (ring_is_deep)
-  static constexpr uint32_t PAIR_COLS = 13312;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
+  static constexpr uint32_t PAIR_COLS = 0;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
   static constexpr uint32_t BY_TILE_M = 4;  // most rows with which the stages of long chunks are handed back one by one
+  static constexpr uint32_t XCH = 0;       // shared memory per compute warp for what its lanes exchange
+  static constexpr bool HAS_ONE = true;    // a variant of the policy for one row
+  using One = DecQ6KOne;
   static constexpr int MAX_M = 2;  // three rows and up spill heavily (twelve weight words and sixteen fragments per column)
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
                                                       uint32_t w1, uint32_t w2) {
@@ -469,6 +479,62 @@ struct DecQ6K {
   }
   __device__ static __forceinline__ float finish(const float (&a)[3], const Lane &LN) {
     return LN.kD * (a[0] + a[1]) - a[2];
+  }
+};
+
+// One row.  Where the SM clock is down at the power limit (the output head: 1455 MHz) the kernel is bound by its instructions and
+// by the integer MMAs beside a stream at the memory's rate.  The same arithmetic in the same order as above, but the strips'
+// scales go to the quad's lanes through shared memory, one store and four loads instead of sixteen shuffles: 128256 x 4096
+// 76.4 -> 74.2 us a call sustained, 14336 x 4096 9.9 -> 9.7, 8192 x 8192 13.8 -> 13.0.  (An MMA of k = 32 a block with the unused
+// half of B zero, which puts both strips' sums in neighbouring registers for packed additions and multiply-adds, was slower:
+// 14336 x 4096 9.9 -> 12.1.  The integer MMAs take their time by k, whatever is in them.)
+struct DecQ6KOne : DecQ6K {
+  static constexpr int MAX_M = 1;
+  static constexpr bool HAS_PEER = false, HAS_ONE = false;
+  static constexpr uint32_t PAIR_COLS = 13312, XCH = 512;
+  struct Lane : DecQ6K::Lane {
+    uint32_t put, get;  // where this lane's scales go; where the row's first four are (four 4 q on: get ^ 16 q)
+    // [row][four 16-byte chunks, their order turned by row / 2]: no conflicts for either
+    __device__ __forceinline__ void set_exchange(uint32_t at, uint32_t lane) {
+      const uint32_t g = lane >> 2, tig = lane & 3;
+      get = at + g * 64 + ((g >> 1) & 3u) * 16, put = get ^ (tig * 16);
+    }
+  };
+  template <int M>
+  __device__ static __forceinline__ void compute(const Data<M> &D, const Lane &LN, float (&acc)[M][3]) {
+    const float d = h2f_bits(D.dd);
+    float ds[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) ds[j] = d * (float)(int)(signed char)((D.sc >> (8 * j)) & 0xFFu);
+    const float4 x0 = D.xs[0][0], x1 = D.xs[0][1];
+    __syncwarp();  // the scales of the span before have been read
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(LN.put), "f"(ds[0] * x0.x), "f"(ds[1] * x0.x), "f"(ds[2] * x1.x), "f"(ds[3] * x1.x) : "memory");
+    __syncwarp();
+    float z = ds[0] * x0.z;
+    z = fmaf(ds[1], x0.w, z), z = fmaf(ds[2], x1.z, z), z = fmaf(ds[3], x1.w, z);
+    acc[0][2] = fmaf(32.f, z, acc[0][2]);
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const float4 t = lds128f(LN.get ^ (16u * q));
+      float c[2][4];
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int i = 2 * q + h, G = i >> 2, k = i & 3;
+        uint32_t a[2];
+#pragma unroll
+        for (int is = 0; is < 2; is++) {
+          const uint32_t lw = D.ql[G * 4 + (k & 1) * 2 + is], hw = D.qh[G * 2 + is];
+          const uint32_t lo = (k >> 1) ? (lw >> 4) : lw;
+          const uint32_t hi = k == 0 ? (hw << 4) : k == 1 ? (hw << 2) : k == 2 ? hw : (hw >> 2);
+          a[is] = (lo & 0x0F0F0F0Fu) | (hi & 0x30303030u);
+        }
+        mma_u8s8_k16(c[h], a[0], a[1], word(D.b[0][G], k));
+      }
+      acc[0][0] = fmaf(t.x, c[0][0] - MMA_BIAS, acc[0][0]);
+      acc[0][1] = fmaf(t.y, c[0][3] - MMA_BIAS, acc[0][1]);
+      acc[0][0] = fmaf(t.z, c[1][0] - MMA_BIAS, acc[0][0]);
+      acc[0][1] = fmaf(t.w, c[1][3] - MMA_BIAS, acc[0][1]);
+    }
   }
 };
 

@@ -29,6 +29,8 @@ struct DecQ5K {
   static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
   static constexpr uint32_t PAIR_COLS = 12288;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
   static constexpr uint32_t BY_TILE_M = 4;  // most rows with which the stages of long chunks are handed back one by one
+  static constexpr uint32_t XCH = 0;       // shared memory per compute warp for what its lanes exchange
+  static constexpr bool HAS_ONE = false;   // a variant of the policy for one row
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
                                                       uint32_t w1, uint32_t w2) {
     store_digits_natural(row_img, PS, e0, w0, w1, w2);
@@ -169,6 +171,8 @@ struct DecQ3K {
   static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
   static constexpr uint32_t PAIR_COLS = 11008;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
   static constexpr uint32_t BY_TILE_M = 4;  // most rows with which the stages of long chunks are handed back one by one
+  static constexpr uint32_t XCH = 0;       // shared memory per compute warp for what its lanes exchange
+  static constexpr bool HAS_ONE = false;   // a variant of the policy for one row
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
                                                       uint32_t w1, uint32_t w2) {
     store_digits_natural(row_img, PS, e0, w0, w1, w2);
@@ -249,6 +253,8 @@ struct DecQ2K {
   static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
   static constexpr uint32_t PAIR_COLS = 0;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
   static constexpr uint32_t BY_TILE_M = 4;  // most rows with which the stages of long chunks are handed back one by one
+  static constexpr uint32_t XCH = 0;       // shared memory per compute warp for what its lanes exchange
+  static constexpr bool HAS_ONE = false;   // a variant of the policy for one row
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
                                                       uint32_t w1, uint32_t w2) {
     store_digits_natural(row_img, PS, e0, w0, w1, w2);

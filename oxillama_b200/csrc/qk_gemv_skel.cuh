@@ -73,6 +73,7 @@ struct SmemMma {
   uint32_t empty;                // chunks of several k-tiles: a stage's tile has been used (one arrival per warp of the group)
   uint32_t prog;                 // chunks the reducer warp has read so far (one word, polled by the producer warp)
   uint32_t issued;               // DEEP: tiles issued so far (one word, polled by the compute warps)
+  uint32_t xch;                  // F::XCH bytes per compute warp
   uint32_t pbar, pair;           // PAIR: per chunk, the mbarrier and the 8 x M sums that the other CTA sends
   uint32_t red, ximg, stage;
   uint32_t PS;         // digit plane stride, bytes
@@ -658,6 +659,7 @@ __global__ void __launch_bounds__((CW + 2 + (MODE == 1 ? 1 : 0)) * 32, 1)
   const uint32_t g = lane >> 2, tig = lane & 3;
   typename F::Lane LN;  // this lane's constants: which bytes, digits and scales it handles
   LN.init(lane, wl, sbase + S.ximg, S.PS, S.xs_off, Kp);
+  if constexpr (F::XCH != 0) LN.set_exchange(sbase + S.xch + warp * F::XCH, lane);
 
   pdl_wait();  // x may be the previous kernel's output; y may be read or written by it
   QK_STAMP(warp == 0, 121);
@@ -758,7 +760,8 @@ struct PlanMma {
 };
 
 // xsb: bytes per 32-column block in the activation scale table (F::XSB).  pair: for CTAs that take half of K each.
-inline bool make_plan_mma(const QkLayout &full, uint32_t m, PlanMma *P, uint32_t xsb, bool pair = false) {
+// xch: bytes per compute warp for what its lanes exchange.
+inline bool make_plan_mma(const QkLayout &full, uint32_t m, PlanMma *P, uint32_t xsb, bool pair = false, uint32_t xch = 0) {
   if (full.nb == 0 || full.chunks == 0) return false;  // nothing to stream: the callers handle empty shapes
   if (full.nb * full.bs % 256u) return false;          // the kernels walk K in spans of 256 columns
   QkLayout L = full;
@@ -783,6 +786,7 @@ inline bool make_plan_mma(const QkLayout &full, uint32_t m, PlanMma *P, uint32_t
   S.pbar = S.pair = off;
   if (pair) off += PAIR_CHUNKS * 8, S.pair = off, off += PAIR_CHUNKS * 8 * m * 4;
   off = (off + 127u) & ~127u;
+  S.xch = off, off += MAX_CW * xch;
   S.red = off, off += MAX_SLOT * MAX_CW * m * 8 * 4;
   off = (off + 127u) & ~127u;
   S.PS = Kp + 64;
@@ -924,7 +928,7 @@ template <class F>
 inline bool pair_pays(const QkLayout &L, int sm_count, PlanMma *P) {
   const uint32_t sms = (uint32_t)sm_count, pairs = sms / 2;
   return L.nb * L.bs >= F::PAIR_COLS && L.chunks <= PAIR_CHUNKS * pairs && 2 * ((L.chunks + sms - 1) / sms) > (L.chunks + pairs - 1) / pairs &&
-         make_plan_mma(L, 1, P, F::XSB, true);
+         make_plan_mma(L, 1, P, F::XSB, true, F::XCH);
 }
 
 template <class F, int M>
@@ -989,6 +993,14 @@ cudaError_t launch_mma_m(const QkLayout &L, const uint8_t *W, const float *x, fl
 }
 
 
+// Whether one row goes to the format's variant for it: where every CTA splits the activations itself.
+template <class F>
+inline bool one_pays(const QkLayout &L, int sm_count, PlanMma *P) {
+  using O = typename F::One;
+  PlanMma pair;
+  return (L.nb * L.bs <= QK_SPLIT_IN_CTA || pair_pays<O>(L, sm_count, &pair)) && make_plan_mma(L, 1, P, O::XSB, false, O::XCH);
+}
+
 // The public faces of one format's kernels.
 template <class F>
 bool supported(const QkLayout &L, uint32_t m) {
@@ -1009,6 +1021,10 @@ cudaError_t launch(const QkLayout &L, const uint8_t *tiled, const float *x, floa
                    unsigned *status, unsigned char *scratch, int sm_count, cudaStream_t s, const QkPeers *peers,
                    const uint8_t *tiled2 = nullptr, bool host_x = false) {
   PlanMma P;
+  if constexpr (F::HAS_ONE) {
+    if (m == 1 && !peers && !tiled2 && !host_x && one_pays<F>(L, sm_count, &P))
+      return launch_mma_m<typename F::One, 1>(L, tiled, x, y, ldy, status, scratch, sm_count, P, s, nullptr, nullptr, false);
+  }
   if (!make_plan_mma(L, m, &P, F::XSB)) return cudaErrorInvalidConfiguration;
   if (m < 1 || m > (uint32_t)F::MAX_M) return cudaErrorInvalidConfiguration;
   if ((tiled2 && (!F::HAS_DUAL || peers)) || (peers && !F::HAS_PEER)) return cudaErrorInvalidConfiguration;

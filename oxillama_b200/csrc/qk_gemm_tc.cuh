@@ -562,12 +562,12 @@ struct ConvArgs {
   const int *counts, *lists;      // grouped: live rows per group; rows to gather (row t of group e = x[lists[e][t] / list_div])
   uint32_t m, cols, Kp, n_zero, cap, list_stride, list_div, n_act;
 };
-// Which row a conversion CTA takes, as group * cap + place in the group: without counts the CTA's own number, with them the
-// blockIdx.x-th live one.  (A CTA per reserved row, most of which left at once, held up the live ones, for which silu(g) * u
+// Which row conversion CTA (or cluster) i takes, as group * cap + place in the group: without counts i itself, with them the
+// i-th live one.  (A CTA per reserved row, most of which left at once, held up the live ones, for which silu(g) * u
 // has three places on an SM: 16 experts of 1024 x 2048 by 300 tokens, top 2, 94.6 -> 78.7 us, of it some 4 from
 // qk_moe_group_plan_kernel.)
-__device__ __forceinline__ bool conv_row(const ConvArgs &A, uint32_t &t) {
-  t = blockIdx.x;
+__device__ __forceinline__ bool conv_row(const ConvArgs &A, uint32_t i, uint32_t &t) {
+  t = i;
   if (!A.counts) return true;
   const uint32_t lane = threadIdx.x & 31, c = lane < A.n_act ? min((uint32_t)__ldg(A.counts + lane), A.cap) : 0u;
   uint32_t end = c;
@@ -576,10 +576,10 @@ __device__ __forceinline__ bool conv_row(const ConvArgs &A, uint32_t &t) {
     const uint32_t v = __shfl_up_sync(0xffffffffu, end, o);
     if (lane >= (uint32_t)o) end += v;
   }
-  const uint32_t mine = __ballot_sync(0xffffffffu, lane < A.n_act && blockIdx.x < end);
+  const uint32_t mine = __ballot_sync(0xffffffffu, lane < A.n_act && i < end);
   if (!mine) return false;
   const uint32_t e = __ffs(mine) - 1;
-  t = e * A.cap + blockIdx.x - __shfl_sync(0xffffffffu, end - c, e);
+  t = e * A.cap + i - __shfl_sync(0xffffffffu, end - c, e);
   return true;
 }
 
@@ -645,7 +645,7 @@ __global__ void __launch_bounds__(CT, CT == 256 ? 6 : 1) qk_x16_kernel(const Con
   if (blockIdx.x == 0)
     for (uint32_t i = threadIdx.x; i < A.n_zero; i += CT) A.zero[i] = 0u;
   uint32_t t;
-  if (!conv_row(A, t)) return;  // (rows past the live ones: never stored, their values do not matter)
+  if (!conv_row(A, blockIdx.x, t)) return;  // (rows past the live ones: never stored, their values do not matter)
   const float *xr = A.x + (uint64_t)t * A.cols, *ur = A.x2 + (uint64_t)t * A.cols;
   if (A.lists) xr = A.x + (uint64_t)(A.lists[(uint64_t)(t / A.cap) * A.list_stride + t % A.cap] / (int)A.list_div) * A.cols;
   const bool vec = (A.cols & 3u) == 0 && (((uintptr_t)xr | (GLU ? (uintptr_t)ur : 0u)) & 15u) == 0;
@@ -692,22 +692,27 @@ __global__ void __launch_bounds__(CT, CT == 256 ? 6 : 1) qk_x16_kernel(const Con
 
 // silu(x) * x2 rows through shared memory: 512 threads of 40 registers and a row of 14336 columns leave room
 // for three CTAs on an SM, where the form above holds one (78 registers) that loads, computes and stores in
-// turn.  Up to one row per SM 1024 threads share it.  14336 columns by 512 rows: 27 -> 9 us.
-template <int T, int CT>
+// turn (14336 columns by 512 rows: 27 -> 9 us).  CL CTAs, a cluster, share a row and meet once for its largest magnitude:
+// exp and the rounded division keep one SM busy for 2 us with a row of 14336.  Eight or four CTAs a row as long as they are no
+// more than the SMs, twice as many where rows are long; above, one CTA of 1024 threads a row, from a row per SM on of 512
+// (us, a feed-forward block of 4096 x 14336, one CTA a row / clusters: by 8 40.9 / 39.9, by 19 43.0 / 41.6, by 37 44.7 / 43.8, by 48
+// 44.6 / 43.7, by 74 52.2 / 52.5; two CTAs a row by 64 45.8 / 47.2, by 512 192 / 196; 2048 x 5632 by 37 23.8 / 23.2, by 50 23.5 / 23.6).
+template <int T, int CT, int CL>
 __global__ void __launch_bounds__(CT, CT == 512 ? 3 : 1) qk_glu16_kernel(const ConvArgs A) {
   extern __shared__ __align__(16) float glu_row[];
-  __shared__ float red[CT / 32];
+  __shared__ float red[CT / 32], parts[CL];
   pdl_launch_dependents();
   pdl_wait();
   if (blockIdx.x == 0)
     for (uint32_t i = threadIdx.x; i < A.n_zero; i += CT) A.zero[i] = 0u;
   uint32_t t;
-  if (!conv_row(A, t)) return;
+  if (!conv_row(A, blockIdx.x / CL, t)) return;
+  const uint32_t rank = blockIdx.x % CL, per = (A.Kp / 256u + CL - 1) / CL * 256u, k0 = min(rank * per, A.Kp), k1 = min(k0 + per, A.Kp);
   const float *xr = A.x + (uint64_t)t * A.cols, *ur = A.x2 + (uint64_t)t * A.cols;
   const bool vec = (A.cols & 3u) == 0 && (((uintptr_t)xr | (uintptr_t)ur) & 15u) == 0;
   float amax = 0.f;
 #pragma unroll 2
-  for (uint32_t k = threadIdx.x * 4; k < A.Kp; k += CT * 4) {
+  for (uint32_t k = k0 + threadIdx.x * 4; k < k1; k += CT * 4) {
     float4 g = make_float4(0.f, 0.f, 0.f, 0.f), u = g;
     if (vec && k < A.cols) {
       g = __ldg(reinterpret_cast<const float4 *>(xr + k)), u = __ldg(reinterpret_cast<const float4 *>(ur + k));
@@ -719,7 +724,7 @@ __global__ void __launch_bounds__(CT, CT == 512 ? 3 : 1) qk_glu16_kernel(const C
     }
     const float4 h = make_float4(silu_mul(g.x, u.x), silu_mul(g.y, u.y), silu_mul(g.z, u.z), silu_mul(g.w, u.w));
     amax = fmaxf(fmaxf(fmaxf(amax, fabsf(h.x)), fmaxf(fabsf(h.y), fabsf(h.z))), fabsf(h.w));
-    *reinterpret_cast<float4 *>(glu_row + k) = h;
+    *reinterpret_cast<float4 *>(glu_row + (k - k0)) = h;
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
@@ -728,11 +733,17 @@ __global__ void __launch_bounds__(CT, CT == 512 ? 3 : 1) qk_glu16_kernel(const C
   amax = red[threadIdx.x % (CT / 32)];
 #pragma unroll
   for (int o = CT / 64; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  if (CL > 1) {
+    if (threadIdx.x < CL) st_cluster(smem_u32(&parts[rank]), threadIdx.x, amax);
+    cluster_sync();
+#pragma unroll
+    for (int c = 0; c < CL; c++) amax = fmaxf(amax, parts[c]);
+  }
   const float scale = conv_scale(amax), inv = 1.f / scale;  // a power of two: exact
-  if (threadIdx.x == 0) A.scales[t] = scale;
-  for (uint32_t c = threadIdx.x; c < A.Kp / 8; c += CT) {
+  if (threadIdx.x == 0 && rank == 0) A.scales[t] = scale;
+  for (uint32_t c = k0 / 8 + threadIdx.x; c < k1 / 8; c += CT) {
     const uint32_t ka = T == QK_T_Q4_K ? (c >> 3) * 64 + (c & 7u) * 4 : c * 8, kb = T == QK_T_Q4_K ? ka + 32 : ka + 4;
-    const float4 fa = *reinterpret_cast<const float4 *>(glu_row + ka), fb = *reinterpret_cast<const float4 *>(glu_row + kb);
+    const float4 fa = *reinterpret_cast<const float4 *>(glu_row + (ka - k0)), fb = *reinterpret_cast<const float4 *>(glu_row + (kb - k0));
     const float a[4] = {fa.x, fa.y, fa.z, fa.w}, b[4] = {fb.x, fb.y, fb.z, fb.w};
     float v[8];
     conv_order<T>(a, b, v);
@@ -1428,6 +1439,22 @@ cudaError_t launch_main(const TcPlan &P, const TcArgs &A, __half *x16, const QkT
   return cudaLaunchKernelEx(&cfg, kern, A, M);
 }
 
+template <int T, int CT, int CL>
+cudaError_t launch_glu16(const ConvArgs &C, uint32_t rows, cudaStream_t s) {
+  static QkPerDevice attr_set;
+  if (attr_set.first()) {
+    cudaError_t e = cudaFuncSetAttribute(qk_glu16_kernel<T, CT, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GLU_SMEM);
+    if (e != cudaSuccess) return attr_set.reset(), e;
+  }
+  cudaLaunchAttribute at[2] = {pdl_attr(), {}};
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = CL, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(rows * CL), cfg.blockDim = dim3(CT), cfg.dynamicSmemBytes = (C.Kp / 256u + CL - 1) / CL * 1024u, cfg.stream = s;
+  cfg.attrs = at, cfg.numAttrs = CL > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, qk_glu16_kernel<T, CT, CL>, C);
+}
+
 template <int T>
 cudaError_t launch_fmt(const QkTcCall &c, unsigned *status, unsigned char *scratch, int sm_count, cudaStream_t s) {
   const QkLayout &L = *c.L;
@@ -1452,15 +1479,11 @@ cudaError_t launch_fmt(const QkTcCall &c, unsigned *status, unsigned char *scrat
   c0.gridDim = dim3(c.counts && c.live < all_rows ? c.live : all_rows), c0.blockDim = dim3(narrow ? 256 : 512), c0.stream = s, c0.attrs = &at, c0.numAttrs = 1;
   cudaError_t e;
   if (c.x2 && !c.lists && Kp * 4 <= GLU_SMEM) {
-    static QkPerDevice attr_set;
-    if (attr_set.first()) {
-      e = cudaFuncSetAttribute(qk_glu16_kernel<T, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GLU_SMEM);
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(qk_glu16_kernel<T, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GLU_SMEM);
-      if (e != cudaSuccess) return attr_set.reset(), e;
-    }
-    const bool few = !c.counts && c0.gridDim.x <= (uint32_t)sm_count;
-    c0.blockDim = dim3(few ? 1024 : 512), c0.dynamicSmemBytes = Kp * 4;
-    e = few ? cudaLaunchKernelEx(&c0, qk_glu16_kernel<T, 1024>, C) : cudaLaunchKernelEx(&c0, qk_glu16_kernel<T, 512>, C);
+    const uint32_t rows = c0.gridDim.x, sms = (uint32_t)sm_count, room = Kp > 8192 ? 2 * sms : sms;
+    if (!c.counts && rows * 8 <= room) e = launch_glu16<T, 512, 8>(C, rows, s);
+    else if (!c.counts && rows * 4 <= room) e = launch_glu16<T, 512, 4>(C, rows, s);
+    else if (!c.counts && rows <= sms) e = launch_glu16<T, 1024, 1>(C, rows, s);
+    else e = launch_glu16<T, 512, 1>(C, rows, s);
   } else if (c.x2) {
     c0.blockDim = dim3(512);
     e = cudaLaunchKernelEx(&c0, qk_x16_kernel<T, true, 512, 4>, C);

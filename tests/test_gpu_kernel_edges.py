@@ -676,3 +676,27 @@ def test_device_call_arguments(native, monkeypatch):
     dw.free()
     with pytest.raises(QuantError):
         dw.gemv(x, y)
+
+
+# silu(g) * u by clusters of eight and four CTAs a row and by one: the last batch of each and the first of the next (148 SMs;
+# rows above 8192 columns twice as many), rows with fewer super-blocks than CTAs, parts of unequal length, a ragged last block.
+# The bound: three chained products, each within 1e-3 of its largest value.
+@pytest.mark.parametrize("t,hidden,inter,ms", [(S.Q4_K, 256, 512, (5, 18, 19, 37, 38)), (S.Q8_0, 256, 2336, (18, 37)), (S.Q6_K, 256, 8448, (37, 38, 74, 75)),
+                                               (S.IQ4_XS, 256, 4864, (18, 19)), (S.Q4_0, 512, 1312, (9, 30))])
+def test_ffn_conversion_by_clusters(t, hidden, inter, ms):
+    import torch
+    from oxillama_b200.device import DeviceWeights, check_device_status, ffn
+    shapes = [(inter, hidden), (inter, hidden), (hidden, inter)]
+    ws = [S.gen_weight(t, r, c, seed=181, stream=i, d_range=(1e-3, 3e-3)) for i, (r, c) in enumerate(shapes)]
+    g, u, d = (O.dequant_matrix(t, w, r, c).astype(np.float64) for w, (r, c) in zip(ws, shapes))
+    dw = [DeviceWeights(t, w, r, c) for w, (r, c) in zip(ws, shapes)]
+    for m in ms:
+        x = S.gen_acts(m, hidden, seed=182) * np.float32(0.25)
+        hg = x.astype(np.float64) @ g.T
+        ref = (hg / (1 + np.exp(-hg)) * (x.astype(np.float64) @ u.T)) @ d.T
+        y = torch.full((m, hidden), float("nan"), device="cuda")
+        ffn(*dw, torch.from_numpy(x).cuda(), y, m)
+        check_device_status()
+        assert np.abs(y.cpu().numpy() - ref).max() <= 3e-3 * np.abs(ref).max()
+    for w in dw:
+        w.free()

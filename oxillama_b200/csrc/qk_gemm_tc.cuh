@@ -553,7 +553,10 @@ struct WFmt<QK_T_IQ4_XS> {  // super-block of 256: f16 d, scales_h, scales_l[4],
 // (where the crossing was measured): 37 rows 11.1 (apart) against 11.5 us (beside), 64 rows 13.8 against 12.6, 128
 // rows 19.7 against 18.3.  Short rows keep few of 512 threads busy, so the smaller CTAs pay for Q6_K as well, whose
 // matmul stays at 80 registers: 4096 x 4096 by 64 rows 15.6 -> 13.7 us, by 2048 66.8 -> 62.2, 300 x 256 by 4096 27.0 -> 16.9.  And for
-// the experts of a mixture, whose rows are mostly not live: 16 experts of 1024 x 1024, 900 tokens top 2, 156 -> 129.
+// the experts of a mixture, whose rows are mostly not live: 16 experts of 1024 x 1024, 900 tokens top 2, 156 -> 129.  Beside gate
+// and up together (80 registers) the smaller CTAs pay from two rows an SM on, six of them being on an SM where there are three of
+// 512: feed-forward blocks of 4096 x 14336 by 200 94.5 -> 98.8, by 700 243.5 -> 238.8, 2048 x 5632 by 512 59.0 -> 57.3, by 2048
+// 176.3 -> 168.0.
 struct ConvArgs {
   const float *x, *x2;
   __half *out;
@@ -1468,11 +1471,11 @@ cudaError_t launch_fmt(const QkTcCall &c, unsigned *status, unsigned char *scrat
   C.x = c.x, C.x2 = c.x2, C.out = x16, C.scales = scales, C.zero = cnt, C.n_zero = (uint32_t)sm_count * 2;
   C.counts = c.counts, C.lists = c.lists, C.m = c.m, C.cols = L.cols, C.Kp = Kp, C.cap = c.xcap;
   C.list_stride = c.list_stride, C.list_div = c.list_div ? c.list_div : 1u, C.n_act = c.n_act;
-  const bool narrow = (c.counts || (c.n == 1 && c.m >= 64)) && Kp <= 4096;
+  const bool narrow = (c.counts || c.m >= (c.n == 1 ? 64u : 2 * (uint32_t)sm_count)) && Kp <= 4096;
   // Single CTAs beside the conversion (72 registers).  Q6_K only where the conversion has more rows than a tile: its
   // expansion wants the 80 (us, 80 / 72 registers: 4096 x 4096 by 80 16.5 / 14.4, by 160 17.1 / 15.4; 14336 x 4096 by
   // 64 16.1 / 16.9).
-  const bool beside = narrow && !c.counts && (T != QK_T_Q6_K || c.m > 64);
+  const bool beside = narrow && c.n == 1 && !c.counts && (T != QK_T_Q6_K || c.m > 64);
   cudaLaunchAttribute at = pdl_attr();
   cudaLaunchConfig_t c0 = {};
   const uint32_t all_rows = c.counts || c.n_act > 1 ? c.n_act * c.xcap : c.m;

@@ -33,7 +33,7 @@ struct DecQ4K {
   static constexpr uint32_t PAIR_COLS = 0;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
   static constexpr uint32_t BY_TILE_M = 4;  // most rows with which the stages of long chunks are handed back one by one
   static constexpr uint32_t XCH = 0;       // shared memory per compute warp for what its lanes exchange
-  static constexpr bool HAS_ONE = false;   // a variant of the policy for one row
+  static constexpr bool HAS_ONE = false;   // a variant of the policy for one row (of the decode kernel; the experts' has it)
 
   // digit planes in natural column order
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
@@ -108,21 +108,24 @@ struct DecQ4K {
     }
   }
 
-  // acc[m] = {low-nibble sums, 16 x high-nibble sums (scale pre-divided), min terms}
-  template <int M>
-  __device__ static __forceinline__ void compute(const Data<M> &D, const Lane &LN, float (&acc)[M][3]) {
-    // this lane decodes sub-blocks (2 tig, 2 tig + 1) of row g's header:
-    // reference/q4_k.rs:27-49 on four 6-bit fields at a time, then byte -> f32 by
-    // dropping the byte into the mantissa of 2^23
-    const uint4 h = D.h;
+  // This lane's part of row g's header, sub-blocks 2 tig and 2 tig + 1:
+  // reference/q4_k.rs:27-49 on four 6-bit fields at a time, then byte -> f32 by
+  // dropping the byte into the mantissa of 2^23
+  __device__ static __forceinline__ void header(const uint4 &h, const Lane &LN, float &ds0, float &ds1, float &dm0, float &dm1) {
     const float d = h2f_bits(h.x), dmin = h2f_bits(h.x >> 16);
     const uint32_t scw = ((LN.hi_half ? h.w : h.y) & LN.m1) | ((h.y >> 2) & LN.m2);
     const uint32_t mnw = ((LN.hi_half ? (h.w >> 4) : h.z) & LN.m1) | ((h.z >> 2) & LN.m2);
-    const float ds0 = d * (__int_as_float(__byte_perm(scw, 0x4B000000u, LN.sel0)) - 8388608.f);
-    const float ds1 =
-        d * (1.f / 16.f) * (__int_as_float(__byte_perm(scw, 0x4B000000u, LN.sel1)) - 8388608.f);
-    const float dm0 = dmin * (__int_as_float(__byte_perm(mnw, 0x4B000000u, LN.sel0)) - 8388608.f);
-    const float dm1 = dmin * (__int_as_float(__byte_perm(mnw, 0x4B000000u, LN.sel1)) - 8388608.f);
+    ds0 = d * (__int_as_float(__byte_perm(scw, 0x4B000000u, LN.sel0)) - 8388608.f);
+    ds1 = d * (1.f / 16.f) * (__int_as_float(__byte_perm(scw, 0x4B000000u, LN.sel1)) - 8388608.f);
+    dm0 = dmin * (__int_as_float(__byte_perm(mnw, 0x4B000000u, LN.sel0)) - 8388608.f);
+    dm1 = dmin * (__int_as_float(__byte_perm(mnw, 0x4B000000u, LN.sel1)) - 8388608.f);
+  }
+
+  // acc[m] = {low-nibble sums, 16 x high-nibble sums (scale pre-divided), min terms}
+  template <int M>
+  __device__ static __forceinline__ void compute(const Data<M> &D, const Lane &LN, float (&acc)[M][3]) {
+    float ds0, ds1, dm0, dm1;
+    header(D.h, LN, ds0, ds1, dm0, dm1);
 #pragma unroll
     for (int m = 0; m < M; m++) {
       const float tx = ds0 * D.xs[m].x, ty = ds1 * D.xs[m].z;
@@ -147,6 +150,47 @@ struct DecQ4K {
 
   __device__ static __forceinline__ float finish(const float (&a)[3], const Lane &LN) {
     return LN.kD * (a[0] + a[1]) - a[2];
+  }
+};
+
+// One row of the experts' kernel: the same arithmetic in the same order, but the sub-blocks' scales go to the quad's lanes
+// through shared memory, one store and two loads instead of eight shuffles, as DecQ6KOne's.  Layers of 8 experts of 4096 x
+// 14336, two a token: one token 52.0 -> 50.9 us, eight 239.4 -> 233.2; Q6_K 70.3 -> 67.9, six tokens 322 -> 306.  In the decode
+// kernel it is worth 1 % (28672 x 4096 12.2 -> 12.1 us), and with more rows, where the MMAs bound, it costs: 14336 x 4096 by
+// four 16.6 -> 20.8.
+struct DecQ4KOne : DecQ4K {
+  static constexpr int MAX_M = 1;
+  static constexpr uint32_t XCH = 256;
+  struct Lane : DecQ4K::Lane {
+    uint32_t put, get;  // where this lane's two scales go; where the row's first four are, the others 128 bytes on
+    __device__ __forceinline__ void set_exchange(uint32_t at, uint32_t lane) {
+      const uint32_t g = lane >> 2, tig = lane & 3;
+      get = at + g * 16, put = at + (tig >> 1) * 128 + g * 16 + (tig & 1u) * 8;
+    }
+  };
+  template <int M>
+  __device__ static __forceinline__ void compute(const Data<M> &D, const Lane &LN, float (&acc)[M][3]) {
+    float ds0, ds1, dm0, dm1;
+    header(D.h, LN, ds0, ds1, dm0, dm1);
+    __syncwarp();  // the scales of the span before have been read
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(LN.put), "f"(ds0 * D.xs[0].x), "f"(ds1 * D.xs[0].z) : "memory");
+    __syncwarp();
+    acc[0][2] = fmaf(dm0, D.xs[0].y, acc[0][2]);
+    acc[0][2] = fmaf(dm1, D.xs[0].w, acc[0][2]);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const float4 t = lds128f(LN.get + 128u * h);
+      float c[2][4];
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const uint2 w = D.w[2 * h + k], b = D.b[0][2 * h + k];
+        mma_u8s8(c[k], w.x & 0x0F0F0F0Fu, w.x, w.y & 0x0F0F0F0Fu, w.y, b.x, b.y);
+      }
+      acc[0][0] = fmaf(t.x, c[0][0] - MMA_BIAS, acc[0][0]);
+      acc[0][1] = fmaf(t.y, c[0][3] - c[0][1], acc[0][1]);
+      acc[0][0] = fmaf(t.z, c[1][0] - MMA_BIAS, acc[0][0]);
+      acc[0][1] = fmaf(t.w, c[1][3] - c[1][1], acc[0][1]);
+    }
   }
 };
 

@@ -33,7 +33,7 @@ struct MoeArgs {
   uint64_t ldy;
   unsigned *status;
   SmemMma S;
-  uint32_t Kp, stage_bytes, seg;     // seg: byte offset of the CTA's run
+  uint32_t Kp, stage_bytes, seg, xch;  // seg: byte offset of the CTA's run, xch: of what the lanes of its warps exchange
   int nstage, nslot;
 };
 // A CTA's run: per job a range of chunks.
@@ -73,7 +73,8 @@ __global__ void __launch_bounds__(256)
   if ((threadIdx.x & 7) == 0) F::store_xs(row + 3 * PS, e0 / 32, digit_scale(amax, s4 + other), s4 + other, s4, other);
 }
 
-template <class F, bool DUAL, int G>
+// F1: the policy of jobs with one row: F, or its variant for them.
+template <class F, class F1, bool DUAL, int G>
 __global__ void __launch_bounds__((MAX_CW + 2) * 32, 1) qk_gemv_moe_kernel(const __grid_constant__ MoeArgs A) {
   constexpr int CW = MAX_CW, WG = CW / G;
   constexpr uint32_t ND = DUAL ? 2 : 1;
@@ -229,8 +230,9 @@ __global__ void __launch_bounds__((MAX_CW + 2) * 32, 1) qk_gemv_moe_kernel(const
   // ================= compute warps =================
   const uint32_t group = warp / WG, wl = warp % WG;
   const uint32_t g = lane >> 2, tig = lane & 3;
-  typename F::Lane LN;
+  typename F1::Lane LN;  // (F's with what F1 needs besides)
   LN.init(lane, wl, sbase + S.ximg, S.PS, S.xs_off, A.Kp);
+  if constexpr (F1::XCH != 0) LN.set_exchange(sbase + A.xch + warp * F1::XCH, lane);
   pdl_wait();  // the split rows are the previous kernel's work
   uint32_t st = 0, fph = 0, slot = group % nslot;  // next stage and its parity, partial slot of this group's next chunk
   auto skip = [&](uint32_t n) {
@@ -256,7 +258,8 @@ __global__ void __launch_bounds__((MAX_CW + 2) * 32, 1) qk_gemv_moe_kernel(const
     if (!mbar_wait_bounded(sbase + S.xbar, sg & 1u)) dead = true;  // (the wait of the copies in flight, too)
     auto run = [&](auto mtag) {
       constexpr int M = decltype(mtag)::value;
-      using Data = typename F::template Data<M>;
+      using P = std::conditional_t<M == 1, F1, F>;
+      using Data = typename P::template Data<M>;
       for (; c < end && !dead; c += G) {
         float acc[M][3];
 #pragma unroll
@@ -268,7 +271,7 @@ __global__ void __launch_bounds__((MAX_CW + 2) * 32, 1) qk_gemv_moe_kernel(const
             dead = true;
             break;
           }
-          const typename F::Base B = F::base(LN, tile, kt);
+          const typename P::Base B = P::base(LN, tile, kt);
           auto tile_body = [&](auto full_tag) {
             constexpr bool FULL = decltype(full_tag)::value;
             constexpr int NSB = NBT / WG;
@@ -276,8 +279,8 @@ __global__ void __launch_bounds__((MAX_CW + 2) * 32, 1) qk_gemv_moe_kernel(const
               constexpr int J = decltype(jt)::value;
               if (FULL || wl + J * WG < nbt) {
                 Data D;
-                F::template load<M, J, WG>(D, B, LN);
-                F::template compute<M>(D, LN, acc);
+                P::template load<M, J, WG>(D, B, LN);
+                P::template compute<M>(D, LN, acc);
               }
             });
           };
@@ -356,9 +359,9 @@ cudaError_t moe_split(const QkLayout &L, const float *x, uint32_t rows, unsigned
                             (uint64_t)moe_image_stride<F>(L), plan ? *plan : qkmoe::PlanArgs{});
 }
 
-template <class F, bool DUAL, int G>
+template <class F, class F1, bool DUAL, int G>
 cudaError_t moe_launch_g(const MoeArgs &A, uint32_t smem, int sm_count, cudaStream_t s) {
-  auto kern = qk_gemv_moe_kernel<F, DUAL, G>;
+  auto kern = qk_gemv_moe_kernel<F, F1, DUAL, G>;
   static QkPerDevice attr_set;
   if (attr_set.first()) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
@@ -372,8 +375,11 @@ cudaError_t moe_launch_g(const MoeArgs &A, uint32_t smem, int sm_count, cudaStre
   return cudaLaunchKernelEx(&c, kern, A);
 }
 
-// rows_per_job: what the job list was made for (at most moe_rows(L)).
-template <class F>
+template <class P>
+struct MoePolicy { using type = P; };
+// rows_per_job: what the job list was made for (at most moe_rows(L)).  F1: the policy for jobs with one row, where its
+// exchange fits behind the run table (else F itself).
+template <class F, class F1>
 cudaError_t moe_launch(const QkLayout &L, const uint8_t *const *w, const uint8_t *const *w2, uint32_t n, uint32_t rows_per_job,
                        const QkMoeJobs *jobs, const unsigned char *img, uint32_t div, float *y, uint64_t ldy, unsigned *status,
                        int sm_count, cudaStream_t s) {
@@ -384,19 +390,27 @@ cudaError_t moe_launch(const QkLayout &L, const uint8_t *const *w, const uint8_t
   for (uint32_t e = 0; e < n; e++) A.w[e] = w[e], A.w[QK_MOE_MAX + e] = w2 ? w2[e] : nullptr;
   A.y = y, A.ldy = ldy, A.status = status, A.S = p.P.S, A.Kp = p.P.Kp, A.stage_bytes = p.P.stage_bytes, A.seg = p.seg;
   A.nstage = p.P.nstage, A.nslot = p.P.nslot;
-  switch (p.P.groups) {
-    case 4:
-      return w2 ? moe_launch_g<F, true, 4>(A, p.total, sm_count, s) : moe_launch_g<F, false, 4>(A, p.total, sm_count, s);
-    case 2:
-      return w2 ? moe_launch_g<F, true, 2>(A, p.total, sm_count, s) : moe_launch_g<F, false, 2>(A, p.total, sm_count, s);
-    default:
-      return w2 ? moe_launch_g<F, true, 1>(A, p.total, sm_count, s) : moe_launch_g<F, false, 1>(A, p.total, sm_count, s);
-  }
+  A.xch = (p.total + 127u) & ~127u;
+  auto launch = [&](auto policy) {
+    using P1 = typename decltype(policy)::type;
+    const uint32_t total = P1::XCH ? A.xch + MAX_CW * P1::XCH : p.total;
+    switch (p.P.groups) {
+      case 4:
+        return w2 ? moe_launch_g<F, P1, true, 4>(A, total, sm_count, s) : moe_launch_g<F, P1, false, 4>(A, total, sm_count, s);
+      case 2:
+        return w2 ? moe_launch_g<F, P1, true, 2>(A, total, sm_count, s) : moe_launch_g<F, P1, false, 2>(A, total, sm_count, s);
+      default:
+        return w2 ? moe_launch_g<F, P1, true, 1>(A, total, sm_count, s) : moe_launch_g<F, P1, false, 1>(A, total, sm_count, s);
+    }
+  };
+  if constexpr (F1::XCH != 0)
+    if (A.xch + MAX_CW * F1::XCH <= 227u * 1024u) return launch(MoePolicy<F1>{});
+  return launch(MoePolicy<F>{});
 }
 
 }  // namespace qkdec
 
-#define QK_MOE_DEC_DEFINE(NAME, F)                                                                                       \
+#define QK_MOE_DEC_DEFINE(NAME, F, F1)                                                                                       \
   uint32_t qk_moe_dec_##NAME##_rows(const QkLayout &L) { return qkdec::moe_rows<F>(L); }                                 \
   size_t qk_moe_dec_##NAME##_image(const QkLayout &L) { return qkdec::moe_image_stride<F>(L); }                          \
   cudaError_t qk_moe_dec_##NAME##_split(const QkLayout &L, const float *x, uint32_t rows, unsigned char *img, \
@@ -406,5 +420,5 @@ cudaError_t moe_launch(const QkLayout &L, const uint8_t *const *w, const uint8_t
   cudaError_t qk_moe_dec_##NAME##_launch(const QkLayout &L, const uint8_t *const *w, const uint8_t *const *w2, uint32_t n, \
                                          uint32_t rows_per_job, const QkMoeJobs *jobs, const unsigned char *img,         \
                                          uint32_t div, float *y, uint64_t ldy, unsigned *status, int sm_count, cudaStream_t s) { \
-    return qkdec::moe_launch<F>(L, w, w2, n, rows_per_job, jobs, img, div, y, ldy, status, sm_count, s);                  \
+    return qkdec::moe_launch<F, F1>(L, w, w2, n, rows_per_job, jobs, img, div, y, ldy, status, sm_count, s);                  \
   }

@@ -2,4 +2,4 @@
 #include "qk_dec_fmts.cuh"
 #include "qk_gemv_moe.cuh"
 
-QK_MOE_DEC_DEFINE(iq4xs, qkdec::DecIQ4XS)
+QK_MOE_DEC_DEFINE(iq4xs, qkdec::DecIQ4XS, qkdec::DecIQ4XS)

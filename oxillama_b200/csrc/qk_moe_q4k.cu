@@ -2,4 +2,4 @@
 #include "qk_dec_q4k.cuh"
 #include "qk_gemv_moe.cuh"
 
-QK_MOE_DEC_DEFINE(q4k, qkdec::DecQ4K)
+QK_MOE_DEC_DEFINE(q4k, qkdec::DecQ4K, qkdec::DecQ4KOne)

@@ -2,4 +2,4 @@
 #include "qk_dec_fmts.cuh"
 #include "qk_gemv_moe.cuh"
 
-QK_MOE_DEC_DEFINE(q6k, qkdec::DecQ6K)
+QK_MOE_DEC_DEFINE(q6k, qkdec::DecQ6K, qkdec::DecQ6KOne)

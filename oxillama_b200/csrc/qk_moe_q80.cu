@@ -2,4 +2,4 @@
 #include "qk_dec_fmts.cuh"
 #include "qk_gemv_moe.cuh"
 
-QK_MOE_DEC_DEFINE(q80, qkdec::DecQ80)
+QK_MOE_DEC_DEFINE(q80, qkdec::DecQ80, qkdec::DecQ80)

@@ -700,3 +700,33 @@ def test_ffn_conversion_by_clusters(t, hidden, inter, ms):
         assert np.abs(y.cpu().numpy() - ref).max() <= 3e-3 * np.abs(ref).max()
     for w in dw:
         w.free()
+
+
+# Experts' jobs of one row (a single token) and of two, whose scales go to the lanes by different ways: one span of columns for
+# eight warps, one that leaves some of them out, a second tile with a ragged last block; rows that are no multiple of a chunk's.
+# Against each expert's own product in f64; the bound is test_moe_short_rows'.
+@pytest.mark.parametrize("t", [S.Q4_K, S.Q6_K])
+@pytest.mark.parametrize("hidden,inter", [(256, 40), (1284, 264), (4352, 2304)])
+def test_moe_decode_one_row(t, hidden, inter):
+    import torch
+    from oxillama_b200 import moe
+    from oxillama_b200.device import check_device_status
+    n, top_k = 4, 2
+    shapes = [(inter, hidden), (inter, hidden), (hidden, inter)]
+    w = [[S.gen_weight(t, r, c, seed=151, stream=3 * e + k, d_range=(1e-4, 3e-4)) for e in range(n)] for k, (r, c) in enumerate(shapes)]
+    logits = torch.tensor([[3., 1., 2., 0.], [3., 0., 1., 2.]])  # a job of two rows and two of one
+    ex = moe.MoeExperts(t, *w, hidden, inter, n)
+    for tokens in (1, 2):
+        x = S.gen_acts(tokens, hidden, seed=152) * np.float32(0.25)
+        ids, wts = (v.cpu().numpy() for v in moe.route(logits[:tokens].cuda(), top_k))
+        ref = np.zeros((tokens, hidden))
+        for tok in range(tokens):
+            for e, wt in zip(ids[tok], wts[tok]):
+                g, u, d = (O.dequant_matrix(t, ws[e], r, c).astype(np.float64) for ws, (r, c) in zip(w, shapes))
+                hg = g @ x[tok]
+                ref[tok] += wt * (d @ (hg / (1 + np.exp(-hg)) * (u @ x[tok])))
+        y = torch.full((tokens, hidden), float("nan"), device="cuda")
+        ex.forward(logits[:tokens].cuda(), torch.from_numpy(x).cuda(), y, top_k)
+        check_device_status()
+        assert np.abs(y.cpu().numpy() - ref).max() <= 3e-3 * np.abs(ref).max()
+    ex.free()

@@ -696,10 +696,12 @@ __global__ void __launch_bounds__(CT, CT == 256 ? 6 : 1) qk_x16_kernel(const Con
 // silu(x) * x2 rows through shared memory: 512 threads of 40 registers and a row of 14336 columns leave room
 // for three CTAs on an SM, where the form above holds one (78 registers) that loads, computes and stores in
 // turn (14336 columns by 512 rows: 27 -> 9 us).  CL CTAs, a cluster, share a row and meet once for its largest magnitude:
-// exp and the rounded division keep one SM busy for 2 us with a row of 14336.  Eight or four CTAs a row as long as they are no
-// more than the SMs, twice as many where rows are long; above, one CTA of 1024 threads a row, from a row per SM on of 512
-// (us, a feed-forward block of 4096 x 14336, one CTA a row / clusters: by 8 40.9 / 39.9, by 19 43.0 / 41.6, by 37 44.7 / 43.8, by 48
-// 44.6 / 43.7, by 74 52.2 / 52.5; two CTAs a row by 64 45.8 / 47.2, by 512 192 / 196; 2048 x 5632 by 37 23.8 / 23.2, by 50 23.5 / 23.6).
+// exp and the rounded division keep one SM busy for 2 us with a row of 14336.  Eight or four CTAs a row of more than 8192
+// columns as long as they are no more than twice the SMs; else one CTA of 1024 threads a row, from a row per SM on of 512 (us, a
+// feed-forward block, one CTA a row / clusters: 4096 x 14336 by 8 40.9 / 39.9, by 19 43.0 / 41.6, by 37 44.7 / 43.8, by 48 44.6 /
+// 43.7, by 74 52.2 / 52.5; 3584 x 11776 by 5 37.8 / 36.2, by 30 41.4 / 41.5; shorter rows leave most threads of eight CTAs without
+// work: 2048 x 8192 by 12 24.8 / 25.3, by 37 26.2 / 27.6; 2304 x 6144 by 12 21.8 / 21.8; 1536 x 4096 by 12 18.0 / 20.2; 1024 x 2816
+// by 18 15.1 / 18.1; two CTAs a row for many rows: 4096 x 14336 by 64 45.8 / 47.2, by 512 192 / 196).
 template <int T, int CT, int CL>
 __global__ void __launch_bounds__(CT, CT == 512 ? 3 : 1) qk_glu16_kernel(const ConvArgs A) {
   extern __shared__ __align__(16) float glu_row[];
@@ -1482,9 +1484,9 @@ cudaError_t launch_fmt(const QkTcCall &c, unsigned *status, unsigned char *scrat
   c0.gridDim = dim3(c.counts && c.live < all_rows ? c.live : all_rows), c0.blockDim = dim3(narrow ? 256 : 512), c0.stream = s, c0.attrs = &at, c0.numAttrs = 1;
   cudaError_t e;
   if (c.x2 && !c.lists && Kp * 4 <= GLU_SMEM) {
-    const uint32_t rows = c0.gridDim.x, sms = (uint32_t)sm_count, room = Kp > 8192 ? 2 * sms : sms;
-    if (!c.counts && rows * 8 <= room) e = launch_glu16<T, 512, 8>(C, rows, s);
-    else if (!c.counts && rows * 4 <= room) e = launch_glu16<T, 512, 4>(C, rows, s);
+    const uint32_t rows = c0.gridDim.x, sms = (uint32_t)sm_count, room = !c.counts && Kp > 8192 ? 2 * sms : 0u;
+    if (rows * 8 <= room) e = launch_glu16<T, 512, 8>(C, rows, s);
+    else if (rows * 4 <= room) e = launch_glu16<T, 512, 4>(C, rows, s);
     else if (!c.counts && rows <= sms) e = launch_glu16<T, 1024, 1>(C, rows, s);
     else e = launch_glu16<T, 512, 1>(C, rows, s);
   } else if (c.x2) {

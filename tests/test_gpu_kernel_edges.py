@@ -678,11 +678,11 @@ def test_device_call_arguments(native, monkeypatch):
         dw.gemv(x, y)
 
 
-# silu(g) * u by clusters of eight and four CTAs a row and by one: the last batch of each and the first of the next (148 SMs;
-# rows above 8192 columns twice as many), rows with fewer super-blocks than CTAs, parts of unequal length, a ragged last block.
+# silu(g) * u by clusters of eight and four CTAs a row (above 8192 columns) and by one: the last batch of each and the first of the
+# next (148 SMs), parts of unequal length, a ragged last block, and shorter rows, of which one CTA takes a whole one.
 # The bound: three chained products, each within 1e-3 of its largest value.
 @pytest.mark.parametrize("t,hidden,inter,ms", [(S.Q4_K, 256, 512, (5, 18, 19, 37, 38)), (S.Q8_0, 256, 2336, (18, 37)), (S.Q6_K, 256, 8448, (37, 38, 74, 75)),
-                                               (S.IQ4_XS, 256, 4864, (18, 19)), (S.Q4_0, 512, 1312, (9, 30))])
+                                               (S.IQ4_XS, 256, 4864, (18, 19)), (S.Q4_0, 512, 1312, (9, 30)), (S.Q8_0, 256, 9248, (37, 38))])
 def test_ffn_conversion_by_clusters(t, hidden, inter, ms):
     import torch
     from oxillama_b200.device import DeviceWeights, check_device_status, ffn

@@ -695,8 +695,8 @@ __global__ void __launch_bounds__(CT, CT == 256 ? 6 : 1) qk_x16_kernel(const Con
 
 // silu(x) * x2 rows through shared memory: 512 threads of 40 registers and a row of 14336 columns leave room
 // for three CTAs on an SM, where the form above holds one (78 registers) that loads, computes and stores in
-// turn (14336 columns by 512 rows: 27 -> 9 us).  CL CTAs, a cluster, share a row and meet once for its largest magnitude:
-// exp and the rounded division keep one SM busy for 2 us with a row of 14336.  Eight or four CTAs a row of more than 8192
+// turn (14336 columns by 512 rows alone 27 -> 9 us; behind the matmul that writes them it costs 26 to 30).  CL CTAs, a cluster,
+// share a row and meet once for its largest magnitude: exp and the rounded division keep one SM busy for 2 us with a row of 14336.  Eight or four CTAs a row of more than 8192
 // columns as long as they are no more than twice the SMs; else one CTA of 1024 threads a row, from a row per SM on of 512 (us, a
 // feed-forward block, one CTA a row / clusters: 4096 x 14336 by 8 40.9 / 39.9, by 19 43.0 / 41.6, by 37 44.7 / 43.8, by 48 44.6 /
 // 43.7, by 74 52.2 / 52.5; 3584 x 11776 by 5 37.8 / 36.2, by 30 41.4 / 41.5; shorter rows leave most threads of eight CTAs without

@@ -707,6 +707,7 @@ __global__ void __launch_bounds__(CT, CT == 512 ? 3 : 1) qk_glu16_kernel(const C
   extern __shared__ __align__(16) float glu_row[];
   __shared__ float red[CT / 32], parts[CL];
   pdl_launch_dependents();
+  if (CL > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // (waited for ahead of the stores into other CTAs)
   pdl_wait();
   if (blockIdx.x == 0)
     for (uint32_t i = threadIdx.x; i < A.n_zero; i += CT) A.zero[i] = 0u;
@@ -739,7 +740,10 @@ __global__ void __launch_bounds__(CT, CT == 512 ? 3 : 1) qk_glu16_kernel(const C
 #pragma unroll
   for (int o = CT / 64; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
   if (CL > 1) {
+    // A CTA whose part of the row is empty comes here at once: the others must have started before it stores into them.
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (threadIdx.x < CL) st_cluster(smem_u32(&parts[rank]), threadIdx.x, amax);
+    __syncwarp();
     cluster_sync();
 #pragma unroll
     for (int c = 0; c < CL; c++) amax = fmaxf(amax, parts[c]);

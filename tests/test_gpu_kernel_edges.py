@@ -678,13 +678,18 @@ def test_device_call_arguments(native, monkeypatch):
         dw.gemv(x, y)
 
 
-# silu(g) * u by clusters of eight and four CTAs a row (above 8192 columns) and by one: the last batch of each and the first of the
-# next (148 SMs), parts of unequal length, a ragged last block, and shorter rows, of which one CTA takes a whole one.
+# silu(g) * u by clusters of eight and four CTAs a row of more than 8192 columns, as long as they are no more than twice the SMs
+# (148: up to 37 and 74 rows), by one from there on and for shorter rows.  8448 and 8500 columns are 33 and 34 spans: of eight parts
+# of five spans the last is empty, its CTA comes to the meeting at once; 9248 leaves the last part short and its last span ragged.  Every format,
+# Q4_K with its order of 64 columns.  Many calls in turn give the same bits.
 # The bound: three chained products, each within 1e-3 of its largest value.
-@pytest.mark.parametrize("t,hidden,inter,ms", [(S.Q4_K, 256, 512, (5, 18, 19, 37, 38)), (S.Q8_0, 256, 2336, (18, 37)), (S.Q6_K, 256, 8448, (37, 38, 74, 75)),
-                                               (S.IQ4_XS, 256, 4864, (18, 19)), (S.Q4_0, 512, 1312, (9, 30)), (S.Q8_0, 256, 9248, (37, 38))])
+@pytest.mark.parametrize("t,hidden,inter,ms", [(S.Q4_K, 256, 512, (5, 18, 38)), (S.Q8_0, 256, 2336, (18, 37)), (S.IQ4_XS, 256, 4864, (18, 19)),
+                                               (S.Q4_0, 512, 1312, (9, 30)), (S.Q6_K, 256, 8448, (5, 37, 38, 74, 75)), (S.Q8_0, 256, 9248, (37, 38)),
+                                               (S.Q4_K, 256, 8500, (5, 37, 38, 74, 75, 149)), (S.Q4_K, 256, 14336, (8, 38)), (S.IQ4_XS, 256, 8448, (5, 37, 38, 75)),
+                                               (S.Q4_0, 256, 9248, (5, 74))])
 def test_ffn_conversion_by_clusters(t, hidden, inter, ms):
     import torch
+    from launches import launched, sm_count
     from oxillama_b200.device import DeviceWeights, check_device_status, ffn
     shapes = [(inter, hidden), (inter, hidden), (hidden, inter)]
     ws = [S.gen_weight(t, r, c, seed=181, stream=i, d_range=(1e-3, 3e-3)) for i, (r, c) in enumerate(shapes)]
@@ -694,10 +699,19 @@ def test_ffn_conversion_by_clusters(t, hidden, inter, ms):
         x = S.gen_acts(m, hidden, seed=182) * np.float32(0.25)
         hg = x.astype(np.float64) @ g.T
         ref = (hg / (1 + np.exp(-hg)) * (x.astype(np.float64) @ u.T)) @ d.T
-        y = torch.full((m, hidden), float("nan"), device="cuda")
-        ffn(*dw, torch.from_numpy(x).cuda(), y, m)
+        xd, y = torch.from_numpy(x).cuda(), torch.full((m, hidden), float("nan"), device="cuda")
+        cl = next((c for c in (8, 4) if inter > 8192 and m * c <= 2 * sm_count()), 1)
+        glu, = [k for k in launched(lambda: ffn(*dw, xd, y, m)) if k.name == "qk_glu16_kernel"]
+        assert glu.ints[-1] == cl and glu.grid[0] == m * cl, glu
+        y.fill_(float("nan"))
+        ffn(*dw, xd, y, m)
         check_device_status()
         assert np.abs(y.cpu().numpy() - ref).max() <= 3e-3 * np.abs(ref).max()
+        again = torch.empty((20, m, hidden), device="cuda")
+        for z in again:
+            ffn(*dw, xd, z, m)
+        check_device_status()
+        assert all(torch.equal(z, y) for z in again)
     for w in dw:
         w.free()
 

@@ -14,7 +14,7 @@ OBJ = os.path.join(HERE, "_obj")
 LIB = os.path.join(HERE, "libqk_cuda.so")
 EXT = os.path.join(HERE, "_qk_torch.so")  # Python extension over torch's C++ objects (csrc/qk_torch.cpp)
 SOURCES = ["qk_api.cu", "qk_simple.cu", "qk_gemv_mma.cu", "qk_gemv_imma.cu", "qk_dec_q80.cu", "qk_dec_q40.cu",
-           "qk_dec_iq4xs.cu", "qk_dec_q6k.cu", "qk_dec_q5k.cu", "qk_dec_q3k.cu", "qk_dec_q2k.cu", "qk_noalloc.cu", "qk_gemm_tc.cu", "qk_tc_q4k.cu", "qk_tc_q80.cu", "qk_tc_q40.cu", "qk_tc_q6k.cu", "qk_tc_iq4xs.cu", "qk_moe.cu", "qk_moe_q4k.cu", "qk_moe_q80.cu", "qk_moe_q40.cu", "qk_moe_iq4xs.cu", "qk_moe_q6k.cu", "qk_gather.cu", "qk_gguf.cu"]
+           "qk_dec_iq4xs.cu", "qk_dec_q6k.cu", "qk_dec_q5k.cu", "qk_dec_q3k.cu", "qk_dec_q2k.cu", "qk_noalloc.cu", "qk_gemm_tc.cu", "qk_tc_q4k.cu", "qk_tc_q4k_wide.cu", "qk_tc_q80.cu", "qk_tc_q40.cu", "qk_tc_q6k.cu", "qk_tc_q6k_wide.cu", "qk_tc_iq4xs.cu", "qk_moe.cu", "qk_moe_q4k.cu", "qk_moe_q80.cu", "qk_moe_q40.cu", "qk_moe_iq4xs.cu", "qk_moe_q6k.cu", "qk_gather.cu", "qk_gguf.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",

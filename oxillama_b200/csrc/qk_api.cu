@@ -237,7 +237,7 @@ static int upload_impl(qk_ctx *c, int type, const uint8_t *w, size_t n_cols, siz
       if (e == cudaSuccess) e = qk_launch_repack(part, buf, h->dev + r / QK_TILE_ROWS * h->L.chunk_bytes, c->stream);
     }
   } while (0);
-  if (e == cudaSuccess) e = qk_gemm_tc_factors(h->L, h->dev, h->rows, c->stream);
+  if (e == cudaSuccess) e = qk_gemm_tc_factors(h->L, h->dev, h->rows, &h->wide, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   else cudaStreamSynchronize(c->stream);
   if (raw) cudaFree(raw);
@@ -449,7 +449,7 @@ static int gemm_dispatch(qk_ctx *c, QkScratch &sc, const qk_weights *h, const fl
   if (!c->force_simple && (m > QK_GEMV_MAX_M || tc_small) && m < (1u << 30) &&
       qk_gemm_tc_supported(h->L, (uint32_t)m)) {
     QkTcCall call = {};
-    call.L = &h->L, call.maps[0] = h->tmap, call.rows[0] = h->rows, call.n = call.n_act = 1;
+    call.L = &h->L, call.maps[0] = h->tmap, call.rows[0] = h->rows, call.wide = h->wide, call.n = call.n_act = 1;
     call.x = x, call.m = (uint32_t)m, call.y = y, call.ldy = ldy;
     return tc_call(c, sc, call, s);
   }
@@ -554,14 +554,15 @@ extern "C" int qk_moe_ffn_dev(qk_ctx *c, const qk_weights *const *gate, const qk
     gu.y = g, gu.ldy = inter;
     // gate and up as 2 n groups over n activation groups (groups n .. 2 n - 1 write u, behind g)
     const bool one_launch = 2 * n_local <= QK_MAX_GROUPS;
-    for (size_t e = 0; e < n_local; e++) gu.maps[e] = gate[e]->tmap, gu.rows[e] = gate[e]->rows;
+    for (size_t e = 0; e < n_local; e++) gu.maps[e] = gate[e]->tmap, gu.rows[e] = gate[e]->rows, gu.wide |= gate[e]->wide;
     if (one_launch)
-      for (size_t e = 0; e < n_local; e++) gu.maps[n_local + e] = up[e]->tmap, gu.rows[n_local + e] = up[e]->rows;
+      for (size_t e = 0; e < n_local; e++) gu.maps[n_local + e] = up[e]->tmap, gu.rows[n_local + e] = up[e]->rows, gu.wide |= up[e]->wide;
     gu.n = (uint32_t)(one_launch ? 2 * n_local : n_local);
     int st = tc_call(c, c->scratch, gu, s);
     if (st) return st;
     if (!one_launch) {
-      for (size_t e = 0; e < n_local; e++) gu.maps[e] = up[e]->tmap, gu.rows[e] = up[e]->rows;
+      gu.wide = false;
+      for (size_t e = 0; e < n_local; e++) gu.maps[e] = up[e]->tmap, gu.rows[e] = up[e]->rows, gu.wide |= up[e]->wide;
       gu.y = u;
       if ((st = tc_call(c, c->scratch, gu, s))) return st;
     }
@@ -569,7 +570,7 @@ extern "C" int qk_moe_ffn_dev(qk_ctx *c, const qk_weights *const *gate, const qk
     QkTcCall dn = {};
     dn.L = &down[0]->L, dn.n = dn.n_act = (uint32_t)n_local, dn.counts = cnt, dn.m = (uint32_t)tokens, dn.expect = gu.expect, dn.live = gu.live;
     dn.xcap = dn.ycap = (uint32_t)cap, dn.x = g, dn.x2 = u, dn.y = o, dn.ldy = hidden;
-    for (size_t e = 0; e < n_local; e++) dn.maps[e] = down[e]->tmap, dn.rows[e] = down[e]->rows;
+    for (size_t e = 0; e < n_local; e++) dn.maps[e] = down[e]->tmap, dn.rows[e] = down[e]->rows, dn.wide |= down[e]->wide;
     return tc_call(c, c->scratch, dn, s);
   };
 
@@ -701,12 +702,12 @@ extern "C" int qk_ffn_dev(qk_ctx *c, const qk_weights *gate, const qk_weights *u
     // Batches: gate and up as one tensor-core launch over the activations converted once, and
     // silu(g) * u formed where the down projection's activations are converted.
     QkTcCall gu = {};
-    gu.L = &gate->L, gu.maps[0] = gate->tmap, gu.maps[1] = up->tmap, gu.rows[0] = gate->rows, gu.rows[1] = up->rows, gu.n = 2, gu.n_act = 1;
+    gu.L = &gate->L, gu.maps[0] = gate->tmap, gu.maps[1] = up->tmap, gu.rows[0] = gate->rows, gu.rows[1] = up->rows, gu.wide = gate->wide || up->wide, gu.n = 2, gu.n_act = 1;
     gu.x = x_dev, gu.m = (uint32_t)m, gu.xcap = gu.ycap = (uint32_t)m, gu.y = h, gu.ldy = inter;
     int st = tc_call(c, c->scratch, gu, s);
     if (st) return st;
     QkTcCall dn = {};
-    dn.L = &down->L, dn.maps[0] = down->tmap, dn.rows[0] = down->rows, dn.n = dn.n_act = 1;
+    dn.L = &down->L, dn.maps[0] = down->tmap, dn.rows[0] = down->rows, dn.wide = down->wide, dn.n = dn.n_act = 1;
     dn.x = h, dn.x2 = u, dn.m = (uint32_t)m, dn.y = y_dev, dn.ldy = down->L.rows;
     return tc_call(c, c->scratch, dn, s);
   } else {

@@ -105,7 +105,8 @@ bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
     p.row_blocks = (L.rows + p.cg * BM - 1) / (p.cg * BM);
     p.grid = (uint32_t)sm_count / p.cg;
   } else {
-    const float expand = L.type == QK_T_Q6_K ? 1130.f : L.type == QK_T_Q4_K ? 870.f : 1000.f;
+    // (with a marked matrix as before)
+    const float expand = L.type == QK_T_Q6_K ? (c.wide ? 1170.f : 1130.f) : L.type == QK_T_Q4_K && !c.wide ? 870.f : 1000.f;
     float best = FLT_MAX;
     auto take = [&](float t, uint32_t cg, uint32_t cs, uint32_t bn, uint32_t tbr, uint32_t rbs, uint32_t run, uint32_t grid) {
       if (t < best) best = t, p.cg = cg, p.cs = cs, p.bn = bn, p.tok_blocks = tbr, p.row_blocks = rbs, p.min_run = run, p.grid = grid;
@@ -213,43 +214,71 @@ cudaError_t qk_gemm_tc_map(const QkLayout &L, uint8_t *tiled, void *map) {
   return cudaSuccess;
 }
 
+// (four bytes a row, and the mark)
 size_t qk_gemm_tc_factor_bytes(const QkLayout &L) {
-  return L.type == QK_T_Q4_K || L.type == QK_T_Q6_K ? (size_t)L.chunks * QK_TILE_ROWS * sizeof(float) : 0;
+  return L.chunks && (L.type == QK_T_Q4_K || L.type == QK_T_Q6_K) ? (size_t)L.chunks * QK_TILE_ROWS * sizeof(float) + 16 : 0;
 }
 
 namespace {
-// A warp per row.  With b = the largest |scale| of the row's weights (Q4_K: 63 |d|, and |dmin|; Q6_K: 128 |d|) the factor is
+__device__ __forceinline__ uint32_t max_byte(uint32_t v) {
+  v = __vmaxu4(v, v >> 16);
+  return max(v & 0xFFu, (v >> 8) & 0xFFu);
+}
+__device__ __forceinline__ float abs_half(uint32_t bits) { return fabsf(__half2float(__ushort_as_half((unsigned short)bits))); }
+
+// A warp per row.  With b = the largest scale of the row's blocks (Q4_K: |d sc|, |d|, |dmin|; Q6_K: |d sc|, |d|) the factor is
 // the power of two over which 2^24 b is at most 0.998 of 2^16, about fp16's largest (2^-6 at least: 2^30 is what the kernel
 // takes).  Scales that are not finite do not count
-// (their blocks stay not finite), a row of zeros has factor 1.
-__global__ void __launch_bounds__(256) qk_row_factor_kernel(QkLayout L, const uint8_t *__restrict__ tiled, float *__restrict__ rows) {
+// (their blocks stay not finite), a row of zeros has factor 1.  `mark` is set where what a block of the row reaches is below
+// 2^-10 of its factor (see WFmt): 63 * 15 d of Q4_K (6-bit scales are made with the largest of a block 63; if all are 0,
+// 63 dmin), 32 |d sc| of Q6_K.
+__global__ void __launch_bounds__(256) qk_row_factor_kernel(QkLayout L, const uint8_t *__restrict__ tiled, float *__restrict__ rows, unsigned *__restrict__ mark) {
   const uint32_t row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= L.chunks * QK_TILE_ROWS) return;
-  const int dp = L.type == QK_T_Q4_K ? 0 : (int)L.nplanes - 1;  // the plane that (begins with) d
-  const float times = L.type == QK_T_Q4_K ? 63.f : 128.f;
-  float b = 0.f;
+  float b = 0.f, least = FLT_MAX;
   if (row < L.rows)
     for (uint32_t k = lane; k < L.nb; k += 32) {
-      const uint32_t w = *reinterpret_cast<const uint16_t *>(tiled + qk_byte_offset(L, row, k, dp, 0));
-      const float d = fabsf(__half2float(__ushort_as_half((unsigned short)w))) * times;
-      if (d <= FLT_MAX) b = fmaxf(b, d);
       if (L.type == QK_T_Q4_K) {
-        const float m = fabsf(__half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(tiled + qk_byte_offset(L, row, k, dp, 2)))));
-        if (m <= FLT_MAX) b = fmaxf(b, m);
+        const uint4 h = *reinterpret_cast<const uint4 *>(tiled + qk_byte_offset(L, row, k, 0, 0));
+        const uint32_t sc = max_byte(__vmaxu4(h.y & 0x3F3F3F3Fu, (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u)));
+        const uint32_t mn = max_byte(__vmaxu4(h.z & 0x3F3F3F3Fu, ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u)));
+        const float d = abs_half(h.x), dmin = abs_half(h.x >> 16);
+        if (d <= FLT_MAX) b = fmaxf(b, d * (float)max(sc, 1u));
+        if (dmin <= FLT_MAX) b = fmaxf(b, dmin);
+        if (sc && d > 0.f && d <= FLT_MAX) least = fminf(least, 945.f * d);
+        else if (mn && dmin > 0.f && dmin <= FLT_MAX) least = fminf(least, 63.f * dmin);
+      } else {
+        const uint4 s = *reinterpret_cast<const uint4 *>(tiled + qk_byte_offset(L, row, k, 1, 0));
+        const uint32_t sc = max_byte(__vmaxu4(__vmaxu4(__vabs4(s.x), __vabs4(s.y)), __vmaxu4(__vabs4(s.z), __vabs4(s.w))));
+        const float d = abs_half(*reinterpret_cast<const uint16_t *>(tiled + qk_byte_offset(L, row, k, 2, 0)));
+        if (d <= FLT_MAX) b = fmaxf(b, d * (float)max(sc, 1u));
+        if (sc && d > 0.f && d <= FLT_MAX) least = fminf(least, 32.f * d * (float)sc);
       }
     }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) b = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, o));
+  for (int o = 16; o > 0; o >>= 1) b = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, o)), least = fminf(least, __shfl_xor_sync(0xffffffffu, least, o));
   int e = 0;
   const float f = frexpf(b, &e);  // b = f * 2^e, f in [0.5, 1)
-  if (lane == 0) rows[row] = b > 0.f ? ldexpf(1.f, max(e + 8 + (f > 0.998f ? 1 : 0), -6)) : 1.f;
+  if (lane == 0) {
+    const float factor = b > 0.f ? ldexpf(1.f, max(e + 8 + (f > 0.998f ? 1 : 0), -6)) : 1.f;
+    rows[row] = factor;
+    if (least < factor * 0x1p-10f) atomicOr(mark, 1u);
+  }
 }
 }  // namespace
 
-cudaError_t qk_gemm_tc_factors(const QkLayout &L, const uint8_t *tiled, float *rows, cudaStream_t s) {
+cudaError_t qk_gemm_tc_factors(const QkLayout &L, const uint8_t *tiled, float *rows, bool *wide, cudaStream_t s) {
+  *wide = false;
   if (!qk_gemm_tc_factor_bytes(L)) return cudaSuccess;
-  qk_row_factor_kernel<<<L.chunks, 256, 0, s>>>(L, tiled, rows);
-  return cudaGetLastError();
+  unsigned *mark = reinterpret_cast<unsigned *>(rows + (size_t)L.chunks * QK_TILE_ROWS), m = 0;
+  cudaError_t e = cudaMemsetAsync(mark, 0, sizeof(m), s);
+  if (e != cudaSuccess) return e;
+  qk_row_factor_kernel<<<L.chunks, 256, 0, s>>>(L, tiled, rows, mark);
+  if ((e = cudaGetLastError()) == cudaSuccess) e = cudaMemcpyAsync(&m, mark, sizeof(m), cudaMemcpyDeviceToHost, s);
+  const cudaError_t e2 = cudaStreamSynchronize(s);
+  if (e == cudaSuccess) e = e2;
+  *wide = e == cudaSuccess && m != 0;
+  return e;
 }
 
 size_t qk_gemm_tc_part_bytes(int sm_count) { return (size_t)sm_count * 2 * qktc::MAX_BN * qktc::BM * 4; }

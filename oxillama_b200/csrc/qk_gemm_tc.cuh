@@ -73,6 +73,7 @@ namespace qktc {
 using namespace qkpipe;
 
 constexpr uint32_t BM = 128;       // weight rows per CTA
+constexpr int QK_TC_WIDE = 0x100;  // or-ed to a format: its expansion for rows whose blocks differ widely (see WFmt)
 constexpr int FIRST_DW = 4;        // first expanding warp
 constexpr int NDW = 16;            // expanding warps: two sets of eight (three sets of 64 registers a thread: 3 to 10 % slower)
 constexpr int FIRST_EW = FIRST_DW + NDW, NTHREADS = (FIRST_EW + 4) * 32;
@@ -274,11 +275,18 @@ __device__ __forceinline__ float4 ldcg4(const float *p) { return __ldcg(reinterp
 // now: Q4_K 14336 x 4096 by 8 tokens 13.1 / 11.6, by 37 14.4 / 12.6, 4096 x 14336 by 8 15.5 / 14.3, 4096 x 4096 by 128 14.9 /
 // 13.1; Q6_K 4096 x 14336 by 8 16.65 / 16.2, 4096 x 4096 by 37 10.8 / 10.5.  Q8_0 and Q4_0, whose scales change with every 32
 // columns, gained nothing: 4096 x 4096 by 8 9.06 / 9.12, 8.31 / 8.33.)  scale 2^24 fits a half because the weights of a row
-// are expanded over a power of two of the row's own, its factor; the epilogue multiplies the row's results by it again.  Both
-// are exact: the weights are those of before over a power of two, but for the ones below 2^-10 of the row's largest (Q6_K
-// 2^-11), which fall among the subnormals and keep 2^-21 of it (2^-22).
+// are expanded over a power of two of the row's own, its factor; the epilogue multiplies the row's results by it again.
+// Scale and weights may be up to 2^-8 of the factor this way, which leaves few bits to the weights far below that: under
+// 2^-14 of the factor they are subnormals themselves, rounded to 2^-24 of it, and so is the minimum or offset of a block.
+// As long as every block's scale is at least 2^-10 of the factor (945 d and 32 d sc: the weights that a block reaches), the
+// products of any single block are within 2 % as exact as from weights in full halves (emulated in f64, activations in that
+// block alone; at 2^-12 a third less exact, at 2^-14 four times).  A matrix with a row whose blocks differ by more is
+// marked when it is uploaded (qk_gemm_tc_factors), and a call with such a matrix takes the former expansion: the fields as
+// whole halves, weights over 2^-17 of the factor, normal halves from 2^15 down to 2^-14 (QK_TC_WIDE; us, by a matrix without
+// the mark / with it: Q4_K 14336 x 4096 by 8 11.7 / 13.1, 4096 x 14336 by 37 15.3 / 16.7; Q6_K 14.4 / 14.7, 17.8 / 18.3).
 //
-//   SCALED    whether that is how the format is expanded and its rows have factors (qk_gemm_tc_factors)
+//   SCALED    whether the format's rows have factors (qk_gemm_tc_factors); UP, BACK: its scales are taken times 2^UP over the
+//             factor (rf, an Rf), and sums of products come out over BACK of it
 //   BB, BPS   bytes of a block of one row; blocks per super-block.  A staged super-block is
 //             [16 chunks][BPS blocks][8 rows x BB bytes], block-major as in HBM
 //   Hd        what the four quarters share (scales), head() fetches it (p: the row's chunk, rf: see above)
@@ -335,11 +343,12 @@ __device__ __forceinline__ void nibbles_to_halves(uint32_t w, __half2 (&e)[4]) {
   e[0] = bits_h2(w & 0x000F000Fu), e[1] = bits_h2(wj & 0x000F000Fu);
   e[2] = bits_h2(w & 0x00F000F0u), e[3] = bits_h2(wj & 0x00F000F0u);
 }
-// rf as the product of two halves, since it may be up to 2^30 (all that it is multiplied with stays exact on the way).
+// rf as the product of two halves, since it may be up to 2^30.  (All that it is multiplied with stays exact on the way, but for
+// scales d of a marked Q4_K matrix below 2^-16 of the row's largest where that is above 4.)
 struct RowScale {
   uint32_t a, b;
-  __device__ __forceinline__ void set(float factor) {  // 2^24 / factor
-    const int e = 24 + 127 - (int)(__float_as_uint(factor) >> 23), ea = max(min(e, 15), -14);
+  __device__ __forceinline__ void set(float factor, int up) {  // 2^up / factor
+    const int e = up + 127 - (int)(__float_as_uint(factor) >> 23), ea = max(min(e, 15), -14);
     a = (uint32_t)(15 + ea) * 0x04000400u, b = (uint32_t)(15 + e - ea) * 0x04000400u;
   }
   __device__ __forceinline__ __half2 times(__half2 v) const { return __hmul2(__hmul2(v, bits_h2(a)), bits_h2(b)); }
@@ -353,6 +362,9 @@ template <>
 struct WFmt<QK_T_Q4_K> {  // d, dmin, 12 bytes of 6-bit scales / mins, 128 bytes of nibbles (reference/q4_k.rs:27-102)
   static constexpr uint32_t BB = 144, BPS = 1, LUT = 0;
   static constexpr bool SCALED = true;
+  using Rf = RowScale;
+  static constexpr int UP = 24;
+  static constexpr float BACK = 1.f;
   __device__ static void fill_lut(unsigned char *, uint32_t, uint32_t) {}
   // position 8 i + j of a 64-group <- column 4 i + {0,2,1,3}[j & 3] + 32 (j >> 2): byte 4 i + b of
   // the group's 32 holds column 4 i + b (low nibble) and 32 + 4 i + b (high nibble)
@@ -388,10 +400,41 @@ struct WFmt<QK_T_Q4_K> {  // d, dmin, 12 bytes of 6-bit scales / mins, 128 bytes
   }
 };
 
+// Rows whose blocks differ widely (see above).  d * sc and dmin * mn have 17 bits at most, so the fp16 products are the f32 ones
+// rounded once; q is exact after the subtraction, then one fused q * scale - min.  |d sc| and |dmin| being at most 2^-8 of the
+// factor, a weight is at most 78 2^9, and |d| 2^9.
+template <>
+struct WFmt<QK_T_Q4_K | QK_TC_WIDE> : WFmt<QK_T_Q4_K> {
+  static constexpr int UP = 17;
+  static constexpr float BACK = 0x1p-17f;
+  __device__ static void expand(const Qt &t, const Hd &c, uint32_t k, uint32_t (&o)[16], uint32_t) {
+    const __half2 k1024 = __float2half2_rn(1024.f), k_hi = __float2half2_rn(64.f);
+    const __half2 d = __low2half2(bits_h2(c.d)), m = __hneg2(__high2half2(bits_h2(c.d)));
+    const uint32_t lo = 0x4040u + (k >> 1) * 0x0202u, hi = lo + 0x0101u;  // the 64-group's two sub-blocks
+    const __half2 s_lo = __hmul2(__hsub2(bits_h2(prmt(c.scw, 0x64646464u, lo)), k1024), d);
+    const __half2 s_hi = __hmul2(__hsub2(bits_h2(prmt(c.scw, 0x64646464u, hi)), k1024), d);
+    const __half2 m_lo = __hmul2(__hsub2(bits_h2(prmt(c.mnw, 0x64646464u, lo)), k1024), m);
+    const __half2 m_hi = __hmul2(__hsub2(bits_h2(prmt(c.mnw, 0x64646464u, hi)), k1024), m);
+    const NibbleMagic km = nibble_magic();
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      uint32_t e[4];
+      nibbles_to_magic(word(t.q, i), km, e);
+      o[4 * i + 0] = h2_bits(__hfma2(__hsub2(bits_h2(e[0]), k1024), s_lo, m_lo));
+      o[4 * i + 1] = h2_bits(__hfma2(__hsub2(bits_h2(e[1]), k1024), s_lo, m_lo));
+      o[4 * i + 2] = h2_bits(__hfma2(__hsub2(bits_h2(e[2]), k_hi), s_hi, m_hi));
+      o[4 * i + 3] = h2_bits(__hfma2(__hsub2(bits_h2(e[3]), k_hi), s_hi, m_hi));
+    }
+  }
+};
+
 template <>
 struct WFmt<QK_T_Q8_0> {  // block of 32: f16 d, 32 int8 (reference/q8_0.rs)
   static constexpr uint32_t BB = 34, BPS = 8, LUT = 0;
   static constexpr bool SCALED = false;
+  using Rf = RowScale;
+  static constexpr int UP = 0;
+  static constexpr float BACK = 1.f;
   __device__ static void fill_lut(unsigned char *, uint32_t, uint32_t) {}
   __host__ __device__ static uint32_t src(uint32_t p) { return p; }
   struct Hd {};
@@ -420,6 +463,9 @@ template <>
 struct WFmt<QK_T_Q4_0> {  // block of 32: f16 d, 16 bytes; byte j = elements 2 j (low nibble) and 2 j + 1 (high) (reference/q4_0.rs:36-46)
   static constexpr uint32_t BB = 18, BPS = 8, LUT = 0;
   static constexpr bool SCALED = false;
+  using Rf = RowScale;
+  static constexpr int UP = 0;
+  static constexpr float BACK = 1.f;
   __device__ static void fill_lut(unsigned char *, uint32_t, uint32_t) {}
   // a word yields its eight elements as (byte 0, byte 2), (byte 1, byte 3) low nibbles, then the
   // same of the high nibbles
@@ -455,6 +501,9 @@ template <>
 struct WFmt<QK_T_Q6_K> {  // super-block of 256: ql 128, qh 64, 16 int8 scales, f16 d (reference/q6_k.rs)
   static constexpr uint32_t BB = 210, BPS = 1, LUT = 0;
   static constexpr bool SCALED = true;
+  using Rf = RowScale;
+  static constexpr int UP = 24;
+  static constexpr float BACK = 1.f;
   __device__ static void fill_lut(unsigned char *, uint32_t, uint32_t) {}
   // half hh = ql[64 hh ..], qh[32 hh ..]; its quarter k (columns 32 k ..) = nibble k >> 1 of ql bytes
   // 32 (k & 1) + l and bit pair 2 k of qh byte l
@@ -489,6 +538,42 @@ struct WFmt<QK_T_Q6_K> {  // super-block of 256: ql 128, qh 64, 16 int8 scales, 
   }
 };
 
+// Rows whose blocks differ widely (see above): (1024 + q) - 1056 = q - 32, exact, then one rounding in the product.  |d sc|
+// being at most 2^-8 of the factor, a weight is at most 2^14.  (The scales through f32: with pairs of halves, as above,
+// 4096 x 14336 by 8 takes 17.4 us instead of 17.0, 14336 x 4096 by 8 15.5 instead of 14.7.)
+template <>
+struct WFmt<QK_T_Q6_K | QK_TC_WIDE> : WFmt<QK_T_Q6_K> {
+  static constexpr int UP = 17;
+  static constexpr float BACK = 0x1p-17f;
+  struct Rf {
+    float f;
+    __device__ __forceinline__ void set(float factor, int up) { f = __uint_as_float((uint32_t)(127 + up) << 23) / factor; }
+  };
+  struct Hd { uint4 qh[2]; uint2 sc; float d; };
+  __device__ static void head(Hd &c, uint32_t p, uint32_t rr, uint32_t hh, Rf rf) {
+    const uint32_t q = p + rr * 16;
+    c.qh[0] = lds128(q + (8 + 2 * hh) * 128), c.qh[1] = lds128(q + (9 + 2 * hh) * 128);
+    c.sc = lds64(q + 1536 + 8 * hh);
+    c.d = h2f_bits(lds16(p + 1664 + 2 * rr)) * rf.f;
+  }
+  __device__ static void expand(const Qt &t, const Hd &c, uint32_t k, uint32_t (&o)[16], uint32_t) {
+    const __half2 off = __float2half2_rn(1056.f);
+    const uint32_t scw = ((k >> 1) ? c.sc.y : c.sc.x) >> (16 * (k & 1u)), nib = 4 * (k >> 1), rot = (4 - 2 * k) & 31u;
+    __half2 s[2];  // 16 columns per scale
+#pragma unroll
+    for (int i = 0; i < 2; i++) s[i] = __float2half2_rn(c.d * (float)(int)(signed char)((scw >> (8 * i)) & 0xFF));
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const uint32_t lw = word(t.ql[i >> 2], i & 3) >> nib, hw = word(c.qh[i >> 2], i & 3);
+      const uint32_t q6 = (lw & 0x0F0F0F0Fu) | (__funnelshift_l(hw, hw, rot) & 0x30303030u);
+      uint32_t a, b2;
+      bytes_to_magic(q6, a, b2);
+      o[2 * i] = h2_bits(__hmul2(__hsub2(bits_h2(a), off), s[i >> 2]));
+      o[2 * i + 1] = h2_bits(__hmul2(__hsub2(bits_h2(b2), off), s[i >> 2]));
+    }
+  }
+};
+
 template <>
 struct WFmt<QK_T_IQ4_XS> {  // super-block of 256: f16 d, scales_h, scales_l[4], 128 nibble bytes (reference/iq4_xs.rs:47-97)
   // sub-block s = nibble bytes 16 s ..; byte j holds elements 2 j (low) and 2 j + 1 (high); value =
@@ -497,6 +582,9 @@ struct WFmt<QK_T_IQ4_XS> {  // super-block of 256: f16 d, scales_h, scales_l[4],
   // a copy of its own in its own bank (32 KB), so the look-ups of a warp never conflict.
   static constexpr uint32_t BB = 136, BPS = 1, LUT = 32768;
   static constexpr bool SCALED = false;  // (the table holds whole numbers as they are: one product)
+  using Rf = RowScale;
+  static constexpr int UP = 0;
+  static constexpr float BACK = 1.f;
   __host__ __device__ static uint32_t src(uint32_t p) { return p; }
   __device__ static void fill_lut(unsigned char *lut, uint32_t tid, uint32_t nthreads) {
     constexpr uint32_t K0 = 0xBFAD9881u, K1 = 0xF6EADDCFu, K2 = 0x26190D01u, K3 = 0x71594535u;  // K[0..15] as bytes
@@ -830,7 +918,7 @@ __device__ __forceinline__ bool walk_segment(uint32_t s0, uint32_t s1, bool wide
 }
 
 // ---------------------------------------------------------------- main kernel
-// T: weight format.  CG: CTAs per tile (see the top).  NG: 1 = one matrix; otherwise up to NG matrices
+// T: weight format, with QK_TC_WIDE for marked matrices.  CG: CTAs per tile (see the top).  NG: 1 = one matrix; otherwise up to NG matrices
 // of one shape and format (the projections of a feed-forward block, the experts of a mixture), each
 // multiplying its own group of activation rows.
 // REGS: registers per thread: 80, or 72 to leave room for CTAs of the conversion beside it, and for the pairs of one
@@ -958,9 +1046,11 @@ __global__ void __maxnreg__(REGS)
   auto box_of = [&](uint32_t n) { return NG > 1 ? (n / CG + hq - 1) / hq : 1u; };  // the how-manieth box (from 1)
   auto box_rows = [&](uint32_t n) { return NG > 1 ? min(box_of(n) * hq, A.hn / CG) : A.hn / CG; };
 
-  // The factors of four rows (a multiple of 4 the first; the table has whole chunks of 8)
+  // What the results of four rows are multiplied with (a multiple of 4 the first; the table has whole chunks of 8)
   auto factors4 = [&](uint32_t g, uint32_t row) {
-    return F::SCALED && row < A.L.rows ? __ldg(reinterpret_cast<const float4 *>(M.rows[g] + row)) : make_float4(1.f, 1.f, 1.f, 1.f);
+    float4 f = F::SCALED && row < A.L.rows ? __ldg(reinterpret_cast<const float4 *>(M.rows[g] + row)) : make_float4(1.f, 1.f, 1.f, 1.f);
+    f.x *= F::BACK, f.y *= F::BACK, f.z *= F::BACK, f.w *= F::BACK;
+    return f;
   };
   // The last contributor of a split tile adds the partials up, in the order of their K runs: a warp four
   // tokens at a time, a lane four rows.
@@ -1196,7 +1286,7 @@ __global__ void __maxnreg__(REGS)
       const uint32_t row0 = (q.rb * CG + rank) * BM, row = row0 + r;
       const float *sp = A.xscale + (NG > 1 ? (q.g % A.n_act) * A.xcap : 0u) + q.t0;
       float *yt = A.y + (uint64_t)((NG > 1 ? q.g * A.ycap : 0u) + q.t0) * ldy;  // the tile's first token
-      const float rk = F::SCALED && !split && row < A.L.rows ? __ldg(M.rows[NG > 1 ? q.g : 0] + row) : 1.f;
+      const float rk = F::SCALED && !split && row < A.L.rows ? F::BACK * __ldg(M.rows[NG > 1 ? q.g : 0] + row) : 1.f;
       // partial tiles: [slot][token][128 rows]
       const uint32_t slot = A.bn * BM;
       float *mine = A.part + (blockIdx.x * 2 + (i == sc.whole ? 0u : 1u)) * slot + r;
@@ -1310,16 +1400,16 @@ __global__ void __maxnreg__(REGS)
       sched.get(i, tile, s0, s1);
       return s1 - s0;
     };
-    RowScale rf = {};
+    typename F::Rf rf = {};
     float next_factor = 1.f;
-    if (F::SCALED && n_sb) rf.set(row_of(0)), next_factor = row_of(1), seg_end = seg_len(0);
+    if (F::SCALED && n_sb) rf.set(row_of(0), F::UP), next_factor = row_of(1), seg_end = seg_len(0);
     const uint32_t w_bytes = S.w_stage, nst = S.w_stages, w0 = sbase + S.w + (r >> 3) * CHB;
     const uint32_t ta0 = tmem + ((32 * quarter) << 16) + a_col + hh * 64u, a_full0 = in_first<CG>(sbase + S.a_full);
     uint32_t ws = set, wph = 0;      // ring stage and parity of this set's next super-block
     uint32_t ab = set, auses = 0;                       // its buffer, and how often that has been used (set < na)
     for (uint32_t j = set; j < n_sb; j += 2) {
       if (F::SCALED)
-        while (j >= seg_end) rf.set(next_factor), next_factor = row_of(++seg + 1), seg_end += seg_len(seg);
+        while (j >= seg_end) rf.set(next_factor, F::UP), next_factor = row_of(++seg + 1), seg_end += seg_len(seg);
       if (!warp_wait(sbase + S.w_full + ws * 8, wph)) {
         dead = true;  // warp-uniform: these warps execute .aligned tcgen05 instructions
         break;
@@ -1464,6 +1554,19 @@ cudaError_t launch_glu16(const ConvArgs &C, uint32_t rows, cudaStream_t s) {
   return cudaLaunchKernelEx(&cfg, qk_glu16_kernel<T, CT, CL>, C);
 }
 
+// The matmul itself.  beside: single CTAs of 72 registers.
+template <int T>
+cudaError_t launch_matmul(const TcPlan &P, const TcArgs &A, __half *x16, const QkTcCall &c, bool beside, cudaStream_t s) {
+  if (c.n == 1 && !c.counts) {
+    if (P.cg == 2) return launch_main<T, 2, 1, 72>(P, A, x16, c, s);
+    return beside ? launch_main<T, 1, 1, 72>(P, A, x16, c, s) : launch_main<T, 1, 1>(P, A, x16, c, s);
+  }
+  return P.cg == 1 ? launch_main<T, 1, QK_MAX_GROUPS>(P, A, x16, c, s) : launch_main<T, 2, QK_MAX_GROUPS>(P, A, x16, c, s);
+}
+// With a marked matrix (qk_tc_q4k_wide.cu, qk_tc_q6k_wide.cu)
+cudaError_t launch_wide_q4k(const TcPlan &P, const TcArgs &A, __half *x16, const QkTcCall &c, bool beside, cudaStream_t s);
+cudaError_t launch_wide_q6k(const TcPlan &P, const TcArgs &A, __half *x16, const QkTcCall &c, bool beside, cudaStream_t s);
+
 template <int T>
 cudaError_t launch_fmt(const QkTcCall &c, unsigned *status, unsigned char *scratch, int sm_count, cudaStream_t s) {
   const QkLayout &L = *c.L;
@@ -1509,11 +1612,11 @@ cudaError_t launch_fmt(const QkTcCall &c, unsigned *status, unsigned char *scrat
   // us), and clusters gain nothing (Q4_K 4096 x 4096 by 8 8.2 -> 8.4); else 14336 x 4096 by 8 13.8 -> 13.1, IQ4_XS by 37
   // 16.7 -> 15.9.
   A.ahead = P.cg == 1 && !c.counts && P.cs == 1 && c.m < 64 ? 2u : 0u;
-  if (c.n == 1 && !c.counts) {
-    if (P.cg == 2) return launch_main<T, 2, 1, 72>(P, A, x16, c, s);
-    return beside ? launch_main<T, 1, 1, 72>(P, A, x16, c, s) : launch_main<T, 1, 1>(P, A, x16, c, s);
-  }
-  return P.cg == 1 ? launch_main<T, 1, QK_MAX_GROUPS>(P, A, x16, c, s) : launch_main<T, 2, QK_MAX_GROUPS>(P, A, x16, c, s);
+  if constexpr (T == QK_T_Q4_K)
+    if (c.wide) return launch_wide_q4k(P, A, x16, c, beside, s);
+  if constexpr (T == QK_T_Q6_K)
+    if (c.wide) return launch_wide_q6k(P, A, x16, c, beside, s);
+  return launch_matmul<T>(P, A, x16, c, beside, s);
 }
 
 }  // namespace qktc

@@ -321,7 +321,7 @@ extern "C" int qk_weights_upload_gguf(qk_ctx *c, const qk_gguf *g, const char *n
     }
     if (st != QK_OK || e != cudaSuccess) break;
     e = qk_launch_repack(h->L, raw, h->dev, c->stream);
-    if (e == cudaSuccess) e = qk_gemm_tc_factors(h->L, h->dev, h->rows, c->stream);
+    if (e == cudaSuccess) e = qk_gemm_tc_factors(h->L, h->dev, h->rows, &h->wide, c->stream);
   } while (0);
   cudaError_t e2 = cudaStreamSynchronize(c->stream);
   if (e == cudaSuccess) e = e2;

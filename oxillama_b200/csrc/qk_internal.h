@@ -13,7 +13,8 @@ struct qk_weights {
   uint8_t *dev;
   int device;
   size_t algo_bytes;
-  float *rows = nullptr;  // factors of the rows for the same (behind the matrix in `dev`)
+  float *rows = nullptr;  // factors of the rows for the tcgen05 matmul (behind the matrix in `dev`)
+  bool wide = false;      // and whether a row's blocks differ widely (qk_gemm_tc_factors)
   alignas(64) unsigned char tmap[128];  // tensor map of `dev` for the tcgen05 matmul (formats it serves)
   uint64_t fp = 0;  // content fingerprint of the host buffer it was uploaded from (host-pointer cache only)
 };

@@ -154,6 +154,7 @@ struct QkTcCall {
   const QkLayout *L;                 // of every matrix
   const void *maps[QK_MAX_GROUPS];   // their tensor maps (qk_gemm_tc_map, 128 bytes each)
   const float *rows[QK_MAX_GROUPS];  // and the factors of their rows (qk_gemm_tc_factors)
+  bool wide;                         // one of them is marked
   uint32_t n, n_act;                 // matrices; activation groups: matrix e multiplies group e % n_act
   // Activation row i of group e is x row e * xcap + i; with `lists` (device) it is x row
   // lists[e * list_stride + i] / list_div.  x2 != null: the row is silu(x) * x2 instead.
@@ -173,9 +174,10 @@ bool qk_gemm_tc_supported(const QkLayout &L, uint32_t m);
 uint64_t qk_gemm_tc_pad_bytes(const QkLayout &L);
 cudaError_t qk_gemm_tc_map(const QkLayout &L, uint8_t *tiled, void *map);
 // A power of two per row (whole chunks of rows) over which the kernel expands its weights: bytes of the table, 0 where the
-// format has none, and its computation from the tiled matrix.
+// format has none, and its computation from the tiled matrix.  *wide: the matrix has a row whose blocks differ so widely that
+// its calls expand another way (the mark).  Waits for the stream.
 size_t qk_gemm_tc_factor_bytes(const QkLayout &L);
-cudaError_t qk_gemm_tc_factors(const QkLayout &L, const uint8_t *tiled, float *rows, cudaStream_t s);
+cudaError_t qk_gemm_tc_factors(const QkLayout &L, const uint8_t *tiled, float *rows, bool *wide, cudaStream_t s);
 // Scratch of a call: the fp16 activations (rows in sixteens), their scales and, at their most for every call, the
 // partial tiles of a K split (two per CTA): which plan a shape gets does not change what it needs.
 size_t qk_gemm_tc_part_bytes(int sm_count);

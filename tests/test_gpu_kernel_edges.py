@@ -608,6 +608,107 @@ def test_matmul_row_scales(t, rows, cols, m):
     assert np.all(y[:, 17] == 0)
 
 
+# Rows whose blocks differ widely, and calls in which only the small blocks count: the activations are 0 where a row's large block
+# lies, or smaller there by as much as its scale is larger.  A row's weights are expanded over one factor, so the small blocks would
+# keep few of their bits: from a spread on (2^5 and 2^8 lie on either side) the matrix is expanded another way.  Scales near
+# fp16's largest, negative ones, blocks whose minima or a single sub-scale make them large; all ways of writing out.  The bound is
+# assert_product's, whatever the spread.
+def unequal_blocks(t, rows, cols, ratio, seed, kind="d", d=1e-3):
+    bb, nb = S.BLOCK_BYTES[t], cols // 256
+    w = S.gen_weight(t, rows, cols, seed=seed, d_range=(1e-3, 2e-3)).reshape(rows, nb, bb).copy()
+    at = 208 if t == S.Q6_K else 0
+    for o in ([208] if t == S.Q6_K else [0, 2]):
+        f = w[:, :, o:o + 2].copy().view(np.float16).astype(np.float64) * (d / 1e-3)
+        w[:, :, o:o + 2] = f.astype(np.float16).view(np.uint8)
+    big = np.float16(1.5 * d * 2.0 ** ratio)
+    if kind == "d" or t == S.Q6_K:
+        w[:, 1, at:at + 2] = np.array([big]).view(np.uint8)
+        w[1::3, 1, at + 1] |= 0x80  # negative
+    else:  # "dmin": its minima alone make the block large; "unused": not even they, being 0 times that
+        w[:, 1, 2:4] = np.array([big]).view(np.uint8)
+        if kind == "unused":
+            w[:, 1, 4:16] = np.array([1, 2, 3, 4, 0, 0, 0, 0, 7, 8, 9, 10], np.uint8)
+    return w.reshape(-1)
+
+
+@pytest.mark.parametrize("t", [S.Q4_K, S.Q6_K])
+@pytest.mark.parametrize("rows,cols,m", [(200, 1024, 9), (4096, 2048, 33), (600, 1024, 130), (130, 8192, 300)])
+@pytest.mark.parametrize("ratio,d", [(0, 1e-3), (5, 1e-3), (8, 1e-3), (12, 1e-3), (16, 1e-3), (15, 1.2), (12, 2e-5)])
+def test_matmul_unequal_blocks(t, rows, cols, m, ratio, d):
+    w = unequal_blocks(t, rows, cols, ratio, seed=155, d=d)
+    wd = O.dequant_matrix(t, w, rows, cols)
+    for small in (0.0, 2.0 ** -ratio):
+        x = S.gen_acts(m, cols, seed=156)
+        x[:, 256:512] *= np.float32(small)
+        assert_product(device_product(t, w, x, rows, cols, m), x, wd, half=True)
+
+
+@pytest.mark.parametrize("kind", ["dmin", "unused"])
+def test_matmul_large_minima(kind):
+    t, rows, cols, m = S.Q4_K, 264, 1024, 24
+    for ratio in (4, 9, 14, 18):
+        w = unequal_blocks(t, rows, cols, ratio, seed=157, kind=kind)
+        x = S.gen_acts(m, cols, seed=158)
+        x[:, 256:512] = 0
+        assert_product(device_product(t, w, x, rows, cols, m), x, O.dequant_matrix(t, w, rows, cols), half=True)
+
+
+# One marked matrix among those of a call: gate or up of a feed-forward block, an expert's; and that it is the marked calls, and they
+# alone, that go the other way.
+@pytest.mark.parametrize("t", [S.Q4_K, S.Q6_K])
+def test_unequal_blocks_among_others(t):
+    import torch
+    from launches import launched
+    from oxillama_b200 import moe
+    from oxillama_b200.device import DeviceWeights, check_device_status, ffn
+    hidden, inter, m, n = 512, 768, 40, 4
+    shapes = [(inter, hidden), (inter, hidden), (hidden, inter)]
+    WIDE = 0x100
+
+    def formats(call):
+        return [k.ints[0] for k in launched(call) if k.name == "qk_gemm_tc_kernel"]
+
+    def block(x, g, u, d):
+        hg = x @ g.T
+        return (hg / (1 + np.exp(-hg)) * (x @ u.T)) @ d.T
+
+    x = S.gen_acts(m, hidden, seed=162) * np.float32(0.25)
+    x[:, 256:512] *= np.float32(2.0 ** -12)
+    xd, y = torch.from_numpy(x).cuda(), torch.empty((m, hidden), device="cuda")
+    for marked in (None, 0, 1, 2):
+        ws = [unequal_blocks(t, r, c, 12 if k == marked else 0, seed=163 + k) for k, (r, c) in enumerate(shapes)]
+        if marked == 2:  # its large block would drown the others
+            ws[2] = unequal_blocks(t, hidden, inter, -12, seed=165)
+        dw = [DeviceWeights(t, w, r, c) for w, (r, c) in zip(ws, shapes)]
+        g, u, d = (O.dequant_matrix(t, w, r, c).astype(np.float64) for w, (r, c) in zip(ws, shapes))
+        assert formats(lambda: ffn(*dw, xd, y, m)) == [t | (WIDE if marked in (0, 1) else 0), t | (WIDE if marked == 2 else 0)]
+        ref = block(x.astype(np.float64), g, u, d)
+        y.fill_(float("nan"))
+        ffn(*dw, xd, y, m)
+        check_device_status()
+        assert np.abs(y.cpu().numpy() - ref).max() <= 3e-3 * np.abs(ref).max()
+        for w in dw:
+            w.free()
+    for marked in (None, 1, 2):
+        w = [[unequal_blocks(t, r, c, (12 if k == 1 else -12) if k == marked and e == 2 else 0, seed=170 + 3 * e + k) for e in range(n)]
+             for k, (r, c) in enumerate(shapes)]
+        logits = S.gen_acts(m, n, seed=168)
+        ids, wts = (v.cpu().numpy() for v in moe.route(torch.from_numpy(logits).cuda(), 2))
+        ref = np.zeros((m, hidden))
+        for e in range(n):
+            g, u, d = (O.dequant_matrix(t, ws[e], r, c).astype(np.float64) for ws, (r, c) in zip(w, shapes))
+            at, slot = np.nonzero(ids == e)
+            np.add.at(ref, at, wts[at, slot][:, None] * block(x[at].astype(np.float64), g, u, d))
+        ex = moe.MoeExperts(t, *w, hidden, inter, n)
+        ld = torch.from_numpy(logits).cuda()
+        assert formats(lambda: ex.forward(ld, xd, y, 2)) == [t | (WIDE if marked == 1 else 0), t | (WIDE if marked == 2 else 0)]
+        y.fill_(float("nan"))
+        ex.forward(ld, xd, y, 2)
+        check_device_status()
+        ex.free()
+        assert np.abs(y.cpu().numpy() - ref).max() <= 3e-3 * np.abs(ref).max()
+
+
 # Chunks of several k-tiles through a ring that hands its stages back one by one: as many tiles as stages, one more, and many
 # rounds, with one, two and four groups of warps.
 @pytest.mark.parametrize("t,m,rows,cols", [(S.Q4_K, 1, 1184, 16384), (S.Q4_K, 1, 1200, 16384), (S.Q4_K, 2, 9600, 14336), (S.Q4_K, 4, 5000, 8448),

@@ -115,4 +115,13 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_qk_torch", nullptr, -1, methods, 
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__qk_torch() { return PyModule_Create(&module); }
+// The accessors of at::Tensor are inlined, so their offsets are those of the torch that this was compiled with, and a file left
+// over from another one can still be loaded: the importer compares both.
+PyMODINIT_FUNC PyInit__qk_torch() {
+  PyObject *m = PyModule_Create(&module);
+  if (m && (PyModule_AddStringConstant(m, "torch_version", QK_TORCH_VERSION) < 0 || PyModule_AddIntConstant(m, "python_version", PY_VERSION_HEX >> 16) < 0)) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}

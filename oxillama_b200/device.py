@@ -6,6 +6,8 @@ launched by libqk_cuda.so on the stream torch reports as current.
 from __future__ import annotations
 
 import ctypes as C
+import sys
+import warnings
 
 import numpy as np
 import torch
@@ -13,10 +15,23 @@ import torch
 from . import _lib
 from .kernels import Context, QuantError, default_context
 
-try:
-    from . import _qk_torch as _native  # what a call needs, without ctypes (csrc/qk_torch.cpp)
-except ImportError:  # not built, or for another torch: the same calls through Python
-    _native = None
+
+def _extension():
+    """What a call needs, without ctypes (csrc/qk_torch.cpp); None where it is not built, or was built for another torch or
+    another Python, whose objects it would misread: the same calls then go through Python."""
+    try:
+        from . import _qk_torch as ext
+    except ImportError:
+        return None
+    made_for = (getattr(ext, "torch_version", None), getattr(ext, "python_version", None))
+    if made_for != (str(torch.__version__), sys.hexversion >> 16):
+        warnings.warn(f"{getattr(ext, '__file__', ext)} was built for torch {made_for[0]}, not {torch.__version__}: "
+                      "run `python -m oxillama_b200.build`; until then device calls go through ctypes")
+        return None
+    return ext
+
+
+_native = _extension()
 
 
 _F32 = torch.float32

@@ -856,16 +856,14 @@ cudaError_t launch_mma(const QkLayout &L, const uint8_t *W, const float *x, floa
     use_pdl = (e && e[0] == '0') ? 0 : 1;
   }
   cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  at[1].id = cudaLaunchAttributeClusterDimension;
-  at[1].val.clusterDim.x = 2, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
+  unsigned n_at = 0;
+  if (use_pdl) at[n_at].id = cudaLaunchAttributeProgrammaticStreamSerialization, at[n_at++].val.programmaticStreamSerializationAllowed = 1;
 
   if (!INCTA) {
     const uint32_t quads = (uint32_t)M * P.Kp / 4;
     cudaLaunchConfig_t c0 = {};
     c0.gridDim = dim3((quads + 255) / 256), c0.blockDim = dim3(256), c0.stream = s;
-    c0.attrs = at, c0.numAttrs = use_pdl ? 1 : 0;
+    c0.attrs = at, c0.numAttrs = n_at;
     cudaError_t e = cudaLaunchKernelEx(&c0, qk_xsplit_kernel<F>, x, (uint32_t)M, L.cols, P.Kp,
                                        P.S.PS, P.S.xs_off, ximg, peers ? peers->wait_slots : nullptr,
                                        peers ? peers->wait_epoch : nullptr, peers ? peers->wait_ld : (uint64_t)0, status);
@@ -884,7 +882,11 @@ cudaError_t launch_mma(const QkLayout &L, const uint8_t *W, const float *x, floa
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid), cfg.blockDim = dim3((CW + 2 + ((MODE == 1 && peers && peers->unpack_n) ? 1 : 0)) * 32);
   cfg.dynamicSmemBytes = P.total + (uint32_t)(nstage - P.nstage) * P.stage_bytes, cfg.stream = s;
-  cfg.attrs = at, cfg.numAttrs = MODE == 3 ? 2 : use_pdl ? 1 : 0;
+  if (MODE == 3) {
+    at[n_at].id = cudaLaunchAttributeClusterDimension;
+    at[n_at].val.clusterDim.x = 2, at[n_at].val.clusterDim.y = 1, at[n_at].val.clusterDim.z = 1, n_at++;
+  }
+  cfg.attrs = at, cfg.numAttrs = n_at;
   QkPeers pv = {};
   if (peers) pv = *peers;
   // Weight tiles issued before the wait on the previous kernel; the rest of the ring follows

@@ -3,10 +3,11 @@
 A size chosen to reach a kernel falls out of a test unnoticed when the rule of a dispatch moves; with this the test says
 which kernel it means.
 """
+import ctypes as C
 import re
 
 import torch
-from cuda.bindings import driver, runtime
+from cuda.bindings import driver
 
 
 class Kernel:
@@ -67,12 +68,13 @@ def launched(call):
 def programmatic_edges(call):
     """How many launches of call() may start before the one ahead of them has ended, and how many edges there are."""
     g = _graph(call)
-    h = runtime.cudaGraph_t(g.raw_cuda_graph())
-    n = _ok(runtime.cudaGraphGetEdges_v2(h))[-1]
-    data = _ok(runtime.cudaGraphGetEdges_v2(h, n))[2] if n else []
-    kinds = [d.type for d in data]
+    get, n = C.CDLL("libcuda.so.1").cuGraphGetEdges_v2, C.c_size_t()  # (cuda.bindings 12.9 gives edge data of freed memory)
+    h = C.c_void_p(g.raw_cuda_graph())
+    assert get(h, None, None, None, C.byref(n)) == 0
+    before, after, data = (C.c_void_p * n.value)(), (C.c_void_p * n.value)(), (C.c_uint8 * (8 * n.value))()
+    assert get(h, before, after, data, C.byref(n)) == 0
     del g
-    return sum(int(k) == int(runtime.cudaGraphDependencyType.cudaGraphDependencyTypeProgrammatic) for k in kinds), len(kinds)
+    return sum(data[8 * i + 2] == 1 for i in range(n.value)), n.value  # {from port, to port, type, 5 reserved}; 1: programmatic
 
 
 def sm_count():

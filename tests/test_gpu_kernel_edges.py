@@ -578,6 +578,33 @@ def test_decode_pairs(t, rows, cols):
     assert np.array_equal(y, device_product(t, w, x, rows, cols, 1))  # the same bits on every run
 
 
+# Decode launches may start before the one ahead has ended, and with QK_PDL=0, by which a developer's build rules that out, none
+# may, those of pairs of CTAs included.  (Read once per process; other builds do not know the knob.)
+@pytest.mark.parametrize("pdl", [0, 1])
+def test_pdl_knob(pdl):
+    import os
+    import subprocess
+    import sys
+    from oxillama_b200 import _lib
+    if pdl == 0 and b"QK_PDL" not in open(_lib.LIB_PATH, "rb").read():
+        pytest.skip("built without QK_DEV_KNOBS")
+    code = f"""
+import sys; sys.path[:0] = [{os.path.dirname(__file__)!r}, {os.path.dirname(os.path.dirname(__file__))!r}]
+import torch
+from launches import launched, programmatic_edges
+from oxillama_b200 import synth as S
+from oxillama_b200.device import DeviceWeights
+for t, rows, cols, mode in ((S.Q6_K, 592, 14336, 3), (S.Q6_K, 592, 4096, 0), (S.Q4_K, 592, 4096, 0)):
+    w = DeviceWeights(t, S.gen_weight(t, rows, cols, seed=1), rows, cols)
+    x, y = torch.zeros(cols, device="cuda"), torch.zeros(rows, device="cuda")
+    call = lambda: (w.gemv(x, y), w.gemv(x, y))
+    assert [k.ints[4] for k in launched(call)] == [mode, mode], launched(call)
+    assert programmatic_edges(call) == ({pdl}, 1), programmatic_edges(call)
+"""
+    r = subprocess.run([sys.executable, "-c", code], env={**os.environ, "QK_PDL": str(pdl)}, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+
+
 # Rows whose scales lie anywhere in fp16's range (each row is expanded over a power of two of its own): rows of subnormal
 # scales, of the largest, and of both kinds of blocks in one row; a row of zeros; all ways of writing out (whole tiles in one
 # CTA and in pairs, clusters, partials through the workspace).  Weights of up to 65504 * 63 * 15 stay within f32 sums.

@@ -99,6 +99,8 @@ struct DecQ80 {
   static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
   static constexpr uint32_t PAIR_COLS = 0;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
   static constexpr uint32_t BY_TILE_M = 4;  // most rows with which the stages of long chunks are handed back one by one
+  static constexpr uint32_t SHORT_M = 0;  // rows (bit m) with which matrices of a single k-tile have a kernel of their own (launch_mma)
+  static constexpr bool OWN_SPLIT = false;  // any number of rows may have to be split by every CTA itself (no scratch in a capture)
   static constexpr uint32_t XCH = 0;       // shared memory per compute warp for what its lanes exchange
   static constexpr bool HAS_ONE = false;   // a variant of the policy for one row
   // digit order inside a 32-column block: the lane's 8 bytes are columns 4 tig .. + 3 and
@@ -174,6 +176,8 @@ struct DecQ40 {
   static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
   static constexpr uint32_t PAIR_COLS = 0;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
   static constexpr uint32_t BY_TILE_M = 4;  // most rows with which the stages of long chunks are handed back one by one
+  static constexpr uint32_t SHORT_M = 1u << 3;  // rows (bit m) with which matrices of a single k-tile have a kernel of their own (launch_mma)
+  static constexpr bool OWN_SPLIT = false;  // any number of rows may have to be split by every CTA itself (no scratch in a capture)
   static constexpr uint32_t XCH = 0;       // shared memory per compute warp for what its lanes exchange
   static constexpr bool HAS_ONE = false;   // a variant of the policy for one row
   // The lane's word (bytes 4 tig .. + 3 of the block) holds elements 8 tig .. + 7: low
@@ -259,6 +263,8 @@ struct DecIQ4XS {
   static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
   static constexpr uint32_t PAIR_COLS = 13312;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
   static constexpr uint32_t BY_TILE_M = 1;  // the same (two rows, bound by issue: 4096 x 14336 16.2 -> 16.6 us, a layer of experts 156 -> 160)
+  static constexpr uint32_t SHORT_M = 0;  // rows (bit m) with which matrices of a single k-tile have a kernel of their own (launch_mma)
+  static constexpr bool OWN_SPLIT = false;  // any number of rows may have to be split by every CTA itself (no scratch in a capture)
   static constexpr uint32_t XCH = 0;       // shared memory per compute warp for what its lanes exchange
   static constexpr bool HAS_ONE = false;   // a variant of the policy for one row
   __device__ static __forceinline__ void store_digits(unsigned char *row_img, uint32_t PS, uint32_t e0, uint32_t w0,
@@ -359,6 +365,8 @@ struct DecQ6K {
   static constexpr bool ANY_DEPTH = true;  // ring depths that are no multiple of the groups (ring_is_deep)
   static constexpr uint32_t PAIR_COLS = 0;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
   static constexpr uint32_t BY_TILE_M = 4;  // most rows with which the stages of long chunks are handed back one by one
+  static constexpr uint32_t SHORT_M = 0;  // rows (bit m) with which matrices of a single k-tile have a kernel of their own (launch_mma)
+  static constexpr bool OWN_SPLIT = false;  // any number of rows may have to be split by every CTA itself (no scratch in a capture)
   static constexpr uint32_t XCH = 0;       // shared memory per compute warp for what its lanes exchange
   static constexpr bool HAS_ONE = true;    // a variant of the policy for one row
   using One = DecQ6KOne;

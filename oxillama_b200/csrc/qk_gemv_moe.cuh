@@ -73,8 +73,9 @@ __global__ void __launch_bounds__(256)
   if ((threadIdx.x & 7) == 0) F::store_xs(row + 3 * PS, e0 / 32, digit_scale(amax, s4 + other), s4 + other, s4, other);
 }
 
-// F1: the policy of jobs with one row: F, or its variant for them.
-template <class F, class F1, bool DUAL, int G>
+// F1: the policy of jobs with one row: F, or its variant for them.  BY_TILE: chunks of several k-tiles, whose stages are handed
+// back one by one, as in the decode kernel.
+template <class F, class F1, bool DUAL, int G, bool BY_TILE>
 __global__ void __launch_bounds__((MAX_CW + 2) * 32, 1) qk_gemv_moe_kernel(const __grid_constant__ MoeArgs A) {
   constexpr int CW = MAX_CW, WG = CW / G;
   constexpr uint32_t ND = DUAL ? 2 : 1;
@@ -87,7 +88,7 @@ __global__ void __launch_bounds__((MAX_CW + 2) * 32, 1) qk_gemv_moe_kernel(const
   MoeSeg *segs = reinterpret_cast<MoeSeg *>(smem + A.seg);
   volatile uint32_t *meta = reinterpret_cast<volatile uint32_t *>(smem + A.seg + QK_MOE_JOBS * sizeof(MoeSeg));  // segments, chunks
 
-  const bool by_tile = L.ktiles > 1 && A.rows <= F::BY_TILE_M;  // as in the decode kernel
+  constexpr bool by_tile = BY_TILE;
   if (A.early) pdl_launch_dependents();
   if (threadIdx.x == 0) {
     for (int s = 0; s < nstage; s++) mbar_init(sbase + S.full + s * 8, 1);
@@ -359,9 +360,9 @@ cudaError_t moe_split(const QkLayout &L, const float *x, uint32_t rows, unsigned
                             (uint64_t)moe_image_stride<F>(L), plan ? *plan : qkmoe::PlanArgs{});
 }
 
-template <class F, class F1, bool DUAL, int G>
-cudaError_t moe_launch_g(const MoeArgs &A, uint32_t smem, int sm_count, cudaStream_t s) {
-  auto kern = qk_gemv_moe_kernel<F, F1, DUAL, G>;
+template <class F, class F1, bool DUAL, int G, bool BY_TILE>
+cudaError_t moe_launch_t(const MoeArgs &A, uint32_t smem, int sm_count, cudaStream_t s) {
+  auto kern = qk_gemv_moe_kernel<F, F1, DUAL, G, BY_TILE>;
   static QkPerDevice attr_set;
   if (attr_set.first()) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
@@ -373,6 +374,15 @@ cudaError_t moe_launch_g(const MoeArgs &A, uint32_t smem, int sm_count, cudaStre
   cudaLaunchConfig_t c = {};
   c.gridDim = dim3((unsigned)sm_count), c.blockDim = dim3((MAX_CW + 2) * 32), c.dynamicSmemBytes = smem, c.stream = s, c.attrs = at, c.numAttrs = 1;
   return cudaLaunchKernelEx(&c, kern, A);
+}
+
+// Two kernels.  (As in launch_mma, the hand-overs that rows of a single k-tile never come to move the allocation as a condition
+// in the loop.  us a layer of experts, with the condition / a kernel each: 8 Q6_K of 2048 x 4096, top 2, two tokens 35.7 / 34.0, 16
+// of 1024 x 1536, top 3, eight 57.6 / 54.3, Q4_K 2048 x 2048, top 1, five 30.2 / 28.7; 0.98 to 1.00 over the formats.)
+template <class F, class F1, bool DUAL, int G>
+cudaError_t moe_launch_g(const MoeArgs &A, uint32_t smem, int sm_count, cudaStream_t s) {
+  return A.L.ktiles > 1 && A.rows <= F::BY_TILE_M ? moe_launch_t<F, F1, DUAL, G, true>(A, smem, sm_count, s)
+                                                  : moe_launch_t<F, F1, DUAL, G, false>(A, smem, sm_count, s);
 }
 
 template <class P>

@@ -402,7 +402,8 @@ __device__ __forceinline__ void unpack_slots(const QkPeers &peers, unsigned uwan
 // 3 = one matrix, each chunk by the two CTAs of a cluster, either half of K (see pair_pays); the reducer of the CTA that
 // does not own the chunk (they take turns) sends its sums into the other's shared memory.
 // DEEP: the ring has every stage that fits, not a multiple of the groups' (see make_plan_mma).
-template <class F, int M, bool INCTA, int CW, int G, int MODE, bool DEEP>
+// LONG: the variant that can hand stages back one by one (see the producer and launch_mma).
+template <class F, int M, bool INCTA, int CW, int G, int MODE, bool DEEP, bool LONG>
 __global__ void __launch_bounds__((CW + 2 + (MODE == 1 ? 1 : 0)) * 32, 1)
     qk_gemv_imma_kernel(QkLayout L, const uint8_t *__restrict__ W, const uint8_t *__restrict__ W2,
                            const float *__restrict__ x,
@@ -424,7 +425,7 @@ __global__ void __launch_bounds__((CW + 2 + (MODE == 1 ? 1 : 0)) * 32, 1)
   const uint32_t ktiles = PAIR ? (nb + L.nbt - 1) / L.nbt : L.ktiles;
   auto tile_blocks = [&](uint32_t kt) { return min(nb - kt * L.nbt, L.nbt); };
   const uint32_t my_items = my_chunks * ktiles;
-  const bool by_tile = M <= (int)F::BY_TILE_M && ktiles > 1 && my_items > (uint32_t)nstage;  // stages are handed back one by one (see the producer)
+  const bool by_tile = LONG && ktiles > 1 && my_items > (uint32_t)nstage;  // stages are handed back one by one (see the producer)
 
   QK_STAMP(warp == 0, 0);
   pdl_launch_dependents();
@@ -839,11 +840,11 @@ inline bool ring_is_deep(const QkLayout &L, const PlanMma &P, int sm_count, bool
   return F::ANY_DEPTH && P.deep > P.nstage && (L.chunks + grid - 1) / grid * ktiles * (dual ? 2u : 1u) > (uint32_t)P.nstage;
 }
 
-template <class F, int M, bool INCTA, int CW, int G, int MODE = 0, bool DEEP = false>
-cudaError_t launch_mma(const QkLayout &L, const uint8_t *W, const float *x, float *y, uint64_t ldy,
-                       unsigned *status, unsigned char *ximg, int sm_count, const PlanMma &P,
-                       cudaStream_t s, const QkPeers *peers = nullptr, const uint8_t *W2 = nullptr) {
-  auto kern = qk_gemv_imma_kernel<F, M, INCTA, CW, G, MODE, DEEP>;
+template <class F, int M, bool INCTA, int CW, int G, int MODE, bool DEEP, bool LONG>
+cudaError_t launch_mma_kernel(const QkLayout &L, const uint8_t *W, const float *x, float *y, uint64_t ldy,
+                              unsigned *status, unsigned char *ximg, int sm_count, const PlanMma &P,
+                              cudaStream_t s, const QkPeers *peers, const uint8_t *W2) {
+  auto kern = qk_gemv_imma_kernel<F, M, INCTA, CW, G, MODE, DEEP, LONG>;
   static QkPerDevice attr_set;
   if (attr_set.first()) {
     cudaError_t e =
@@ -903,6 +904,27 @@ cudaError_t launch_mma(const QkLayout &L, const uint8_t *W, const float *x, floa
   if (npre > nstage) npre = nstage;
   return cudaLaunchKernelEx(&cfg, kern, L, W, W2, x, (const unsigned char *)ximg, y, ldy, status,
                             nstage, nstage + 1, P.stage_bytes, P.S, P.Kp, pv, npre);
+}
+
+// The variant of the kernel.  Where stages can be handed back one by one, that is a condition inside the loop over the tiles,
+// and it moves the compiler's allocation at the cap of 96 registers one way or the other, also for rows of a single k-tile, which
+// never come to it.  F::SHORT_M names the numbers of rows (bit m) where those are faster with a kernel that has no such
+// condition (us, with it / without: Q4_0 by three 896 x 3584 4.9 / 4.35, 3072 x 3072 6.4 / 5.9, Q4_K by three 320 x 1280 3.9 /
+// 3.6, a feed-forward block of 1024 x 2816 11.0 / 10.4; Q2_K by three, as two and one, 896 x 3584 10.5 / 9.7, Q3_K 11.7 / 10.9; but Q4_K
+// by four 3072 x 3072 6.5 / 6.9, Q8_0 by four 4096 x 4096 9.1 / 9.4).
+template <class F, int M, bool INCTA, int CW, int G, int MODE = 0, bool DEEP = false>
+cudaError_t launch_mma(const QkLayout &L, const uint8_t *W, const float *x, float *y, uint64_t ldy,
+                       unsigned *status, unsigned char *ximg, int sm_count, const PlanMma &P,
+                       cudaStream_t s, const QkPeers *peers = nullptr, const uint8_t *W2 = nullptr) {
+  constexpr bool SHORT = M > (int)F::BY_TILE_M || (F::SHORT_M >> M & 1u) != 0;  // rows of a single k-tile have a variant of their own
+  // (several rows of more than one k-tile are split by a launch of their own, but in formats with OWN_SPLIT)
+  if constexpr (M <= (int)F::BY_TILE_M && (!SHORT || M == 1 || !INCTA || F::OWN_SPLIT)) {
+    const uint32_t ktiles = MODE == 3 ? (half_blocks(L) + L.nbt - 1) / L.nbt : L.ktiles;
+    if (!SHORT || ktiles > 1)
+      return launch_mma_kernel<F, M, INCTA, CW, G, MODE, DEEP, true>(L, W, x, y, ldy, status, ximg, sm_count, P, s, peers, W2);
+  }
+  if constexpr (SHORT) return launch_mma_kernel<F, M, INCTA, CW, G, MODE, DEEP, false>(L, W, x, y, ldy, status, ximg, sm_count, P, s, peers, W2);
+  return cudaErrorInvalidConfiguration;
 }
 
 // Every CTA redoing the split costs ~M*K/512 quads per thread; past this size the

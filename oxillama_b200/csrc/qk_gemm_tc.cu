@@ -85,7 +85,8 @@ static uint32_t round_up(uint32_t v, uint32_t to) { return (v + to - 1) / to * t
 // round of hand-overs (expanding warps -> issuer -> tensor pipe -> back).  A tile whose partials go through the
 // workspace costs some 7000 cycles and 40 per token (writing them out, the fence, the counter, reading them back);
 // through the cluster 4300 and 17 per token (with 4600 for any width IQ4_XS 2048 x 2048 by 64 took 9.5 us in clusters, 8.1
-// without).
+// without).  4200 for Q6_K: with 4300, and super-blocks that expand faster, its rows of six by up to 16 tokens went to a CTA a tile
+// (1536 x 1536 by 8 6.66 us, in clusters 6.15; no other of 400 shapes changes).
 bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
   const QkLayout &L = *c.L;
   const uint32_t w_stage = 16u * 8u * L.bb * (256u / L.bs), lut = L.type == QK_T_IQ4_XS ? WFmt<QK_T_IQ4_XS>::LUT : 0u;
@@ -153,7 +154,7 @@ bool make_plan(const QkTcCall &c, int sm_count, TcPlan *P) {
         if (cg == 1 && c.n == 1)
           for (uint32_t cs = 4; cs <= 8 && cs <= p.nsb; cs <<= 1)
             if (tiles * cs <= (uint32_t)sm_count * (cs == 4 ? 14u : 12u) / 16u)
-              take((float)((p.nsb + cs - 1) / cs) * sb + 4300.f + 17.f * bn + out, 1, cs, bn, tbr, rbs, 1, (uint32_t)tiles * cs);
+              take((float)((p.nsb + cs - 1) / cs) * sb + (L.type == QK_T_Q6_K ? 4200.f : 4300.f) + 17.f * bn + out, 1, cs, bn, tbr, rbs, 1, (uint32_t)tiles * cs);
       }
     }
   }

@@ -40,16 +40,25 @@ def assert_product(y, x, wd, half):
     assert np.all(np.abs(y - ref) <= 7 * sigma * s + 1e-30), float((np.abs(y - ref) / (sigma * s + 1e-30)).max())
 
 
-def device_product(t, w, x, rows, cols, m):
+def device_product(t, w, x, rows, cols, m, launches=None):
+    """The product, and in `launches` what such a call launches."""
     import torch
     from oxillama_b200.device import DeviceWeights, check_device_status
     dw = DeviceWeights(t, w, rows, cols)
     y = torch.full((m, rows), float("nan"), device="cuda")
     xd = torch.from_numpy(x).cuda()
-    if m == 1:
-        dw.gemv(xd, y)
-    else:
-        dw.gemm(xd, y, m)
+
+    def call():
+        if m == 1:
+            dw.gemv(xd, y)
+        else:
+            dw.gemm(xd, y, m)
+
+    if launches is not None:
+        from launches import launched
+        launches += launched(call)
+        y.fill_(float("nan"))
+    call()
     check_device_status()
     dw.free()
     return y.cpu().numpy()
@@ -564,16 +573,26 @@ def test_moe_group_plan(n, top_k, tokens, begin, local):
     assert np.abs(y.cpu().numpy() - ref).max() <= 3e-3 * np.abs(ref).max()
 
 
-# One row by pairs of CTAs, half of K each (148 SMs: where 2 ceil(chunks / 148) > ceil(chunks / 74)): a single chunk, one and
-# two chunks for some pairs, the most chunks that a pair takes; halves of equal and of unequal length, the last block ragged;
-# and neighbours that stay with whole chunks (even shares, halves of 33 and 32 spans).
-@pytest.mark.parametrize("t,rows,cols", [(t, *s) for t in (S.Q6_K, S.Q5_K) for s in [
-    (3, 14336), (592, 13568), (593, 13500), (1190, 14592), (1777, 16128), (18352, 13312), (18353, 13312), (1184, 14336), (600, 16640)]] + [
-    (S.IQ4_XS, 4096, 13312), (S.Q3_K, 600, 11264)])
-def test_decode_pairs(t, rows, cols):
+# One row by pairs of CTAs, half of K each (148 SMs: where 2 ceil(chunks / 148) > ceil(chunks / 74)): a single chunk, one and two
+# for some pairs, the most that a pair can be given; halves of equal and of unequal length, the last block ragged; and neighbours
+# that stay with whole chunks: even shares, a chunk or a column less than it takes, halves of 33 and 32 spans.
+PAIRS = [(3, 14336), (592, 13568), (592, 13500), (1190, 14592), (1185, 14400), (1776, 16128), (18352, 13312)]
+WHOLE = [(593, 13500), (1777, 16128), (18353, 13312), (1184, 14336), (592, 16640)]
+
+
+@pytest.mark.parametrize("t,rows,cols,pair", [(t, *s, True) for t in (S.Q6_K, S.Q5_K) for s in PAIRS] +
+                         [(t, *s, False) for t in (S.Q6_K, S.Q5_K) for s in WHOLE] +
+                         [(S.IQ4_XS, 4096, 13824, True), (S.IQ4_XS, 592, 14000, True), (S.IQ4_XS, 592, 13568, False), (S.Q3_K, 592, 11264, True),
+                          (S.Q3_K, 4096, 11008, True), (S.Q3_K, 1190, 11200, True), (S.Q3_K, 592, 10752, False), (S.Q6_K, 592, 13056, False),
+                          (S.Q5_K, 592, 12288, True), (S.Q5_K, 592, 12032, False), (S.Q4_K, 592, 14336, False)])
+def test_decode_pairs(t, rows, cols, pair):
+    from launches import sm_count
+    assert sm_count() == 148
     w = S.gen_weight(t, rows, cols, seed=141)
     x = S.gen_acts(1, cols, seed=142)
-    y = device_product(t, w, x, rows, cols, 1)
+    ks = []
+    y = device_product(t, w, x, rows, cols, 1, ks)
+    assert ((ks[-1].name, ks[-1].ints[4]) == ("qk_gemv_imma_kernel", 3)) == pair, ks
     assert_product(y, x, O.dequant_matrix(t, w, rows, cols), half=False)
     assert np.array_equal(y, device_product(t, w, x, rows, cols, 1))  # the same bits on every run
 
@@ -608,8 +627,7 @@ for t, rows, cols, mode in ((S.Q6_K, 592, 14336, 3), (S.Q6_K, 592, 4096, 0), (S.
 # Rows whose scales lie anywhere in fp16's range (each row is expanded over a power of two of its own): rows of subnormal
 # scales, of the largest, and of both kinds of blocks in one row; a row of zeros; all ways of writing out (whole tiles in one
 # CTA and in pairs, clusters, partials through the workspace).  Weights of up to 65504 * 63 * 15 stay within f32 sums.
-# The bound is assert_product's, whose weights are the largest of their block: what falls among fp16's subnormals is below
-# 2^-10 of the row's largest weight, and keeps 2^-21 of that.
+# The bound is assert_product's.
 @pytest.mark.parametrize("t", [S.Q4_K, S.Q6_K])
 @pytest.mark.parametrize("rows,cols,m", [(200, 512, 9), (4096, 2048, 33), (600, 1024, 130), (130, 8192, 300), (40, 256, 5)])
 def test_matmul_row_scales(t, rows, cols, m):
@@ -626,12 +644,7 @@ def test_matmul_row_scales(t, rows, cols, m):
     x = S.gen_acts(m, cols, seed=152)
     wd = O.dequant_matrix(t, w, rows, cols)
     y = device_product(t, w, x, rows, cols, m)
-    ref = x.astype(np.float64) @ wd.astype(np.float64).T
-    # 2^-11 for the activations, 2^-11 for the weights, and 2^-21 of the row's largest weight
-    sq = (x.astype(np.float64) ** 2) @ (wd.astype(np.float64) ** 2).T
-    low = (x.astype(np.float64) ** 2).sum(1)[:, None] * (np.abs(wd).max(1)[None, :].astype(np.float64) * 2.0 ** -21) ** 2
-    assert np.all(np.isfinite(y))
-    assert np.all(np.abs(y - ref) <= 7 * (2.0 ** -11 * np.sqrt(2 * sq) + np.sqrt(low)) + 1e-30)
+    assert_product(y, x, wd, half=True)
     assert np.all(y[:, 17] == 0)
 
 
@@ -736,17 +749,38 @@ def test_unequal_blocks_among_others(t):
         assert np.abs(y.cpu().numpy() - ref).max() <= 3e-3 * np.abs(ref).max()
 
 
-# Chunks of several k-tiles through a ring that hands its stages back one by one: as many tiles as stages, one more, and many
-# rounds, with one, two and four groups of warps.
-@pytest.mark.parametrize("t,m,rows,cols", [(S.Q4_K, 1, 1184, 16384), (S.Q4_K, 1, 1200, 16384), (S.Q4_K, 2, 9600, 14336), (S.Q4_K, 4, 5000, 8448),
-                                           (S.Q8_0, 1, 9480, 12288), (S.Q6_K, 1, 9481, 8192), (S.Q6_K, 2, 4800, 12032), (S.Q4_0, 3, 4736, 8192),
-                                           (S.IQ4_XS, 1, 9480, 8448), (S.Q5_K, 4, 2400, 12288), (S.Q2_K, 2, 2400, 12288)])
-def test_decode_ring_by_tile(t, m, rows, cols):
-    w = S.gen_weight(t, rows, cols, seed=161)
-    x = S.gen_acts(m, cols, seed=162)
-    y = device_product(t, w, x, rows, cols, m)
-    assert_product(y, x, O.dequant_matrix(t, w, rows, cols), half=False)
-    assert np.array_equal(y, device_product(t, w, x, rows, cols, m))
+# Chunks of several k-tiles through a ring that hands its stages back one by one, where a CTA has more tiles than the ring stages
+# (twelve at most): every depth of the ring is reached, passed by one chunk and gone round, with one, two and four groups of warps;
+# matrices with a chunk that some CTAs do not have; and rows of a single k-tile, which go to a kernel without the hand-over where the
+# format has one.  (Kernels: without it 0, with it 1.)
+@pytest.mark.parametrize("t,m,cols", [(S.Q4_K, 1, 16384), (S.Q4_K, 2, 14336), (S.Q4_K, 4, 8448), (S.Q8_0, 1, 12288), (S.Q6_K, 1, 8192),
+                                      (S.Q6_K, 2, 12032), (S.Q4_0, 3, 8192), (S.IQ4_XS, 1, 8448), (S.Q5_K, 4, 12288), (S.Q3_K, 2, 8448),
+                                      (S.Q2_K, 2, 12288)])
+def test_decode_ring_by_tile(t, m, cols):
+    from launches import sm_count
+    sms, ktiles = sm_count(), -(-cols // 4096)
+    most = -(-13 // ktiles)  # chunks whose tiles are more than any ring holds
+    for chunks in (1, 2, 3, most, most + 1):
+        rows = 8 * sms * chunks - (1000 if chunks == most else 3)
+        w = S.gen_weight(t, rows, cols, seed=161)
+        x = S.gen_acts(m, cols, seed=162)
+        ks = []
+        y = device_product(t, w, x, rows, cols, m, ks)
+        assert ks[-1].name == "qk_gemv_imma_kernel" and ks[-1].ints[-1] == 1, ks
+        assert_product(y, x, O.dequant_matrix(t, w, rows, cols), half=False)
+        assert np.array_equal(y, device_product(t, w, x, rows, cols, m))
+
+
+@pytest.mark.parametrize("t,m,by_tile", [(S.Q4_K, 3, 0), (S.Q4_K, 4, 1), (S.Q4_0, 3, 0), (S.Q4_0, 2, 1), (S.Q3_K, 2, 0), (S.Q2_K, 2, 0), (S.Q2_K, 1, 1),
+                                         (S.Q8_0, 3, 1), (S.IQ4_XS, 2, 0), (S.Q5_K, 4, 1), (S.Q6_K, 2, 1)])
+def test_decode_ring_of_single_tiles(t, m, by_tile):
+    for rows, cols in ((320, 1280), (9481, 3584), (2400, 4096)):
+        w = S.gen_weight(t, rows, cols, seed=163)
+        x = S.gen_acts(m, cols, seed=164)
+        ks = []
+        y = device_product(t, w, x, rows, cols, m, ks)
+        assert [(k.name, k.ints[0], k.ints[-1]) for k in ks if k.name != "qk_xsplit_kernel"] == [("qk_gemv_imma_kernel", m, by_tile)], ks
+        assert_product(y, x, O.dequant_matrix(t, w, rows, cols), half=False)
 
 
 # What DeviceWeights.gemv / .gemm take and refuse is the same with the extension and without it.
@@ -846,7 +880,10 @@ def test_ffn_conversion_by_clusters(t, hidden, inter, ms):
 
 # Experts' jobs of one row (a single token) and of two, whose scales go to the lanes by different ways: one span of columns for
 # eight warps, one that leaves some of them out, a second tile with a ragged last block; rows that are no multiple of a chunk's.
-# Against each expert's own product in f64; the bound is test_moe_short_rows'.
+# Against each expert's own product in f64.  The bound is that of f32-grade sums for each of the three products (top of this file;
+# a block's largest value is up to 2 times the root mean square of these weights, 2.5 times that of these activations and 4 times that
+# of silu(g) u), which are independent, and half as much again for what silu makes of an error.  (7e-6 to 3e-5; with two digits of the
+# activations for three the result is off by 2e-5 to 8e-5 at the same sizes.)
 @pytest.mark.parametrize("t", [S.Q4_K, S.Q6_K])
 @pytest.mark.parametrize("hidden,inter", [(256, 40), (1284, 264), (4352, 2304)])
 def test_moe_decode_one_row(t, hidden, inter):
@@ -870,5 +907,6 @@ def test_moe_decode_one_row(t, hidden, inter):
         y = torch.full((tokens, hidden), float("nan"), device="cuda")
         ex.forward(logits[:tokens].cuda(), torch.from_numpy(x).cuda(), y, top_k)
         check_device_status()
-        assert np.abs(y.cpu().numpy() - ref).max() <= 3e-3 * np.abs(ref).max()
+        sigma = [2.0 ** -23 * (1 + np.sqrt(2 * k / 32)) * 2 * a for k, a in ((hidden, 2.5), (hidden, 2.5), (inter, 4))]
+        assert np.linalg.norm(y.cpu().numpy() - ref) <= 1.5 * np.linalg.norm(sigma) * np.linalg.norm(ref)
     ex.free()

@@ -98,6 +98,7 @@ struct DecQ80 {
   static constexpr bool HAS_DUAL = true, HAS_PEER = true;
   static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
   static constexpr uint32_t PAIR_COLS = 0;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
+  static constexpr bool PAIR_FULL = true;  // pairs also where every one has a single chunk (pair_pays)
   static constexpr uint32_t BY_TILE_M = 4;  // most rows with which the stages of long chunks are handed back one by one
   static constexpr uint32_t SHORT_M = 0;  // rows (bit m) with which matrices of a single k-tile have a kernel of their own (launch_mma)
   static constexpr bool OWN_SPLIT = false;  // any number of rows may have to be split by every CTA itself (no scratch in a capture)
@@ -175,6 +176,7 @@ struct DecQ40 {
   static constexpr bool HAS_DUAL = true, HAS_PEER = true;
   static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
   static constexpr uint32_t PAIR_COLS = 0;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
+  static constexpr bool PAIR_FULL = true;  // pairs also where every one has a single chunk (pair_pays)
   static constexpr uint32_t BY_TILE_M = 4;  // most rows with which the stages of long chunks are handed back one by one
   static constexpr uint32_t SHORT_M = 1u << 3;  // rows (bit m) with which matrices of a single k-tile have a kernel of their own (launch_mma)
   static constexpr bool OWN_SPLIT = false;  // any number of rows may have to be split by every CTA itself (no scratch in a capture)
@@ -261,7 +263,8 @@ struct DecIQ4XS {
   static constexpr int MAX_M = 4;
   static constexpr bool HAS_DUAL = true, HAS_PEER = true;
   static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
-  static constexpr uint32_t PAIR_COLS = 13312;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
+  static constexpr uint32_t PAIR_COLS = 13824;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
+  static constexpr bool PAIR_FULL = false;  // pairs also where every one has a single chunk (pair_pays)
   static constexpr uint32_t BY_TILE_M = 1;  // the same (two rows, bound by issue: 4096 x 14336 16.2 -> 16.6 us, a layer of experts 156 -> 160)
   static constexpr uint32_t SHORT_M = 0;  // rows (bit m) with which matrices of a single k-tile have a kernel of their own (launch_mma)
   static constexpr bool OWN_SPLIT = false;  // any number of rows may have to be split by every CTA itself (no scratch in a capture)
@@ -364,6 +367,7 @@ struct DecQ6K {
   static constexpr bool HAS_DUAL = false, HAS_PEER = true;
   static constexpr bool ANY_DEPTH = true;  // ring depths that are no multiple of the groups (ring_is_deep)
   static constexpr uint32_t PAIR_COLS = 0;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
+  static constexpr bool PAIR_FULL = true;  // pairs also where every one has a single chunk (pair_pays)
   static constexpr uint32_t BY_TILE_M = 4;  // most rows with which the stages of long chunks are handed back one by one
   static constexpr uint32_t SHORT_M = 0;  // rows (bit m) with which matrices of a single k-tile have a kernel of their own (launch_mma)
   static constexpr bool OWN_SPLIT = false;  // any number of rows may have to be split by every CTA itself (no scratch in a capture)

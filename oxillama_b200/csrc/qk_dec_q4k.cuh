@@ -31,6 +31,7 @@ struct DecQ4K {
   static constexpr bool HAS_DUAL = true, HAS_PEER = true;
   static constexpr bool ANY_DEPTH = false;  // ring depths that are no multiple of the groups (ring_is_deep)
   static constexpr uint32_t PAIR_COLS = 0;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
+  static constexpr bool PAIR_FULL = true;  // pairs also where every one has a single chunk (pair_pays)
   static constexpr uint32_t BY_TILE_M = 4;  // most rows with which the stages of long chunks are handed back one by one
   static constexpr uint32_t SHORT_M = 1u << 3;  // rows (bit m) with which matrices of a single k-tile have a kernel of their own (launch_mma)
   static constexpr bool OWN_SPLIT = false;  // any number of rows may have to be split by every CTA itself (no scratch in a capture)

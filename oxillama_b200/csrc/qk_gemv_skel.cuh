@@ -944,15 +944,19 @@ inline bool split_in_cta(const PlanMma &P, uint32_t m) {
 // long (F::PAIR_COLS; 0: never) that what drops out is worth the meeting of the pair: the launch that splits the activations,
 // and an image of them that leaves the ring few stages.  us, whole chunks / halves, a feed-forward block with this matrix last
 // (4096 rows: 4 chunks / 7 halves a CTA): Q6_K 14336 columns 27.4 / 26.1, 12288 23.1 / 23.4, 11008 22.0 / 22.4; Q5_K 26.0 /
-// 24.9, 12288 22.0 / 22.0, 11008 20.5 / 21.0; Q3_K 27.4 / 26.4, 11008 23.4 / 22.6; IQ4_XS 34.0 / 34.2, with 5120 rows of
-// 13824 40.8 / 39.3; Q8_0 33.8 / 33.7.  The matvec alone: Q6_K 13.0 / 12.9, Q5_K 13.1 / 11.2, Q3_K 14.6 / 12.7, IQ4_XS 13.3 /
-// 12.9.  Q4_K and Q4_0 have rings that are long enough; even shares gain little or lose (Q6_K, 1024 rows: one chunk or two
-// halves, 6.1 / 6.7), two rows and more mostly lose (Q4_K 1024 x 14336 6.2 / 8.5).
+// 24.9, 12288 22.0 / 22.0, 11008 20.5 / 21.0; Q3_K 27.4 / 26.4, 11008 23.4 / 22.6; IQ4_XS 34.3 / 34.4,
+// 13824 34.2 / 33.5, 13312 32.6 / 33.1, with 5120 rows of 13824 41.7 / 39.4; Q8_0 33.8 / 33.7.  The matvec alone: Q6_K 13.0 / 12.9,
+// Q5_K 13.1 / 11.2, Q3_K 14.6 / 12.7, IQ4_XS 14.1 / 13.1.  Q4_K and Q4_0 have rings that are long enough; even shares gain little or
+// lose (Q6_K, 1024 rows: one chunk or two halves, 6.1 / 6.7), two rows and more mostly lose (Q4_K 1024 x 14336 6.2 / 8.5).
+// With one chunk a pair the next launch becomes resident on the SMs that are left; where none are, the gain is small, and IQ4_XS,
+// bound by issue, loses (14336 columns, 400, 480 and 592 rows 6.0 / 5.6, 6.1 / 5.9, 6.0 / 6.7; Q5_K 6.3 / 5.1, 6.3 / 5.3, 6.2 / 5.9; Q3_K 7.1 / 5.8,
+// 7.1 / 6.0, 7.0 / 6.9; as the last of a block IQ4_XS by 512 rows of 13824 15.3 / 15.5):
+// F::PAIR_FULL.
 template <class F>
 inline bool pair_pays(const QkLayout &L, int sm_count, PlanMma *P) {
   const uint32_t sms = (uint32_t)sm_count, pairs = sms / 2;
   return L.nb * L.bs >= F::PAIR_COLS && L.chunks <= PAIR_CHUNKS * pairs && 2 * ((L.chunks + sms - 1) / sms) > (L.chunks + pairs - 1) / pairs &&
-         make_plan_mma(L, 1, P, F::XSB, true, F::XCH);
+         (F::PAIR_FULL || L.chunks > pairs || L.chunks * 4 <= pairs * 3) && make_plan_mma(L, 1, P, F::XSB, true, F::XCH);
 }
 
 template <class F, int M>

@@ -575,14 +575,16 @@ def test_moe_group_plan(n, top_k, tokens, begin, local):
 
 # One row by pairs of CTAs, half of K each (148 SMs: where 2 ceil(chunks / 148) > ceil(chunks / 74)): a single chunk, one and two
 # for some pairs, the most that a pair can be given; halves of equal and of unequal length, the last block ragged; and neighbours
-# that stay with whole chunks: even shares, a chunk or a column less than it takes, halves of 33 and 32 spans.
+# that stay with whole chunks: even shares, a chunk or a column less than it takes, halves of 33 and 32 spans, and IQ4_XS with a
+# chunk for nearly every pair.
 PAIRS = [(3, 14336), (592, 13568), (592, 13500), (1190, 14592), (1185, 14400), (1776, 16128), (18352, 13312)]
 WHOLE = [(593, 13500), (1777, 16128), (18353, 13312), (1184, 14336), (592, 16640)]
 
 
 @pytest.mark.parametrize("t,rows,cols,pair", [(t, *s, True) for t in (S.Q6_K, S.Q5_K) for s in PAIRS] +
                          [(t, *s, False) for t in (S.Q6_K, S.Q5_K) for s in WHOLE] +
-                         [(S.IQ4_XS, 4096, 13824, True), (S.IQ4_XS, 592, 14000, True), (S.IQ4_XS, 592, 13568, False), (S.Q3_K, 592, 11264, True),
+                         [(S.IQ4_XS, 4096, 13824, True), (S.IQ4_XS, 1190, 14000, True), (S.IQ4_XS, 440, 14000, True), (S.IQ4_XS, 441, 14000, False),
+                          (S.IQ4_XS, 592, 14336, False), (S.IQ4_XS, 4096, 13568, False), (S.Q3_K, 592, 11264, True),
                           (S.Q3_K, 4096, 11008, True), (S.Q3_K, 1190, 11200, True), (S.Q3_K, 592, 10752, False), (S.Q6_K, 592, 13056, False),
                           (S.Q5_K, 592, 12288, True), (S.Q5_K, 592, 12032, False), (S.Q4_K, 592, 14336, False)])
 def test_decode_pairs(t, rows, cols, pair):

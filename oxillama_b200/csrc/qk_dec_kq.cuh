@@ -30,7 +30,7 @@ struct DecQ5K {
   static constexpr uint32_t PAIR_COLS = 12288;  // fewest columns of which a pair of CTAs takes half each (pair_pays)
   static constexpr bool PAIR_FULL = true;  // pairs also where every one has a single chunk (pair_pays)
   static constexpr uint32_t BY_TILE_M = 4;  // most rows with which the stages of long chunks are handed back one by one
-  static constexpr uint32_t SHORT_M = 0;  // rows (bit m) with which matrices of a single k-tile have a kernel of their own (launch_mma)
+  static constexpr uint32_t SHORT_M = 1u << 3;  // rows (bit m) with which matrices of a single k-tile have a kernel of their own (launch_mma)
   static constexpr bool OWN_SPLIT = true;  // any number of rows may have to be split by every CTA itself (no scratch in a capture)
   static constexpr uint32_t XCH = 0;       // shared memory per compute warp for what its lanes exchange
   static constexpr bool HAS_ONE = false;   // a variant of the policy for one row

@@ -910,8 +910,9 @@ cudaError_t launch_mma_kernel(const QkLayout &L, const uint8_t *W, const float *
 // and it moves the compiler's allocation at the cap of 96 registers one way or the other, also for rows of a single k-tile, which
 // never come to it.  F::SHORT_M names the numbers of rows (bit m) where those are faster with a kernel that has no such
 // condition (us, with it / without: Q4_0 by three 896 x 3584 4.9 / 4.35, 3072 x 3072 6.4 / 5.9, Q4_K by three 320 x 1280 3.9 /
-// 3.6, a feed-forward block of 1024 x 2816 11.0 / 10.4; Q2_K by three, as two and one, 896 x 3584 10.5 / 9.7, Q3_K 11.7 / 10.9; but Q4_K
-// by four 3072 x 3072 6.5 / 6.9, Q8_0 by four 4096 x 4096 9.1 / 9.4).
+// 3.6, a feed-forward block of 1024 x 2816 11.0 / 10.4; Q2_K by three, as two and one, 896 x 3584 10.5 / 9.7, Q3_K 11.7 / 10.9; Q5_K by three
+// 9600 x 512 5.3 / 5.1, a feed-forward block of 1024 x 2816 11.4 / 11.0; but Q4_K by four 3072 x 3072 6.5 / 6.9, Q8_0 by four 4096 x
+// 4096 9.1 / 9.4, Q6_K by two 14336 x 4096 14.8 / 15.7; all other numbers of rows within 1 to 3 % either way).
 template <class F, int M, bool INCTA, int CW, int G, int MODE = 0, bool DEEP = false>
 cudaError_t launch_mma(const QkLayout &L, const uint8_t *W, const float *x, float *y, uint64_t ldy,
                        unsigned *status, unsigned char *ximg, int sm_count, const PlanMma &P,

@@ -774,7 +774,7 @@ def test_decode_ring_by_tile(t, m, cols):
 
 
 @pytest.mark.parametrize("t,m,by_tile", [(S.Q4_K, 3, 0), (S.Q4_K, 4, 1), (S.Q4_0, 3, 0), (S.Q4_0, 2, 1), (S.Q3_K, 2, 0), (S.Q2_K, 2, 0), (S.Q2_K, 1, 1),
-                                         (S.Q8_0, 3, 1), (S.IQ4_XS, 2, 0), (S.Q5_K, 4, 1), (S.Q6_K, 2, 1)])
+                                         (S.Q8_0, 3, 1), (S.IQ4_XS, 2, 0), (S.Q5_K, 3, 0), (S.Q5_K, 4, 1), (S.Q6_K, 2, 1)])
 def test_decode_ring_of_single_tiles(t, m, by_tile):
     for rows, cols in ((320, 1280), (9481, 3584), (2400, 4096)):
         w = S.gen_weight(t, rows, cols, seed=163)

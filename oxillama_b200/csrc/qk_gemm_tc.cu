@@ -227,16 +227,23 @@ __device__ __forceinline__ uint32_t max_byte(uint32_t v) {
 }
 __device__ __forceinline__ float abs_half(uint32_t bits) { return fabsf(__half2float(__ushort_as_half((unsigned short)bits))); }
 
-// A warp per row.  With b = the largest scale of the row's blocks (Q4_K: |d sc|, |d|, |dmin|; Q6_K: |d sc|, |d|) the factor is
-// the power of two over which 2^24 b is at most 0.998 of 2^16, about fp16's largest (2^-6 at least: 2^30 is what the kernel
-// takes).  Scales that are not finite do not count
-// (their blocks stay not finite), a row of zeros has factor 1.  `mark` is set where what a block of the row reaches is below
-// 2^-10 of its factor (see WFmt): 63 * 15 d of Q4_K (6-bit scales are made with the largest of a block 63; if all are 0,
-// 63 dmin), 32 |d sc| of Q6_K.
-__global__ void __launch_bounds__(256) qk_row_factor_kernel(QkLayout L, const uint8_t *__restrict__ tiled, float *__restrict__ rows, unsigned *__restrict__ mark) {
+// The power of two over which 2^24 b is at most 0.998 of 2^16, about fp16's largest (2^-6 at least: 2^30 is what the kernel takes)
+__device__ __forceinline__ float factor_over(float b) {
+  int e = 0;
+  const float f = frexpf(b, &e);  // b = f * 2^e, f in [0.5, 1)
+  return b > 0.f ? ldexpf(1.f, max(e + 8 + (f > 0.998f ? 1 : 0), -6)) : 1.f;
+}
+
+// A warp per row.  Its factor is that of the largest scale that its blocks can have by their d (Q4_K: 63 |d|, |dmin|; Q6_K: 128
+// |d|), which keeps the results of such matrices, bit for bit, what they are for any sub-scales; where that is more than 8 times the
+// factor of the largest scale in use (|d sc|, |d|, |dmin|; Q6_K: |d sc|, |d|), or with `in_use`, the latter.  Scales that are not
+// finite do not count (their blocks stay not finite), a row of zeros has factor 1.  `mark` is set where what a block of the row
+// reaches is below 2^-10 of the factor in use or 2^-12 of its own (see WFmt): 63 * 15 d of Q4_K (6-bit scales are made with the
+// largest of a block 63; if all are 0, 63 dmin), 32 |d sc| of Q6_K.
+__global__ void __launch_bounds__(256) qk_row_factor_kernel(QkLayout L, const uint8_t *__restrict__ tiled, float *__restrict__ rows, unsigned *__restrict__ mark, bool in_use) {
   const uint32_t row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= L.chunks * QK_TILE_ROWS) return;
-  float b = 0.f, least = FLT_MAX;
+  float b = 0.f, top = 0.f, least = FLT_MAX;
   if (row < L.rows)
     for (uint32_t k = lane; k < L.nb; k += 32) {
       if (L.type == QK_T_Q4_K) {
@@ -244,26 +251,27 @@ __global__ void __launch_bounds__(256) qk_row_factor_kernel(QkLayout L, const ui
         const uint32_t sc = max_byte(__vmaxu4(h.y & 0x3F3F3F3Fu, (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u)));
         const uint32_t mn = max_byte(__vmaxu4(h.z & 0x3F3F3F3Fu, ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u)));
         const float d = abs_half(h.x), dmin = abs_half(h.x >> 16);
-        if (d <= FLT_MAX) b = fmaxf(b, d * (float)max(sc, 1u));
-        if (dmin <= FLT_MAX) b = fmaxf(b, dmin);
+        if (d <= FLT_MAX) b = fmaxf(b, d * (float)max(sc, 1u)), top = fmaxf(top, 63.f * d);
+        if (dmin <= FLT_MAX) b = fmaxf(b, dmin), top = fmaxf(top, dmin);
         if (sc && d > 0.f && d <= FLT_MAX) least = fminf(least, 945.f * d);
         else if (mn && dmin > 0.f && dmin <= FLT_MAX) least = fminf(least, 63.f * dmin);
       } else {
         const uint4 s = *reinterpret_cast<const uint4 *>(tiled + qk_byte_offset(L, row, k, 1, 0));
         const uint32_t sc = max_byte(__vmaxu4(__vmaxu4(__vabs4(s.x), __vabs4(s.y)), __vmaxu4(__vabs4(s.z), __vabs4(s.w))));
         const float d = abs_half(*reinterpret_cast<const uint16_t *>(tiled + qk_byte_offset(L, row, k, 2, 0)));
-        if (d <= FLT_MAX) b = fmaxf(b, d * (float)max(sc, 1u));
+        if (d <= FLT_MAX) b = fmaxf(b, d * (float)max(sc, 1u)), top = fmaxf(top, 128.f * d);
         if (sc && d > 0.f && d <= FLT_MAX) least = fminf(least, 32.f * d * (float)sc);
       }
     }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) b = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, o)), least = fminf(least, __shfl_xor_sync(0xffffffffu, least, o));
-  int e = 0;
-  const float f = frexpf(b, &e);  // b = f * 2^e, f in [0.5, 1)
+  for (int o = 16; o > 0; o >>= 1) {
+    b = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, o)), top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    least = fminf(least, __shfl_xor_sync(0xffffffffu, least, o));
+  }
   if (lane == 0) {
-    const float factor = b > 0.f ? ldexpf(1.f, max(e + 8 + (f > 0.998f ? 1 : 0), -6)) : 1.f;
+    const float used = factor_over(b), by_d = factor_over(top), factor = in_use || by_d > 8.f * used ? used : by_d;
     rows[row] = factor;
-    if (least < factor * 0x1p-10f) atomicOr(mark, 1u);
+    if (least < fmaxf(used * 0x1p-10f, factor * 0x1p-12f)) atomicOr(mark, 1u);
   }
 }
 }  // namespace
@@ -274,10 +282,15 @@ cudaError_t qk_gemm_tc_factors(const QkLayout &L, const uint8_t *tiled, float *r
   unsigned *mark = reinterpret_cast<unsigned *>(rows + (size_t)L.chunks * QK_TILE_ROWS), m = 0;
   cudaError_t e = cudaMemsetAsync(mark, 0, sizeof(m), s);
   if (e != cudaSuccess) return e;
-  qk_row_factor_kernel<<<L.chunks, 256, 0, s>>>(L, tiled, rows, mark);
+  qk_row_factor_kernel<<<L.chunks, 256, 0, s>>>(L, tiled, rows, mark, false);
   if ((e = cudaGetLastError()) == cudaSuccess) e = cudaMemcpyAsync(&m, mark, sizeof(m), cudaMemcpyDeviceToHost, s);
-  const cudaError_t e2 = cudaStreamSynchronize(s);
+  cudaError_t e2 = cudaStreamSynchronize(s);
   if (e == cudaSuccess) e = e2;
+  if (e == cudaSuccess && m) {  // (the other expansion reaches 2^16 down from the largest scale in use)
+    qk_row_factor_kernel<<<L.chunks, 256, 0, s>>>(L, tiled, rows, mark, true);
+    e = cudaGetLastError(), e2 = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) e = e2;
+  }
   *wide = e == cudaSuccess && m != 0;
   return e;
 }

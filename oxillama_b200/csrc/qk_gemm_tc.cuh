@@ -1,6 +1,7 @@
 // Batched dequant-matmul (more than four activation rows) on the 5th-generation tensor cores.
 //
-//   y[t][n] = sum_k  w(n, k) * x[t][k]          w as the format's dequant_block gives it, rounded to fp16
+//   y[t][n] = sum_k  w(n, k) * x[t][k]          w as the format's dequant_block gives it, rounded to fp16 (Q4_K and Q6_K: over a
+//                                               power of two of the row, see WFmt)
 //
 // A real dense contraction, so it goes to tcgen05.mma: 128 weight rows are the MMA's M, up to
 // 256 activation rows (tokens) its N, fp16 operands, f32 accumulation in tensor memory.
@@ -280,7 +281,8 @@ __device__ __forceinline__ float4 ldcg4(const float *p) { return __ldcg(reinterp
 // 2^-14 of the factor they are subnormals themselves, rounded to 2^-24 of it, and so is the minimum or offset of a block.
 // As long as every block's scale is at least 2^-10 of the factor (945 d and 32 d sc: the weights that a block reaches), the
 // products of any single block are within 2 % as exact as from weights in full halves (emulated in f64, activations in that
-// block alone; at 2^-12 a third less exact, at 2^-14 four times).  A matrix with a row whose blocks differ by more is
+// block alone; at 2^-12, which blocks whose sub-scales leave most of their range unused may come to, a third less exact, at 2^-14
+// four times).  A matrix with a row whose blocks differ by more is
 // marked when it is uploaded (qk_gemm_tc_factors), and a call with such a matrix takes the former expansion: the fields as
 // whole halves, weights over 2^-17 of the factor, normal halves from 2^15 down to 2^-14 (QK_TC_WIDE; us, by a matrix without
 // the mark / with it: Q4_K 14336 x 4096 by 8 11.7 / 13.1, 4096 x 14336 by 37 15.3 / 16.7; Q6_K 14.4 / 14.7, 17.8 / 18.3).

@@ -650,6 +650,38 @@ def test_matmul_row_scales(t, rows, cols, m):
     assert np.all(y[:, 17] == 0)
 
 
+# The arithmetic of rows of ordinary blocks, restated: weights rounded once to fp16's grid (subnormals included) over the power of two
+# of the largest scale that the blocks' d allows, whatever sub-scales are in use (here a quarter to an eighth of the int8 range), and
+# activations over a power of two of their row.  What is left is the f32 sums'.
+@pytest.mark.parametrize("rows,cols,m", [(200, 1024, 24), (1024, 4096, 8), (300, 2048, 130)])
+def test_matmul_q6k_row_factor(rows, cols, m):
+    t, bb, nb = S.Q6_K, S.BLOCK_BYTES[S.Q6_K], cols // 256
+    w = S.gen_weight(t, rows, cols, seed=171, d_range=(1e-4, 2e-3)).reshape(rows, nb, bb).copy()
+    w[:, :, 192:208] = np.random.default_rng(172).integers(-32, 32, (rows, nb, 16)).astype(np.int8).view(np.uint8)
+    w[:, 1, 208:210] = np.array([1e-4], np.float16).view(np.uint8)
+    w[:, 2, 208:210] = np.array([2e-3], np.float16).view(np.uint8)
+    x = S.gen_acts(m, cols, seed=173)
+    x[:, :256] = x[:, 512:] = 0  # the block with the smallest scale alone, whose weights lie near the subnormals
+    y = device_product(t, w.reshape(-1), x, rows, cols, m)
+    d = w[:, :, 208:210].copy().view(np.float16).astype(np.float64)[:, :, 0]
+    top = 128 * np.abs(d).max(1)
+    f, e = np.frexp(top)
+    factor = 2.0 ** (e + 8 + (f > 0.998))
+    half = lambda v: v.astype(np.float16).astype(np.float64)
+    s = half(w[:, :, 192:208].view(np.int8) * (d * 2.0 ** 24 / factor[:, None])[:, :, None])
+    off = half(s * -(2.0 ** -19))
+    blk = w[:, :, :192].astype(np.int64)
+    q = np.empty((rows, nb, 256), np.int64)
+    for g in range(2):
+        for k in range(4):
+            lo = blk[:, :, 64 * g + 32 * (k & 1):64 * g + 32 * (k & 1) + 32] >> (4 * (k >> 1)) & 15
+            q[:, :, 128 * g + 32 * k:128 * g + 32 * k + 32] = lo | (blk[:, :, 128 + 32 * g:160 + 32 * g] >> (2 * k) & 3) << 4
+    wt = half(q * 2.0 ** -24 * np.repeat(s, 16, 2) + np.repeat(off, 16, 2)).reshape(rows, cols) * factor[:, None]
+    scale = 2.0 ** (np.frexp(np.abs(x).max(1).astype(np.float64))[1] - 10)[:, None]
+    ref = half(x / scale) * scale @ wt.T
+    assert np.linalg.norm(y - ref) <= 3e-6 * np.linalg.norm(ref)
+
+
 # Rows whose blocks differ widely, and calls in which only the small blocks count: the activations are 0 where a row's large block
 # lies, or smaller there by as much as its scale is larger.  A row's weights are expanded over one factor, so the small blocks would
 # keep few of their bits: from a spread on (2^5 and 2^8 lie on either side) the matrix is expanded another way.  Scales near

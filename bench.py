@@ -194,7 +194,7 @@ def layer_rates(torch, ctx, ms, stream, copies=3):
             check_device_status(ctx, stream)
             out["us_per_layer_separate_calls"] = out["us_per_layer"]
             out["us_per_layer"] = us
-            out["note"] = "feed-forward block through qk_ffn_dev (5 launches per layer instead of 7)"
+            out["note"] = "feed-forward block through qk_ffn_dev (6 launches per layer instead of 7: q, k, v, o, gate and up, down)"
             yqkv = torch.empty(m, qkv_rows, device="cuda")
 
             def fn_qkv():
@@ -206,7 +206,7 @@ def layer_rates(torch, ctx, ms, stream, copies=3):
             check_device_status(ctx, stream)
             out["us_per_layer_qkv_rows_as_one_matrix"] = us_qkv
             out["note_qkv"] = ("the same layer with the rows of q, k and v uploaded as one 6144 x 4096 matrix at load "
-                               "(3 launches per layer, the same arithmetic per row); not in us_per_layer / frac")
+                               "(4 launches per layer, the same arithmetic per row); not in us_per_layer / frac")
         if m <= 64:
             peak, which = peaks()
             out.update({"weight_gbs": nbytes / us / 1e3, "frac": nbytes / us / 1e3 / peak, "bound": "hbm",
